@@ -37,7 +37,7 @@ def test_quantizer_oracle_matches_reference_packed_tensor():
     assert eq["q"] >= 0.9999 and eq["qs"] >= 0.9995 and eq["qm"] >= 0.9995 and eq["d"] >= 0.999 and eq["dm"] >= 0.999
 
 
-@pytest.mark.skipif(not os.path.isdir(REF), reason="reference tree not present")
+@pytest.mark.skipif(not os.path.isdir(os.path.join(REF, "rwkv_quant")), reason="reference tree not present")
 @pytest.mark.parametrize("bits,search,aw", [(4, True, False), (5, True, False), (6, False, False), (4, True, True), (6, True, True)])
 def test_quantizer_oracle_matches_reference_live(bits, search, aw):
     sys.path.insert(0, REF)
@@ -60,7 +60,7 @@ def test_quantizer_oracle_matches_reference_live(bits, search, aw):
     assert abs(e_our - e_ref[0]) <= 1e-3 * e_ref[0]
 
 
-@pytest.mark.skipif(not os.path.isdir(REF), reason="reference tree not present")
+@pytest.mark.skipif(not os.path.isdir(os.path.join(REF, "rwkv_quant")), reason="reference tree not present")
 @pytest.mark.parametrize("bits,search,aw", [(6, True, False), (8, True, False), (6, False, False), (8, True, True)])
 def test_sym_quantizer_oracle_matches_reference_live(bits, search, aw):
     sys.path.insert(0, REF)
