@@ -1,0 +1,23 @@
+// Time-mix core of long sequences (rwkvq_wkv_chunk.cu): interface for the one-call forward.
+#pragma once
+#include "rwkvq_common.cuh"
+
+namespace rwkvq {
+
+struct WkvChunkArgs {
+    const float *r, *k, *v, *yw, *ya, *yv, *v_first, *g;      // [B, T, H * 64]; yv / v_first null on layer 0
+    const float *w0, *a0, *v0, *k_k, *k_a, *r_k, *ln_w, *ln_b;  // [H * 64]
+    const float* h_in;                                        // [B, H, 64, 64] or null (zeros)
+    float* h_out;                                             // [B, H, 64, 64]
+    float* og;                                                // [B, T, H * 64]
+    float* ops;                                               // scratch: wkv_chunk_floats(B, T, H)
+    float* dp;                                                // scratch: [B, T, H]
+    float* y;                                                 // scratch: [B, T, H * 64]
+    int* status;                                              // receives RWKVQ_E_TIMEOUT if a bounded wait ran out
+    int B, T, H;
+};
+size_t wkv_chunk_floats(int B, int T, int H);
+// decay, gates, key normalisation, the scan and the tail (group norm + bonus + gate); 16-byte aligned arrays
+int launch_wkv_chunked(const WkvChunkArgs& a, cudaStream_t s);
+
+}  // namespace rwkvq
