@@ -206,13 +206,13 @@ int rwkvq_gemv_batch(const rwkvq_qtensor* t, const float* x, int N, int64_t ldx,
  * batched decode):  y[n, o] = epi( sum_c W[o, c] x[n, c] ),  n < M.
  * Stands behind the N >= 128 branch of GwQuantLinear.__call__ / SymQuantLinear.__call__
  * (backends/metal/quant_linear_gw.py:846-849, quant_linear_sym.py:481-484: dequantise to
- * fp16, then a dense matmul) with the dequantisation fused into the operand producer, so
- * no dense copy of W is ever written.  Operands are fp16 (weights: fp16(q*s+m); tokens:
+ * fp16, then a dense matmul).  The weights are converted into scratch in row chunks that stay in L2
+ * and read back by TMA.  Operands are fp16 (weights: fp16(q*s+m); tokens:
  * scaled per row by a power of two), accumulation fp32 in tensor memory.
- *   x [M, ldx] fp32, y [M, ldy] fp32, sb6 / sym tensors only.
+ *   x [M, ldx] fp32, y [M, ldy] fp32, sb6 / sym tensors of at most 32768 columns.
  *   workspace: rwkvq_gemm_workspace_bytes_for(M, IN) bytes, 256-byte aligned (or
- *   rwkvq_gemm_workspace_bytes(M), which covers IN <= 16384); it holds the fp16 copy of x the
- *   TMA loads read, the split-K accumulator tiles and a header.  Its first int32 is a status word the
+ *   rwkvq_gemm_workspace_bytes(M), which covers IN <= 16384); it holds the fp16 copy of x and of a
+ *   chunk of the weights.  Its first int32 is a status word the
  *   kernel sets to RWKVQ_E_TIMEOUT if a bounded wait on the tensor-core pipeline ran out
  *   (read it after synchronising the stream; 0 = ok).
  */
@@ -222,8 +222,8 @@ int rwkvq_gemm(const rwkvq_qtensor* t, const float* x, int M, int64_t ldx, float
                int epilogue, const float* resid, void* workspace, size_t workspace_bytes, void* stream);
 /* The same product on activations the caller has already brought into the form the kernel reads
  * (rwkvq_seq_ln_shift_mix_prep writes it): x16 fp16 [M, rwkvq_gemm_x16_pitch(IN)] = x * row_scale[m],
- * row_scale [M] fp32 powers of two.  The workspace (same size rule) then only carries the header
- * and the split-K tiles. */
+ * row_scale [M] fp32 powers of two.  The workspace (rwkvq_gemm_workspace_bytes_for(M, 0)) then only
+ * carries the status word and the weights. */
 size_t rwkvq_gemm_x16_pitch(int cols);
 int rwkvq_gemm_x16(const rwkvq_qtensor* t, const void* x16, const float* row_scale, int M, float* y, int64_t ldy,
                    int epilogue, const float* resid, void* workspace, size_t workspace_bytes, void* stream);
@@ -400,6 +400,29 @@ int rwkvq_decode_step(const rwkvq_model* m_host, int B, const int64_t* tokens,
                       float* const* wkv_host, float* const* tshift_host, float* const* cshift_host,
                       void* workspace, size_t workspace_bytes, float* logits, int64_t* next_tokens,
                       void* stream);
+
+/*
+ * The whole forward pass over B sequences of T tokens in one call: embedding, all layers, head.
+ * Stands behind QuantRWKV7.forward_stateful with T > 1 (backends/metal/quant_model.py:964-990).
+ *   tokens [B, T] int64 on the device
+ *   *_in   host arrays [n_layer] of device pointers: wkv [B, H, 64, 64], shift rows [B, D] fp32 (not
+ *          modified; NULL entries: zeros).  *_out: where the carried states go (an entry may equal its
+ *          wkv_in entry; the shift rows of a layer must not alias their inputs)
+ *   hidden [B, T, D] the final-LayerNorm rows, or NULL;  logits [B, tail, vocab] of the last `tail`
+ *          positions (tail = 0: none)
+ * Rows N = B * T up to 64 run on the fp32-grade small-batch linears (rwkvq_gemv_batch), more on fp16
+ * tensor-core operands (the arithmetic of rwkvq_gemm; LoRA products with x as an fp16 pair).
+ * rwkvq_forward_seq_ok: 1 if every tensor of the model has a layout this serves at n_rows rows (sb6 / sym
+ * linears with their relayouted streams; per-row int8 up to 64 rows; LoRA shapes of rwkvq_lora_pair;
+ * n_embd a multiple of 128 up to 4096).  workspace: rwkvq_forward_seq_workspace_bytes, 256-byte
+ * aligned; its first int32 is a status word (RWKVQ_E_TIMEOUT if a bounded device-side wait ran out).
+ */
+int rwkvq_forward_seq_ok(const rwkvq_model* m_host, int64_t n_rows);
+size_t rwkvq_forward_seq_workspace_bytes(const rwkvq_model* m_host, int B, int T, int tail);
+int rwkvq_forward_seq(const rwkvq_model* m_host, int B, int T, const int64_t* tokens,
+                      const float* const* wkv_in, const float* const* tshift_in, const float* const* cshift_in,
+                      float* const* wkv_out, float* const* tshift_out, float* const* cshift_out,
+                      int tail, float* hidden, float* logits, void* workspace, size_t workspace_bytes, void* stream);
 
 /*
  * Load-time relayout of the side streams of an sb6 / sym tensor for the decode

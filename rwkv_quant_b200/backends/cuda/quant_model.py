@@ -8,9 +8,8 @@ states, last_only, tail_only)``, ``forward_hidden``, ``__call__(idx)``; plus
 
 Two execution paths share the same weights (kept packed on the device):
   T == 1   one call of ``rwkvq_decode_step`` (all kernels of a token launched from C)
-  T  > 1   per-layer ops over all B*T positions: quantized linears, LoRA products,
-           ``wkv7_infer`` and ``wkv_tail`` are library kernels; layer norms, lerps and
-           gates are elementwise torch ops on the device.
+  T  > 1   one call of ``rwkvq_forward_seq``; models with a tensor it has no path for (per-row
+           layouts in long calls, ragged LoRA ranks) run per-layer ops over all B*T positions
 Weight precision follows the reference's loader (quant_model.py:128-154, 245-262):
 quantized linears are used exactly as coded; every other tensor is rounded to bf16,
 then to fp16 when it is 2-D with min(shape) >= 32 (LoRA, embedding, r_k).
@@ -112,6 +111,7 @@ class QuantRWKV7:
                             for L in self.blocks)
         self._build_struct()
         self._ws = {}
+        self._seq_ok = {}
         self._lora_dense = {}
         self.fused_prep = True       # sequence path: LN/shift/lerp rows written in their consumers' forms
         torch.cuda.synchronize(dev)
@@ -328,9 +328,44 @@ class QuantRWKV7:
             rows = ops.dequant(bufs, meta, torch.float32, True)
         return rows.half().float()[inv].reshape(*idx.shape, self.n_embd)
 
+    def _one_call_ok(self, n_rows: int) -> bool:
+        """Whether ``rwkvq_forward_seq`` serves calls of this many rows (layouts, shapes); the answer
+        depends on the regime only."""
+        if self._model_c is None or not self.fused_prep:
+            return False
+        small = n_rows <= self.batch_max
+        if small not in self._seq_ok:
+            self._seq_ok[small] = bool(_lib.load().rwkvq_forward_seq_ok(C.byref(self._model_c), n_rows))
+        return self._seq_ok[small]
+
+    def _forward_one_call(self, idx, states, tail, want_hidden):
+        """idx [B, T] on the device -> (hidden or None, logits [B, tail, V] or None, new states): every
+        launch of the pass issued by one library call."""
+        B, T = idx.shape
+        L, H, S, D, dev = self.n_layer, self.n_head, self.head_size, self.n_embd, self.device
+        lib = _lib.load()
+        idx = idx.contiguous()
+        ins = [[None if st[k] is None else st[k].reshape(shape).contiguous().float() for st in states]
+               for k, shape in ((0, (B, H, S, S)), (1, (B, D)), (2, (B, D)))]
+        f32 = dict(dtype=torch.float32, device=dev)
+        outs = [torch.empty((L, B, H, S, S), **f32), torch.empty((L, B, 1, D), **f32), torch.empty((L, B, 1, D), **f32)]
+        hidden = torch.empty((B, T, D), **f32) if want_hidden else None
+        logits = torch.empty((B, tail, self.vocab_size), **f32) if tail else None
+        nws = lib.rwkvq_forward_seq_workspace_bytes(C.byref(self._model_c), B, T, tail)
+        ws = torch.empty(nws, dtype=torch.uint8, device=dev)
+        table = C.c_void_p * L
+        arr_in = [table(*[None if t is None else t.data_ptr() for t in ts]) for ts in ins]
+        arr_out = [table(*[o.data_ptr() + i * o.stride(0) * 4 for i in range(L)]) for o in outs]
+        _lib.check(lib.rwkvq_forward_seq(C.byref(self._model_c), B, T, idx.data_ptr(), *arr_in, *arr_out, tail, _lib.ptr(hidden),
+                                         _lib.ptr(logits), ws.data_ptr(), nws, _lib.stream_ptr()), "rwkvq_forward_seq")
+        return hidden, logits, list(zip(*(o.unbind(0) for o in outs)))
+
     def forward_hidden(self, idx, states):
         idx = torch.as_tensor(idx, device=self.device).long()
         B, T = idx.shape
+        if B * T > 1 and self._one_call_ok(B * T):
+            hidden, _, new_states = self._forward_one_call(idx, states, 0, True)
+            return hidden, new_states
         states = self._materialize(states, B)
         if self.emb.outliers is None and self.n_embd <= 4096:
             x = ops.seq_embed_ln0(self.emb, idx.clamp(0, self.vocab_size - 1), *self.ln0)     # gather + LN0: one kernel
@@ -353,6 +388,10 @@ class QuantRWKV7:
             st = self._materialize(states, B)
             logits = self._decode(idx.reshape(B).contiguous(), st)
             return logits.reshape(B, 1, self.vocab_size), st
+        if self._one_call_ok(B * T):
+            tail = 1 if last_only else tail_only if tail_only and T > tail_only else T
+            _, logits, new_states = self._forward_one_call(idx, states, tail, False)
+            return logits, new_states
         x, new_states = self.forward_hidden(idx, states)
         if last_only:
             x = x[:, -1:]

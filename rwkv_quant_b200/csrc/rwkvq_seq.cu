@@ -8,6 +8,8 @@
 //                      kk = l2norm_head(k * k_k), k' = k (1 + (a - 1) k_a),
 //                      v' = v + (v_first - v) sigmoid(yv + v0) (layers > 0); emits w, k', v',
 //                      -kk and kk*a, the operands of the WKV-7 scan       (quant_model.py:700-712)
+#include "rwkvq_seq.cuh"
+
 #include "rwkvq_decode_parts.cuh"
 
 namespace rwkvq {
@@ -75,18 +77,6 @@ __global__ void __launch_bounds__(kSeqThreads) seq_ln_shift_mix_kernel(const flo
 // split [hi | lo]), or both; writing those forms here saves the fp32 round trip through HBM and
 // one launch per consumer.  The conversions are those of the GEMM's own pre-pass (scale =
 // 2^(14 - exponent of the row maximum)) and of split_fp16_kernel.
-constexpr int kPrepScaled = 1, kPrepSplit = 2, kPrepF32 = 4;
-struct SeqPrepArgs {
-    const float *x, *ln_w, *ln_b, *shift_in, *mix;
-    float* shift_out;
-    __half* x16[6];        // [N, D + 64]
-    float* scale[6];       // [N]
-    __half* split[6];      // [N, 2 D]
-    float* f32[6];         // [N, D]
-    int mode[6];
-    int T, D, n_mix;
-};
-
 __device__ __forceinline__ float block_max(float v, float* red) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
@@ -105,6 +95,12 @@ __global__ void __launch_bounds__(kSeqThreads, 3) seq_ln_shift_mix_prep_kernel(c
     const long long tok = blockIdx.x;
     const int D = a.D, b = static_cast<int>(tok / a.T), t = static_cast<int>(tok % a.T);
     const float* row = a.x + tok * D;
+    pdl_launch_dependents();
+    pdl_wait();
+    if (threadIdx.x == 0) {
+        if (a.zero_a != nullptr) a.zero_a[tok] = 0.f;
+        if (a.zero_b != nullptr) a.zero_b[tok] = 0.f;
+    }
     float2 v[kPairs], pv[kPairs];
     const float2 zero = make_float2(0.f, 0.f);
 #pragma unroll
@@ -183,6 +179,17 @@ __global__ void __launch_bounds__(kSeqThreads, 3) seq_ln_shift_mix_prep_kernel(c
         }
         const int mode = a.mode[m];
         float sc = 1.f;
+        if (m == 0 && a.n2 != nullptr) {
+            float q = 0.f;
+#pragma unroll
+            for (int i = 0; i < kPairs; ++i) q += val[i].x * val[i].x + val[i].y * val[i].y;
+            q = block_sum(q, red);
+            if (threadIdx.x == 0) a.n2[tok] = q;
+        }
+        if (mode & kPrepAmax) {
+            amax = block_max(amax, red);
+            if (threadIdx.x == 0) a.scale[m][tok] = amax;
+        }
         if (mode & kPrepScaled) {
             amax = block_max(amax, red);
             int e = 0;
@@ -208,6 +215,324 @@ __global__ void __launch_bounds__(kSeqThreads, 3) seq_ln_shift_mix_prep_kernel(c
     }
 }
 
+// The same for few tokens and D a multiple of 256: a CTA per token (or run of tokens) and mix, so that the
+// mixes run side by side; D / 8 threads own 8 consecutive columns each (16-byte stores of the fp16 forms),
+// parameters and lerp vector loaded before the launch wait.  Bound: the latency of the two sums.
+constexpr int kSeqVecWarps = 16;
+__device__ __forceinline__ void prep_load8(const float* p, float (&o)[8]) {
+    const float4 x = *reinterpret_cast<const float4*>(p), y = *reinterpret_cast<const float4*>(p + 4);
+    o[0] = x.x; o[1] = x.y; o[2] = x.z; o[3] = x.w; o[4] = y.x; o[5] = y.y; o[6] = y.z; o[7] = y.w;
+}
+__device__ __forceinline__ void prep_load8cg(const float* p, float (&o)[8]) {
+    const float4 x = __ldcg(reinterpret_cast<const float4*>(p)), y = __ldcg(reinterpret_cast<const float4*>(p) + 1);
+    o[0] = x.x; o[1] = x.y; o[2] = x.z; o[3] = x.w; o[4] = y.x; o[5] = y.y; o[6] = y.z; o[7] = y.w;
+}
+__device__ __forceinline__ void prep_store8(float* p, const float (&v)[8]) {
+    *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    *reinterpret_cast<float4*>(p + 4) = make_float4(v[4], v[5], v[6], v[7]);
+}
+__device__ __forceinline__ uint4 prep_pack8(const float (&v)[8]) {
+    uint4 r;
+    __half2 h;
+    h = __floats2half2_rn(v[0], v[1]); r.x = *reinterpret_cast<uint32_t*>(&h);
+    h = __floats2half2_rn(v[2], v[3]); r.y = *reinterpret_cast<uint32_t*>(&h);
+    h = __floats2half2_rn(v[4], v[5]); r.z = *reinterpret_cast<uint32_t*>(&h);
+    h = __floats2half2_rn(v[6], v[7]); r.w = *reinterpret_cast<uint32_t*>(&h);
+    return r;
+}
+__device__ __forceinline__ float warp_add(float v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
+    return v;
+}
+// power of two with |x| * 2^s <= 2^14 for max|x| = amax
+__device__ __forceinline__ float prep_scale(float amax) {
+    int e = 0;
+    if (amax > 0.f && amax < INFINITY) frexpf(amax, &e);
+    return ldexpf(1.f, 14 - e);
+}
+// 8 columns of mix row m of token tok in the forms `mode` selects
+__device__ __forceinline__ void prep_emit8(const SeqPrepArgs& a, int m, int mode, long long tok, int d0, float (&o)[8], float sc) {
+    const int D = a.D;
+    if (mode & kPrepF32) prep_store8(a.f32[m] + tok * D + d0, o);
+    if (mode & kPrepSplit) {
+        float lo[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) lo[i] = o[i] - __half2float(__float2half_rn(o[i]));
+        __half* p = a.split[m] + tok * 2 * D + d0;
+        *reinterpret_cast<uint4*>(p) = prep_pack8(o);
+        *reinterpret_cast<uint4*>(p + D) = prep_pack8(lo);
+    }
+    if (mode & kPrepScaled) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) o[i] *= sc;
+        *reinterpret_cast<uint4*>(a.x16[m] + tok * (D + 64) + d0) = prep_pack8(o);
+    }
+}
+
+__global__ void __launch_bounds__(kSeqVecWarps * 32) seq_prep_vec_kernel(const SeqPrepArgs a, long long n_tokens, int run) {
+    __shared__ float red_s[kSeqVecWarps], red_q[kSeqVecWarps];
+    __shared__ float2 red_m[kSeqVecWarps];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
+    const int D = a.D, d0 = tid * 8, m = blockIdx.y, mode = a.mode[m];
+    const long long tok0 = static_cast<long long>(blockIdx.x) * run, tok1 = min(tok0 + run, n_tokens);
+    float lw[8], lb[8], mx[8];
+    prep_load8(a.ln_w + d0, lw);
+    prep_load8(a.ln_b + d0, lb);
+    prep_load8(a.mix + static_cast<size_t>(m) * D + d0, mx);
+    const bool want_n2 = a.n2 != nullptr && m == 0, want_max = (mode & (kPrepScaled | kPrepAmax)) != 0;
+    pdl_launch_dependents();
+    pdl_wait();
+    if (m == 0)
+        for (long long t = tok0 + tid; t < tok1; t += blockDim.x) {
+            if (a.zero_a != nullptr) a.zero_a[t] = 0.f;
+            if (a.zero_b != nullptr) a.zero_b[t] = 0.f;
+        }
+    // two-pass LayerNorm; the barriers of the two sums also separate the uses of each buffer
+    auto normalise = [&](float (&y)[8]) {
+        float s = warp_add(((y[0] + y[1]) + (y[2] + y[3])) + ((y[4] + y[5]) + (y[6] + y[7])));
+        if (lane == 0) red_s[warp] = s;
+        __syncthreads();
+        s = 0.f;
+        for (int w = 0; w < nw; ++w) s += red_s[w];
+        const float mean = s / D;
+        float q = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) { const float c = y[i] - mean; q = fmaf(c, c, q); }
+        q = warp_add(q);
+        if (lane == 0) red_q[warp] = q;
+        __syncthreads();
+        q = 0.f;
+        for (int w = 0; w < nw; ++w) q += red_q[w];
+        const float inv = 1.0f / sqrtf(q / D + 1e-5f);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) y[i] = (y[i] - mean) * inv * lw[i] + lb[i];
+    };
+    float nx[8], pv[8];
+    prep_load8cg(a.x + tok0 * D + d0, nx);
+    int t = static_cast<int>(tok0 % a.T), b = static_cast<int>(tok0 / a.T);
+    if (t > 0) {
+        prep_load8cg(a.x + (tok0 - 1) * D + d0, pv);
+        normalise(pv);
+    }
+    for (long long tok = tok0; tok < tok1; ++tok) {
+        float v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = nx[i];
+        if (tok + 1 < tok1) prep_load8cg(a.x + (tok + 1) * D + d0, nx);
+        if (t == 0) {
+            if (a.shift_in) prep_load8(a.shift_in + static_cast<size_t>(b) * D + d0, pv);
+            else {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) pv[i] = 0.f;
+            }
+        }
+        normalise(v);
+        if (t == a.T - 1 && m == 0) prep_store8(a.shift_out + static_cast<size_t>(b) * D + d0, v);
+        float o[8], am = 0.f, n2 = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            o[i] = v[i] + (pv[i] - v[i]) * mx[i];
+            am = fmaxf(am, fabsf(o[i]));
+            n2 = fmaf(o[i], o[i], n2);
+            pv[i] = v[i];
+        }
+        float sc = 1.f;
+        if (want_max || want_n2) {
+#pragma unroll
+            for (int q = 16; q > 0; q >>= 1) {
+                am = fmaxf(am, __shfl_xor_sync(0xFFFFFFFFu, am, q));
+                n2 += __shfl_xor_sync(0xFFFFFFFFu, n2, q);
+            }
+            if (lane == 0) red_m[warp] = make_float2(am, n2);
+            __syncthreads();
+            n2 = 0.f;
+            for (int w = 0; w < nw; ++w) { am = fmaxf(am, red_m[w].x); n2 += red_m[w].y; }
+            sc = prep_scale(am);
+            if (tid == 0) {
+                if (want_n2) a.n2[tok] = n2;
+                if (want_max) a.scale[m][tok] = (mode & kPrepScaled) ? sc : am;
+            }
+        }
+        prep_emit8(a, m, mode, tok, d0, o, sc);
+        if (++t == a.T) { t = 0; ++b; }
+    }
+}
+
+// Many tokens, D a multiple of 512: 64 threads per token (a barrier of two warps, not of a CTA, behind
+// every sum), four tokens side by side in a CTA that share the parameters and lerp vectors in shared
+// memory; a group walks a run of consecutive tokens and keeps the normalised row for its successor.
+// Bound: HBM writes of the six rows.
+constexpr int kPrepGroup = 64, kPrepGroups = 4;
+template <int CH>      // chunks of 512 columns
+__global__ void __launch_bounds__(kPrepGroup * kPrepGroups, 2) seq_prep_group_kernel(const SeqPrepArgs a, long long n_tokens, int run) {
+    extern __shared__ __align__(16) float params[];      // [2 + n_mix][D]
+    __shared__ float red_s[kPrepGroups][2], red_q[kPrepGroups][2];
+    __shared__ float red_m[kPrepGroups][2][8];
+    constexpr int D = CH * 512;
+    const int grp = threadIdx.x / kPrepGroup, tid = threadIdx.x % kPrepGroup, wp = tid >> 5, lane = tid & 31, n_mix = a.n_mix;
+    for (int i = threadIdx.x; i < D / 4; i += kPrepGroup * kPrepGroups) {
+        reinterpret_cast<float4*>(params)[i] = __ldg(reinterpret_cast<const float4*>(a.ln_w) + i);
+        reinterpret_cast<float4*>(params + D)[i] = __ldg(reinterpret_cast<const float4*>(a.ln_b) + i);
+        for (int m = 0; m < n_mix; ++m)
+            reinterpret_cast<float4*>(params + (2 + m) * D)[i] = __ldg(reinterpret_cast<const float4*>(a.mix + static_cast<size_t>(m) * D) + i);
+    }
+    bool any_max = a.n2 != nullptr;
+    for (int m = 0; m < n_mix; ++m) any_max |= (a.mode[m] & (kPrepScaled | kPrepAmax)) != 0;
+    pdl_launch_dependents();
+    __syncthreads();
+    pdl_wait();
+    auto group_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "n"(kPrepGroup) : "memory"); };
+    const long long tok0 = (static_cast<long long>(blockIdx.x) * kPrepGroups + grp) * run, tok1 = min(tok0 + run, n_tokens);
+    if (tok0 >= tok1) return;
+    for (long long t = tok0 + tid; t < tok1; t += kPrepGroup) {
+        if (a.zero_a != nullptr) a.zero_a[t] = 0.f;
+        if (a.zero_b != nullptr) a.zero_b[t] = 0.f;
+    }
+    auto load_row = [&](const float* row, float (&y)[CH][8]) {
+#pragma unroll
+        for (int c = 0; c < CH; ++c) prep_load8cg(row + 8 * (tid + kPrepGroup * c), y[c]);
+    };
+    auto normalise = [&](float (&y)[CH][8]) {
+        float s = 0.f;
+#pragma unroll
+        for (int c = 0; c < CH; ++c)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) s += y[c][i];
+        s = warp_add(s);
+        if (lane == 0) red_s[grp][wp] = s;
+        group_sync();
+        const float mean = (red_s[grp][0] + red_s[grp][1]) / D;
+        float q = 0.f;
+#pragma unroll
+        for (int c = 0; c < CH; ++c)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) { const float e = y[c][i] - mean; q = fmaf(e, e, q); }
+        q = warp_add(q);
+        if (lane == 0) red_q[grp][wp] = q;
+        group_sync();
+        const float inv = 1.0f / sqrtf((red_q[grp][0] + red_q[grp][1]) / D + 1e-5f);
+#pragma unroll
+        for (int c = 0; c < CH; ++c) {
+            float w[8], b[8];
+            prep_load8(params + 8 * (tid + kPrepGroup * c), w);
+            prep_load8(params + D + 8 * (tid + kPrepGroup * c), b);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) y[c][i] = (y[c][i] - mean) * inv * w[i] + b[i];
+        }
+    };
+    float v[CH][8], pv[CH][8];
+    int t = static_cast<int>(tok0 % a.T), b = static_cast<int>(tok0 / a.T);
+    if (t > 0) load_row(a.x + (tok0 - 1) * D, pv);
+    load_row(a.x + tok0 * D, v);
+    if (t > 0) normalise(pv);
+    for (long long tok = tok0;;) {
+        if (t == 0) {
+#pragma unroll
+            for (int c = 0; c < CH; ++c) {
+                if (a.shift_in) prep_load8(a.shift_in + static_cast<size_t>(b) * D + 8 * (tid + kPrepGroup * c), pv[c]);
+                else {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) pv[c][i] = 0.f;
+                }
+            }
+        }
+        normalise(v);
+        if (t == a.T - 1) {
+#pragma unroll
+            for (int c = 0; c < CH; ++c) prep_store8(a.shift_out + static_cast<size_t>(b) * D + 8 * (tid + kPrepGroup * c), v[c]);
+        }
+#pragma unroll
+        for (int c = 0; c < CH; ++c)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) pv[c][i] -= v[c][i];     // xx = prev - cur
+        if (any_max) {
+            float n2 = 0.f;
+            for (int m = 0; m < n_mix; ++m) {
+                float x = 0.f;
+#pragma unroll
+                for (int c = 0; c < CH; ++c) {
+                    float mx[8];
+                    prep_load8(params + (2 + m) * D + 8 * (tid + kPrepGroup * c), mx);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const float o = v[c][i] + pv[c][i] * mx[i];
+                        x = fmaxf(x, fabsf(o));
+                        if (m == 0) n2 = fmaf(o, o, n2);
+                    }
+                }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) x = fmaxf(x, __shfl_xor_sync(0xFFFFFFFFu, x, o));
+                if (lane == 0) red_m[grp][wp][m] = x;
+            }
+            n2 = warp_add(n2);
+            if (lane == 0) red_m[grp][wp][6] = n2;
+            group_sync();
+            if (a.n2 != nullptr && tid == 0) a.n2[tok] = red_m[grp][0][6] + red_m[grp][1][6];
+        }
+        for (int m = 0; m < n_mix; ++m) {
+            const int mode = a.mode[m];
+            float sc = 1.f;
+            if (mode & (kPrepScaled | kPrepAmax)) {
+                const float am = fmaxf(red_m[grp][0][m], red_m[grp][1][m]);
+                sc = prep_scale(am);
+                if (tid == 0) a.scale[m][tok] = (mode & kPrepScaled) ? sc : am;
+            }
+#pragma unroll
+            for (int c = 0; c < CH; ++c) {
+                const int d0 = 8 * (tid + kPrepGroup * c);
+                float mx[8], o[8];
+                prep_load8(params + (2 + m) * D + d0, mx);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) o[i] = v[c][i] + pv[c][i] * mx[i];
+                prep_emit8(a, m, mode, tok, d0, o, sc);
+            }
+        }
+        if (++tok == tok1) break;
+#pragma unroll
+        for (int c = 0; c < CH; ++c)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) pv[c][i] = v[c][i];
+        load_row(a.x + tok * D, v);
+        if (++t == a.T) { t = 0; ++b; }
+    }
+}
+
+template <int CH>
+static cudaError_t launch_prep_group(const SeqPrepArgs& a, long long n_tokens, cudaStream_t s) {
+    const size_t smem = sizeof(float) * (2 + a.n_mix) * CH * 512;
+    cudaError_t e = cudaFuncSetAttribute(seq_prep_group_kernel<CH>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(8 * sizeof(float) * CH * 512));
+    if (e != cudaSuccess) return e;
+    const long long wave = 148 * 2 * kPrepGroups;                // groups resident at once
+    const int run = static_cast<int>((n_tokens + wave - 1) / wave);
+    const long long groups = (n_tokens + run - 1) / run;
+    return launch_pdl(seq_prep_group_kernel<CH>, dim3(static_cast<unsigned>((groups + kPrepGroups - 1) / kPrepGroups)),
+                      dim3(kPrepGroup * kPrepGroups), smem, s, a, n_tokens, run);
+}
+
+int launch_seq_prep(const SeqPrepArgs& a, long long n_tokens, cudaStream_t s) {
+    cudaError_t e;
+    // rows on 16-byte boundaries throughout, as the vector forms read and write them
+    bool vec = a.D % 256 == 0 && a.D <= kSeqVecWarps * 256 && aligned(a.x, 16) && aligned(a.ln_w, 16) && aligned(a.ln_b, 16) &&
+               aligned(a.mix, 16) && aligned(a.shift_in, 16) && aligned(a.shift_out, 16);
+    for (int m = 0; m < a.n_mix; ++m) vec = vec && aligned(a.x16[m], 16) && aligned(a.split[m], 16) && aligned(a.f32[m], 16);
+    // one wave of CTAs (two per SM) with a token and mix each, then groups of 64 threads per token
+    const bool few = n_tokens * a.n_mix <= 2 * 148;
+    if (vec && !few && a.D == 2048) e = launch_prep_group<4>(a, n_tokens, s);
+    else if (vec && !few && a.D == 2560) e = launch_prep_group<5>(a, n_tokens, s);
+    else if (vec && !few && a.D == 1024) e = launch_prep_group<2>(a, n_tokens, s);
+    else if (vec) {
+        long long run = n_tokens * a.n_mix / (148 * 8);
+        run = run < 1 ? 1 : run > 16 ? 16 : run;
+        e = launch_pdl(seq_prep_vec_kernel, dim3(static_cast<unsigned>((n_tokens + run - 1) / run), a.n_mix), dim3(a.D / 8), 0, s, a, n_tokens,
+                       static_cast<int>(run));
+    } else {
+        e = launch_pdl(seq_ln_shift_mix_prep_kernel, dim3(static_cast<unsigned>(n_tokens)), dim3(kSeqThreads), 0, s, a);
+    }
+    if (e != cudaSuccess) return fail(RWKVQ_E_LAUNCH, "seq_ln_shift_mix_prep: %s", cudaGetErrorString(e));
+    return RWKVQ_OK;
+}
+
 struct TmixPreArgs {
     const float *k, *v, *yw, *ya, *yv, *v_first;     // [N, D]; yv / v_first null on layer 0
     const float *w0, *a0, *v0, *k_k, *k_a;           // [D]
@@ -220,6 +545,8 @@ struct TmixPreArgs {
 // loads and stores).
 __global__ void __launch_bounds__(256) seq_tmix_pre_kernel(const TmixPreArgs p) {
     const long long pair = blockIdx.x * 8ll + (threadIdx.x >> 5);
+    pdl_launch_dependents();
+    pdl_wait();
     if (pair >= p.n_pairs) return;
     const int lane = threadIdx.x & 31, hd = static_cast<int>(pair % p.H);
     const size_t i = static_cast<size_t>(pair) * 64 + 2 * lane;
@@ -325,8 +652,8 @@ int rwkvq_seq_ln_shift_mix_prep(const float* x, const float* ln_w, const float* 
             a.f32[m] = out_f32[m];
         }
     }
-    seq_ln_shift_mix_prep_kernel<<<static_cast<unsigned>(n), kSeqThreads, 0, static_cast<cudaStream_t>(stream)>>>(a);
-    return check_launch("rwkvq_seq_ln_shift_mix_prep");
+    int rc = launch_seq_prep(a, n, static_cast<cudaStream_t>(stream));
+    return rc ? rc : check_launch("rwkvq_seq_ln_shift_mix_prep");
 }
 
 int rwkvq_seq_tmix_pre(const float* k, const float* v, const float* yw, const float* ya, const float* yv,
@@ -345,7 +672,7 @@ int rwkvq_seq_tmix_pre(const float* k, const float* v, const float* yw, const fl
     TmixPreArgs p{k, v, yw, ya, yv, v_first, w0, a0, v0, k_k, k_a, w, k2, v2, neg_kk, kk_a, n_tokens * H, H};
     const long long blocks = (p.n_pairs + 7) / 8;
     RWKVQ_REQUIRE(blocks < (1ll << 31), RWKVQ_E_LIMIT, "rwkvq_seq_tmix_pre: too many tokens");
-    seq_tmix_pre_kernel<<<static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(p);
+    launch_pdl(seq_tmix_pre_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, static_cast<cudaStream_t>(stream), p);
     return check_launch("rwkvq_seq_tmix_pre");
 }
 

@@ -1,0 +1,30 @@
+// Launchers of the sequence-path glue kernels (rwkvq_seq.cu, rwkvq_wkv.cu) for the one-call forward.
+#pragma once
+#include "rwkvq_common.cuh"
+
+namespace rwkvq {
+
+// Forms a mix row can be written in (bits of SeqPrepArgs::mode)
+constexpr int kPrepScaled = 1;      // scaled fp16 copy + scale, the operand of the fp16 GEMM
+constexpr int kPrepSplit = 2;       // fp16 pair [hi | lo]
+constexpr int kPrepF32 = 4;
+constexpr int kPrepAmax = 8;        // max|row| into scale[m] (beside kPrepF32: what the small-batch linears read)
+
+struct SeqPrepArgs {
+    const float *x, *ln_w, *ln_b, *shift_in, *mix;
+    float* shift_out;
+    __half* x16[6];        // [N, D + 64]
+    float* scale[6];       // [N]
+    __half* split[6];      // [N, 2 D]
+    float* f32[6];         // [N, D]
+    int mode[6];
+    int T, D, n_mix;
+    float* n2;             // optional [N]: squared norm of mix row 0 (unscaled)
+    float *zero_a, *zero_b;    // optional [N]: cleared
+};
+int launch_seq_prep(const SeqPrepArgs& a, long long n_tokens, cudaStream_t s);
+
+int launch_wkv_tail(const float* wkv, const float* r, const float* k, const float* v, const float* r_k, const float* ln_w,
+                    const float* ln_b, const float* g, float* out, int N, int H, float eps, float* og_amax, cudaStream_t s);
+
+}  // namespace rwkvq

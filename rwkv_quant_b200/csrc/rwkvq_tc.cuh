@@ -1,4 +1,4 @@
-// Device-side building blocks shared by the tcgen05 kernels (rwkvq_gemm_tc.cu: prefill and large
+// Device-side building blocks shared by the tcgen05 kernels (rwkvq_gemm_f16.cu: prefill and large
 // batches; rwkvq_gemm_tcb.cu: small decode batches): PTX wrappers for mbarriers, tensor memory and
 // tcgen05.mma, the 128-byte-swizzled K-major operand layout, and the weight producer that turns
 // packed file bytes into fp16 operand rows.

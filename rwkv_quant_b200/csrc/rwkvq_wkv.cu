@@ -7,7 +7,7 @@
 // independent, so a CTA owns one (batch, head) and its threads keep tiles of the state in
 // registers for the whole scan; the two dot products per step end in shuffles.  The
 // r/w/k/v/a/b rows of following steps are staged in shared memory ahead of time (see below).
-#include "rwkvq_common.cuh"
+#include "rwkvq_seq.cuh"
 
 namespace rwkvq {
 
@@ -226,8 +226,10 @@ __global__ void __launch_bounds__(512 / R / SPLIT, 4) wkv7_kernel(const WkvArgs 
 __global__ void __launch_bounds__(128) wkv_tail_kernel(const float* wkv, const float* r, const float* k,
                                                        const float* v, const float* r_k, const float* ln_w,
                                                        const float* ln_b, const float* g, float* out,
-                                                       int n_pairs, int H, float eps) {
+                                                       int n_pairs, int H, float eps, float* og_amax) {
     const int pair = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    pdl_launch_dependents();
+    pdl_wait();
     if (pair >= n_pairs) return;
     const int hd = pair % H;
     const size_t base = static_cast<size_t>(pair) * kS;
@@ -246,9 +248,25 @@ __global__ void __launch_bounds__(128) wkv_tail_kernel(const float* wkv, const f
                r[base + lane + 32] * k[base + lane + 32] * r_k[hb + lane + 32];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) dp += __shfl_xor_sync(0xFFFFFFFFu, dp, o);
-    out[base + lane] = (d0 * inv * ln_w[hb + lane] + ln_b[hb + lane] + dp * v[base + lane]) * g[base + lane];
-    out[base + lane + 32] =
-        (d1 * inv * ln_w[hb + lane + 32] + ln_b[hb + lane + 32] + dp * v[base + lane + 32]) * g[base + lane + 32];
+    const float o0 = (d0 * inv * ln_w[hb + lane] + ln_b[hb + lane] + dp * v[base + lane]) * g[base + lane];
+    const float o1 = (d1 * inv * ln_w[hb + lane + 32] + ln_b[hb + lane + 32] + dp * v[base + lane + 32]) * g[base + lane + 32];
+    out[base + lane] = o0;
+    out[base + lane + 32] = o1;
+    if (og_amax != nullptr) {                 // |o| as int bits orders like the float, a NaN above every number
+        int m = max(__float_as_int(fabsf(o0)), __float_as_int(fabsf(o1)));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
+        if (lane == 0) atomicMax(reinterpret_cast<int*>(og_amax) + pair / H, m);
+    }
+}
+
+int launch_wkv_tail(const float* wkv, const float* r, const float* k, const float* v, const float* r_k, const float* ln_w,
+                    const float* ln_b, const float* g, float* out, int N, int H, float eps, float* og_amax, cudaStream_t s) {
+    const int pairs = N * H;
+    cudaError_t e = launch_pdl(wkv_tail_kernel, dim3((pairs + 3) / 4), dim3(128), 0, s, wkv, r, k, v, r_k, ln_w, ln_b, g, out, pairs, H,
+                               eps, og_amax);
+    if (e != cudaSuccess) return fail(RWKVQ_E_LAUNCH, "wkv_tail: %s", cudaGetErrorString(e));
+    return RWKVQ_OK;
 }
 
 }  // namespace rwkvq
@@ -271,6 +289,8 @@ int rwkvq_wkv7(const float* r, const float* w, const float* k, const float* v, c
     // few (batch, head) pairs: smaller tiles and several CTAs per pair, so that a step is short;
     // full grids: the largest tile (least shared-memory traffic and issue per state element)
     const int pairs = B * H;
+    // (plain launches: CTAs that start while the kernel before still fills the chip pile up on the SMs it
+    // leaves first, and the scan of one batch element takes 300 us instead of 100)
     if (pairs > 2 * 148) wkv7_kernel<8, 1><<<pairs, 64, kWkvSmemBytes, st>>>(p);
     else if (pairs > 74) wkv7_kernel<4, 1><<<pairs, 128, kWkvSmemBytes, st>>>(p);
     else wkv7_kernel<2, 4><<<pairs * 4, 64, kWkvSmemBytes, st>>>(p);
@@ -283,9 +303,8 @@ int rwkvq_wkv_tail(const float* wkv, const float* r, const float* k, const float
     RWKVQ_REQUIRE(wkv && r && k && v && r_k && ln_w && ln_b && g && out, RWKVQ_E_NULL, "rwkvq_wkv_tail: null pointer");
     RWKVQ_REQUIRE(head_size == kS, RWKVQ_E_SHAPE, "rwkvq_wkv_tail: head size %d, only 64 is built", head_size);
     RWKVQ_REQUIRE(N >= 1 && H >= 1, RWKVQ_E_SHAPE, "rwkvq_wkv_tail: N=%d H=%d", N, H);
-    const int pairs = N * H;
-    wkv_tail_kernel<<<(pairs + 3) / 4, 128, 0, static_cast<cudaStream_t>(stream)>>>(wkv, r, k, v, r_k, ln_w, ln_b, g,
-                                                                                  out, pairs, H, eps);
+    int rc = launch_wkv_tail(wkv, r, k, v, r_k, ln_w, ln_b, g, out, N, H, eps, nullptr, static_cast<cudaStream_t>(stream));
+    if (rc) return rc;
     return check_launch("rwkvq_wkv_tail");
 }
 

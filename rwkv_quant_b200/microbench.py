@@ -214,7 +214,7 @@ def gemm_sweep(recipe="compression", Ms=(64, 512, 8192), reps=20, acc_mode=0):
     """rwkvq_gemm (pre-pass + tensor-core kernel) on the four linear shapes of a 1.5B layer
     and the head: microseconds per call (CUDA-graph replay, so that host time does not
     count) and TFLOP/s = 2 * M * OUT * IN / time.  acc_mode: 0 the launcher's tile choice,
-    1 128-row tiles only, 2 256-row tiles wherever legal."""
+    1 single-CTA tiles only, 2 CTA pairs only."""
     f = _lib.load().rwkvq_profiling_gemm_acc_mode      # rwkvq_profiling.h: not part of the C ABI
     f.restype, f.argtypes = None, [C.c_int]
     f(acc_mode)
@@ -387,35 +387,6 @@ def gemm_once(layout="sb6", bits=5, rows=2048, cols=2048, M=8192, launches=3):
         y = ops.gemm(dq, x, check=True)
     torch.cuda.synchronize()
     print("ok", float(y.abs().sum()))
-
-
-def gemm_timeline(layout="sb6", bits=5, rows=2048, cols=2048, M=8192, acc_mode=0):
-    """Pipeline timeline of CTA (0,0,0) of one rwkvq_gemm launch: per macro-iteration
-    when its weight stage was free, converted, seen full by the issuer and issued."""
-    import numpy as np
-    f = _lib.load().rwkvq_profiling_gemm_acc_mode      # rwkvq_profiling.h: not part of the C ABI
-    f.restype, f.argtypes = None, [C.c_int]
-    f(acc_mode)
-    dq = _tensor(layout, bits, rows, cols)
-    x = torch.randn(M, cols, device="cuda")
-    ops.gemm(dq, x, check=True)
-    buf = torch.zeros(512, dtype=torch.int64, device="cuda")
-    lib = _lib.load()
-    _trace = lib.rwkvq_profiling_gemm_trace          # rwkvq_profiling.h: not part of the C ABI
-    _trace.restype, _trace.argtypes = None, [C.c_void_p]
-    _trace(buf.data_ptr())
-    ops.gemm(dq, x)
-    torch.cuda.synchronize()
-    _trace(None)
-    t = buf.cpu().numpy().astype(np.float64)
-    t0 = t[0]
-    n = sum(1 for i in range(120) if t[8 + 4 * i] > 0)
-    us = lambda v: (v - t0) / 1e3
-    print(f"gemm timeline {layout}@{bits} [{rows},{cols}] M={M}: accumulator complete {us(t[1]):.2f} us, CTA end {us(t[2]):.2f} us, {n} macro-iterations")
-    print("  i  stage free  converted  issuer full  issued")
-    for i in range(n):
-        r = t[8 + 4 * i: 12 + 4 * i]
-        print(f"{i:3d} {us(r[1]) if r[1] else 0:10.2f} {us(r[0]):10.2f} {us(r[2]):12.2f} {us(r[3]):7.2f}")
 
 
 def prefill(layers=24, recipe="reduction", T=512, batch=1, model="1.5b", reps=3):
@@ -626,9 +597,6 @@ def main():
     bt.add_argument("--recipe", default="compression"); bt.add_argument("--model", default="1.5b")
     bs = sub.add_parser("batch-sweep")
     bs.add_argument("--recipe", default="compression")
-    gt = sub.add_parser("gemm-timeline")
-    gt.add_argument("--M", type=int, default=8192); gt.add_argument("--rows", type=int, default=2048)
-    gt.add_argument("--cols", type=int, default=2048); gt.add_argument("--acc-mode", type=int, default=0); gt.add_argument("--bits", type=int, default=5)
     gs = sub.add_parser("gemm-sweep"); gs.add_argument("--acc-mode", type=int, default=0)
     gs.add_argument("--recipe", default="compression")
     wk = sub.add_parser("wkv")
@@ -658,9 +626,6 @@ def main():
         return
     if a.cmd == "batch-sweep":
         batch_sweep(a.recipe)
-        return
-    if a.cmd == "gemm-timeline":
-        gemm_timeline("sb6", a.bits, a.rows, a.cols, a.M, a.acc_mode)
         return
     if a.cmd == "quantize":
         quantize_time()
