@@ -159,6 +159,10 @@ int rwkvq_outlier_tail(const int32_t* row_ptr, const int32_t* cols, const float*
  */
 int rwkvq_quantize_sb6(const float* w, int64_t ldw, int rows, int cols, int bits, int search, const float* ex2,
                        uint8_t* q, uint8_t* qs, int8_t* qm, void* d, void* dm, void* stream);
+/* The same, written as the file's buffers in the same pass: codes_packed [rows, cols/2], qh / qh2
+ * [rows, cols/8] (from 5 / 6 bits on, else ignored), qsqm [rows, cols/256, 12]. */
+int rwkvq_quantize_sb6_packed(const float* w, int64_t ldw, int rows, int cols, int bits, int search, const float* ex2,
+                              uint8_t* codes_packed, uint8_t* qh, uint8_t* qh2, uint8_t* qsqm, void* d, void* dm, void* stream);
 
 /*
  * The same for the symmetric layout (blocks of 16, int8 block-scale codes against one fp16 per 256 weights);
@@ -170,6 +174,9 @@ int rwkvq_quantize_sb6(const float* w, int64_t ldw, int rows, int cols, int bits
  */
 int rwkvq_quantize_sym(const float* w, int64_t ldw, int rows, int cols, int bits, const float* factors, int n_factors,
                        const float* ex2, int8_t* q, int8_t* qs, void* d, void* stream);
+/* 6-bit codes written as the file's buffers in the same pass: codes_packed [rows, cols/2], qh / qh2 [rows, cols/8] */
+int rwkvq_quantize_sym6_packed(const float* w, int64_t ldw, int rows, int cols, const float* factors, int n_factors, const float* ex2,
+                               uint8_t* codes_packed, uint8_t* qh, uint8_t* qh2, int8_t* qs, void* d, void* stream);
 
 /*
  * The same product for a SMALL BATCH of right-hand sides (decode streams, short verify runs)

@@ -1,9 +1,13 @@
 // Block quantizers for the sb6 and sym layouts on the device.  sb6: the search the reference runs in torch on the
 // host (rwkv_quant/calibration/groupwise.py:207-300, `_gw_one` with 8 blocks of 32 per super-block).
 //
-// One warp owns one (row, super-block) = 256 weights: lane l holds element l of each of the 8
-// blocks, so every per-block reduction (min, max, the weighted means, covariance, variance, squared
-// error) is a 5-step shuffle tree and nothing touches shared memory.
+// One THREAD owns one block (32 weights, 16 in the sym layout): its weights stay in registers, so the sums,
+// extremes and errors of the search are plain register arithmetic (a warp per super-block with shuffle
+// trees took 1263 us for [10240, 2560] at 4 bits, five shuffles for every sum of 32); 8 (16) adjacent lanes hold a
+// super-block.  Sums add in the order of a butterfly over the block (i with i + 16, then + 8, ..).
+// A code rint(u / s) is found as rint(u * (1 / s)) by adding and subtracting 1.5 * 2^23; only where a product
+// comes within its error of a half does the block repeat the step with the rounded division, so every
+// code is the division's.  The packed entry points write the file buffers from the same registers.
 //   per block      s0 = max((max - min) / qmax, 1e-8); with search, for each factor f of
 //                  {0.7 .. 1.05}: q = clamp(rint((w - min) / (f s0))), the closed-form least-squares
 //                  (s, m) for those codes (weights E[x^2] of the input channel when given), the codes
@@ -24,168 +28,305 @@ namespace rwkvq {
 
 namespace {
 
-__device__ __forceinline__ float wsum(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-    return v;
-}
-__device__ __forceinline__ float wmax(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
-    return v;
-}
-__device__ __forceinline__ float wmin(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
-    return v;
-}
 __device__ __forceinline__ float hrt(float x) { return __half2float(__float2half_rn(x)); }
 __device__ __forceinline__ float clampf(float v, float lo, float hi) { return fminf(fmaxf(v, lo), hi); }
 
-__global__ void __launch_bounds__(256) quant_sb6_kernel(const float* __restrict__ w, long long ldw, int rows, int nsb, int bits,
-                                                         int search, const float* __restrict__ ex2, uint8_t* __restrict__ q,
-                                                         uint8_t* __restrict__ qs_out, int8_t* __restrict__ qm_out,
-                                                         __half* __restrict__ d_out, __half* __restrict__ dm_out) {
-    const int lane = threadIdx.x & 31;
-    const long long unit = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
-    if (unit >= static_cast<long long>(rows) * nsb) return;          // whole warps leave together
-    const int row = static_cast<int>(unit / nsb), sbk = static_cast<int>(unit % nsb);
-    const float* wp = w + static_cast<size_t>(row) * ldw + sbk * 256 + lane;
-    const float qmax = static_cast<float>((1 << bits) - 1);
-    float wv[8], ev[8];
+// sum of N values in butterfly order
+template <int N>
+__device__ __forceinline__ float tree(float (&v)[N]) {
 #pragma unroll
-    for (int b = 0; b < 8; ++b) {
-        wv[b] = wp[b * 32];
-        ev[b] = ex2 ? fmaxf(ex2[sbk * 256 + b * 32 + lane], 1e-12f) : 1.f;
-    }
-    float my_s = 0.f, my_m = 0.f;          // lane b keeps the pair of block b
+    for (int h = N / 2; h > 0; h >>= 1)
 #pragma unroll
-    for (int b = 0; b < 8; ++b) {
-        const float x = wv[b];
-        float mn = wmin(x);
-        const float mx = wmax(x);
-        float scale = fmaxf(__fdiv_rn(mx - mn, qmax), 1e-8f);
-        if (search) {
-            const float e = ev[b];
-            const float es = ex2 ? wsum(e) : 32.f;
-            const float wm = __fdiv_rn(ex2 ? wsum(e * x) : wsum(x), es);
-            float best_s = 0.f, best_m = 0.f, best_e = 0.f;
-            const float factors[8] = {0.7f, 0.75f, 0.8f, 0.85f, 0.9f, 0.95f, 1.0f, 1.05f};
+        for (int i = 0; i < N / 2; ++i)
+            if (i < h) v[i] = __fadd_rn(v[i], v[i + h]);
+    return v[0];
+}
+// maximum over the G adjacent lanes of a super-block
+template <int G>
+__device__ __forceinline__ float gmax(float v) {
 #pragma unroll
-            for (int fi = 0; fi < 8; ++fi) {
-                const float sc = scale * factors[fi];
-                const float qq = clampf(rintf(__fdiv_rn(x - mn, sc)), 0.f, qmax);
-                const float qm_ = __fdiv_rn(ex2 ? wsum(e * qq) : wsum(qq), es);
-                const float dq = qq - qm_;
-                const float cov = wsum(ex2 ? e * dq * (x - wm) : dq * (x - wm));
-                const float var = fmaxf(wsum(ex2 ? e * dq * dq : dq * dq), 1e-12f);
-                float s_ls = __fdiv_rn(cov, var);
-                const float m_ls = __fsub_rn(wm, __fmul_rn(s_ls, qm_));       // separate multiply and subtract, as in torch
-                s_ls = s_ls > 1e-8f ? s_ls : sc;
-                const float q2 = clampf(rintf(__fdiv_rn(x - m_ls, s_ls)), 0.f, qmax);
-                const float r = __fadd_rn(__fmul_rn(q2, s_ls), m_ls) - x;        // (q2 * s + m) - w, no contraction
-                const float err = wsum(ex2 ? e * (r * r) : r * r);
-                if (fi == 0 || err < best_e) { best_s = s_ls; best_m = m_ls; best_e = err; }
-            }
-            scale = fmaxf(best_s, 1e-8f);
-            mn = best_m;
+    for (int o = G / 2; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
+    return v;
+}
+
+// q[i] = clamp(rint((x[i] - m) / s), lo, hi) for a block, as the rounded division gives it.  With |u / s| <= hi + 1
+// (beyond, the clamp decides) the product u * (1 / s) and the rounded quotient are both within
+// 2.4e-7 (hi + 1) of the true one.
+template <int N, bool EXACT>
+__device__ __forceinline__ float codes_once(const float (&x)[N], float m, float s, float inv, float lo, float hi, float (&q)[N]) {
+    float dev = 0.f;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const float u = __fsub_rn(x[i], m);
+        float r;
+        if (EXACT) {
+            r = rintf(__fdiv_rn(u, s));
+        } else {
+            const float t = __fmul_rn(u, inv);
+            r = __fadd_rn(__fadd_rn(t, 12582912.f), -12582912.f);
+            dev = fmaxf(dev, fabsf(__fsub_rn(t, r)));
         }
-        if (lane == b) { my_s = scale; my_m = mn; }
+        q[i] = clampf(r, lo, hi);
     }
-    // super-block: lanes 0-7 hold (s, m) of the 8 blocks
-    const bool holder = lane < 8;
-    const float smax_v = wmax(holder ? my_s : 0.f);
-    const float mabs = wmax(holder ? fabsf(my_m) : 0.f);
-    const float d = hrt(fmaxf(__fdiv_rn(smax_v, 63.f), 1e-12f));
-    const float dm = hrt(fmaxf(__fdiv_rn(mabs, 31.f), 1e-12f));
-    const float qsv = clampf(rintf(__fdiv_rn(my_s, d)), 1.f, 63.f);
+    return dev;
+}
+template <int N>
+__device__ __forceinline__ void codes_of(const float (&x)[N], float m, float s, float lo, float hi, float (&q)[N]) {
+    const float inv = __fdiv_rn(1.0f, s);
+    // products beyond 2^22 leave the reach of the rounding trick with dev > 0.5 and take the division too
+    if (codes_once<N, false>(x, m, s, inv, lo, hi, q) > 0.5f - 2.4e-7f * (hi + 1.0f)) codes_once<N, true>(x, m, s, inv, lo, hi, q);
+}
+
+struct QuantOut {                    // unpacked parts, or file buffers (those that are null are not written)
+    uint8_t* q;                      // [rows, cols] codes (sym: int8)
+    uint8_t* qs;                     // [rows, blocks]
+    int8_t* qm;                      // [rows, blocks] (sb6)
+    __half *d, *dm;
+    uint8_t *packed, *qh, *qh2, *qsqm;
+};
+
+template <bool AW>
+__global__ void __launch_bounds__(128) quant_sb6_kernel(const float* __restrict__ w, long long ldw, int rows, int nsb, int bits, int search,
+                                                        const float* __restrict__ ex2, const QuantOut o) {
+    const long long blk = static_cast<long long>(blockIdx.x) * 128 + threadIdx.x, n_blocks = static_cast<long long>(rows) * nsb * 8;
+    const bool live = blk < n_blocks;                     // whole super-blocks (8 adjacent lanes) together
+    const long long bb = live ? blk : n_blocks - 1;
+    const int nb = nsb * 8, row = static_cast<int>(bb / nb), bi = static_cast<int>(bb % nb);
+    const float4* wp = reinterpret_cast<const float4*>(w + static_cast<size_t>(row) * ldw + bi * 32);
+    const float qmax = static_cast<float>((1 << bits) - 1);
+    float x[32], e[AW ? 32 : 1];
+    if ((reinterpret_cast<uintptr_t>(wp) & 15) == 0) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float4 v = __ldg(wp + i);
+            x[4 * i] = v.x; x[4 * i + 1] = v.y; x[4 * i + 2] = v.z; x[4 * i + 3] = v.w;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) x[i] = __ldg(reinterpret_cast<const float*>(wp) + i);
+    }
+    if (AW) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) e[AW ? i : 0] = fmaxf(__ldg(ex2 + bi * 32 + i), 1e-12f);
+    }
+    float mn = x[0], mx = x[0];
+#pragma unroll
+    for (int i = 1; i < 32; ++i) { mn = fminf(mn, x[i]); mx = fmaxf(mx, x[i]); }
+    float scale = fmaxf(__fdiv_rn(__fsub_rn(mx, mn), qmax), 1e-8f);
+    if (search) {
+        float t[32];
+        float es = 32.f;
+        if (AW) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) t[i] = e[AW ? i : 0];
+            es = tree(t);
+        }
+#pragma unroll
+        for (int i = 0; i < 32; ++i) t[i] = AW ? __fmul_rn(e[AW ? i : 0], x[i]) : x[i];
+        const float wm = __fdiv_rn(tree(t), es);
+        float best_s = 0.f, best_m = 0.f, best_e = 0.f;
+        const float factors[8] = {0.7f, 0.75f, 0.8f, 0.85f, 0.9f, 0.95f, 1.0f, 1.05f};
+#pragma unroll 1
+        for (int fi = 0; fi < 8; ++fi) {
+            const float sc = __fmul_rn(scale, factors[fi]);
+            float q[32];
+            codes_of<32>(x, mn, sc, 0.f, qmax, q);
+#pragma unroll
+            for (int i = 0; i < 32; ++i) t[i] = AW ? __fmul_rn(e[AW ? i : 0], q[i]) : q[i];
+            const float qmean = __fdiv_rn(tree(t), es);
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+                q[i] = __fsub_rn(q[i], qmean);
+                const float dx = __fsub_rn(x[i], wm);
+                t[i] = AW ? __fmul_rn(__fmul_rn(e[AW ? i : 0], q[i]), dx) : __fmul_rn(q[i], dx);
+            }
+            const float cov = tree(t);
+#pragma unroll
+            for (int i = 0; i < 32; ++i) t[i] = AW ? __fmul_rn(__fmul_rn(e[AW ? i : 0], q[i]), q[i]) : __fmul_rn(q[i], q[i]);
+            const float var = fmaxf(tree(t), 1e-12f);
+            float s_ls = __fdiv_rn(cov, var);
+            const float m_ls = __fsub_rn(wm, __fmul_rn(s_ls, qmean));       // separate multiply and subtract, as in torch
+            s_ls = s_ls > 1e-8f ? s_ls : sc;
+            codes_of<32>(x, m_ls, s_ls, 0.f, qmax, q);
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+                const float r = __fsub_rn(__fadd_rn(__fmul_rn(q[i], s_ls), m_ls), x[i]);        // (q * s + m) - w, no contraction
+                t[i] = AW ? __fmul_rn(e[AW ? i : 0], __fmul_rn(r, r)) : __fmul_rn(r, r);
+            }
+            const float err = tree(t);
+            if (fi == 0 || err < best_e) { best_s = s_ls; best_m = m_ls; best_e = err; }
+        }
+        scale = fmaxf(best_s, 1e-8f);
+        mn = best_m;
+    }
+    // super-block: 8 adjacent lanes
+    const float d = hrt(fmaxf(__fdiv_rn(fmaxf(gmax<8>(scale), 0.f), 63.f), 1e-12f));
+    const float dm = hrt(fmaxf(__fdiv_rn(gmax<8>(fabsf(mn)), 31.f), 1e-12f));
+    const float qsv = clampf(rintf(__fdiv_rn(scale, d)), 1.f, 63.f);
     // an all-zero super-block has dm = fp16(1e-12) = 0: min code 0 (the reference's 0 / 0 leaves NaN there)
-    const float qmv = (dm > 0.f || my_m != 0.f) ? clampf(rintf(__fdiv_rn(my_m, dm)), -31.f, 31.f) : 0.f;
+    const float qmv = (dm > 0.f || mn != 0.f) ? clampf(rintf(__fdiv_rn(mn, dm)), -31.f, 31.f) : 0.f;
     const float s2 = fmaxf(hrt(__fmul_rn(qsv, d)), 1e-8f);
     const float m2 = hrt(__fmul_rn(qmv, dm));
-    const size_t nb = static_cast<size_t>(nsb) * 8;
-    if (holder) {
-        qs_out[static_cast<size_t>(row) * nb + sbk * 8 + lane] = static_cast<uint8_t>(qsv);
-        qm_out[static_cast<size_t>(row) * nb + sbk * 8 + lane] = static_cast<int8_t>(qmv);
-    }
-    if (lane == 0) {
-        d_out[static_cast<size_t>(row) * nsb + sbk] = __float2half_rn(d);
-        dm_out[static_cast<size_t>(row) * nsb + sbk] = __float2half_rn(dm);
-    }
-    uint8_t* qp = q + static_cast<size_t>(row) * (static_cast<size_t>(nsb) * 256) + sbk * 256 + lane;
+    float q[32];
+    codes_of<32>(x, m2, s2, 0.f, qmax, q);
+    // the super-block's 8 scale and 8 min codes as two 48-bit streams, for the lane that stores them
+    uint64_t ss = 0, ms = 0;
+    const uint32_t mine = static_cast<uint32_t>(qsv) | (static_cast<uint32_t>(static_cast<int>(qmv) + 31) << 8);
 #pragma unroll
-    for (int b = 0; b < 8; ++b) {
-        const float sb_ = __shfl_sync(0xFFFFFFFFu, s2, b), mb_ = __shfl_sync(0xFFFFFFFFu, m2, b);
-        qp[b * 32] = static_cast<uint8_t>(clampf(rintf(__fdiv_rn(wv[b] - mb_, sb_)), 0.f, qmax));
+    for (int i = 0; i < 8; ++i) {
+        const uint32_t v = __shfl_sync(0xFFFFFFFFu, mine, i, 8);
+        ss |= static_cast<uint64_t>(v & 63u) << (6 * i);
+        ms |= static_cast<uint64_t>((v >> 8) & 63u) << (6 * i);
+    }
+    if (!live) return;
+    const size_t B = static_cast<size_t>(blk);
+    uint32_t c[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) c[i] = static_cast<uint32_t>(q[i]);
+    if ((bi & 7) == 0) {
+        o.d[B >> 3] = __float2half_rn(d);
+        o.dm[B >> 3] = __float2half_rn(dm);
+        if (o.qsqm) {
+            uint32_t* p = reinterpret_cast<uint32_t*>(o.qsqm + (B >> 3) * 12);
+            p[0] = static_cast<uint32_t>(ss);
+            p[1] = static_cast<uint32_t>(ss >> 32) | (static_cast<uint32_t>(ms) << 16);
+            p[2] = static_cast<uint32_t>(ms >> 16);
+        }
+    }
+    if (o.q) {
+        uint32_t b[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) b[i] = c[4 * i] | (c[4 * i + 1] << 8) | (c[4 * i + 2] << 16) | (c[4 * i + 3] << 24);
+        uint4* p = reinterpret_cast<uint4*>(o.q + B * 32);
+        p[0] = make_uint4(b[0], b[1], b[2], b[3]);
+        p[1] = make_uint4(b[4], b[5], b[6], b[7]);
+        o.qs[B] = static_cast<uint8_t>(qsv);
+        o.qm[B] = static_cast<int8_t>(qmv);
+    }
+    if (o.packed) {                   // byte j of a block: column j (low nibble), column j + 16 (high nibble)
+        uint32_t b[4] = {0, 0, 0, 0}, h = 0, h2 = 0;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) b[i >> 2] |= ((c[i] & 15u) | ((c[i + 16] & 15u) << 4)) << (8 * (i & 3));
+#pragma unroll
+        for (int i = 0; i < 32; ++i) { h |= ((c[i] >> 4) & 1u) << i; h2 |= ((c[i] >> 5) & 1u) << i; }
+        reinterpret_cast<uint4*>(o.packed)[B] = make_uint4(b[0], b[1], b[2], b[3]);
+        if (o.qh) reinterpret_cast<uint32_t*>(o.qh)[B] = h;
+        if (o.qh2) reinterpret_cast<uint32_t*>(o.qh2)[B] = h2;
     }
 }
 
-
 // The symmetric layout (blocks of 16, int8 block-scale codes against one fp16 per 256 weights;
-// calibration/groupwise.py:358-473 `_sym_one`): a warp owns a super-block, a half-warp a block, two
-// blocks per round.  Per block s0 = max(max|w|, 1e-12) / qmax and, over the caller's factors (the
+// calibration/groupwise.py:358-473 `_sym_one`): 16 adjacent lanes hold a super-block.  Per block
+// s0 = max(max|w|, 1e-12) / qmax and, over the caller's factors (the
 // reference's 19 float32 nodes of linspace(0.7, 1.15), or 1.0 alone), the s = f s0 with the
 // smallest (weighted) squared error of w - clamp(rint(w / s)) s, the first on ties; then
 // d = fp16(max s / 127), qs = clamp(rint(s / d), -128, 127), s' = fp16(qs d) and
 // q = clamp(rint(w / s')) (0 where s' is 0).
-__device__ __forceinline__ float hsum16(float v) {
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-    return v;
-}
-__device__ __forceinline__ float hmax16(float v) {
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
-    return v;
-}
-
-__global__ void __launch_bounds__(256) quant_sym_kernel(const float* __restrict__ w, long long ldw, int rows, int nsb, int bits,
-                                                         const float* __restrict__ factors, int n_factors,
-                                                         const float* __restrict__ ex2, int8_t* __restrict__ q,
-                                                         int8_t* __restrict__ qs_out, __half* __restrict__ d_out) {
-    const int lane = threadIdx.x & 31, hl = lane & 15, hw = lane >> 4;
-    const long long unit = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
-    if (unit >= static_cast<long long>(rows) * nsb) return;
-    const int row = static_cast<int>(unit / nsb), sbk = static_cast<int>(unit % nsb);
-    const float* wp = w + static_cast<size_t>(row) * ldw + sbk * 256;
+template <bool AW>
+__global__ void __launch_bounds__(128) quant_sym_kernel(const float* __restrict__ w, long long ldw, int rows, int nsb, int bits,
+                                                        const float* __restrict__ factors, int n_factors, const float* __restrict__ ex2,
+                                                        const QuantOut o) {
+    const long long blk = static_cast<long long>(blockIdx.x) * 128 + threadIdx.x, n_blocks = static_cast<long long>(rows) * nsb * 16;
+    const bool live = blk < n_blocks;
+    const long long bb = live ? blk : n_blocks - 1;
+    const int nb = nsb * 16, row = static_cast<int>(bb / nb), bi = static_cast<int>(bb % nb);
+    const float* wp = w + static_cast<size_t>(row) * ldw + bi * 16;
     const float qmax = static_cast<float>((1 << (bits - 1)) - 1), qmin = -qmax - 1.f;
-    float wv[8];
-    float my_s = 0.f;                       // lane b (< 16) keeps the scale of block b
+    float x[16], e[AW ? 16 : 1];
+    if ((reinterpret_cast<uintptr_t>(wp) & 15) == 0) {
 #pragma unroll
-    for (int r = 0; r < 8; ++r) {           // round r: blocks 2r (lanes 0-15) and 2r + 1 (lanes 16-31)
-        const int col = (2 * r + hw) * 16 + hl;
-        const float x = wp[col];
-        wv[r] = x;
-        const float e = ex2 ? fmaxf(ex2[sbk * 256 + col], 1e-12f) : 1.f;
-        const float base = __fdiv_rn(fmaxf(hmax16(fabsf(x)), 1e-12f), qmax);
-        float best_s = base, best_e = 0.f;
-        for (int fi = 0; fi < n_factors; ++fi) {
-            const float s = __fmul_rn(base, factors[fi]);
-            const float qv = clampf(rintf(__fdiv_rn(x, s)), qmin, qmax);
-            const float dlt = __fsub_rn(x, __fmul_rn(qv, s));
-            const float err = hsum16(ex2 ? e * (dlt * dlt) : dlt * dlt);
-            if (fi == 0 || err < best_e) { best_s = s; best_e = err; }
+        for (int i = 0; i < 4; ++i) {
+            const float4 v = __ldg(reinterpret_cast<const float4*>(wp) + i);
+            x[4 * i] = v.x; x[4 * i + 1] = v.y; x[4 * i + 2] = v.z; x[4 * i + 3] = v.w;
         }
-        // both half-warps hand their block's scale to the lane with the block's number
-        const float s_even = __shfl_sync(0xFFFFFFFFu, best_s, 0), s_odd = __shfl_sync(0xFFFFFFFFu, best_s, 16);
-        if (lane == 2 * r) my_s = s_even;
-        if (lane == 2 * r + 1) my_s = s_odd;
+    } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) x[i] = __ldg(wp + i);
     }
-    const bool holder = lane < 16;
-    const float d = hrt(fmaxf(__fdiv_rn(wmax(holder ? my_s : 0.f), 127.f), 1e-12f));
-    float qsv = clampf(rintf(__fdiv_rn(my_s, d)), -128.f, 127.f);
+    float mx = 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        if (AW) e[AW ? i : 0] = fmaxf(__ldg(ex2 + bi * 16 + i), 1e-12f);
+        mx = fmaxf(mx, fabsf(x[i]));
+    }
+    const float base = __fdiv_rn(fmaxf(mx, 1e-12f), qmax);
+    float best_s = base, best_e = 0.f, q[16], t[16];
+#pragma unroll 1
+    for (int fi = 0; fi < n_factors; ++fi) {
+        const float s = __fmul_rn(base, __ldg(factors + fi));
+        codes_of<16>(x, 0.f, s, qmin, qmax, q);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const float dlt = __fsub_rn(x[i], __fmul_rn(q[i], s));
+            t[i] = AW ? __fmul_rn(e[AW ? i : 0], __fmul_rn(dlt, dlt)) : __fmul_rn(dlt, dlt);
+        }
+        const float err = tree(t);
+        if (fi == 0 || err < best_e) { best_s = s; best_e = err; }
+    }
+    const float d = hrt(fmaxf(__fdiv_rn(fmaxf(gmax<16>(best_s), 0.f), 127.f), 1e-12f));
+    float qsv = clampf(rintf(__fdiv_rn(best_s, d)), -128.f, 127.f);
     if (!(qsv == qsv)) qsv = 0.f;           // 0 / 0: code 0, as the reference writes
     const float s2 = hrt(__fmul_rn(qsv, d));
-    const size_t nb = static_cast<size_t>(nsb) * 16;
-    if (holder) qs_out[static_cast<size_t>(row) * nb + sbk * 16 + lane] = static_cast<int8_t>(qsv);
-    if (lane == 0) d_out[static_cast<size_t>(row) * nsb + sbk] = __float2half_rn(d);
-    int8_t* qp = q + static_cast<size_t>(row) * (static_cast<size_t>(nsb) * 256) + sbk * 256;
+    if (fabsf(s2) > 0.f) {
+        codes_of<16>(x, 0.f, s2, qmin, qmax, q);
+    } else {
 #pragma unroll
-    for (int r = 0; r < 8; ++r) {
-        const float sb_ = __shfl_sync(0xFFFFFFFFu, s2, 2 * r + hw);
-        const float qv = fabsf(sb_) > 0.f ? clampf(rintf(__fdiv_rn(wv[r], sb_)), qmin, qmax) : 0.f;
-        qp[(2 * r + hw) * 16 + hl] = static_cast<int8_t>(qv);
+        for (int i = 0; i < 16; ++i) q[i] = 0.f;
     }
+    if (!live) return;
+    const size_t B = static_cast<size_t>(blk);
+    o.qs[B] = static_cast<uint8_t>(static_cast<int8_t>(qsv));
+    if ((bi & 15) == 0) o.d[B >> 4] = __float2half_rn(d);
+    if (o.q) {
+        uint32_t b[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            b[i] = 0;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) b[i] |= (static_cast<uint32_t>(static_cast<int>(q[4 * i + k])) & 0xFFu) << (8 * k);
+        }
+        reinterpret_cast<uint4*>(o.q)[B] = make_uint4(b[0], b[1], b[2], b[3]);
+    }
+    if (o.packed) {                   // stored code = value + 32; byte j of a block: column j (low nibble), column j + 8 (high nibble)
+        uint32_t c[16], b[2] = {0, 0}, h = 0, h2 = 0;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            c[i] = static_cast<uint32_t>(static_cast<int>(q[i]) + 32);
+            h |= ((c[i] >> 4) & 1u) << i;
+            h2 |= ((c[i] >> 5) & 1u) << i;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) b[i >> 2] |= ((c[i] & 15u) | ((c[i + 8] & 15u) << 4)) << (8 * (i & 3));
+        reinterpret_cast<uint2*>(o.packed)[B] = make_uint2(b[0], b[1]);
+        reinterpret_cast<unsigned short*>(o.qh)[B] = static_cast<unsigned short>(h);
+        reinterpret_cast<unsigned short*>(o.qh2)[B] = static_cast<unsigned short>(h2);
+    }
+}
+
+int run_sb6(const char* who, const float* w, int64_t ldw, int rows, int cols, int bits, int search, const float* ex2, const QuantOut& o,
+            cudaStream_t s) {
+    RWKVQ_REQUIRE(rows >= 1 && cols >= 256 && cols % 256 == 0 && ldw >= cols, RWKVQ_E_SHAPE,
+                  "%s: [%d, %d] (columns in multiples of 256), ldw %lld", who, rows, cols, (long long)ldw);
+    RWKVQ_REQUIRE(bits >= 4 && bits <= 6, RWKVQ_E_DTYPE, "%s: %d bits (4, 5 or 6)", who, bits);
+    const int nsb = cols / 256;
+    const long long ctas = (static_cast<long long>(rows) * nsb * 8 + 127) / 128;
+    RWKVQ_REQUIRE(ctas <= 0x7FFFFFFFLL, RWKVQ_E_LIMIT, "%s: tensor too large for one launch", who);
+    if (ex2 && search) quant_sb6_kernel<true><<<static_cast<unsigned>(ctas), 128, 0, s>>>(w, ldw, rows, nsb, bits, search, ex2, o);
+    else quant_sb6_kernel<false><<<static_cast<unsigned>(ctas), 128, 0, s>>>(w, ldw, rows, nsb, bits, search, ex2, o);
+    return check_launch(who);
+}
+int run_sym(const char* who, const float* w, int64_t ldw, int rows, int cols, int bits, const float* factors, int n_factors,
+            const float* ex2, const QuantOut& o, cudaStream_t s) {
+    RWKVQ_REQUIRE(rows >= 1 && cols >= 256 && cols % 256 == 0 && ldw >= cols, RWKVQ_E_SHAPE,
+                  "%s: [%d, %d] (columns in multiples of 256), ldw %lld", who, rows, cols, (long long)ldw);
+    RWKVQ_REQUIRE(bits == 6 || bits == 8, RWKVQ_E_DTYPE, "%s: %d bits (6 or 8)", who, bits);
+    RWKVQ_REQUIRE(n_factors >= 1 && n_factors <= 64, RWKVQ_E_LIMIT, "%s: %d factors", who, n_factors);
+    const int nsb = cols / 256;
+    const long long ctas = (static_cast<long long>(rows) * nsb * 16 + 127) / 128;
+    RWKVQ_REQUIRE(ctas <= 0x7FFFFFFFLL, RWKVQ_E_LIMIT, "%s: tensor too large for one launch", who);
+    if (ex2) quant_sym_kernel<true><<<static_cast<unsigned>(ctas), 128, 0, s>>>(w, ldw, rows, nsb, bits, factors, n_factors, ex2, o);
+    else quant_sym_kernel<false><<<static_cast<unsigned>(ctas), 128, 0, s>>>(w, ldw, rows, nsb, bits, factors, n_factors, ex2, o);
+    return check_launch(who);
 }
 
 }  // namespace
@@ -196,28 +337,38 @@ using namespace rwkvq;
 extern "C" int rwkvq_quantize_sb6(const float* w, int64_t ldw, int rows, int cols, int bits, int search, const float* ex2,
                                   uint8_t* q, uint8_t* qs, int8_t* qm, void* d, void* dm, void* stream) {
     RWKVQ_REQUIRE(w && q && qs && qm && d && dm, RWKVQ_E_NULL, "rwkvq_quantize_sb6: null pointer");
-    RWKVQ_REQUIRE(rows >= 1 && cols >= 256 && cols % 256 == 0 && ldw >= cols, RWKVQ_E_SHAPE,
-                  "rwkvq_quantize_sb6: [%d, %d] (columns in multiples of 256), ldw %lld", rows, cols, (long long)ldw);
-    RWKVQ_REQUIRE(bits >= 4 && bits <= 6, RWKVQ_E_DTYPE, "rwkvq_quantize_sb6: %d bits (4, 5 or 6)", bits);
-    const int nsb = cols / 256;
-    const long long units = static_cast<long long>(rows) * nsb;
-    RWKVQ_REQUIRE((units + 7) / 8 <= 0x7FFFFFFFLL, RWKVQ_E_LIMIT, "rwkvq_quantize_sb6: tensor too large for one launch");
-    quant_sb6_kernel<<<static_cast<unsigned int>((units + 7) / 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        w, static_cast<long long>(ldw), rows, nsb, bits, search, ex2, q, qs, qm, static_cast<__half*>(d), static_cast<__half*>(dm));
-    return check_launch("rwkvq_quantize_sb6");
+    RWKVQ_REQUIRE(aligned(q, 16), RWKVQ_E_ALIGN, "rwkvq_quantize_sb6: q must be 16-byte aligned");
+    QuantOut o{};
+    o.q = q; o.qs = qs; o.qm = qm; o.d = static_cast<__half*>(d); o.dm = static_cast<__half*>(dm);
+    return run_sb6("rwkvq_quantize_sb6", w, ldw, rows, cols, bits, search, ex2, o, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int rwkvq_quantize_sb6_packed(const float* w, int64_t ldw, int rows, int cols, int bits, int search, const float* ex2,
+                                         uint8_t* codes_packed, uint8_t* qh, uint8_t* qh2, uint8_t* qsqm, void* d, void* dm, void* stream) {
+    RWKVQ_REQUIRE(w && codes_packed && qsqm && d && dm && (bits < 5 || qh) && (bits < 6 || qh2), RWKVQ_E_NULL,
+                  "rwkvq_quantize_sb6_packed: null pointer");
+    RWKVQ_REQUIRE(aligned(codes_packed, 16) && aligned(qh, 4) && aligned(qh2, 4) && aligned(qsqm, 4), RWKVQ_E_ALIGN,
+                  "rwkvq_quantize_sb6_packed: unaligned buffer");
+    QuantOut o{};
+    o.packed = codes_packed; o.qh = bits >= 5 ? qh : nullptr; o.qh2 = bits >= 6 ? qh2 : nullptr; o.qsqm = qsqm;
+    o.d = static_cast<__half*>(d); o.dm = static_cast<__half*>(dm);
+    return run_sb6("rwkvq_quantize_sb6_packed", w, ldw, rows, cols, bits, search, ex2, o, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int rwkvq_quantize_sym(const float* w, int64_t ldw, int rows, int cols, int bits, const float* factors, int n_factors,
                                   const float* ex2, int8_t* q, int8_t* qs, void* d, void* stream) {
     RWKVQ_REQUIRE(w && q && qs && d && factors, RWKVQ_E_NULL, "rwkvq_quantize_sym: null pointer");
-    RWKVQ_REQUIRE(rows >= 1 && cols >= 256 && cols % 256 == 0 && ldw >= cols, RWKVQ_E_SHAPE,
-                  "rwkvq_quantize_sym: [%d, %d] (columns in multiples of 256), ldw %lld", rows, cols, (long long)ldw);
-    RWKVQ_REQUIRE(bits == 6 || bits == 8, RWKVQ_E_DTYPE, "rwkvq_quantize_sym: %d bits (6 or 8)", bits);
-    RWKVQ_REQUIRE(n_factors >= 1 && n_factors <= 64, RWKVQ_E_LIMIT, "rwkvq_quantize_sym: %d factors", n_factors);
-    const int nsb = cols / 256;
-    const long long units = static_cast<long long>(rows) * nsb;
-    RWKVQ_REQUIRE((units + 7) / 8 <= 0x7FFFFFFFLL, RWKVQ_E_LIMIT, "rwkvq_quantize_sym: tensor too large for one launch");
-    quant_sym_kernel<<<static_cast<unsigned int>((units + 7) / 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        w, static_cast<long long>(ldw), rows, nsb, bits, factors, n_factors, ex2, q, qs, static_cast<__half*>(d));
-    return check_launch("rwkvq_quantize_sym");
+    RWKVQ_REQUIRE(aligned(q, 16), RWKVQ_E_ALIGN, "rwkvq_quantize_sym: q must be 16-byte aligned");
+    QuantOut o{};
+    o.q = reinterpret_cast<uint8_t*>(q); o.qs = reinterpret_cast<uint8_t*>(qs); o.d = static_cast<__half*>(d);
+    return run_sym("rwkvq_quantize_sym", w, ldw, rows, cols, bits, factors, n_factors, ex2, o, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int rwkvq_quantize_sym6_packed(const float* w, int64_t ldw, int rows, int cols, const float* factors, int n_factors,
+                                          const float* ex2, uint8_t* codes_packed, uint8_t* qh, uint8_t* qh2, int8_t* qs, void* d, void* stream) {
+    RWKVQ_REQUIRE(w && codes_packed && qh && qh2 && qs && d && factors, RWKVQ_E_NULL, "rwkvq_quantize_sym6_packed: null pointer");
+    RWKVQ_REQUIRE(aligned(codes_packed, 8) && aligned(qh, 2) && aligned(qh2, 2), RWKVQ_E_ALIGN, "rwkvq_quantize_sym6_packed: unaligned buffer");
+    QuantOut o{};
+    o.packed = codes_packed; o.qh = qh; o.qh2 = qh2; o.qs = reinterpret_cast<uint8_t*>(qs); o.d = static_cast<__half*>(d);
+    return run_sym("rwkvq_quantize_sym6_packed", w, ldw, rows, cols, 6, factors, n_factors, ex2, o, static_cast<cudaStream_t>(stream));
 }

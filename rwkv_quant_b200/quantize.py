@@ -2,20 +2,19 @@
 
 The counterpart of the reference's host-side packer for its block formats
 (`formats/writer.py:236-269` `_make_qt_gw_sb6` over `calibration/groupwise.py:207-300`): the
-scale search and code selection run in one CUDA kernel (`rwkvq_quantize_sb6`, a warp per
-super-block of 256 weights), the bit packing into the file buffers with the package's packers.
+scale search, the code selection and the bit packing into the file buffers run in one CUDA kernel
+(`rwkvq_quantize_sb6_packed`, a thread per block of 32 weights).
 The result is a `QuantizedTensor` a `.rwkvq` file can hold and the kernels can read.
 """
 from __future__ import annotations
 
-import ctypes as C
+import functools
 from typing import Optional
 
 import torch
 
 from . import _lib
 from .formats import QuantizedTensor
-from .synth import pack_6bit, pack_bitplane, pack_nibbles_blocklocal
 
 MODES = {"asym_sb6": False, "asym_sb6_search": True, "asym_sb6_aw": True}
 SYM_MODES = ("sym", "sym_aw", "sym_plain")
@@ -27,19 +26,31 @@ def sym_factors() -> torch.Tensor:
     return torch.linspace(0.7, 1.15, 19)
 
 
-def quantize_sb6_parts(w: torch.Tensor, bits: int, search: bool = True, ex2: Optional[torch.Tensor] = None):
-    """(q u8 [OUT, IN], qs u8 [OUT, IN/32], qm i8 [OUT, IN/32], d f16 [OUT, IN/256], dm f16) on the device."""
+@functools.lru_cache(maxsize=16)
+def _factors(search: bool, device: torch.device) -> torch.Tensor:
+    """The search's scale factors on a device (19 constants: uploaded once)."""
+    return (sym_factors() if search else torch.ones(1)).to(device)
+
+
+def _prepared(who: str, w: torch.Tensor, ex2: Optional[torch.Tensor]):
+    """(w fp32 contiguous, ex2 fp32 on its device or None) of a quantizer call."""
     if not w.is_cuda or w.dim() != 2:
-        raise ValueError("quantize_sb6: a 2-D CUDA tensor is required")
-    o, n = w.shape
+        raise ValueError(f"{who}: a 2-D CUDA tensor is required")
+    n = w.shape[1]
     if n % 256:
-        raise ValueError(f"quantize_sb6: IN={n} is not a multiple of 256")
-    w32 = w.float().contiguous()
+        raise ValueError(f"{who}: IN={n} is not a multiple of 256")
     e = None
     if ex2 is not None:
         e = ex2.to(device=w.device, dtype=torch.float32).contiguous()
         if e.numel() != n:
-            raise ValueError("quantize_sb6: ex2 needs one value per input channel")
+            raise ValueError(f"{who}: ex2 needs one value per input channel")
+    return w.float().contiguous(), e
+
+
+def quantize_sb6_parts(w: torch.Tensor, bits: int, search: bool = True, ex2: Optional[torch.Tensor] = None):
+    """(q u8 [OUT, IN], qs u8 [OUT, IN/32], qm i8 [OUT, IN/32], d f16 [OUT, IN/256], dm f16) on the device."""
+    w32, e = _prepared("quantize_sb6", w, ex2)
+    o, n = w32.shape
     dev = w.device
     q = torch.empty((o, n), dtype=torch.uint8, device=dev)
     qs = torch.empty((o, n // 32), dtype=torch.uint8, device=dev)
@@ -63,32 +74,31 @@ def quantize_sb6(key: str, group: str, w: torch.Tensor, bits: int, mode: str = "
         raise ValueError(f"quantize_sb6: mode {mode!r}")
     if (mode == "asym_sb6_aw") != (ex2 is not None):
         raise ValueError("quantize_sb6: ex2 goes with mode asym_sb6_aw, and only with it")
-    q, qs, qm, d, dm = quantize_sb6_parts(w, bits, MODES[mode], ex2)
-    o, n = w.shape
-    qsqm = torch.cat([pack_6bit(qs.reshape(o, -1, 8)), pack_6bit((qm.to(torch.int16) + 31).to(torch.uint8).reshape(o, -1, 8))], dim=-1)
-    return QuantizedTensor(
-        key=key, group=group, bits=bits, shape=(o, n), gw_mode="sb6", gw_gs=32, gw_sb=8,
-        codes_packed=pack_nibbles_blocklocal(q & 0xF, 32),
-        gw_qh=pack_bitplane((q >> 4) & 1) if bits >= 5 else None,
-        gw_qh2=pack_bitplane((q >> 5) & 1) if bits >= 6 else None,
-        gw_qsqm=qsqm.contiguous(), gw_d=d, gw_dm=dm)
+    if not 4 <= bits <= 6:
+        raise ValueError(f"quantize_sb6: {bits} bits (4, 5 or 6)")
+    w32, e = _prepared("quantize_sb6", w, ex2)
+    (o, n), dev = w32.shape, w32.device
+    u8 = dict(dtype=torch.uint8, device=dev)
+    packed = torch.empty((o, n // 2), **u8)
+    qh = torch.empty((o, n // 8), **u8) if bits >= 5 else None
+    qh2 = torch.empty((o, n // 8), **u8) if bits >= 6 else None
+    qsqm = torch.empty((o, n // 256, 12), **u8)
+    d = torch.empty((o, n // 256), dtype=torch.float16, device=dev)
+    dm = torch.empty_like(d)
+    lib = _lib.load(check_device=True)
+    with torch.cuda.device(dev):
+        _lib.check(lib.rwkvq_quantize_sb6_packed(w32.data_ptr(), n, o, n, bits, 1 if MODES[mode] else 0, _lib.ptr(e) or None,
+                                                 packed.data_ptr(), _lib.ptr(qh) or None, _lib.ptr(qh2) or None, qsqm.data_ptr(),
+                                                 d.data_ptr(), dm.data_ptr(), _lib.stream_ptr()), "rwkvq_quantize_sb6_packed")
+    return QuantizedTensor(key=key, group=group, bits=bits, shape=(o, n), gw_mode="sb6", gw_gs=32, gw_sb=8,
+                           codes_packed=packed, gw_qh=qh, gw_qh2=qh2, gw_qsqm=qsqm, gw_d=d, gw_dm=dm)
 
 
 def quantize_sym_parts(w: torch.Tensor, bits: int, search: bool = True, ex2: Optional[torch.Tensor] = None):
     """(q i8 [OUT, IN], qs i8 [OUT, IN/16], d f16 [OUT, IN/256]) on the device."""
-    if not w.is_cuda or w.dim() != 2:
-        raise ValueError("quantize_sym: a 2-D CUDA tensor is required")
-    o, n = w.shape
-    if n % 256:
-        raise ValueError(f"quantize_sym: IN={n} is not a multiple of 256")
-    w32 = w.float().contiguous()
-    dev = w.device
-    e = None
-    if ex2 is not None:
-        e = ex2.to(device=dev, dtype=torch.float32).contiguous()
-        if e.numel() != n:
-            raise ValueError("quantize_sym: ex2 needs one value per input channel")
-    f = (sym_factors() if search else torch.ones(1)).to(dev)
+    w32, e = _prepared("quantize_sym", w, ex2)
+    (o, n), dev = w32.shape, w32.device
+    f = _factors(search, dev)
     q = torch.empty((o, n), dtype=torch.int8, device=dev)
     qs = torch.empty((o, n // 16), dtype=torch.int8, device=dev)
     d = torch.empty((o, n // 256), dtype=torch.float16, device=dev)
@@ -108,14 +118,23 @@ def quantize_sym(key: str, group: str, w: torch.Tensor, bits: int, mode: str = "
         raise ValueError(f"quantize_sym: mode {mode!r}")
     if (mode == "sym_aw") != (ex2 is not None):
         raise ValueError("quantize_sym: ex2 goes with mode sym_aw, and only with it")
-    q, qs, d = quantize_sym_parts(w, bits, mode != "sym_plain", ex2)
-    o, n = w.shape
-    qt = QuantizedTensor(key=key, group=group, bits=bits, shape=(o, n), gw_mode="sym", gw_gs=16, gw_sb=16, gw_qs=qs, gw_d=d)
     if bits == 8:
-        qt.codes = q
-    else:
-        u = (q.to(torch.int16) + 32).to(torch.uint8)
-        qt.codes_packed = pack_nibbles_blocklocal(u & 0xF, 16)
-        qt.gw_qh = pack_bitplane((u >> 4) & 1)
-        qt.gw_qh2 = pack_bitplane((u >> 5) & 1)
-    return qt
+        q, qs, d = quantize_sym_parts(w, bits, mode != "sym_plain", ex2)
+        return QuantizedTensor(key=key, group=group, bits=8, shape=tuple(w.shape), gw_mode="sym", gw_gs=16, gw_sb=16, gw_qs=qs, gw_d=d, codes=q)
+    if bits != 6:
+        raise ValueError(f"quantize_sym: {bits} bits (6 or 8)")
+    w32, e = _prepared("quantize_sym", w, ex2)
+    (o, n), dev = w32.shape, w32.device
+    f = _factors(mode != "sym_plain", dev)
+    packed = torch.empty((o, n // 2), dtype=torch.uint8, device=dev)
+    qh = torch.empty((o, n // 8), dtype=torch.uint8, device=dev)
+    qh2 = torch.empty_like(qh)
+    qs = torch.empty((o, n // 16), dtype=torch.int8, device=dev)
+    d = torch.empty((o, n // 256), dtype=torch.float16, device=dev)
+    lib = _lib.load(check_device=True)
+    with torch.cuda.device(dev):
+        _lib.check(lib.rwkvq_quantize_sym6_packed(w32.data_ptr(), n, o, n, f.data_ptr(), f.numel(), _lib.ptr(e) or None,
+                                                  packed.data_ptr(), qh.data_ptr(), qh2.data_ptr(), qs.data_ptr(), d.data_ptr(),
+                                                  _lib.stream_ptr()), "rwkvq_quantize_sym6_packed")
+    return QuantizedTensor(key=key, group=group, bits=6, shape=(o, n), gw_mode="sym", gw_gs=16, gw_sb=16, codes_packed=packed,
+                           gw_qh=qh, gw_qh2=qh2, gw_qs=qs, gw_d=d)
