@@ -73,6 +73,8 @@ _PROTOS = {
                                      C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
     "rwkvq_quantize_sym": (C.c_int, [C.c_void_p, C.c_int64, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_int, C.c_void_p,
                                      C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
+    "rwkvq_quantize_sb6_packed": (C.c_int, [C.c_void_p, C.c_int64, C.c_int, C.c_int, C.c_int, C.c_int] + [C.c_void_p] * 8),
+    "rwkvq_quantize_sym6_packed": (C.c_int, [C.c_void_p, C.c_int64, C.c_int, C.c_int, C.c_void_p, C.c_int] + [C.c_void_p] * 7),
     "rwkvq_gemv_batch_workspace_bytes": (C.c_size_t, [C.c_int]),
     "rwkvq_gemv_batch": (C.c_int, [C.POINTER(QTensorStruct), C.c_void_p, C.c_int, C.c_int64, C.c_void_p, C.c_int64,
                                    C.c_int, C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p]),
@@ -173,5 +175,13 @@ def ptr(t) -> int:
     return 0 if t is None else t.data_ptr()
 
 
+# the handle alone: building a Stream object costs more than the rest of an operator call
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_device_index = getattr(torch._C, "_cuda_getDevice", None)
+
+
 def stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """cudaStream_t of the current device's current stream."""
+    if _raw_stream is None or _device_index is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(_device_index())

@@ -94,6 +94,14 @@ class DeviceQT:
         if oi is not None and oi.numel() > 0:
             self._attach_outliers(oi, qt.outlier_values, dev)
 
+    @property
+    def struct_ref(self):
+        """``struct`` as the pointer argument of a library call."""
+        ref = self.__dict__.get("_struct_ref")
+        if ref is None or ref[0] is not self.struct:
+            ref = self.__dict__["_struct_ref"] = (self.struct, C.byref(self.struct))
+        return ref[1]
+
     def _attach_outliers(self, oi, ov, dev):
         """Sparse overrides of per-row tensors (formats/codec.py:279-292): W[r, c] = value.  Kept
         sorted by (row, column); ``delta`` = value - quantized value is what a product over the
@@ -128,7 +136,7 @@ class DeviceQT:
         CSR tail kernel adds every row's override terms in column order (deterministic) and applies the
         epilogue (the reference's per-row kernels carry the same tail, quant_linear_v2.py:47-55)."""
         if self.outliers is None:
-            return gemv(self.bufs, self.meta, x, epilogue, resid)
+            return gemv_direct(self, x, epilogue, resid)
         delta, row_ptr, cols32 = self.outliers[3:6]
         y = gemv(self.bufs, self.meta, x, 0, None)
         _lib.check(_lib.load().rwkvq_outlier_tail(row_ptr.data_ptr(), cols32.data_ptr(), delta.data_ptr(), self.rows,
@@ -238,6 +246,19 @@ def _(bufs, meta, x, epilogue, resid):
     return torch.empty((x.shape[0], meta[2]), dtype=torch.float32, device=x.device)
 
 
+def gemv_direct(dq: "DeviceQT", x: torch.Tensor, epilogue: int = 0, resid: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """``gemv`` on the tensor's own descriptor, past the operator dispatcher (40 us of the 50 us a
+    single-row call took); a graph being traced gets the registered operator."""
+    if torch.compiler.is_compiling():
+        return gemv(dq.bufs, dq.meta, x, epilogue, resid)
+    _require_cuda(x, resid)
+    n = x.shape[0]
+    y = torch.empty((n, dq.rows), dtype=torch.float32, device=x.device)
+    _lib.check(_lib.load().rwkvq_gemv(dq.struct_ref, x.data_ptr(), _lib.DTYPE_CODE[x.dtype], n, x.stride(0), y.data_ptr(),
+                                      dq.rows, epilogue, _lib.ptr(resid), _lib.stream_ptr()), "rwkvq_gemv")
+    return y
+
+
 @torch.library.custom_op("rwkvq::gemv_t", mutates_args=())
 def gemv_t(bufs: Sequence[torch.Tensor], meta: Sequence[int], x: torch.Tensor, act: int,
            round_w: bool) -> torch.Tensor:
@@ -288,7 +309,7 @@ def gemv_batch(dq: "DeviceQT", x: torch.Tensor, epilogue: int = 0, resid: Option
     y = torch.empty((n, dq.rows), dtype=torch.float32, device=x.device)
     nws = lib.rwkvq_gemv_batch_workspace_bytes(n)
     ws = torch.empty(nws, dtype=torch.uint8, device=x.device)
-    _lib.check(lib.rwkvq_gemv_batch(C.byref(dq.struct), x.data_ptr(), n, x.stride(0), y.data_ptr(), y.stride(0),
+    _lib.check(lib.rwkvq_gemv_batch(dq.struct_ref, x.data_ptr(), n, x.stride(0), y.data_ptr(), y.stride(0),
                                     epilogue, _lib.ptr(resid), ws.data_ptr(), nws, _lib.stream_ptr()), "rwkvq_gemv_batch")
     if check:          # synchronises: the kernel's own report that a bounded pipeline wait ran out
         _lib.check(int(ws[:4].view(torch.int32).item()), "rwkvq_gemv_batch(kernel status)")
@@ -333,7 +354,7 @@ def gemm(dq: "DeviceQT", x: torch.Tensor, epilogue: int = 0, resid: Optional[tor
     nws = lib.rwkvq_gemm_workspace_bytes_for(m, dq.cols)
     ws = torch.empty(nws, dtype=torch.uint8, device=x.device)
     y = torch.empty((m, dq.rows), dtype=torch.float32, device=x.device)
-    _lib.check(lib.rwkvq_gemm(C.byref(dq.struct), x.data_ptr(), m, x.stride(0), y.data_ptr(), y.stride(0),
+    _lib.check(lib.rwkvq_gemm(dq.struct_ref, x.data_ptr(), m, x.stride(0), y.data_ptr(), y.stride(0),
                               epilogue, _lib.ptr(resid), ws.data_ptr(), nws, _lib.stream_ptr()), "rwkvq_gemm")
     if check:
         st = int(ws[:4].view(torch.int32).item())
@@ -362,7 +383,7 @@ def gemm_x16(dq: "DeviceQT", rows: PreparedRows, epilogue: int = 0, resid: Optio
     nws = lib.rwkvq_gemm_workspace_bytes_for(m, 0)
     ws = torch.empty(nws, dtype=torch.uint8, device=rows.x16.device)
     y = torch.empty((m, dq.rows), dtype=torch.float32, device=rows.x16.device)
-    _lib.check(lib.rwkvq_gemm_x16(C.byref(dq.struct), rows.x16.data_ptr(), rows.scale.data_ptr(), m, y.data_ptr(),
+    _lib.check(lib.rwkvq_gemm_x16(dq.struct_ref, rows.x16.data_ptr(), rows.scale.data_ptr(), m, y.data_ptr(),
                                   y.stride(0), epilogue, _lib.ptr(resid), ws.data_ptr(), nws, _lib.stream_ptr()),
                "rwkvq_gemm_x16")
     return y
@@ -484,7 +505,7 @@ def as_rows(x: torch.Tensor, n_in: int):
     if x.shape[-1] != n_in:
         raise AssertionError(f"last dim {x.shape[-1]} != in_features {n_in}")
     lead = x.shape[:-1]
-    x2 = x.reshape(-1, n_in)
+    x2 = x if x.dim() == 2 else x.reshape(-1, n_in)
     if x2.dtype not in _lib.DTYPE_CODE:
         x2 = x2.float()
     if x2.stride(-1) != 1 or (x2.stride(0) * x2.element_size()) % 16 or x2.data_ptr() % 16:

@@ -306,7 +306,7 @@ int rwkvq_forward_seq(const rwkvq_model* m, int B, int T, const int64_t* tokens,
         }
         rc = launch_dequant_f16(L.Wo, 0, D, w.w16, nullptr, s);
         if (rc) return rc;
-        rc = launch_row_scale(w.og, D, D, N, w.scale + 3 * N, w.og16, static_cast<long long>(pitch16(D)), s);
+        rc = launch_row_scale(w.og, D, D, N, w.scale + 3 * N, w.og16, static_cast<long long>(pitch16(D)), nullptr, s);
         if (rc) return rc;
         HgProb p = ps.prob(w.w16, D, D, w.og16, w.scale + 3 * N);
         p.out = HG_F32; p.epilogue = RWKVQ_EPI_ADD; p.y32 = w.x; p.resid = w.x; p.ldy = D;

@@ -594,11 +594,12 @@ __global__ void __launch_bounds__(kHgThreads, 1) gemm_one_kernel(const __grid_co
 // Pre-pass for fp32 activations, one CTA per token: power-of-two scale with |x * scale| <= 2^14 and the
 // scaled row as fp16 (the tensor the TMA loads read).
 __global__ void __launch_bounds__(256) row_scale_kernel(const float* __restrict__ x, long long ldx, int cols, float* __restrict__ scale,
-                                                        __half* __restrict__ x16, long long pitch) {
+                                                        __half* __restrict__ x16, long long pitch, int* __restrict__ status) {
     __shared__ float red[8];
     constexpr int kKeep = 4;                             // float4 per thread held between the two uses (4096 columns)
     pdl_launch_dependents();
     pdl_wait();
+    if (status != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *status = 0;      // of the product that follows
     const float4* row = reinterpret_cast<const float4*>(x + blockIdx.x * ldx);
     const int n4 = cols >> 2;
     float4 keep[kKeep];
@@ -634,8 +635,8 @@ __global__ void __launch_bounds__(256) row_scale_kernel(const float* __restrict_
     for (int i = threadIdx.x + 256 * kKeep; i < n4; i += 256) put(i, __ldcg(row + i));
 }
 
-int launch_row_scale(const float* x, long long ldx, int cols, int M, float* scale, __half* x16, long long pitch, cudaStream_t s) {
-    cudaError_t e = launch_pdl(row_scale_kernel, dim3(M), dim3(256), 0, s, x, ldx, cols, scale, x16, pitch);
+int launch_row_scale(const float* x, long long ldx, int cols, int M, float* scale, __half* x16, long long pitch, int* status, cudaStream_t s) {
+    cudaError_t e = launch_pdl(row_scale_kernel, dim3(M), dim3(256), 0, s, x, ldx, cols, scale, x16, pitch, status);
     if (e != cudaSuccess) return fail(RWKVQ_E_LAUNCH, "row_scale: %s", cudaGetErrorString(e));
     return RWKVQ_OK;
 }
@@ -852,8 +853,7 @@ int rwkvq_gemm(const rwkvq_qtensor* t, const float* x, int M, int64_t ldx, float
     int* status = reinterpret_cast<int*>(ws);
     float* scale = reinterpret_cast<float*>(ws + 256);
     __half* x16 = reinterpret_cast<__half*>(ws + ws_x16_off(M));
-    if (cudaMemsetAsync(status, 0, sizeof(int), s) != cudaSuccess) return check_launch("rwkvq_gemm(status)");
-    rc = launch_row_scale(x, ldx, t->cols, M, scale, x16, static_cast<long long>(x16_pitch(t->cols)), s);
+    rc = launch_row_scale(x, ldx, t->cols, M, scale, x16, static_cast<long long>(x16_pitch(t->cols)), status, s);
     if (rc) return rc;
     rc = gemm_chunks(t, x16, scale, M, y, ldy, epilogue, resid, reinterpret_cast<__half*>(ws + ws_w_off(M, t->cols)), status, s);
     return rc ? rc : check_launch("rwkvq_gemm");

@@ -40,8 +40,9 @@ struct HgProb {
 // status: device word that receives RWKVQ_E_TIMEOUT if a bounded wait ran out
 int launch_gemm_f16(const HgProb* probs, int n_probs, int M, int* status, cudaStream_t s);
 
-// fp32 rows -> x16 = fp16(x * scale) with the power of two scale[tok] that brings max|x| below 2^14
-int launch_row_scale(const float* x, long long ldx, int cols, int M, float* scale, __half* x16, long long pitch, cudaStream_t s);
+// fp32 rows -> x16 = fp16(x * scale) with the power of two scale[tok] that brings max|x| below 2^14;
+// status (optional) is cleared
+int launch_row_scale(const float* x, long long ldx, int cols, int M, float* scale, __half* x16, long long pitch, int* status, cudaStream_t s);
 
 // Packed sb6 / sym rows [row0, row0 + rows) -> fp16(q * s + m) [rows, cols] (pitch cols).
 // n2 (optional, [cols / 256], zeroed by the caller): merged with the largest squared norm of a row's
