@@ -265,6 +265,7 @@ int launch_gemv_batch(const rwkvq_qtensor* ts, int n_mats, const void* const* xs
 bool gemm_tcb_ok(const rwkvq_qtensor& t);
 bool batch_fast();        // RWKVQ_BATCH_FAST=1: single fp16 operands in the small-batch linears (faster, ~5e-4 per linear)
 bool tcb_enabled();
+int tcb_forced_ks();      // ... and the cluster size it asks for
 bool tcb_forced();        // a profiling override asks for the tcgen05 kernel at every batch size
 int launch_gemm_tcb(const rwkvq_qtensor* ts, int n_mats, const void* const* xs, bool half_in, const float* const* scales,
                     int N, long long ldx, float* const* ys, long long ldy, int epilogue, const float* const* resids,

@@ -19,6 +19,7 @@
 // Every mbarrier wait is bounded; on expiry the status word is set, all roles run to the common end, and
 // tensor memory is freed.
 #include "rwkvq_gemm_f16.cuh"
+#include "rwkvq_gemm_sb.cuh"
 
 #include <cooperative_groups.h>
 
@@ -662,21 +663,6 @@ EncodeTiledFn encode_tiled() {
     return fn;
 }
 
-// fp16 [rows, cols] row-major; box = [box_rows, 64 columns], 128-byte swizzle, zero fill beyond the edges
-int make_map(CUtensorMap* map, const __half* base, long long rows, long long cols, long long pitch, int box_rows) {
-    EncodeTiledFn enc = encode_tiled();
-    RWKVQ_REQUIRE(enc != nullptr, RWKVQ_E_ARCH, "gemm_f16: cuTensorMapEncodeTiled is not available");
-    const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
-    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(pitch) * sizeof(__half)};
-    const cuuint32_t box[2] = {kGmK, static_cast<cuuint32_t>(box_rows)};
-    const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half*>(base), dims, strides, box, estr,
-                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    RWKVQ_REQUIRE(r == CUDA_SUCCESS, RWKVQ_E_LAUNCH, "gemm_f16: cuTensorMapEncodeTiled failed (%d)", static_cast<int>(r));
-    return RWKVQ_OK;
-}
-
 // the attribute belongs to the (function, device) pair: remembered per device of this process
 template <typename K>
 int smem_attr(K kernel, size_t bytes, bool (&configured)[64]) {
@@ -713,6 +699,21 @@ int launch_one(const HgArgs& a, const HgMaps& maps, int ks, cudaStream_t s) {
 }
 
 }  // namespace
+
+// fp16 [rows, cols] row-major; box = [box_rows, 64 columns], 128-byte swizzle, zero fill beyond the edges
+int make_half_map(CUtensorMap* map, const __half* base, long long rows, long long cols, long long pitch, int box_rows) {
+    EncodeTiledFn enc = encode_tiled();
+    RWKVQ_REQUIRE(enc != nullptr, RWKVQ_E_ARCH, "gemm_f16: cuTensorMapEncodeTiled is not available");
+    const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
+    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(pitch) * sizeof(__half)};
+    const cuuint32_t box[2] = {kGmK, static_cast<cuuint32_t>(box_rows)};
+    const cuuint32_t estr[2] = {1, 1};
+    const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half*>(base), dims, strides, box, estr,
+                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    RWKVQ_REQUIRE(r == CUDA_SUCCESS, RWKVQ_E_LAUNCH, "gemm_f16: cuTensorMapEncodeTiled failed (%d)", static_cast<int>(r));
+    return RWKVQ_OK;
+}
 
 // Which kernel and tile: the smallest modelled time of the slowest SM in tensor cycles.  A stage of 64
 // columns costs four MMAs: 512 cycles for the pair's 256-token tile, 200 / 300 for one CTA's 64- / 128-token
@@ -766,9 +767,9 @@ int launch_gemm_f16(const HgProb* probs, int n_probs, int M, int* status, cudaSt
         d.out = p.out; d.epilogue = p.epilogue; d.act = p.act; d.lo_off = p.lo_off; d.n_w_n2 = p.n_w_n2;
         d.row_scale = p.row_scale; d.resid = p.resid; d.w_n2 = p.w_n2; d.x_n2 = p.x_n2;
         d.y32 = p.y32; d.y16 = p.y16; d.out_scale = p.out_scale; d.ldy = p.ldy;
-        int rc = make_map(&maps.w[i], p.w, p.w_rows ? p.w_rows : p.rows, p.k, p.w_pitch, kGmRows);
+        int rc = make_half_map(&maps.w[i], p.w, p.w_rows ? p.w_rows : p.rows, p.k, p.w_pitch, kGmRows);
         if (rc) return rc;
-        rc = make_map(&maps.x[i], p.x, M, static_cast<long long>(p.k) * p.terms, p.x_pitch, nt == 0 ? kPairTok / 2 : nt);
+        rc = make_half_map(&maps.x[i], p.x, M, static_cast<long long>(p.k) * p.terms, p.x_pitch, nt == 0 ? kPairTok / 2 : nt);
         if (rc) return rc;
     }
     if (nt == 128) return launch_one<128>(a, maps, ks, s);

@@ -1,0 +1,614 @@
+// Quantized linear for small batches (some 17 to 256 right-hand sides) on the tcgen05 tensor cores at fp32 grade:
+// packed weights converted on the way into the operands, every byte read once per 128 tokens.
+//
+//     y[n, o] = epi( sum_c W[o, c] x[n, c] )
+//
+// Both operands are carried as two fp16 terms (weights: p = fp16(q s) and its exact rounding error e;
+// activations: hi + lo of x * 2^s, |x * 2^s| <= 2^9); per 16 columns p and e each multiply [hi | lo] side by side as one
+// MMA of 2 NT token columns into one fp32 accumulator in tensor memory, so that shared memory delivers a weight once for
+// both terms of x.  sb6 block mins (fp16 by definition) times the block sums of x (as a pair too) are one more MMA of 16
+// columns per super-block.
+//
+// A CTA owns 128 rows and a K slice (cluster of ks CTAs along K, reduced through distributed shared memory in rank
+// order) and is a pipeline over stages of 64 columns:
+//   warps 0-15   weights: packed bytes arrive by cp.async in per-thread slots, up to six stages ahead, so that the HBM
+//                latency of a dependent launch is paid once; two groups of 8 warps take the stages in turn (one
+//                group: 1 us a stage whatever the batch), one item of 32 weights per thread and stage
+//   warp 16      TMA of the activation pairs, which split_rows_kernel or the LayerNorm kernels have made once (converting
+//                in every CTA cost 8 more warps and 0.8 us a stage at 64 tokens)
+//   warp 17      MMAs, the loop run by the whole warp so that descriptors stay in uniform registers (one lane
+//                under a branch: 0.65 us for the nine MMAs of a stage)
+// The mma.sync form of the same product (rwkvq_gemv_batch.cu) issues 3 MMAs of 16 x 8 x 16 per warp and step and tops out
+// at 0.92 G MMA/s per SM.
+// Every mbarrier wait is bounded; on expiry the status word is set and all roles run to the common end.
+#include "rwkvq_gemm_sb.cuh"
+
+#include <cooperative_groups.h>
+
+#include <algorithm>
+#include <cstdlib>
+
+#include "rwkvq_gemv_mma.cuh"
+#include "rwkvq_tc.cuh"
+
+namespace cg = cooperative_groups;
+
+namespace rwkvq {
+
+constexpr int kSbGroup = 256;                     // weight threads of one stage; two groups take the stages in turn
+constexpr int kSbWeightThreads = 2 * kSbGroup, kSbThreads = kSbWeightThreads + 64;
+constexpr int kSbTmaWarp = kSbWeightThreads / 32, kSbMmaWarp = kSbTmaWarp + 1;
+constexpr int kSbAhead = 3;                       // stages of packed weights a group has in flight
+constexpr int kSbSlab = kGmRows * 128;            // 128 rows x 64 columns of fp16
+constexpr int kSbPitch = kGmRows + 4;             // partial tile [NT][kSbPitch]
+constexpr int kSbMaxMats = 4;
+
+struct SbArgs {
+    QView t[kSbMaxMats];
+    const __half* sums[kSbMaxMats];
+    const float* unscale[kSbMaxMats];
+    float* y[kSbMaxMats];
+    const float* resid[kSbMaxMats];
+    float* amax_out[kSbMaxMats];
+    long long ldy;
+    int n_tokens, epilogue;
+    int row_tiles;                                // of one matrix
+    int n_tiles;                                  // matrices * row_tiles
+    int n_sb;                                     // super-blocks of a row
+    int ks;
+    int* status;
+};
+struct SbMaps { CUtensorMap hi[kSbMaxMats], lo[kSbMaxMats]; };
+
+template <int L>
+struct SbLayout {
+    static constexpr bool SB6 = L <= ML_SB6_6;
+    static constexpr int CODE_BYTES = L == ML_SYM8 ? 32 : 16;
+    static constexpr int PLANES = L == ML_SB6_5 ? 1 : (L == ML_SB6_6 || L == ML_SYM6) ? 2 : 0;
+    static constexpr int RAW = kSbGroup * (CODE_BYTES + 4 * PLANES);               // bytes of one stage
+};
+
+template <int L, int NT>
+struct SbGeo {
+    static constexpr int ST = NT > 64 ? 2 : 3;                       // operand buffers
+    static constexpr int BSLAB = 2 * NT * 128;
+    static constexpr int MA = SbLayout<L>::SB6 ? kGmRows * 32 : 0, MB = SbLayout<L>::SB6 ? 2 * NT * 32 : 0;     // min operands of a super-block
+    static constexpr int OFF_E = ST * kSbSlab, OFF_B = 2 * ST * kSbSlab, OFF_MA = OFF_B + ST * BSLAB, OFF_MB = OFF_MA + 2 * MA,
+                         OFF_RAW = OFF_MB + 2 * MB, OFF_REC = OFF_RAW + 2 * kSbAhead * SbLayout<L>::RAW, SMEM = OFF_REC + 2 * 3 * kGmRows * 16;
+    static constexpr size_t BYTES = SMEM + 1024;
+    static_assert(NT * kSbPitch * 4 <= OFF_MA, "partial tile over the operands");
+    static_assert(BYTES <= 226 * 1024, "shared memory");
+};
+
+__device__ __forceinline__ void sb_cp16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void sb_cp4(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+template <int NC>
+__device__ __forceinline__ void sb_tmem_ld(uint32_t taddr, float (&v)[NC]) {
+    uint32_t r[NC];
+    if constexpr (NC == 4) {
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr));
+    } else if constexpr (NC == 8) {
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                     : "r"(taddr));
+    } else {
+        static_assert(NC == 16, "columns");
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+                       "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                     : "r"(taddr));
+    }
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < NC; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// 32 weights of row r, item `it` of its super-block: codes * scale as product and rounding error into the two
+// operand slabs; returns the block's min (fp16 by the codec's definition; zero for sym).  decode_item with the layout
+// known at compile time.
+template <int L>
+__device__ __forceinline__ __half sb_convert(const Packed& p, bool in_rec, int r, int it, int half, unsigned char* p_slab, unsigned char* e_slab) {
+    uint32_t bytes[8];
+    __half2 s2[2], m2 = __float2half2_rn(0.f), bias;
+    const uint32_t w[4] = {p.c0.x, p.c0.y, p.c0.z, p.c0.w};
+    if constexpr (SbLayout<L>::SB6) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {              // byte k of the block: column k (low), k + 16 (high)
+            bytes[i] = w[i] & 0x0F0F0F0Fu;
+            bytes[4 + i] = (w[i] >> 4) & 0x0F0F0F0Fu;
+            if (L != ML_SB6_4) {
+                bytes[i] |= spread_nibble<4>((p.h >> (4 * i)) & 0xFu);
+                bytes[4 + i] |= spread_nibble<4>((p.h >> (16 + 4 * i)) & 0xFu);
+            }
+            if (L == ML_SB6_6) {
+                bytes[i] |= spread_nibble<5>((p.h2 >> (4 * i)) & 0xFu);
+                bytes[4 + i] |= spread_nibble<5>((p.h2 >> (16 + 4 * i)) & 0xFu);
+            }
+        }
+        float s, m;
+        if (in_rec) {
+            const int tt = it >> 1;                // record word it / 2: codes of blocks 2 (it / 2), + 1 and one byte of d | dm << 16
+            const uint32_t w4 = (tt & 2) ? ((tt & 1) ? p.rec.w : p.rec.z) : ((tt & 1) ? p.rec.y : p.rec.x);
+            const uint32_t dd = __byte_perm(p.rec.x, p.rec.y, 0x0073) & 0xFFFFu, dm = __byte_perm(p.rec.z, p.rec.w, 0x0073) & 0xFFFFu;
+            s = fmaxf(half_roundtrip(__fmul_rn(static_cast<float>((w4 >> (6 * half)) & 0x3Fu), half_bits_to_float(dd))), 1e-8f);
+            m = half_roundtrip(__fmul_rn(static_cast<float>(static_cast<int>((w4 >> (12 + 6 * half)) & 0x3Fu) - 31), half_bits_to_float(dm)));
+        } else {
+            sb6_scale_min(p.rec.x, p.rec.y, p.rec.z, it, half_bits_to_float(p.rec.w & 0xFFFFu), half_bits_to_float(p.rec.w >> 16), s, m);
+        }
+        s2[0] = s2[1] = __float2half2_rn(s);
+        m2 = __float2half2_rn(m);
+        bias = __float2half2_rn(1024.f);
+    } else {
+        const float d = half_bits_to_float(p.rec.y);
+#pragma unroll
+        for (int b = 0; b < 2; ++b)
+            s2[b] = __float2half2_rn(half_roundtrip(__fmul_rn(static_cast<float>(static_cast<int8_t>((p.rec.x >> (8 * b)) & 0xFFu)), d)));
+        if constexpr (L == ML_SYM8) {
+            const uint32_t w8[8] = {p.c0.x, p.c0.y, p.c0.z, p.c0.w, p.c1.x, p.c1.y, p.c1.z, p.c1.w};
+#pragma unroll
+            for (int i = 0; i < 8; ++i) bytes[i] = w8[i] ^ 0x80808080u;      // code + 128
+            bias = __float2half2_rn(1152.f);
+        } else {
+#pragma unroll
+            for (int b = 0; b < 2; ++b)            // block b: words 2b, 2b + 1; byte k: column k (low), k + 8 (high)
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const int cl = 16 * b + 4 * i, ch = cl + 8;
+                    bytes[4 * b + i] = (w[2 * b + i] & 0x0F0F0F0Fu) | spread_nibble<4>((p.h >> cl) & 0xFu) | spread_nibble<5>((p.h2 >> cl) & 0xFu);
+                    bytes[4 * b + 2 + i] =
+                        ((w[2 * b + i] >> 4) & 0x0F0F0F0Fu) | spread_nibble<4>((p.h >> ch) & 0xFu) | spread_nibble<5>((p.h2 >> ch) & 0xFu);
+                }
+            bias = __float2half2_rn(1056.f);       // stored code = value + 32
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        uint2 pa, ea, pb, eb;
+        bytes_to_half4_pair(bytes[2 * j], bias, s2[j >> 1], pa, ea);
+        bytes_to_half4_pair(bytes[2 * j + 1], bias, s2[j >> 1], pb, eb);
+        const uint32_t off = sw128_offset(r, 4 * half + j);
+        *reinterpret_cast<uint4*>(p_slab + off) = make_uint4(pa.x, pa.y, pb.x, pb.y);
+        *reinterpret_cast<uint4*>(e_slab + off) = make_uint4(ea.x, ea.y, eb.x, eb.y);
+    }
+    return __low2half(m2);
+}
+
+template <int L, int NT>
+__global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_constant__ SbArgs a, const __grid_constant__ SbMaps maps) {
+    using G = SbGeo<L, NT>;
+    using Y = SbLayout<L>;
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    // the operands of a stage are complete (8 weight warps + the TMA bytes) / have been multiplied.  A super-block's min
+    // operands are part of its stages: mins with the weights of each, block sums with the activations of the first.
+    // Two buffers of them need no barrier of their own: the stage that writes buffer s % 2 again has waited for a stage
+    // behind the MMA that read it.
+    __shared__ uint64_t bar_full[G::ST], bar_empty[G::ST], bar_done;
+    __shared__ uint32_t s_tmem;
+    __shared__ volatile int s_fail;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int ks = a.ks, z = blockIdx.x % ks, first_tile = blockIdx.x / ks, tile_step = gridDim.x / ks;
+    const int n0 = blockIdx.y * NT, nn = min(NT, a.n_tokens - n0);
+    const int sb0 = a.n_sb * z / ks, n_super = a.n_sb * (z + 1) / ks - sb0, n_stages = n_super * 4;     // this CTA's K slice
+    const int n_my = (a.n_tiles - first_tile + tile_step - 1) / tile_step;
+    constexpr uint32_t COLS = 2 * NT;
+
+    if (tid == 0) {
+        for (int s = 0; s < G::ST; ++s) { mbar_init(&bar_full[s], kSbGroup / 32 + 1); mbar_init(&bar_empty[s], 1); }
+        mbar_init(&bar_done, 1);
+        s_fail = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    pdl_launch_dependents();
+    if (warp == kSbMmaWarp) tmem_alloc(&s_tmem, COLS);
+    if (Y::SB6) {                                                    // K 8-15 of the min operands and the rows beyond nn stay zero
+        for (int i = tid; i < 2 * (G::MA + G::MB) / 16; i += kSbThreads) reinterpret_cast<uint4*>(smem + G::OFF_MA)[i] = make_uint4(0, 0, 0, 0);
+        fence_async_smem();
+    }
+
+    // ---- weight threads: group grp takes stages grp, grp + 2, ..; item = (row wt / 2, 32-column block wt & 1 of the stage)
+    const int grp = tid / kSbGroup, wt = tid % kSbGroup, wrow = wt >> 1, wblk = wt & 1;
+    unsigned char* raw = smem + G::OFF_RAW + grp * kSbAhead * Y::RAW;
+    unsigned char* recs = smem + G::OFF_REC + grp * 3 * kGmRows * 16;
+    int c_ti = 0, c_st = grp, c_slot = 0, c_rec = 0;                 // copy side: tile of this CTA, stage in it, ring positions
+    const uint8_t *c_codes = nullptr, *c_h = nullptr, *c_h2 = nullptr, *c_meta = nullptr;
+    bool c_long = true;                                              // a 16-byte record (else the 12 bytes of the file)
+    auto copy_tile = [&]() {                                         // source pointers of tile c_ti at stage grp
+        const int tile = first_tile + c_ti * tile_step;
+        const QView& t = a.t[tile / a.row_tiles];
+        const size_t R = static_cast<size_t>(min((tile % a.row_tiles) * kGmRows + wrow, t.rows - 1));
+        const int col = sb0 * 256 + grp * 64 + wblk * 32;
+        c_codes = t.codes + (L == ML_SYM8 ? R * t.cols + col : R * (t.cols >> 1) + (col >> 1));
+        if (Y::PLANES >= 1) c_h = t.qh + R * (t.cols >> 3) + (col >> 3);
+        if (Y::PLANES == 2) c_h2 = t.qh2 + R * (t.cols >> 3) + (col >> 3);
+        c_long = !Y::SB6 || t.dev_meta != nullptr;
+        if (!Y::SB6) c_meta = reinterpret_cast<const uint8_t*>(t.qs) + R * (t.cols >> 4) + sb0 * 16;
+        else c_meta = c_long ? t.dev_meta + (R * (t.cols >> 8) + sb0) * 16 : t.qsqm + (R * (t.cols >> 8) + sb0) * 12;
+    };
+    auto copy_stage = [&]() {
+        if (c_ti < n_my) {
+            unsigned char* slot = raw + c_slot * Y::RAW;
+            sb_cp16(slot + wt * 16, c_codes);
+            if (L == ML_SYM8) sb_cp16(slot + kSbGroup * 16 + wt * 16, c_codes + 16);
+            if (Y::PLANES >= 1) sb_cp4(slot + kSbGroup * Y::CODE_BYTES + wt * 4, c_h);
+            if (Y::PLANES == 2) sb_cp4(slot + kSbGroup * (Y::CODE_BYTES + 4) + wt * 4, c_h2);
+            if ((c_st & 2) == 0) {                                   // the row's scale record, once per super-block (2 stages of this group)
+                if (wblk == 0) {
+                    unsigned char* rec = recs + c_rec * (kGmRows * 16) + wrow * 16;
+                    if (c_long) sb_cp16(rec, c_meta);
+                    else { sb_cp4(rec, c_meta); sb_cp4(rec + 4, c_meta + 4); sb_cp4(rec + 8, c_meta + 8); }
+                }
+                c_meta += c_long ? 16 : 12;
+                c_rec = c_rec == 2 ? 0 : c_rec + 1;
+            }
+            c_codes += 2 * (L == ML_SYM8 ? 64 : 32);
+            if (Y::PLANES >= 1) c_h += 16;
+            if (Y::PLANES == 2) c_h2 += 16;
+            c_slot = c_slot == kSbAhead - 1 ? 0 : c_slot + 1;
+            c_st += 2;
+            if (c_st >= n_stages) {
+                c_st = grp;
+                if (++c_ti < n_my) copy_tile();
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");         // empty groups keep the count uniform
+    };
+    if (tid < kSbWeightThreads) {                                    // weights do not depend on the producer of x
+        copy_tile();
+        for (int i = 0; i < kSbAhead; ++i) copy_stage();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = s_tmem;
+    if (warp == kSbTmaWarp) pdl_wait();                              // the activations; the others wait before they read or store
+
+    int r_slot = 0, r_rec = 0;                                       // read side of the rings
+    int it = 0;                                                      // stages of the tiles before
+    uint32_t done_phase = 0;
+    for (int ti = 0; ti < n_my; ++ti) {
+        const int tile = first_tile + ti * tile_step, mat = tile / a.row_tiles, row0 = (tile % a.row_tiles) * kGmRows;
+        const QView& t = a.t[mat];
+        if (warp == kSbMmaWarp) {
+            // ------------------------------------------------------------------ MMA issuer (whole warp, one lane elected)
+            const uint32_t id = umma_idesc(2 * NT);
+            const uint64_t p0 = umma_desc(smem_addr(smem)), e0 = umma_desc(smem_addr(smem + G::OFF_E)), b0 = umma_desc(smem_addr(smem + G::OFF_B));
+            const uint64_t ma0 = umma_desc_plain(smem_addr(smem + G::OFF_MA), kGmRows * 16, 128);
+            const uint64_t mb0 = umma_desc_plain(smem_addr(smem + G::OFF_MB), 2 * NT * 16, 128);
+            uint32_t elected;
+            asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xFFFFFFFF;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(elected));
+            bool ok = true;
+            int st = it % G::ST, ph = (it / G::ST) & 1;
+            for (int i = 0; i < n_stages; ++i) {
+                if (!mbar_wait_bounded(&bar_full[st], ph)) { ok = false; break; }
+                tc_fence_after();
+                const uint64_t pd = p0 + (static_cast<uint64_t>(st * kSbSlab) >> 4), ed = e0 + (static_cast<uint64_t>(st * kSbSlab) >> 4);
+                const uint64_t bd = b0 + (static_cast<uint64_t>(st * G::BSLAB) >> 4);
+                if (elected) {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {                    // small terms first
+                        umma_f16(tmem, ed + 2 * k, bd + 2 * k, id, (i | k) ? 1u : 0u);
+                        umma_f16(tmem, pd + 2 * k, bd + 2 * k, id, 1u);
+                    }
+                    if (Y::SB6 && (i & 3) == 3) {                    // the super-block's mins are complete with its last stage
+                        const int ms = ((it + i) >> 2) & 1;
+                        umma_f16(tmem, ma0 + (static_cast<uint64_t>(ms * G::MA) >> 4), mb0 + (static_cast<uint64_t>(ms * G::MB) >> 4), id, 1u);
+                    }
+                    umma_commit(&bar_empty[st]);
+                }
+                __syncwarp();
+                if (++st == G::ST) { st = 0; ph ^= 1; }
+            }
+            if (ok && elected) umma_commit(&bar_done);
+            if (!ok) s_fail = 1;
+        } else if (warp == kSbTmaWarp) {
+            // ------------------------------------------------------------------ activation pairs
+            if (lane == 0) {
+                for (int i = 0; i < n_stages; ++i) {
+                    const int g = it + i, st = g % G::ST;
+                    if (g >= G::ST && !mbar_wait_bounded(&bar_empty[st], (g / G::ST - 1) & 1)) { s_fail = 1; break; }
+                    unsigned char* b = smem + G::OFF_B + st * G::BSLAB;
+                    const bool with_sums = Y::SB6 && (i & 3) == 0;
+                    mbar_expect_tx(&bar_full[st], G::BSLAB + (with_sums ? 2 * nn * 16 : 0));
+                    tma_load_2d(b, &maps.hi[mat], sb0 * 256 + i * 64, n0, &bar_full[st]);
+                    tma_load_2d(b + NT * 128, &maps.lo[mat], sb0 * 256 + i * 64, n0, &bar_full[st]);
+                    if (with_sums) {
+                        unsigned char* m = smem + G::OFF_MB + ((g >> 2) & 1) * G::MB;
+#pragma unroll
+                        for (int h = 0; h < 2; ++h)
+                            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                                             smem_addr(m + h * NT * 16)),
+                                         "l"(a.sums[mat] + ((static_cast<size_t>(sb0 + (i >> 2)) * 2 + h) * a.n_tokens + n0) * 8), "r"(nn * 16),
+                                         "r"(smem_addr(&bar_full[st]))
+                                         : "memory");
+                    }
+                }
+            }
+        } else {
+            // ------------------------------------------------------------------ weights
+            // super-scales that are not part of the staged record (sym d; sb6 d | dm without the relayouted record), one
+            // super-block ahead
+            const bool in_rec = Y::SB6 && t.dev_meta != nullptr;
+            const size_t drow = static_cast<size_t>(min(row0 + wrow, t.rows - 1)) * (t.cols >> 8) + sb0;
+            uint32_t dd = 0, dd_next = 0;
+            auto load_d = [&](int sb) {
+                if (in_rec || sb >= n_super) return;
+                dd_next = __half_as_ushort(__ldg(t.d + drow + sb));
+                if (Y::SB6) dd_next |= static_cast<uint32_t>(__half_as_ushort(__ldg(t.dm + drow + sb))) << 16;
+            };
+            load_d(0);
+#pragma unroll 1
+            for (int i = grp; i < n_stages; i += 2) {
+                const int g = it + i, st = g % G::ST;
+                asm volatile("cp.async.wait_group %0;" ::"n"(kSbAhead - 1) : "memory");
+                __syncwarp();                                        // the pair lane's record
+                const unsigned char* slot = raw + r_slot * Y::RAW;
+                Packed p{};
+                p.c0 = *reinterpret_cast<const uint4*>(slot + wt * 16);
+                if (L == ML_SYM8) p.c1 = *reinterpret_cast<const uint4*>(slot + kSbGroup * 16 + wt * 16);
+                if (Y::PLANES >= 1) p.h = *reinterpret_cast<const uint32_t*>(slot + kSbGroup * Y::CODE_BYTES + wt * 4);
+                if (Y::PLANES == 2) p.h2 = *reinterpret_cast<const uint32_t*>(slot + kSbGroup * (Y::CODE_BYTES + 4) + wt * 4);
+                const int item = (i & 3) * 2 + wblk;                 // of the super-block
+                const unsigned char* rec = recs + r_rec * (kGmRows * 16) + wrow * 16;
+                r_slot = r_slot == kSbAhead - 1 ? 0 : r_slot + 1;
+                if (i & 2) r_rec = r_rec == 2 ? 0 : r_rec + 1;
+                if ((i & 2) == 0) { dd = dd_next; load_d((i >> 2) + 1); }
+                if (Y::SB6) {
+                    p.rec = *reinterpret_cast<const uint4*>(rec);
+                    if (!in_rec) p.rec.w = dd;
+                } else {
+                    p.rec.x = *reinterpret_cast<const unsigned short*>(rec + item * 2);
+                    p.rec.y = dd;
+                }
+                if (g >= G::ST) {                                    // the MMAs that read this buffer have completed
+                    if (lane == 0 && !s_fail && !mbar_wait_bounded(&bar_empty[st], (g / G::ST - 1) & 1)) s_fail = 1;
+                    __syncwarp();
+                }
+                const __half mn = sb_convert<L>(p, in_rec, wrow, item, wblk, smem + st * kSbSlab, smem + G::OFF_E + st * kSbSlab);
+                if (Y::SB6) reinterpret_cast<__half*>(smem + G::OFF_MA + ((g >> 2) & 1) * G::MA + wrow * 16)[item] = mn;
+                fence_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bar_full[st]);
+                copy_stage();                                        // every lane of the warp has read its slot
+            }
+        }
+        it += n_stages;
+        // ---------------------------------------------------------------------- epilogue of the tile
+        __syncwarp();
+        if (warp != kSbTmaWarp) {
+            if (lane == 0 && !s_fail && !mbar_wait_bounded(&bar_done, done_phase)) s_fail = 1;
+            __syncwarp();
+            done_phase ^= 1;
+            tc_fence_after();
+            if (ti == 0) pdl_wait();                                 // token scales, residual, output
+        }
+        constexpr int TPW = NT / 4;                                  // tokens per warp: four warps share a lane quadrant
+        constexpr int TC = TPW < 16 ? TPW : 16;                      // ... in chunks of at most 16
+        const int q = warp & 3, tg = warp >> 2, rl = q * 32 + lane;
+        float* y = a.y[mat] + static_cast<size_t>(n0) * a.ldy;
+        const float* rs = a.resid[mat] ? a.resid[mat] + static_cast<size_t>(n0) * a.ldy : nullptr;
+        float* am_out = a.amax_out[mat] ? a.amax_out[mat] + n0 : nullptr;
+        const float* un = a.unscale[mat] + n0;
+        auto store = [&](float v, int n, int row) {                  // whole warps; the 32 lanes hold 32 consecutive rows
+            const bool in = n < nn && row < t.rows && !s_fail;
+            const size_t o = static_cast<size_t>(n) * a.ldy + row;
+            if (a.epilogue == RWKVQ_EPI_RELU2) { v = fmaxf(v, 0.f); v = v * v; }
+            else if (a.epilogue == RWKVQ_EPI_ADD && in) v = __fadd_rn(v, __ldcg(rs + o));
+            if (in) y[o] = v;
+            if (am_out != nullptr && n < nn) {                       // |v| as bits orders like the float, a NaN above every number
+                const unsigned m = __reduce_max_sync(0xFFFFFFFFu, in ? __float_as_uint(fabsf(v)) : 0u);
+                if (lane == 0 && m != 0u) atomicMax(reinterpret_cast<unsigned*>(am_out) + n, m);
+            }
+        };
+        float* part = reinterpret_cast<float*>(smem);                // every MMA that read the operands has completed
+        if (warp < kSbTmaWarp) {
+#pragma unroll
+            for (int c0 = 0; c0 < TPW; c0 += TC) {
+                float v[TC], lo[TC];
+                const uint32_t base = tmem + (static_cast<uint32_t>(q * 32) << 16) + tg * TPW + c0;
+                sb_tmem_ld<TC>(base, v);
+                sb_tmem_ld<TC>(base + NT, lo);
+#pragma unroll
+                for (int j = 0; j < TC; ++j) {
+                    const int n = tg * TPW + c0 + j;
+                    v[j] = n < nn ? (v[j] + lo[j]) * __ldcg(un + n) : 0.f;
+                    if (ks == 1) store(v[j], n, row0 + rl);
+                    else part[n * kSbPitch + rl] = v[j];
+                }
+            }
+            tc_fence_before();
+        }
+        if (ks == 1) {                                               // the accumulator is free for the next tile
+            if (warp != kSbTmaWarp) asm volatile("bar.sync 1, %0;" ::"n"(kSbThreads - 32) : "memory");
+            tc_fence_after();
+        } else {
+            cluster.sync();
+            if (warp < kSbTmaWarp) {                                 // this CTA's share of the tokens, ranks added in order
+                const int per = (NT + ks - 1) / ks, n1 = min(nn, (z + 1) * per);
+                constexpr int UT = 4;                                // tokens whose remote loads are in flight together
+                for (int nb = z * per + tg; nb < n1; nb += 4 * UT) {
+                    float s4[UT];
+#pragma unroll
+                    for (int j = 0; j < UT; ++j) s4[j] = 0.f;
+                    for (int u = 0; u < ks; u += 2) {
+                        const float* p0 = cluster.map_shared_rank(part, u);
+                        const float* p1 = cluster.map_shared_rank(part, u + 1 < ks ? u + 1 : u);
+                        float v0[UT], v1[UT];
+#pragma unroll
+                        for (int j = 0; j < UT; ++j) {
+                            const int n = min(nb + 4 * j, NT - 1);
+                            v0[j] = p0[n * kSbPitch + rl];
+                            v1[j] = u + 1 < ks ? p1[n * kSbPitch + rl] : 0.f;
+                        }
+#pragma unroll
+                        for (int j = 0; j < UT; ++j) s4[j] = (s4[j] + v0[j]) + v1[j];
+                    }
+#pragma unroll
+                    for (int j = 0; j < UT; ++j)
+                        if (nb + 4 * j < n1) store(s4[j], nb + 4 * j, row0 + rl);
+                }
+            }
+            cluster.sync();                                          // nobody leaves while a peer still reads its partial tile
+        }
+    }
+    if (tid < kSbWeightThreads) asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    if (tid == 0 && s_fail) atomicCAS(a.status, 0, RWKVQ_E_TIMEOUT);
+    tc_fence_after();
+    if (warp == kSbMmaWarp) tmem_dealloc(tmem, COLS);
+}
+
+// fp32 rows -> pairs, one CTA per row.  Bound: latency (a load, a block maximum, the stores); rows of up to 8192 columns
+// stay in registers between the two uses.
+__global__ void __launch_bounds__(512) split_rows_kernel(const float* __restrict__ x, long long ldx, int cols, const SbRows o, int N, int* status) {
+    __shared__ float red[16];
+    pdl_launch_dependents();
+    pdl_wait();
+    if (status != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *status = 0;      // of the product that follows
+    const int n = blockIdx.x, n8 = cols >> 3;                        // n8 is a multiple of 32: whole warps take a pass together
+    const float4* row = reinterpret_cast<const float4*>(x + static_cast<size_t>(n) * ldx);
+    constexpr int kKeep = 2;
+    float4 f[kKeep][2];
+    float m = 0.f;
+    auto upd = [&](const float4& v) {
+        m = fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+        if (!(fabsf(v.x) + fabsf(v.y) + fabsf(v.z) + fabsf(v.w) < INFINITY)) m = INFINITY;
+    };
+#pragma unroll
+    for (int k = 0; k < kKeep; ++k) {
+        const int i = threadIdx.x + k * 512;
+        f[k][0] = i < n8 ? __ldcg(row + 2 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        f[k][1] = i < n8 ? __ldcg(row + 2 * i + 1) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int k = 0; k < kKeep; ++k) { upd(f[k][0]); upd(f[k][1]); }
+    for (int i = threadIdx.x + kKeep * 512; i < n8; i += 512) { upd(__ldcg(row + 2 * i)); upd(__ldcg(row + 2 * i + 1)); }
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, s));
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+    __syncthreads();
+    m = red[threadIdx.x & 15];
+#pragma unroll
+    for (int s = 8; s > 0; s >>= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, s));
+    float s1, u1;
+    sb_scale(m, s1, u1);
+    if (threadIdx.x == 0) o.unscale[n] = u1;
+    auto put = [&](int i, const float4& a, const float4& b) {
+        const float v[8] = {a.x * s1, a.y * s1, a.z * s1, a.w * s1, b.x * s1, b.y * s1, b.z * s1, b.w * s1};
+        sb_store_pair(o, n, N, i, v);
+    };
+#pragma unroll
+    for (int k = 0; k < kKeep; ++k)
+        if (static_cast<int>(threadIdx.x) + k * 512 < n8) put(threadIdx.x + k * 512, f[k][0], f[k][1]);
+    for (int i = threadIdx.x + kKeep * 512; i < n8; i += 512) put(i, __ldcg(row + 2 * i), __ldcg(row + 2 * i + 1));
+}
+
+int launch_split_rows(const float* x, long long ldx, int cols, int N, const SbRows& o, int* status, cudaStream_t s) {
+    cudaError_t e = launch_pdl(split_rows_kernel, dim3(N), dim3(512), 0, s, x, ldx, cols, o, N, status);
+    if (e != cudaSuccess) return fail(RWKVQ_E_LAUNCH, "split_rows: %s", cudaGetErrorString(e));
+    return RWKVQ_OK;
+}
+
+namespace {
+
+int sb_layout_of(const rwkvq_qtensor& t) {
+    if (t.kind == RWKVQ_KIND_SB6) return ML_SB6_4 + (t.bits - 4);
+    return t.bits == 8 ? ML_SYM8 : ML_SYM6;
+}
+
+template <int L, int NT>
+int launch_sb(SbArgs& a, const SbMaps& maps, int groups, cudaStream_t s) {
+    static bool configured[64] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) dev = 0;
+    if (dev >= 64 || !configured[dev]) {
+        cudaError_t e = cudaFuncSetAttribute(gemm_sb_kernel<L, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(SbGeo<L, NT>::BYTES));
+        if (e != cudaSuccess) return fail(RWKVQ_E_LIMIT, "gemm_sb: %zu bytes of shared memory: %s", SbGeo<L, NT>::BYTES, cudaGetErrorString(e));
+        if (dev < 64) configured[dev] = true;
+    }
+    cudaLaunchConfig_t cfg{};
+    // one wave of persistent CTAs where K is not split
+    cfg.gridDim = dim3(a.ks > 1 ? a.n_tiles * a.ks : std::min(a.n_tiles, std::max(1, 148 / groups)), groups);
+    cfg.blockDim = dim3(kSbThreads);
+    cfg.dynamicSmemBytes = SbGeo<L, NT>::BYTES;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = a.ks; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_sb_kernel<L, NT>, a, maps);
+    if (e != cudaSuccess) return fail(RWKVQ_E_LAUNCH, "gemm_sb: %s", cudaGetErrorString(e));
+    return RWKVQ_OK;
+}
+
+template <int L>
+int launch_sb_nt(SbArgs& a, const SbMaps& maps, int nt, int groups, cudaStream_t s) {
+    switch (nt) {
+        case 16: return launch_sb<L, 16>(a, maps, groups, s);
+        case 32: return launch_sb<L, 32>(a, maps, groups, s);
+        case 64: return launch_sb<L, 64>(a, maps, groups, s);
+        default: return launch_sb<L, 128>(a, maps, groups, s);
+    }
+}
+
+}  // namespace
+
+// Whether this kernel takes a product the mma.sync kernel serves too.
+bool gemm_sb_pays(const rwkvq_qtensor& t, int N) {
+    static const int least = [] { const char* e = getenv("SBMIN"); return e ? atoi(e) : 17; }();
+    return tcb_enabled() && gemm_tcb_ok(t) && N >= least;
+}
+
+int launch_gemm_sb(const rwkvq_qtensor* ts, int n_mats, const SbRows* rows, int N, float* const* ys, long long ldy, int epilogue,
+                   const float* const* resids, float* const* amax_outs, int* status, int force_ks, cudaStream_t s) {
+    RWKVQ_REQUIRE(n_mats >= 1 && n_mats <= kSbMaxMats, RWKVQ_E_LIMIT, "gemm_sb: %d matrices", n_mats);
+    SbArgs a{};
+    SbMaps maps;
+    const int nt = N <= 16 ? 16 : N <= 32 ? 32 : N <= 64 ? 64 : 128, groups = (N + nt - 1) / nt;
+    for (int k = 0; k < n_mats; ++k) {
+        RWKVQ_REQUIRE(gemm_tcb_ok(ts[k]) && ts[k].kind == ts[0].kind && ts[k].bits == ts[0].bits && ts[k].rows == ts[0].rows &&
+                          ts[k].cols == ts[0].cols, RWKVQ_E_SHAPE, "gemm_sb: fused matrices must share layout and shape");
+        RWKVQ_REQUIRE(rows[k].hi && rows[k].lo && rows[k].sums && rows[k].unscale && ys[k], RWKVQ_E_NULL, "gemm_sb: x pairs or y is null");
+        a.t[k] = make_view(ts[k]);
+        a.sums[k] = rows[k].sums; a.unscale[k] = rows[k].unscale; a.y[k] = ys[k];
+        a.resid[k] = resids ? resids[k] : nullptr;
+        a.amax_out[k] = amax_outs ? amax_outs[k] : nullptr;
+        RWKVQ_REQUIRE(epilogue != RWKVQ_EPI_ADD || a.resid[k], RWKVQ_E_NULL, "gemm_sb: resid is null");
+        int rc = make_half_map(&maps.hi[k], rows[k].hi, N, ts[0].cols, rows[k].pitch, nt);
+        if (rc) return rc;
+        rc = make_half_map(&maps.lo[k], rows[k].lo, N, ts[0].cols, rows[k].pitch, nt);
+        if (rc) return rc;
+    }
+    a.ldy = ldy; a.n_tokens = N; a.epilogue = epilogue; a.status = status;
+    a.row_tiles = (ts[0].rows + kGmRows - 1) / kGmRows;
+    a.n_tiles = a.row_tiles * n_mats;
+    a.n_sb = ts[0].cols / 256;
+    // K split into up to 8 slices of whole super-blocks: modelled cycles of the slowest SM = waves of CTAs (one per SM) x
+    // (ramp + stages) + the cluster reduction; without a split the CTAs are persistent and pay the ramp once
+    const double stage = nt == 128 ? 1150.0 : nt == 64 ? 850.0 : 800.0;
+    double best = 1e300;
+    a.ks = 1;
+    for (int c = 1; c <= 8 && c <= a.n_sb; ++c) {
+        const double waves = static_cast<double>((a.n_tiles * groups * c + 147) / 148), work = ((a.n_sb + c - 1) / c) * 4 * stage;
+        const double t = c == 1 ? waves * (work + 2000.0) + 4000.0 : waves * (work + 4000.0) + 3500.0 + 150.0 * c;
+        if (t < best) { best = t; a.ks = c; }
+    }
+    if (force_ks > 0 && force_ks <= 8 && force_ks <= a.n_sb) a.ks = force_ks;
+    switch (sb_layout_of(ts[0])) {
+        case ML_SB6_4: return launch_sb_nt<ML_SB6_4>(a, maps, nt, groups, s);
+        case ML_SB6_5: return launch_sb_nt<ML_SB6_5>(a, maps, nt, groups, s);
+        case ML_SB6_6: return launch_sb_nt<ML_SB6_6>(a, maps, nt, groups, s);
+        case ML_SYM6: return launch_sb_nt<ML_SYM6>(a, maps, nt, groups, s);
+        default: return launch_sb_nt<ML_SYM8>(a, maps, nt, groups, s);
+    }
+}
+
+}  // namespace rwkvq

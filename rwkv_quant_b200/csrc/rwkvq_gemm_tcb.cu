@@ -462,8 +462,8 @@ bool tcb_enabled() {
     static const bool on = [] { const char* e = getenv("RWKVQ_TCB"); return !(e && e[0] == '0'); }();
     return on && g_tcb_force_ks >= 0;          // rwkvq_profiling_tcb_force(-1) switches it off at run time
 }
-bool tcb_forced() { return g_tcb_force_ks > 0;
-}
+bool tcb_forced() { return g_tcb_force_ks > 0; }
+int tcb_forced_ks() { return g_tcb_force_ks > 0 ? g_tcb_force_ks : 0; }
 
 // Whether the tcgen05 small-batch kernel serves the tensor: sb6 / sym in the layouts the prefill
 // kernel's producer reads (block 32 x 8 and 16 x 16), columns a multiple of 256.

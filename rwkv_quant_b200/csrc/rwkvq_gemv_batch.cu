@@ -38,6 +38,7 @@
 #include <algorithm>
 #include <cstdlib>
 
+#include "rwkvq_gemm_sb.cuh"
 #include "rwkvq_gemv_mma.cuh"
 
 namespace cg = cooperative_groups;
@@ -751,8 +752,12 @@ extern "C" void rwkvq_profiling_batch_force(int force_ks, int rows, int cols) {
     g_batch_force_cols = cols;
 }
 
-// [status word, padded to 256 bytes][N floats: max|x| per row]
-extern "C" size_t rwkvq_gemv_batch_workspace_bytes(int N) { return N > 0 ? 256 + ((static_cast<size_t>(N) * sizeof(float) + 255) / 256) * 256 : 0; }
+// [status word, padded to 256 bytes][N floats: max|x| per row, or 2^-s of the pairs][pairs of up to kPairCols columns]
+namespace {
+constexpr int kPairCols = 16384;
+inline size_t batch_ws_pairs(int N) { return 256 + ((static_cast<size_t>(N) * sizeof(float) + 255) / 256) * 256; }
+}
+extern "C" size_t rwkvq_gemv_batch_workspace_bytes(int N) { return N > 0 ? batch_ws_pairs(N) + sb_halves(N, kPairCols) * sizeof(__half) : 0; }
 
 extern "C" int rwkvq_gemv_batch(const rwkvq_qtensor* t, const float* x, int N, int64_t ldx, float* y, int64_t ldy,
                                 int epilogue, const float* resid, void* workspace, size_t workspace_bytes, void* stream) {
@@ -764,9 +769,10 @@ extern "C" int rwkvq_gemv_batch(const rwkvq_qtensor* t, const float* x, int N, i
     RWKVQ_REQUIRE(x && y, RWKVQ_E_NULL, "rwkvq_gemv_batch: x or y is null");
     // default: the two-term mma.sync kernel.  The tcgen05 kernel (single fp16 operands) serves more than
     // 32 rows in fast mode, tensors the mma.sync kernel has no layout for, and the profiling override.
-    const bool tcb = tcb_enabled() && gemm_tcb_ok(*t) && ldx % 8 == 0 &&
-                     ((batch_fast() && N > 32) || mma_layout_of(*t) < 0 || tcb_forced());
-    RWKVQ_REQUIRE(tcb || mma_layout_of(*t) >= 0, RWKVQ_E_DTYPE,
+    const bool tcb_ok = tcb_enabled() && gemm_tcb_ok(*t) && t->cols <= kPairCols;
+    const bool tcb = tcb_ok && batch_fast() && ldx % 8 == 0 && (N > 32 || mma_layout_of(*t) < 0 || tcb_forced());
+    const bool sb = tcb_ok && !batch_fast() && (gemm_sb_pays(*t, N) || mma_layout_of(*t) < 0 || tcb_forced());
+    RWKVQ_REQUIRE(tcb || sb || mma_layout_of(*t) >= 0, RWKVQ_E_DTYPE,
                   "rwkvq_gemv_batch: needs an sb6 tensor, a sym tensor or per-row int8 with columns in multiples of 128");
     RWKVQ_REQUIRE(aligned(x, 16) && ldx % 4 == 0, RWKVQ_E_ALIGN, "rwkvq_gemv_batch: x rows must be 16-byte aligned");
     RWKVQ_REQUIRE(aligned(workspace, 16), RWKVQ_E_ALIGN, "rwkvq_gemv_batch: workspace must be 16-byte aligned");
@@ -775,13 +781,20 @@ extern "C" int rwkvq_gemv_batch(const rwkvq_qtensor* t, const float* x, int N, i
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     int* status = static_cast<int*>(workspace);
     float* amax = reinterpret_cast<float*>(static_cast<char*>(workspace) + 256);
+    float* ys[1] = {y};
+    const float* rs[1] = {resid};
+    if (sb) {
+        const SbRows rows = sb_rows(reinterpret_cast<__half*>(static_cast<char*>(workspace) + batch_ws_pairs(N)), amax, N, t->cols);
+        rc = launch_split_rows(x, ldx, t->cols, N, rows, status, s);
+        if (rc) return rc;
+        rc = launch_gemm_sb(t, 1, &rows, N, ys, ldy, epilogue, rs, nullptr, status, tcb_forced_ks(), s);
+        return rc ? rc : check_launch("rwkvq_gemv_batch");
+    }
     rc = launch_row_amax(x, ldx, t->cols, N, amax, status, s);
     if (rc) return rc;
     const void* xs[1] = {x};
     const float* am[1] = {amax};
-    float* ys[1] = {y};
-    const float* rs[1] = {resid};
-    rc = tcb ? launch_gemm_tcb(t, 1, xs, false, am, N, ldx, ys, ldy, epilogue, rs, nullptr, status, s, !batch_fast())
+    rc = tcb ? launch_gemm_tcb(t, 1, xs, false, am, N, ldx, ys, ldy, epilogue, rs, nullptr, status, s)
              : launch_gemv_batch(t, 1, xs, false, am, N, ldx, ys, ldy, epilogue, rs, nullptr, s);
     return rc ? rc : check_launch("rwkvq_gemv_batch");
 }
