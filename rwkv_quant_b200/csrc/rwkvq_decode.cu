@@ -22,6 +22,7 @@
 #include <utility>
 
 #include "rwkvq_decode_parts.cuh"
+#include "rwkvq_seq.cuh"
 
 namespace rwkvq {
 
@@ -170,19 +171,13 @@ __global__ void __launch_bounds__(kRowThreads) ln_shift_mix_kernel(const float* 
                                                                   float* __restrict__ shift,
                                                                   const float* __restrict__ mix,
                                                                   float* __restrict__ out, int B, int D,
-                                                                  __half* __restrict__ x16_out, __half* __restrict__ x16lo_out,
-                                                                  __half* __restrict__ xsum_out,
-                                                                  float* __restrict__ unscale_out, int x16_mask,
+                                                                  __half* __restrict__ x16_out, float* __restrict__ unscale_out, int x16_mask,
                                                                   float* __restrict__ zero_a, float* __restrict__ zero_b) {
     // x16_out (optional) [max(NMIX, 1)][B][D] with unscale_out [max(NMIX, 1)][B]: the rows selected by
     // x16_mask also as fp16(out * 2^s), s chosen from the row's max so that no value leaves the fp16
     // range, and 2^-s: the form the single-term small-batch linear reads (half the bytes, no
-    // conversion there); x16lo_out with xsum_out (optional; D a multiple of 128): the form the two-term
-    // tcgen05 linear reads: s is then chosen for |out * 2^s| <= 2^9, x16lo_out (same shape) takes
-    // fp16(out * 2^s - x16_out) and xsum_out [max(NMIX, 1)][B][D / 128][8] the sums of out * 2^s over the
-    // four 32-column blocks of every 128 columns, 4 high halves then 4 low halves.  With unscale_out
-    // alone, max|out| of the selected rows goes there instead (what the two-term mma.sync linear wants
-    // beside the fp32 rows);
+    // conversion there).  With unscale_out alone, max|out| of the selected rows goes there instead (what the
+    // two-term mma.sync linear wants beside the fp32 rows);
     // zero_a / zero_b (optional) [B]: slots later kernels of the layer merge their own row maxima
     // into, cleared here for stream b
     constexpr int NM = NMIX > 0 ? NMIX : 1;
@@ -262,16 +257,14 @@ __global__ void __launch_bounds__(kRowThreads) ln_shift_mix_kernel(const float* 
                 if ((x16_mask >> threadIdx.x) & 1) unscale_out[threadIdx.x * B + b] = r;
                 return;
             }
-            // |x| * 2^(14 - e) <= 2^14 with max|x| <= 2^e (2^9 for the two-term form, whose block sums must
-            // stay inside the fp16 range); a non-finite row keeps scale 1 and propagates
+            // |x| * 2^(14 - e) <= 2^14 with max|x| <= 2^e; a non-finite row keeps scale 1 and propagates
             float s1 = 1.f, u1 = 1.f;
             if (r > 0.f && r < INFINITY) {
                 int e = 0;
                 frexpf(r, &e);
                 e = max(-100, e);
-                const int top = x16lo_out ? 9 : 14;
-                s1 = ldexpf(1.f, top - e);
-                u1 = ldexpf(1.f, e - top);
+                s1 = ldexpf(1.f, 14 - e);
+                u1 = ldexpf(1.f, e - 14);
             }
             sc_m[threadIdx.x] = s1;
             if ((x16_mask >> threadIdx.x) & 1) unscale_out[threadIdx.x * B + b] = u1;
@@ -284,24 +277,7 @@ __global__ void __launch_bounds__(kRowThreads) ln_shift_mix_kernel(const float* 
             if (d >= D) continue;
             const size_t bd = static_cast<size_t>(b) * D + d;
             const float xn = (v[i] - mean) * inv * lw[i] + lb[i];
-            // d >= D holds for a whole warp or for none of it (D is a multiple of 32 whenever xsum_out is given)
-            auto emit = [&](int m, float sx) {
-                const size_t o = (static_cast<size_t>(m) * B) * D + bd;
-                const __half hi = __float2half_rn(sx);
-                x16_out[o] = hi;
-                if (x16lo_out == nullptr) return;
-                x16lo_out[o] = __float2half_rn(sx - __half2float(hi));
-                float bs = sx;                                   // the warp holds one block of 32 columns
-#pragma unroll
-                for (int sh = 16; sh > 0; sh >>= 1) bs += __shfl_xor_sync(0xFFFFFFFFu, bs, sh);
-                if ((threadIdx.x & 31) == 0) {
-                    const int blk = d >> 5;
-                    __half* sp = xsum_out + ((static_cast<size_t>(m) * B + b) * (D >> 7) + (blk >> 2)) * 8 + (blk & 3);
-                    const __half sh16 = __float2half_rn(bs);
-                    sp[0] = sh16;
-                    sp[4] = __float2half_rn(bs - __half2float(sh16));
-                }
-            };
+            auto emit = [&](int m, float sx) { x16_out[(static_cast<size_t>(m) * B) * D + bd] = __float2half_rn(sx); };
             if (NMIX == 0) { emit(0, xn * sc_m[0]); continue; }
             const float xx = prev[i] - xn;
 #pragma unroll
@@ -683,36 +659,38 @@ inline bool batch_path(int B) { return B > 2 && B <= kBatchMax; }
 // streams on (64 streams: 3.77 against 4.43 ms per step) and loses below (32: 2.87 / 2.68 ms, 8: 2.42 / 2.01 ms):
 // its pass (dependent weight loads -> conversion -> MMA) is longer than a warp-iteration of the mma.sync form
 inline bool tcb_pays(int B) { return batch_fast() && tcb_enabled() && B > 32; }
-// Default (two-term) precision above 32 streams: which linears run on the tcgen05 form of the two-term
-// kernel, fed with fp16 pairs and block sums by the LayerNorm kernels (bit 0 r / k / v, bit 1 ffn key,
-// bit 2 head).  The output projection and the ffn value, whose inputs reach the linear as fp32 rows without
-// a known scale, always stay on the mma.sync form.  Measured on B200 (1.5B, whole decode step, ms):
-//   streams        33    36    40    48    50    52    56    60    64
-//   all mma.sync  3.69  3.72  3.72  3.76  3.92  4.02  4.10  4.13  4.05
-//   head          3.66  3.69  3.72  3.73   -    3.96  4.04  4.07  4.00
-//   r/k/v + head   -    3.70  3.82  3.86  3.80  3.79  3.87  3.92  3.92
-//   all three     3.45  3.47  3.59  3.64  4.14  4.20  4.27  4.32  4.27
-// -> all three up to 48 streams, r / k / v and the head from 49 to 64.
-// RWKVQ_TCB_EXACT in the environment (read once) overrides: 0 none, 1 all three at every such batch.
-int g_tcb_exact = -2;          // -2 environment not read yet, -1 the measured policy, 0 none, 1 all three
-inline int tcx_mask(int B) {
+// Default (two-term) precision: from kSbMinStreams streams on every linear of the step runs on the tcgen05 pipeline
+// (rwkvq_gemm_sb.cu), fed with fp16 pairs and block sums by the LayerNorm kernels and, for the output projection and the
+// ffn value, by a pass over the fp32 rows.  Below, the mma.sync form: few tokens give its 3 MMAs per step little to do.
+// RWKVQ_TCB_EXACT in the environment (read once) overrides: 0 never, 1 at every batch.
+constexpr int kSbMinStreams = 17;
+int g_tcb_exact = -2;          // -2 environment not read yet, -1 by stream count, 0 never, 1 always
+bool sb_wanted(int B) {
     if (g_tcb_exact == -2) {
         const char* e = getenv("RWKVQ_TCB_EXACT");
         g_tcb_exact = (e == nullptr || (e[0] != '0' && e[0] != '1')) ? -1 : e[0] - '0';
     }
-    if (batch_fast() || !tcb_enabled() || B <= 32 || B > kBatchMax || g_tcb_exact == 0) return 0;
-    if (g_tcb_exact == 1) return 7;
-    return B <= 48 ? 7 : B <= 64 ? 5 : 0;
+    if (batch_fast() || !tcb_enabled() || B <= 2 || B > kBatchMax || g_tcb_exact == 0) return false;
+    return g_tcb_exact == 1 || B >= kSbMinStreams;
 }
-
+bool sb_model_ok(const rwkvq_model& m) {
+    if (!seq_prep_in_place_ok(m.n_embd) || !gemm_tcb_ok(m.head)) return false;
+    for (int l = 0; l < m.n_layer; ++l) {
+        const rwkvq_layer& L = m.layers[l];
+        for (const rwkvq_qtensor* t : {&L.Wr, &L.Wk, &L.Wv, &L.Wo, &L.Wfk, &L.Wfv})
+            if (!gemm_tcb_ok(*t)) return false;
+        for (const rwkvq_qtensor* t : {&L.Wk, &L.Wv})
+            if (t->kind != L.Wr.kind || t->bits != L.Wr.bits || t->rows != L.Wr.rows || t->cols != L.Wr.cols) return false;
+    }
+    return true;
+}
 
 struct Workspace {
     float *x, *xs, *rkv, *part, *yl, *og, *xk, *hffn, *xo, *v_first, *logits, *argv, *gscratch, *gemm_ws;
     int* status;             // first word of the workspace: RWKVQ_E_TIMEOUT if a bounded device-side wait of a step ran out
     float* amax;             // [10][B] per-row scale inverses / maxima for the small-batch linears: 6 mix rows, og, xk, hffn, xo
     __half *xs16, *xk16, *xo16;     // fp16 forms of the mix rows, the channel-mix row and the final row
-    __half *xs16lo, *xk16lo, *xo16lo;   // their second terms (two-term tcgen05 linears)
-    __half *xs_sum, *xk_sum, *xo_sum;   // ... and block sums, [rows][B][D / 128][8]
+    SbRows rkv_pair[3], d_pair, f_pair;     // operand rows of the tcgen05 pipeline: r / k / v; og, xk or xo; hffn
     int n_chunks;
     size_t part_floats;
     size_t bytes;
@@ -739,12 +717,15 @@ Workspace carve(const rwkvq_model& m, int B, void* base) {
     w.xs16 = reinterpret_cast<__half*>(take(3 * b * D));
     w.xk16 = reinterpret_cast<__half*>(take((b * D + 1) / 2));
     w.xo16 = reinterpret_cast<__half*>(take((b * D + 1) / 2));
-    w.xs16lo = reinterpret_cast<__half*>(take(3 * b * D));
-    w.xk16lo = reinterpret_cast<__half*>(take((b * D + 1) / 2));
-    w.xo16lo = reinterpret_cast<__half*>(take((b * D + 1) / 2));
-    w.xs_sum = reinterpret_cast<__half*>(take(6 * b * (D / 32 + 4)));
-    w.xk_sum = reinterpret_cast<__half*>(take(b * (D / 32 + 4)));
-    w.xo_sum = reinterpret_cast<__half*>(take(b * (D / 32 + 4)));
+    if (D % 256 == 0 && F % 256 == 0) {
+        auto pair = [&](size_t cols) {
+            float* un = take(b);
+            return sb_rows(reinterpret_cast<__half*>(take((sb_halves(B, static_cast<int>(cols)) + 1) / 2)), un, B, static_cast<int>(cols));
+        };
+        for (int k = 0; k < 3; ++k) w.rkv_pair[k] = pair(D);
+        w.d_pair = pair(D);
+        w.f_pair = pair(F);
+    }
     w.gscratch = take(gemv_mma_scratch_bytes() / sizeof(float));
     w.gemm_ws = take(rwkvq_gemm_workspace_bytes_for(B, static_cast<int>(F > D ? F : D)) / sizeof(float) + 1);
     w.bytes = off;
@@ -755,12 +736,11 @@ Workspace carve(const rwkvq_model& m, int B, void* base) {
 // One quantized linear for B right-hand sides; the single-vector tensor-core kernel gets
 // the K-split scratch, everything else goes through the public entry point.
 // x16 / x_scale: the fp16 form of x with its per-row scale inverses (what the LayerNorm kernels write
-// on the small-batch path), or null with x_scale = max|x| per row for fp32 rows; x16lo: the second fp16
-// term of x, which selects the two-term tcgen05 kernel (the caller has checked gemm_tcb_ok); y_amax:
-// optional slots max|y| per row is merged into.
+// in fast mode), or null with x_scale = max|x| per row for fp32 rows; y_amax: optional slots max|y| per row is
+// merged into.
 int linear(const rwkvq_qtensor* t, const float* x, int B, int in, float* y, int out, int epi, const float* resid,
            float* scratch, void* gemm_ws, void* stream, const __half* x16 = nullptr, const float* x_scale = nullptr,
-           float* y_amax = nullptr, int* status = nullptr, const __half* x16lo = nullptr, const __half* xsum = nullptr) {
+           float* y_amax = nullptr, int* status = nullptr) {
     const int ml = mma_layout_of(*t);
     if (B == 1 && ml >= 0) {
         int rc = validate_qtensor(t, "rwkvq_decode_step(linear)");
@@ -776,11 +756,6 @@ int linear(const rwkvq_qtensor* t, const float* x, int B, int in, float* y, int 
         float* ys[1] = {y};
         const float* rs[1] = {resid};
         float* ao[1] = {y_amax};
-        if (x16 && x16lo) {
-            const void* xl[1] = {x16lo};
-            const void* xm[1] = {xsum};
-            return launch_gemm_tcb(t, 1, xs, true, sc, B, in, ys, out, epi, rs, ao, status, static_cast<cudaStream_t>(stream), true, xl, xm);
-        }
         if (tcb_pays(B) && gemm_tcb_ok(*t))
             return launch_gemm_tcb(t, 1, xs, x16 != nullptr, sc, B, in, ys, out, epi, rs, ao, status, static_cast<cudaStream_t>(stream));
         return launch_gemv_batch(t, 1, xs, x16 != nullptr, sc, B, in, ys, out, epi, rs, ao, static_cast<cudaStream_t>(stream));
@@ -892,7 +867,7 @@ int rwkvq_seq_layer_norm(const float* x, const float* ln_w, const float* ln_b, f
                   (long long)n_rows, D, kRowThreads * kRowPer);
     launch_pdl(D <= 8 * kRowThreads ? ln_shift_mix_kernel<0, 8> : ln_shift_mix_kernel<0, kRowPer>, dim3(static_cast<unsigned>(n_rows)), dim3(kRowThreads), 0, static_cast<cudaStream_t>(stream), x,
                ln_w, ln_b, static_cast<float*>(nullptr), static_cast<const float*>(nullptr), out, static_cast<int>(n_rows), D,
-               static_cast<__half*>(nullptr), static_cast<__half*>(nullptr), static_cast<__half*>(nullptr), static_cast<float*>(nullptr), 0,
+               static_cast<__half*>(nullptr), static_cast<float*>(nullptr), 0,
                static_cast<float*>(nullptr), static_cast<float*>(nullptr));
     return check_launch("rwkvq_seq_layer_norm");
 }
@@ -921,6 +896,14 @@ int rwkvq_decode_step(const rwkvq_model* m, int B, const int64_t* tokens, float*
     int rc = validate_qtensor(&m->emb, "rwkvq_decode_step(emb)");
     if (rc) return rc;
     float* lg = logits ? logits : w.logits;
+    const bool sb = sb_wanted(B) && sb_model_ok(*m);
+    if (sb) {
+        for (int l = 0; l < m->n_layer; ++l)
+            for (const rwkvq_qtensor* t : {&m->layers[l].Wr, &m->layers[l].Wk, &m->layers[l].Wv, &m->layers[l].Wo, &m->layers[l].Wfk, &m->layers[l].Wfv}) {
+                rc = validate_qtensor(t, "rwkvq_decode_step(linear)");
+                if (rc) return rc;
+            }
+    }
 
     launch_pdl(embed_ln0_kernel, dim3(B), dim3(kRowThreads), 0, s, make_view(m->emb),
                reinterpret_cast<const long long*>(tokens), m->ln0_w, m->ln0_b, w.x, D);
@@ -934,16 +917,25 @@ int rwkvq_decode_step(const rwkvq_model* m, int B, const int64_t* tokens, float*
         const int ml = mma_layout_of(L.Wr);
         const bool rkv_fused = ml >= 0 && mma_layout_of(L.Wk) == ml && mma_layout_of(L.Wv) == ml && L.Wk.rows == L.Wr.rows &&
                                L.Wv.rows == L.Wr.rows && L.Wk.cols == L.Wr.cols && L.Wv.cols == L.Wr.cols;
-        // two-term tcgen05 linears: fp16 pairs of their input rows from the LayerNorm kernels
-        const int tcx = tcx_mask(B);
-        const bool x_rkv = (tcx & 1) && rkv_fused && gemm_tcb_ok(L.Wr) && gemm_tcb_ok(L.Wk) && gemm_tcb_ok(L.Wv);
-        const bool x_key = (tcx & 2) && mma_layout_of(L.Wfk) >= 0 && gemm_tcb_ok(L.Wfk);
         float* am = bp ? w.amax : nullptr;
         float *am_og = bp ? w.amax + 6 * B : nullptr, *am_xk = bp ? w.amax + 7 * B : nullptr;
         float *am_h = bp ? w.amax + 8 * B : nullptr;
-        launch_pdl(D <= 8 * kRowThreads ? ln_shift_mix_kernel<6, 8> : ln_shift_mix_kernel<6, kRowPer>, dim3(B), dim3(kRowThreads), 0, s, w.x, L.ln1_w, L.ln1_b, tshift[l], L.x_mix, w.xs, B, D,
-                   (h16 || x_rkv) ? w.xs16 : static_cast<__half*>(nullptr), x_rkv ? w.xs16lo : static_cast<__half*>(nullptr),
-                   x_rkv ? w.xs_sum : static_cast<__half*>(nullptr), am, 0b001101, am_og, am_h);      // scales of the r, k, v rows
+        if (sb) {
+            // LayerNorm 1 + shift + lerps, a CTA per stream and mix; r / k / v rows as operand pairs, the LoRA rows fp32
+            SeqPrepArgs pa{};
+            pa.x = w.x; pa.ln_w = L.ln1_w; pa.ln_b = L.ln1_b; pa.shift_in = tshift[l]; pa.shift_out = tshift[l]; pa.mix = L.x_mix;
+            pa.T = 1; pa.D = D; pa.n_mix = 6;
+            const int lin[3] = {0, 2, 3};
+            for (int q = 0; q < 6; ++q) { pa.f32[q] = w.xs + q * BD; pa.mode[q] = kPrepF32; }
+            for (int q = 0; q < 3; ++q) { pa.pair[lin[q]] = w.rkv_pair[q]; pa.mode[lin[q]] = kPrepPair; }
+            if (!layer0) pa.mode[3] |= kPrepF32;
+            rc = launch_seq_prep(pa, B, s);
+            if (rc) return rc;
+        } else {
+            launch_pdl(D <= 8 * kRowThreads ? ln_shift_mix_kernel<6, 8> : ln_shift_mix_kernel<6, kRowPer>, dim3(B), dim3(kRowThreads), 0, s, w.x, L.ln1_w,
+                       L.ln1_b, tshift[l], L.x_mix, w.xs, B, D, h16 ? w.xs16 : static_cast<__half*>(nullptr), am, 0b001101, am_og,
+                       am_h);      // scales of the r, k, v rows
+        }
         float *xr = w.xs, *xw = w.xs + BD, *xk = w.xs + 2 * BD, *xv = w.xs + 3 * BD, *xa = w.xs + 4 * BD,
               *xg = w.xs + 5 * BD;
         float *r = w.rkv, *k = w.rkv + BD, *v = w.rkv + 2 * BD;
@@ -970,6 +962,11 @@ int rwkvq_decode_step(const rwkvq_model* m, int B, const int64_t* tokens, float*
             const void* x_each[3] = {xr, xk, xv};
             rc = launch_gemv_mma(ml, three, 3, xr, RWKVQ_F32, D, r, D, RWKVQ_EPI_NONE, nullptr, 1, s_rkv, x_each, w.gscratch);
             if (rc) return rc;
+        } else if (sb) {
+            const rwkvq_qtensor three[3] = {L.Wr, L.Wk, L.Wv};
+            float* y3[3] = {r, k, v};
+            rc = launch_gemm_sb(three, 3, w.rkv_pair, B, y3, D, RWKVQ_EPI_NONE, nullptr, nullptr, w.status, 0, s_rkv);
+            if (rc) return rc;
         } else if (bp && rkv_fused) {
             for (const rwkvq_qtensor* t : {&L.Wr, &L.Wk, &L.Wv}) {
                 rc = validate_qtensor(t, "rwkvq_decode_step(r/k/v)");
@@ -977,15 +974,10 @@ int rwkvq_decode_step(const rwkvq_model* m, int B, const int64_t* tokens, float*
             }
             const rwkvq_qtensor three[3] = {L.Wr, L.Wk, L.Wv};
             const void* x3[3] = {w.xs16, w.xs16 + 2 * BD, w.xs16 + 3 * BD};
-            const void* x3lo[3] = {w.xs16lo, w.xs16lo + 2 * BD, w.xs16lo + 3 * BD};
-            const size_t BS = static_cast<size_t>(B) * (D / 128) * 8;     // block sums of one mix row
-            const void* x3sum[3] = {w.xs_sum, w.xs_sum + 2 * BS, w.xs_sum + 3 * BS};
-            if (!h16 && !x_rkv) { x3[0] = xr; x3[1] = xk; x3[2] = xv; }
+            if (!h16) { x3[0] = xr; x3[1] = xk; x3[2] = xv; }
             const float* a3[3] = {am, am + 2 * B, am + 3 * B};
             float* y3[3] = {r, k, v};
-            if (x_rkv)
-                rc = launch_gemm_tcb(three, 3, x3, true, a3, B, D, y3, D, RWKVQ_EPI_NONE, nullptr, nullptr, w.status, s_rkv, true, x3lo, x3sum);
-            else if (tcb_pays(B) && gemm_tcb_ok(L.Wr))
+            if (tcb_pays(B) && gemm_tcb_ok(L.Wr))
                 rc = launch_gemm_tcb(three, 3, x3, h16, a3, B, D, y3, D, RWKVQ_EPI_NONE, nullptr, nullptr, w.status, s_rkv);
             else
                 rc = launch_gemv_batch(three, 3, x3, h16, a3, B, D, y3, D, RWKVQ_EPI_NONE, nullptr, nullptr, s_rkv);
@@ -1015,29 +1007,57 @@ int rwkvq_decode_step(const rwkvq_model* m, int B, const int64_t* tokens, float*
                 return fail(RWKVQ_E_LAUNCH, "rwkvq_decode_step: join of the side stream failed");
         }
         TmixCoreArgs tc{r, k, v, yw, ya, layer0 ? nullptr : yv, yg, L.w0, L.a0, L.v0, L.k_k, L.k_a, L.r_k,
-                        L.lnx_w, L.lnx_b, w.v_first, wkv[l], w.og, D, H, layer0 ? 1 : 0, am_og};
+                        L.lnx_w, L.lnx_b, w.v_first, wkv[l], w.og, D, H, layer0 ? 1 : 0, sb ? nullptr : am_og};
         launch_pdl(tmix_core_kernel, dim3(H, B), dim3(256), 0, s, tc);
+        if (sb) {
+            const float* res[1] = {w.x};
+            float *yx[1] = {w.x}, *yh[1] = {w.hffn};
+            rc = launch_split_rows(w.og, D, D, B, w.d_pair, nullptr, s);
+            if (rc) return rc;
+            rc = launch_gemm_sb(&L.Wo, 1, &w.d_pair, B, yx, D, RWKVQ_EPI_ADD, res, nullptr, w.status, 0, s);
+            if (rc) return rc;
+            SeqPrepArgs pc{};
+            pc.x = w.x; pc.ln_w = L.ln2_w; pc.ln_b = L.ln2_b; pc.shift_in = cshift[l]; pc.shift_out = cshift[l]; pc.mix = L.ffn_x_k;
+            pc.T = 1; pc.D = D; pc.n_mix = 1; pc.mode[0] = kPrepPair; pc.pair[0] = w.d_pair;
+            rc = launch_seq_prep(pc, B, s);
+            if (rc) return rc;
+            rc = launch_gemm_sb(&L.Wfk, 1, &w.d_pair, B, yh, F, RWKVQ_EPI_RELU2, nullptr, nullptr, w.status, 0, s);
+            if (rc) return rc;
+            rc = launch_split_rows(w.hffn, F, F, B, w.f_pair, nullptr, s);
+            if (rc) return rc;
+            rc = launch_gemm_sb(&L.Wfv, 1, &w.f_pair, B, yx, D, RWKVQ_EPI_ADD, res, nullptr, w.status, 0, s);
+            if (rc) return rc;
+            continue;
+        }
         rc = linear(&L.Wo, w.og, B, D, w.x, D, RWKVQ_EPI_ADD, w.x, w.gscratch, w.gemm_ws, stream, nullptr, am_og, nullptr, w.status);
         if (rc) return rc;
         // ---- channel mix
-        launch_pdl(D <= 8 * kRowThreads ? ln_shift_mix_kernel<1, 8> : ln_shift_mix_kernel<1, kRowPer>, dim3(B), dim3(kRowThreads), 0, s, w.x, L.ln2_w, L.ln2_b, cshift[l], L.ffn_x_k, w.xk, B, D,
-                   (h16 || x_key) ? w.xk16 : static_cast<__half*>(nullptr), x_key ? w.xk16lo : static_cast<__half*>(nullptr),
-                   x_key ? w.xk_sum : static_cast<__half*>(nullptr), am_xk, 1, static_cast<float*>(nullptr), static_cast<float*>(nullptr));
-        rc = linear(&L.Wfk, w.xk, B, D, w.hffn, F, RWKVQ_EPI_RELU2, nullptr, w.gscratch, w.gemm_ws, stream, (h16 || x_key) ? w.xk16 : nullptr,
-                    am_xk, am_h, w.status, x_key ? w.xk16lo : nullptr, x_key ? w.xk_sum : nullptr);
+        launch_pdl(D <= 8 * kRowThreads ? ln_shift_mix_kernel<1, 8> : ln_shift_mix_kernel<1, kRowPer>, dim3(B), dim3(kRowThreads), 0, s, w.x, L.ln2_w,
+                   L.ln2_b, cshift[l], L.ffn_x_k, w.xk, B, D, h16 ? w.xk16 : static_cast<__half*>(nullptr), am_xk, 1, static_cast<float*>(nullptr),
+                   static_cast<float*>(nullptr));
+        rc = linear(&L.Wfk, w.xk, B, D, w.hffn, F, RWKVQ_EPI_RELU2, nullptr, w.gscratch, w.gemm_ws, stream, h16 ? w.xk16 : nullptr, am_xk, am_h,
+                    w.status);
         if (rc) return rc;
         rc = linear(&L.Wfv, w.hffn, B, F, w.x, D, RWKVQ_EPI_ADD, w.x, w.gscratch, w.gemm_ws, stream, nullptr, am_h, nullptr, w.status);
         if (rc) return rc;
     }
-    float* am_xo = batch_path(B) ? w.amax + 9 * B : nullptr;
-    const bool x_head = (tcx_mask(B) & 4) && mma_layout_of(m->head) >= 0 && gemm_tcb_ok(m->head);
-    const bool xo_h16 = (am_xo && batch_fast()) || x_head;
-    launch_pdl(D <= 8 * kRowThreads ? ln_shift_mix_kernel<0, 8> : ln_shift_mix_kernel<0, kRowPer>, dim3(B), dim3(kRowThreads), 0, s, w.x, m->lnout_w, m->lnout_b, static_cast<float*>(nullptr), static_cast<const float*>(nullptr), w.xo, B, D,
-               xo_h16 ? w.xo16 : static_cast<__half*>(nullptr), x_head ? w.xo16lo : static_cast<__half*>(nullptr),
-               x_head ? w.xo_sum : static_cast<__half*>(nullptr), am_xo, 1, static_cast<float*>(nullptr), static_cast<float*>(nullptr));
-    rc = linear(&m->head, w.xo, B, D, lg, V, RWKVQ_EPI_NONE, nullptr, w.gscratch, w.gemm_ws, stream, xo_h16 ? w.xo16 : nullptr, am_xo, nullptr,
-                w.status, x_head ? w.xo16lo : nullptr, x_head ? w.xo_sum : nullptr);
-    if (rc) return rc;
+    if (sb) {
+        SeqPrepArgs po{};
+        po.x = w.x; po.ln_w = m->lnout_w; po.ln_b = m->lnout_b; po.T = 1; po.D = D; po.n_mix = 1; po.mode[0] = kPrepPair; po.pair[0] = w.d_pair;
+        rc = launch_seq_prep(po, B, s);
+        if (rc) return rc;
+        rc = launch_gemm_sb(&m->head, 1, &w.d_pair, B, &lg, V, RWKVQ_EPI_NONE, nullptr, nullptr, w.status, 0, s);
+        if (rc) return rc;
+    } else {
+        float* am_xo = batch_path(B) ? w.amax + 9 * B : nullptr;
+        const bool xo_h16 = am_xo && batch_fast();
+        launch_pdl(D <= 8 * kRowThreads ? ln_shift_mix_kernel<0, 8> : ln_shift_mix_kernel<0, kRowPer>, dim3(B), dim3(kRowThreads), 0, s, w.x, m->lnout_w,
+                   m->lnout_b, static_cast<float*>(nullptr), static_cast<const float*>(nullptr), w.xo, B, D, xo_h16 ? w.xo16 : static_cast<__half*>(nullptr),
+                   am_xo, 1, static_cast<float*>(nullptr), static_cast<float*>(nullptr));
+        rc = linear(&m->head, w.xo, B, D, lg, V, RWKVQ_EPI_NONE, nullptr, w.gscratch, w.gemm_ws, stream, xo_h16 ? w.xo16 : nullptr, am_xo, nullptr,
+                    w.status);
+        if (rc) return rc;
+    }
     if (next_tokens) {
         float* pv = w.argv;
         int* pi = reinterpret_cast<int*>(w.argv + static_cast<size_t>(B) * kArgSlices);

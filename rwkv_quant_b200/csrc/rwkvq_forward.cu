@@ -27,6 +27,7 @@ struct ForwardWs {
     float* scale;                      // [4][N] row scales of the r / k / v (or channel-mix) rows and of og
     float* hscale;                     // [N]
     __half *x16, *og16, *h16, *split, *hl, *w16, *lw16;
+    SbRows rkv_pair[3], d_pair, f_pair;      // operand rows of the tcgen05 pipeline (17 rows and more): r / k / v; og or xk; hffn
     void* head_ws;
     size_t head_ws_bytes;
 };
@@ -60,6 +61,15 @@ ForwardWs carve(const rwkvq_model& m, int B, int T, size_t n_tail, void* base) {
     if (N <= kSmallRows) {
         w.xs = f32(6 * N * D); w.hffn = f32(N * F); w.amax = f32(8 * N);
         w.lora_h = f32(4 * static_cast<size_t>(kSmallRows) * m.max_rank);
+        if (D % 256 == 0) {
+            auto pair = [&](size_t cols) {
+                float* un = f32(N);
+                return sb_rows(f16(sb_halves(static_cast<int>(N), static_cast<int>(cols))), un, static_cast<int>(N), static_cast<int>(cols));
+            };
+            for (int k = 0; k < 3; ++k) w.rkv_pair[k] = pair(D);
+            w.d_pair = pair(D);
+            w.f_pair = pair(F);
+        }
     } else {
         w.x16 = f16(3 * N * pitch16(D)); w.og16 = f16(N * pitch16(D)); w.h16 = f16(N * pitch16(F));
         w.split = f16(4 * N * 2 * D); w.hl = f16(4 * N * 2 * up64(m.max_rank));
@@ -228,19 +238,29 @@ int rwkvq_forward_seq(const rwkvq_model* m, int B, int T, const int64_t* tokens,
         a.x = w.x; a.ln_w = L.ln1_w; a.ln_b = L.ln1_b; a.shift_in = tshift_in[l]; a.mix = L.x_mix; a.shift_out = tshift_out[l];
         a.T = T; a.D = D; a.n_mix = 6;
         // mix rows: r, w, k, v, a, g
+        const bool sb = small && D % 256 == 0 && same_shape(L.Wr, L.Wk) && same_shape(L.Wr, L.Wv) && gemm_sb_pays(L.Wr, N) &&
+                        gemm_sb_pays(L.Wo, N) && gemm_sb_pays(L.Wfk, N) && gemm_sb_pays(L.Wfv, N);
         if (small) {
             for (int q = 0; q < 6; ++q) {
                 a.f32[q] = w.xs + q * ND; a.scale[q] = w.amax + q * N;
                 a.mode[q] = kPrepF32 | ((q == 0 || q == 2 || q == 3) ? kPrepAmax : 0);
             }
-            a.zero_a = am_og;
-            a.zero_b = am_h;
+            if (sb) {
+                const int lin[3] = {0, 2, 3};
+                for (int q = 0; q < 3; ++q) { a.pair[lin[q]] = w.rkv_pair[q]; a.mode[lin[q]] = kPrepPair | (q == 2 && !layer0 ? kPrepF32 : 0); }
+            } else {
+                a.zero_a = am_og;
+                a.zero_b = am_h;
+            }
             rc = launch_seq_prep(a, N, s);
             if (rc) return rc;
             const rwkvq_qtensor* t3[3] = {&L.Wr, &L.Wk, &L.Wv};
             const float* x3[3] = {w.xs, w.xs + 2 * ND, w.xs + 3 * ND};
             const float* a3[3] = {w.amax, w.amax + 2 * N, w.amax + 3 * N};
-            if (same_shape(L.Wr, L.Wk) && same_shape(L.Wr, L.Wv)) {
+            if (sb) {
+                const rwkvq_qtensor three[3] = {L.Wr, L.Wk, L.Wv};
+                rc = launch_gemm_sb(three, 3, w.rkv_pair, N, y3, D, RWKVQ_EPI_NONE, nullptr, nullptr, w.status, 0, s);
+            } else if (same_shape(L.Wr, L.Wk) && same_shape(L.Wr, L.Wv)) {
                 rc = small_linear(t3, 3, x3, a3, N, D, y3, D, RWKVQ_EPI_NONE, nullptr, nullptr, s);
             } else {
                 for (int q = 0; q < 3 && !rc; ++q) rc = small_linear(t3 + q, 1, x3 + q, a3 + q, N, D, y3 + q, D, RWKVQ_EPI_NONE, nullptr, nullptr, s);
@@ -282,13 +302,31 @@ int rwkvq_forward_seq(const rwkvq_model* m, int B, int T, const int64_t* tokens,
             if (rc) return rc;
             rc = rwkvq_wkv7(r, dw, k2, v2, na, nb, wkv_in[l], w.out, wkv_out[l], B, T, H, 64, stream);
             if (rc) return rc;
-            rc = launch_wkv_tail(w.out, r, k2, v2, L.r_k, L.lnx_w, L.lnx_b, yg, w.og, N, H, 64e-5f, am_og, s);
+            rc = launch_wkv_tail(w.out, r, k2, v2, L.r_k, L.lnx_w, L.lnx_b, yg, w.og, N, H, 64e-5f, sb ? nullptr : am_og, s);
             if (rc) return rc;
         }
         // ---- output projection, channel mix
         SeqPrepArgs c{};
         c.x = w.x; c.ln_w = L.ln2_w; c.ln_b = L.ln2_b; c.shift_in = cshift_in[l]; c.mix = L.ffn_x_k; c.shift_out = cshift_out[l];
         c.T = T; c.D = D; c.n_mix = 1;
+        if (sb) {
+            const float* res[1] = {w.x};
+            float *yx[1] = {w.x}, *yh[1] = {w.hffn};
+            rc = launch_split_rows(w.og, D, D, N, w.d_pair, nullptr, s);
+            if (rc) return rc;
+            rc = launch_gemm_sb(&L.Wo, 1, &w.d_pair, N, yx, D, RWKVQ_EPI_ADD, res, nullptr, w.status, 0, s);
+            if (rc) return rc;
+            c.mode[0] = kPrepPair; c.pair[0] = w.d_pair;
+            rc = launch_seq_prep(c, N, s);
+            if (rc) return rc;
+            rc = launch_gemm_sb(&L.Wfk, 1, &w.d_pair, N, yh, F, RWKVQ_EPI_RELU2, nullptr, nullptr, w.status, 0, s);
+            if (rc) return rc;
+            rc = launch_split_rows(w.hffn, F, F, N, w.f_pair, nullptr, s);
+            if (rc) return rc;
+            rc = launch_gemm_sb(&L.Wfv, 1, &w.f_pair, N, yx, D, RWKVQ_EPI_ADD, res, nullptr, w.status, 0, s);
+            if (rc) return rc;
+            continue;
+        }
         if (small) {
             const rwkvq_qtensor *to[1] = {&L.Wo}, *tk[1] = {&L.Wfk}, *tv[1] = {&L.Wfv};
             const float *xo[1] = {w.og}, *ao[1] = {am_og}, *xk[1] = {w.xs}, *ak[1] = {w.amax}, *xv[1] = {w.hffn}, *av[1] = {am_h};

@@ -11,9 +11,11 @@
 //
 // A CTA owns 128 rows and a K slice (cluster of ks CTAs along K, reduced through distributed shared memory in rank
 // order) and is a pipeline over stages of 64 columns:
-//   warps 0-15   weights: packed bytes arrive by cp.async in per-thread slots, up to six stages ahead, so that the HBM
-//                latency of a dependent launch is paid once; two groups of 8 warps take the stages in turn (one
-//                group: 1 us a stage whatever the batch), one item of 32 weights per thread and stage
+//   warps 0-15   weights, four groups of 128 threads: group g takes stage g of every super-block, a thread one row's 64
+//                columns.  Packed bytes arrive by cp.async in per-thread slots, 8 to 12 stages ahead, so that the HBM
+//                latency of a dependent launch is paid once; p and e go to tensor memory (the A operand of the MMA:
+//                lane = row), so that shared memory carries the activations only (with p and e in shared memory
+//                their stores and the MMAs' reads bound a stage at 0.52 us for 16 tokens, 0.58 for 64, 0.80 for 128)
 //   warp 16      TMA of the activation pairs, which split_rows_kernel or the LayerNorm kernels have made once (converting
 //                in every CTA cost 8 more warps and 0.8 us a stage at 64 tokens)
 //   warp 17      MMAs, the loop run by the whole warp so that descriptors stay in uniform registers (one lane
@@ -35,11 +37,11 @@ namespace cg = cooperative_groups;
 
 namespace rwkvq {
 
-constexpr int kSbGroup = 256;                     // weight threads of one stage; two groups take the stages in turn
-constexpr int kSbWeightThreads = 2 * kSbGroup, kSbThreads = kSbWeightThreads + 64;
+constexpr int kSbGroups = 4;                      // = stages of a super-block
+constexpr int kSbWeightThreads = kSbGroups * kGmRows, kSbThreads = kSbWeightThreads + 64;
 constexpr int kSbTmaWarp = kSbWeightThreads / 32, kSbMmaWarp = kSbTmaWarp + 1;
-constexpr int kSbAhead = 3;                       // stages of packed weights a group has in flight
-constexpr int kSbSlab = kGmRows * 128;            // 128 rows x 64 columns of fp16
+constexpr int kSbACols = 64;                      // tensor-memory columns of a stage: p 32, e 32
+constexpr uint32_t kSbTmemCols = 512;
 constexpr int kSbPitch = kGmRows + 4;             // partial tile [NT][kSbPitch]
 constexpr int kSbMaxMats = 4;
 
@@ -63,28 +65,48 @@ struct SbMaps { CUtensorMap hi[kSbMaxMats], lo[kSbMaxMats]; };
 template <int L>
 struct SbLayout {
     static constexpr bool SB6 = L <= ML_SB6_6;
-    static constexpr int CODE_BYTES = L == ML_SYM8 ? 32 : 16;
+    static constexpr int CODE_BYTES = L == ML_SYM8 ? 64 : 32;                      // of a row's stage
     static constexpr int PLANES = L == ML_SB6_5 ? 1 : (L == ML_SB6_6 || L == ML_SYM6) ? 2 : 0;
-    static constexpr int RAW = kSbGroup * (CODE_BYTES + 4 * PLANES);               // bytes of one stage
+    // one stage in shared memory: codes and the scale record as planes of 16 bytes a row, bit planes 8 bytes a row
+    static constexpr int RAW = kGmRows * (CODE_BYTES + 16 + 8 * PLANES);
 };
 
 template <int L, int NT>
 struct SbGeo {
-    static constexpr int ST = NT > 64 ? 2 : 3;                       // operand buffers
+    // Operand buffers: as many as groups, so that a group waits for a buffer it filled itself.  (With three, a group that
+    // ran ahead waited for a phase two ahead of the barrier's, which a parity wait takes for the one just past.)
+    static constexpr int ST = kSbGroups;
+    static constexpr int AHEAD = NT > 64 ? 2 : 3;                    // stages of packed weights a group has in flight
     static constexpr int BSLAB = 2 * NT * 128;
     static constexpr int MA = SbLayout<L>::SB6 ? kGmRows * 32 : 0, MB = SbLayout<L>::SB6 ? 2 * NT * 32 : 0;     // min operands of a super-block
-    static constexpr int OFF_E = ST * kSbSlab, OFF_B = 2 * ST * kSbSlab, OFF_MA = OFF_B + ST * BSLAB, OFF_MB = OFF_MA + 2 * MA,
-                         OFF_RAW = OFF_MB + 2 * MB, OFF_REC = OFF_RAW + 2 * kSbAhead * SbLayout<L>::RAW, SMEM = OFF_REC + 2 * 3 * kGmRows * 16;
-    static constexpr size_t BYTES = SMEM + 1024;
-    static_assert(NT * kSbPitch * 4 <= OFF_MA, "partial tile over the operands");
+    static constexpr int PART = NT * kSbPitch * 4;                   // partial tile of a K slice, over the operands
+    static constexpr int OFF_MA = ST * BSLAB, OFF_MB = OFF_MA + 2 * MA, OFF_RAW = OFF_MB + 2 * MB,
+                         SMEM = OFF_RAW + kSbGroups * AHEAD * SbLayout<L>::RAW;
+    // one CTA per SM: two could wait for each other's tensor memory inside a cluster
+    static constexpr size_t BYTES = (SMEM > 119 * 1024 ? SMEM : 119 * 1024) + 1024;
+    static_assert(PART <= SMEM, "partial tile");
+    static_assert(2 * NT + ST * kSbACols <= static_cast<int>(kSbTmemCols), "tensor memory");
     static_assert(BYTES <= 226 * 1024, "shared memory");
 };
 
-__device__ __forceinline__ void sb_cp16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+// through L1: the groups read different parts of the same sectors
+template <int BYTES>
+__device__ __forceinline__ void sb_cp(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_addr(dst)), "l"(src), "n"(BYTES) : "memory");
 }
-__device__ __forceinline__ void sb_cp4(void* dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+__device__ __forceinline__ void sb_tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
+                 "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
+                 "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+                 : "memory");
+}
+// A from tensor memory (lane = row, a 32-bit column = two consecutive k)
+__device__ __forceinline__ void umma_f16_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}" ::"r"(d_tmem),
+        "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
 }
 template <int NC>
 __device__ __forceinline__ void sb_tmem_ld(uint32_t taddr, float (&v)[NC]) {
@@ -107,11 +129,11 @@ __device__ __forceinline__ void sb_tmem_ld(uint32_t taddr, float (&v)[NC]) {
     for (int i = 0; i < NC; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// 32 weights of row r, item `it` of its super-block: codes * scale as product and rounding error into the two
-// operand slabs; returns the block's min (fp16 by the codec's definition; zero for sym).  decode_item with the layout
+// The 32 weights of item `it` of a super-block: codes * scale as product pw and rounding error ew, two per word in
+// column order; returns the block's min (fp16 by the codec's definition; zero for sym).  decode_item with the layout
 // known at compile time.
 template <int L>
-__device__ __forceinline__ __half sb_convert(const Packed& p, bool in_rec, int r, int it, int half, unsigned char* p_slab, unsigned char* e_slab) {
+__device__ __forceinline__ __half sb_convert(const Packed& p, bool in_rec, int it, int half, uint32_t (&pw)[16], uint32_t (&ew)[16]) {
     uint32_t bytes[8];
     __half2 s2[2], m2 = __float2half2_rn(0.f), bias;
     const uint32_t w[4] = {p.c0.x, p.c0.y, p.c0.z, p.c0.w};
@@ -166,13 +188,11 @@ __device__ __forceinline__ __half sb_convert(const Packed& p, bool in_rec, int r
         }
     }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        uint2 pa, ea, pb, eb;
-        bytes_to_half4_pair(bytes[2 * j], bias, s2[j >> 1], pa, ea);
-        bytes_to_half4_pair(bytes[2 * j + 1], bias, s2[j >> 1], pb, eb);
-        const uint32_t off = sw128_offset(r, 4 * half + j);
-        *reinterpret_cast<uint4*>(p_slab + off) = make_uint4(pa.x, pa.y, pb.x, pb.y);
-        *reinterpret_cast<uint4*>(e_slab + off) = make_uint4(ea.x, ea.y, eb.x, eb.y);
+    for (int j = 0; j < 8; ++j) {
+        uint2 pa, ea;
+        bytes_to_half4_pair(bytes[j], bias, s2[j >> 2], pa, ea);
+        pw[2 * j] = pa.x; pw[2 * j + 1] = pa.y;
+        ew[2 * j] = ea.x; ew[2 * j + 1] = ea.y;
     }
     return __low2half(m2);
 }
@@ -183,7 +203,7 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
     using Y = SbLayout<L>;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    // the operands of a stage are complete (8 weight warps + the TMA bytes) / have been multiplied.  A super-block's min
+    // the operands of a stage are complete (4 weight warps + the TMA bytes) / have been multiplied.  A super-block's min
     // operands are part of its stages: mins with the weights of each, block sums with the activations of the first.
     // Two buffers of them need no barrier of their own: the stage that writes buffer s % 2 again has waited for a stage
     // behind the MMA that read it.
@@ -196,33 +216,32 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
     const int n0 = blockIdx.y * NT, nn = min(NT, a.n_tokens - n0);
     const int sb0 = a.n_sb * z / ks, n_super = a.n_sb * (z + 1) / ks - sb0, n_stages = n_super * 4;     // this CTA's K slice
     const int n_my = (a.n_tiles - first_tile + tile_step - 1) / tile_step;
-    constexpr uint32_t COLS = 2 * NT;
 
     if (tid == 0) {
-        for (int s = 0; s < G::ST; ++s) { mbar_init(&bar_full[s], kSbGroup / 32 + 1); mbar_init(&bar_empty[s], 1); }
+        for (int s = 0; s < G::ST; ++s) { mbar_init(&bar_full[s], kGmRows / 32 + 1); mbar_init(&bar_empty[s], 1); }
         mbar_init(&bar_done, 1);
         s_fail = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     pdl_launch_dependents();
-    if (warp == kSbMmaWarp) tmem_alloc(&s_tmem, COLS);
+    if (warp == kSbMmaWarp) tmem_alloc(&s_tmem, kSbTmemCols);
     if (Y::SB6) {                                                    // K 8-15 of the min operands and the rows beyond nn stay zero
         for (int i = tid; i < 2 * (G::MA + G::MB) / 16; i += kSbThreads) reinterpret_cast<uint4*>(smem + G::OFF_MA)[i] = make_uint4(0, 0, 0, 0);
         fence_async_smem();
     }
 
-    // ---- weight threads: group grp takes stages grp, grp + 2, ..; item = (row wt / 2, 32-column block wt & 1 of the stage)
-    const int grp = tid / kSbGroup, wt = tid % kSbGroup, wrow = wt >> 1, wblk = wt & 1;
-    unsigned char* raw = smem + G::OFF_RAW + grp * kSbAhead * Y::RAW;
-    unsigned char* recs = smem + G::OFF_REC + grp * 3 * kGmRows * 16;
-    int c_ti = 0, c_st = grp, c_slot = 0, c_rec = 0;                 // copy side: tile of this CTA, stage in it, ring positions
+    // ---- weight threads: group grp takes stage grp of every super-block, thread wrow its row
+    const int grp = tid / kGmRows, wrow = tid % kGmRows;
+    unsigned char* raw = smem + G::OFF_RAW + (grp % kSbGroups) * G::AHEAD * Y::RAW;
+    constexpr int OFF_R = kGmRows * Y::CODE_BYTES, OFF_H = OFF_R + kGmRows * 16, OFF_H2 = OFF_H + kGmRows * 8;
+    int c_ti = 0, c_sb = 0, c_slot = 0;                              // copy side: tile of this CTA, super-block, ring slot
     const uint8_t *c_codes = nullptr, *c_h = nullptr, *c_h2 = nullptr, *c_meta = nullptr;
     bool c_long = true;                                              // a 16-byte record (else the 12 bytes of the file)
-    auto copy_tile = [&]() {                                         // source pointers of tile c_ti at stage grp
+    auto copy_tile = [&]() {                                         // source pointers of tile c_ti
         const int tile = first_tile + c_ti * tile_step;
         const QView& t = a.t[tile / a.row_tiles];
         const size_t R = static_cast<size_t>(min((tile % a.row_tiles) * kGmRows + wrow, t.rows - 1));
-        const int col = sb0 * 256 + grp * 64 + wblk * 32;
+        const int col = sb0 * 256 + grp * 64;
         c_codes = t.codes + (L == ML_SYM8 ? R * t.cols + col : R * (t.cols >> 1) + (col >> 1));
         if (Y::PLANES >= 1) c_h = t.qh + R * (t.cols >> 3) + (col >> 3);
         if (Y::PLANES == 2) c_h2 = t.qh2 + R * (t.cols >> 3) + (col >> 3);
@@ -233,26 +252,22 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
     auto copy_stage = [&]() {
         if (c_ti < n_my) {
             unsigned char* slot = raw + c_slot * Y::RAW;
-            sb_cp16(slot + wt * 16, c_codes);
-            if (L == ML_SYM8) sb_cp16(slot + kSbGroup * 16 + wt * 16, c_codes + 16);
-            if (Y::PLANES >= 1) sb_cp4(slot + kSbGroup * Y::CODE_BYTES + wt * 4, c_h);
-            if (Y::PLANES == 2) sb_cp4(slot + kSbGroup * (Y::CODE_BYTES + 4) + wt * 4, c_h2);
-            if ((c_st & 2) == 0) {                                   // the row's scale record, once per super-block (2 stages of this group)
-                if (wblk == 0) {
-                    unsigned char* rec = recs + c_rec * (kGmRows * 16) + wrow * 16;
-                    if (c_long) sb_cp16(rec, c_meta);
-                    else { sb_cp4(rec, c_meta); sb_cp4(rec + 4, c_meta + 4); sb_cp4(rec + 8, c_meta + 8); }
-                }
-                c_meta += c_long ? 16 : 12;
-                c_rec = c_rec == 2 ? 0 : c_rec + 1;
+#pragma unroll
+            for (int k = 0; k < Y::CODE_BYTES / 16; ++k) sb_cp<16>(slot + k * (kGmRows * 16) + wrow * 16, c_codes + 16 * k);
+            if (c_long) sb_cp<16>(slot + OFF_R + wrow * 16, c_meta);
+            else {
+#pragma unroll
+                for (int k = 0; k < 3; ++k) sb_cp<4>(slot + OFF_R + wrow * 16 + 4 * k, c_meta + 4 * k);
             }
-            c_codes += 2 * (L == ML_SYM8 ? 64 : 32);
-            if (Y::PLANES >= 1) c_h += 16;
-            if (Y::PLANES == 2) c_h2 += 16;
-            c_slot = c_slot == kSbAhead - 1 ? 0 : c_slot + 1;
-            c_st += 2;
-            if (c_st >= n_stages) {
-                c_st = grp;
+            if (Y::PLANES >= 1) sb_cp<8>(slot + OFF_H + wrow * 8, c_h);
+            if (Y::PLANES == 2) sb_cp<8>(slot + OFF_H2 + wrow * 8, c_h2);
+            c_codes += L == ML_SYM8 ? 256 : 128;
+            c_meta += c_long ? 16 : 12;
+            if (Y::PLANES >= 1) c_h += 32;
+            if (Y::PLANES == 2) c_h2 += 32;
+            c_slot = c_slot == G::AHEAD - 1 ? 0 : c_slot + 1;
+            if (++c_sb == n_super) {
+                c_sb = 0;
                 if (++c_ti < n_my) copy_tile();
             }
         }
@@ -260,7 +275,7 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
     };
     if (tid < kSbWeightThreads) {                                    // weights do not depend on the producer of x
         copy_tile();
-        for (int i = 0; i < kSbAhead; ++i) copy_stage();
+        for (int i = 0; i < G::AHEAD; ++i) copy_stage();
     }
     tc_fence_before();
     __syncthreads();
@@ -268,7 +283,7 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
     const uint32_t tmem = s_tmem;
     if (warp == kSbTmaWarp) pdl_wait();                              // the activations; the others wait before they read or store
 
-    int r_slot = 0, r_rec = 0;                                       // read side of the rings
+    int r_slot = 0;                                                  // read side of the weight ring
     int it = 0;                                                      // stages of the tiles before
     uint32_t done_phase = 0;
     for (int ti = 0; ti < n_my; ++ti) {
@@ -276,8 +291,8 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
         const QView& t = a.t[mat];
         if (warp == kSbMmaWarp) {
             // ------------------------------------------------------------------ MMA issuer (whole warp, one lane elected)
-            const uint32_t id = umma_idesc(2 * NT);
-            const uint64_t p0 = umma_desc(smem_addr(smem)), e0 = umma_desc(smem_addr(smem + G::OFF_E)), b0 = umma_desc(smem_addr(smem + G::OFF_B));
+            const uint32_t id2 = umma_idesc(2 * NT), id1 = umma_idesc(NT);
+            const uint64_t b0 = umma_desc(smem_addr(smem));
             const uint64_t ma0 = umma_desc_plain(smem_addr(smem + G::OFF_MA), kGmRows * 16, 128);
             const uint64_t mb0 = umma_desc_plain(smem_addr(smem + G::OFF_MB), 2 * NT * 16, 128);
             uint32_t elected;
@@ -287,17 +302,17 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
             for (int i = 0; i < n_stages; ++i) {
                 if (!mbar_wait_bounded(&bar_full[st], ph)) { ok = false; break; }
                 tc_fence_after();
-                const uint64_t pd = p0 + (static_cast<uint64_t>(st * kSbSlab) >> 4), ed = e0 + (static_cast<uint64_t>(st * kSbSlab) >> 4);
+                const uint32_t pa = tmem + 2 * NT + st * kSbACols, ea = pa + kSbACols / 2;
                 const uint64_t bd = b0 + (static_cast<uint64_t>(st * G::BSLAB) >> 4);
                 if (elected) {
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {                    // small terms first
-                        umma_f16(tmem, ed + 2 * k, bd + 2 * k, id, (i | k) ? 1u : 0u);
-                        umma_f16(tmem, pd + 2 * k, bd + 2 * k, id, 1u);
+                    for (int k = 0; k < 4; ++k) {                    // e meets the high halves only (e lo is below 2^-22)
+                        umma_f16_ta(tmem, pa + 8 * k, bd + 2 * k, id2, (i | k) ? 1u : 0u);
+                        umma_f16_ta(tmem, ea + 8 * k, bd + 2 * k, id1, 1u);
                     }
                     if (Y::SB6 && (i & 3) == 3) {                    // the super-block's mins are complete with its last stage
                         const int ms = ((it + i) >> 2) & 1;
-                        umma_f16(tmem, ma0 + (static_cast<uint64_t>(ms * G::MA) >> 4), mb0 + (static_cast<uint64_t>(ms * G::MB) >> 4), id, 1u);
+                        umma_f16(tmem, ma0 + (static_cast<uint64_t>(ms * G::MA) >> 4), mb0 + (static_cast<uint64_t>(ms * G::MB) >> 4), id2, 1u);
                     }
                     umma_commit(&bar_empty[st]);
                 }
@@ -312,7 +327,7 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
                 for (int i = 0; i < n_stages; ++i) {
                     const int g = it + i, st = g % G::ST;
                     if (g >= G::ST && !mbar_wait_bounded(&bar_empty[st], (g / G::ST - 1) & 1)) { s_fail = 1; break; }
-                    unsigned char* b = smem + G::OFF_B + st * G::BSLAB;
+                    unsigned char* b = smem + st * G::BSLAB;
                     const bool with_sums = Y::SB6 && (i & 3) == 0;
                     mbar_expect_tx(&bar_full[st], G::BSLAB + (with_sums ? 2 * nn * 16 : 0));
                     tma_load_2d(b, &maps.hi[mat], sb0 * 256 + i * 64, n0, &bar_full[st]);
@@ -342,39 +357,60 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
                 if (Y::SB6) dd_next |= static_cast<uint32_t>(__half_as_ushort(__ldg(t.dm + drow + sb))) << 16;
             };
             load_d(0);
+            const uint32_t lane_base = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + 2 * NT;
 #pragma unroll 1
-            for (int i = grp; i < n_stages; i += 2) {
-                const int g = it + i, st = g % G::ST;
-                asm volatile("cp.async.wait_group %0;" ::"n"(kSbAhead - 1) : "memory");
-                __syncwarp();                                        // the pair lane's record
+            for (int sb = 0; sb < n_super; ++sb) {
+                const int g = it + 4 * sb + grp, st = g % G::ST;
+                asm volatile("cp.async.wait_group %0;" ::"n"(G::AHEAD - 1) : "memory");
                 const unsigned char* slot = raw + r_slot * Y::RAW;
-                Packed p{};
-                p.c0 = *reinterpret_cast<const uint4*>(slot + wt * 16);
-                if (L == ML_SYM8) p.c1 = *reinterpret_cast<const uint4*>(slot + kSbGroup * 16 + wt * 16);
-                if (Y::PLANES >= 1) p.h = *reinterpret_cast<const uint32_t*>(slot + kSbGroup * Y::CODE_BYTES + wt * 4);
-                if (Y::PLANES == 2) p.h2 = *reinterpret_cast<const uint32_t*>(slot + kSbGroup * (Y::CODE_BYTES + 4) + wt * 4);
-                const int item = (i & 3) * 2 + wblk;                 // of the super-block
-                const unsigned char* rec = recs + r_rec * (kGmRows * 16) + wrow * 16;
-                r_slot = r_slot == kSbAhead - 1 ? 0 : r_slot + 1;
-                if (i & 2) r_rec = r_rec == 2 ? 0 : r_rec + 1;
-                if ((i & 2) == 0) { dd = dd_next; load_d((i >> 2) + 1); }
+                r_slot = r_slot == G::AHEAD - 1 ? 0 : r_slot + 1;
+                Packed p[2];
+                uint2 h = make_uint2(0, 0), h2 = h;
+                if (Y::PLANES >= 1) h = *reinterpret_cast<const uint2*>(slot + OFF_H + wrow * 8);
+                if (Y::PLANES == 2) h2 = *reinterpret_cast<const uint2*>(slot + OFF_H2 + wrow * 8);
+                uint4 rec = *reinterpret_cast<const uint4*>(slot + OFF_R + wrow * 16);
+                dd = dd_next;
+                load_d(sb + 1);
                 if (Y::SB6) {
-                    p.rec = *reinterpret_cast<const uint4*>(rec);
-                    if (!in_rec) p.rec.w = dd;
-                } else {
-                    p.rec.x = *reinterpret_cast<const unsigned short*>(rec + item * 2);
-                    p.rec.y = dd;
+                    if (!in_rec) rec.w = dd;
+                } else {                                             // the two scale codes of each block of this stage
+                    const uint32_t w = (grp & 2) ? ((grp & 1) ? rec.w : rec.z) : ((grp & 1) ? rec.y : rec.x);
+                    rec = make_uint4(w, dd, 0, 0);
+                }
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                    constexpr int CB = Y::CODE_BYTES / 32;           // 16-byte pieces of an item
+                    p[b].c0 = *reinterpret_cast<const uint4*>(slot + (CB * b) * (kGmRows * 16) + wrow * 16);
+                    if (L == ML_SYM8) p[b].c1 = *reinterpret_cast<const uint4*>(slot + (CB * b + 1) * (kGmRows * 16) + wrow * 16);
+                    p[b].h = b ? h.y : h.x;
+                    p[b].h2 = b ? h2.y : h2.x;
+                    p[b].rec = rec;
+                    if (!Y::SB6 && b) p[b].rec.x = rec.x >> 16;
                 }
                 if (g >= G::ST) {                                    // the MMAs that read this buffer have completed
                     if (lane == 0 && !s_fail && !mbar_wait_bounded(&bar_empty[st], (g / G::ST - 1) & 1)) s_fail = 1;
                     __syncwarp();
+                    tc_fence_after();
                 }
-                const __half mn = sb_convert<L>(p, in_rec, wrow, item, wblk, smem + st * kSbSlab, smem + G::OFF_E + st * kSbSlab);
-                if (Y::SB6) reinterpret_cast<__half*>(smem + G::OFF_MA + ((g >> 2) & 1) * G::MA + wrow * 16)[item] = mn;
-                fence_async_smem();
+                const uint32_t ta = lane_base + st * kSbACols;
+                __half mn[2];
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                    uint32_t pw[16], ew[16];
+                    mn[b] = sb_convert<L>(p[b], in_rec, 2 * grp + b, b, pw, ew);
+                    sb_tmem_st16(ta + 16 * b, pw);
+                    sb_tmem_st16(ta + kSbACols / 2 + 16 * b, ew);
+                }
+                if (Y::SB6) {
+                    const __half2 m2 = __halves2half2(mn[0], mn[1]);
+                    *reinterpret_cast<__half2*>(smem + G::OFF_MA + ((g >> 2) & 1) * G::MA + wrow * 16 + grp * 4) = m2;
+                    fence_async_smem();
+                }
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&bar_full[st]);
-                copy_stage();                                        // every lane of the warp has read its slot
+                copy_stage();
             }
         }
         it += n_stages;
@@ -460,7 +496,7 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
     __syncthreads();
     if (tid == 0 && s_fail) atomicCAS(a.status, 0, RWKVQ_E_TIMEOUT);
     tc_fence_after();
-    if (warp == kSbMmaWarp) tmem_dealloc(tmem, COLS);
+    if (warp == kSbMmaWarp) tmem_dealloc(tmem, kSbTmemCols);
 }
 
 // fp32 rows -> pairs, one CTA per row.  Bound: latency (a load, a block maximum, the stores); rows of up to 8192 columns
@@ -521,16 +557,53 @@ int sb_layout_of(const rwkvq_qtensor& t) {
     return t.bits == 8 ? ML_SYM8 : ML_SYM6;
 }
 
+// Clusters of c CTAs the device holds at once (one CTA per SM): whole clusters of a GPC, e.g. 16 of 6 but not of 7.
 template <int L, int NT>
-int launch_sb(SbArgs& a, const SbMaps& maps, int groups, cudaStream_t s) {
+int resident_clusters(int dev, int c) {
+    static int known[64][9] = {};
+    if (dev < 64 && known[dev][c] > 0) return known[dev][c];
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(c);
+    cfg.blockDim = dim3(kSbThreads);
+    cfg.dynamicSmemBytes = SbGeo<L, NT>::BYTES;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = c; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, gemm_sb_kernel<L, NT>, &cfg) != cudaSuccess || n < 1) {
+        cudaGetLastError();
+        n = std::max(1, 96 / c);
+    }
+    if (dev < 64) known[dev][c] = n;
+    return n;
+}
+
+template <int L, int NT>
+int launch_sb(SbArgs& a, const SbMaps& maps, int groups, int force_ks, cudaStream_t s) {
     static bool configured[64] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) dev = 0;
     if (dev >= 64 || !configured[dev]) {
         cudaError_t e = cudaFuncSetAttribute(gemm_sb_kernel<L, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(SbGeo<L, NT>::BYTES));
         if (e != cudaSuccess) return fail(RWKVQ_E_LIMIT, "gemm_sb: %zu bytes of shared memory: %s", SbGeo<L, NT>::BYTES, cudaGetErrorString(e));
+        for (int c = 2; c <= 8; ++c) resident_clusters<L, NT>(dev, c);
         if (dev < 64) configured[dev] = true;
     }
+    // K split into up to 8 slices of whole super-blocks, by a model of the slowest CTA in microseconds fitted to
+    // [2048, 2048] .. [65536, 2048] at 8 to 100 rows: 0.36 to 0.55 a stage, 5 for ramp and store, 3.5 for the cluster
+    // reduction; without a split the CTAs are persistent and pay the ramp once
+    const double stage = NT > 64 ? 0.55 : NT > 32 ? 0.41 : 0.37;
+    double best = 1e300;
+    a.ks = 1;
+    for (int c = 1; c <= 8 && c <= a.n_sb; ++c) {
+        const int fit = c == 1 ? 148 : resident_clusters<L, NT>(dev, c);
+        const double waves = static_cast<double>((a.n_tiles * groups + fit - 1) / fit), work = ((a.n_sb + c - 1) / c) * 4 * stage;
+        const double t = c == 1 ? waves * (work + 1.5) + 4.0 : waves * (work + 5.0) + 3.5;
+        if (t < best) { best = t; a.ks = c; }
+    }
+    if (force_ks > 0 && force_ks <= 8 && force_ks <= a.n_sb) a.ks = force_ks;
     cudaLaunchConfig_t cfg{};
     // one wave of persistent CTAs where K is not split
     cfg.gridDim = dim3(a.ks > 1 ? a.n_tiles * a.ks : std::min(a.n_tiles, std::max(1, 148 / groups)), groups);
@@ -550,12 +623,12 @@ int launch_sb(SbArgs& a, const SbMaps& maps, int groups, cudaStream_t s) {
 }
 
 template <int L>
-int launch_sb_nt(SbArgs& a, const SbMaps& maps, int nt, int groups, cudaStream_t s) {
+int launch_sb_nt(SbArgs& a, const SbMaps& maps, int nt, int groups, int force_ks, cudaStream_t s) {
     switch (nt) {
-        case 16: return launch_sb<L, 16>(a, maps, groups, s);
-        case 32: return launch_sb<L, 32>(a, maps, groups, s);
-        case 64: return launch_sb<L, 64>(a, maps, groups, s);
-        default: return launch_sb<L, 128>(a, maps, groups, s);
+        case 16: return launch_sb<L, 16>(a, maps, groups, force_ks, s);
+        case 32: return launch_sb<L, 32>(a, maps, groups, force_ks, s);
+        case 64: return launch_sb<L, 64>(a, maps, groups, force_ks, s);
+        default: return launch_sb<L, 128>(a, maps, groups, force_ks, s);
     }
 }
 
@@ -591,23 +664,12 @@ int launch_gemm_sb(const rwkvq_qtensor* ts, int n_mats, const SbRows* rows, int 
     a.row_tiles = (ts[0].rows + kGmRows - 1) / kGmRows;
     a.n_tiles = a.row_tiles * n_mats;
     a.n_sb = ts[0].cols / 256;
-    // K split into up to 8 slices of whole super-blocks: modelled cycles of the slowest SM = waves of CTAs (one per SM) x
-    // (ramp + stages) + the cluster reduction; without a split the CTAs are persistent and pay the ramp once
-    const double stage = nt == 128 ? 1150.0 : nt == 64 ? 850.0 : 800.0;
-    double best = 1e300;
-    a.ks = 1;
-    for (int c = 1; c <= 8 && c <= a.n_sb; ++c) {
-        const double waves = static_cast<double>((a.n_tiles * groups * c + 147) / 148), work = ((a.n_sb + c - 1) / c) * 4 * stage;
-        const double t = c == 1 ? waves * (work + 2000.0) + 4000.0 : waves * (work + 4000.0) + 3500.0 + 150.0 * c;
-        if (t < best) { best = t; a.ks = c; }
-    }
-    if (force_ks > 0 && force_ks <= 8 && force_ks <= a.n_sb) a.ks = force_ks;
     switch (sb_layout_of(ts[0])) {
-        case ML_SB6_4: return launch_sb_nt<ML_SB6_4>(a, maps, nt, groups, s);
-        case ML_SB6_5: return launch_sb_nt<ML_SB6_5>(a, maps, nt, groups, s);
-        case ML_SB6_6: return launch_sb_nt<ML_SB6_6>(a, maps, nt, groups, s);
-        case ML_SYM6: return launch_sb_nt<ML_SYM6>(a, maps, nt, groups, s);
-        default: return launch_sb_nt<ML_SYM8>(a, maps, nt, groups, s);
+        case ML_SB6_4: return launch_sb_nt<ML_SB6_4>(a, maps, nt, groups, force_ks, s);
+        case ML_SB6_5: return launch_sb_nt<ML_SB6_5>(a, maps, nt, groups, force_ks, s);
+        case ML_SB6_6: return launch_sb_nt<ML_SB6_6>(a, maps, nt, groups, force_ks, s);
+        case ML_SYM6: return launch_sb_nt<ML_SYM6>(a, maps, nt, groups, force_ks, s);
+        default: return launch_sb_nt<ML_SYM8>(a, maps, nt, groups, force_ks, s);
     }
 }
 

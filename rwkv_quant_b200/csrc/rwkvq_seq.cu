@@ -270,6 +270,9 @@ __device__ __forceinline__ void prep_emit8(const SeqPrepArgs& a, int m, int mode
     }
 }
 
+// CLUSTER: the CTAs of a token's mixes form a cluster, so that the shift state can be updated in place: it is
+// written once all of them have read it.
+template <bool CLUSTER>
 __global__ void __launch_bounds__(kSeqVecWarps * 32) seq_prep_vec_kernel(const SeqPrepArgs a, long long n_tokens, int run) {
     __shared__ float red_s[kSeqVecWarps], red_q[kSeqVecWarps];
     __shared__ float2 red_m[kSeqVecWarps];
@@ -279,8 +282,12 @@ __global__ void __launch_bounds__(kSeqVecWarps * 32) seq_prep_vec_kernel(const S
     float lw[8], lb[8], mx[8];
     prep_load8(a.ln_w + d0, lw);
     prep_load8(a.ln_b + d0, lb);
-    prep_load8(a.mix + static_cast<size_t>(m) * D + d0, mx);
-    const bool want_n2 = a.n2 != nullptr && m == 0, want_max = (mode & (kPrepScaled | kPrepAmax)) != 0;
+    if (a.mix != nullptr) prep_load8(a.mix + static_cast<size_t>(m) * D + d0, mx);
+    else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) mx[i] = 0.f;
+    }
+    const bool want_n2 = a.n2 != nullptr && m == 0, want_max = (mode & (kPrepScaled | kPrepAmax | kPrepPair)) != 0;
     pdl_launch_dependents();
     pdl_wait();
     if (m == 0)
@@ -321,14 +328,16 @@ __global__ void __launch_bounds__(kSeqVecWarps * 32) seq_prep_vec_kernel(const S
         for (int i = 0; i < 8; ++i) v[i] = nx[i];
         if (tok + 1 < tok1) prep_load8cg(a.x + (tok + 1) * D + d0, nx);
         if (t == 0) {
-            if (a.shift_in) prep_load8(a.shift_in + static_cast<size_t>(b) * D + d0, pv);
+            if (a.shift_in) prep_load8cg(a.shift_in + static_cast<size_t>(b) * D + d0, pv);
             else {
 #pragma unroll
                 for (int i = 0; i < 8; ++i) pv[i] = 0.f;
             }
         }
+        if (CLUSTER) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
         normalise(v);
-        if (t == a.T - 1 && m == 0) prep_store8(a.shift_out + static_cast<size_t>(b) * D + d0, v);
+        if (CLUSTER) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (t == a.T - 1 && m == 0 && a.shift_out != nullptr) prep_store8(a.shift_out + static_cast<size_t>(b) * D + d0, v);
         float o[8], am = 0.f, n2 = 0.f;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
@@ -351,8 +360,16 @@ __global__ void __launch_bounds__(kSeqVecWarps * 32) seq_prep_vec_kernel(const S
             sc = prep_scale(am);
             if (tid == 0) {
                 if (want_n2) a.n2[tok] = n2;
-                if (want_max) a.scale[m][tok] = (mode & kPrepScaled) ? sc : am;
+                if (mode & (kPrepScaled | kPrepAmax)) a.scale[m][tok] = (mode & kPrepScaled) ? sc : am;
             }
+        }
+        if (mode & kPrepPair) {                          // the mode goes alone or with kPrepF32
+            float s1, u1, q[8];
+            sb_scale(am, s1, u1);
+            if (tid == 0) a.pair[m].unscale[tok] = u1;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) q[i] = o[i] * s1;
+            sb_store_pair(a.pair[m], static_cast<int>(tok), static_cast<int>(n_tokens), tid, q);
         }
         prep_emit8(a, m, mode, tok, d0, o, sc);
         if (++t == a.T) { t = 0; ++b; }
@@ -516,15 +533,33 @@ int launch_seq_prep(const SeqPrepArgs& a, long long n_tokens, cudaStream_t s) {
     bool vec = a.D % 256 == 0 && a.D <= kSeqVecWarps * 256 && aligned(a.x, 16) && aligned(a.ln_w, 16) && aligned(a.ln_b, 16) &&
                aligned(a.mix, 16) && aligned(a.shift_in, 16) && aligned(a.shift_out, 16);
     for (int m = 0; m < a.n_mix; ++m) vec = vec && aligned(a.x16[m], 16) && aligned(a.split[m], 16) && aligned(a.f32[m], 16);
-    // one wave of CTAs (two per SM) with a token and mix each, then groups of 64 threads per token
-    const bool few = n_tokens * a.n_mix <= 2 * 148;
+    bool pair = a.mix == nullptr;
+    for (int m = 0; m < a.n_mix; ++m) pair = pair || (a.mode[m] & kPrepPair) != 0;
+    const bool in_place = a.shift_out != nullptr && a.shift_in == a.shift_out;
+    RWKVQ_REQUIRE(vec || !(pair || in_place), RWKVQ_E_ALIGN, "seq_ln_shift_mix_prep: D %d, rows on 16-byte boundaries", a.D);
+    RWKVQ_REQUIRE(!in_place || a.T == 1, RWKVQ_E_SHAPE, "seq_ln_shift_mix_prep: the shift state in place needs T = 1");
+    // up to one wave of CTAs (two per SM) with a token and mix each, then groups of 64 threads per token
+    const bool few = n_tokens * a.n_mix <= 2 * 148 || pair || in_place;
     if (vec && !few && a.D == 2048) e = launch_prep_group<4>(a, n_tokens, s);
     else if (vec && !few && a.D == 2560) e = launch_prep_group<5>(a, n_tokens, s);
     else if (vec && !few && a.D == 1024) e = launch_prep_group<2>(a, n_tokens, s);
-    else if (vec) {
-        long long run = n_tokens * a.n_mix / (148 * 8);
+    else if (vec && in_place && a.n_mix > 1) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(static_cast<unsigned>(n_tokens), a.n_mix);
+        cfg.blockDim = dim3(a.D / 8);
+        cfg.stream = s;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = a.n_mix; attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = pdl_enabled() ? 2 : 1;
+        e = cudaLaunchKernelEx(&cfg, seq_prep_vec_kernel<true>, a, n_tokens, 1);
+    } else if (vec) {
+        long long run = in_place ? 1 : n_tokens * a.n_mix / (148 * 8);
         run = run < 1 ? 1 : run > 16 ? 16 : run;
-        e = launch_pdl(seq_prep_vec_kernel, dim3(static_cast<unsigned>((n_tokens + run - 1) / run), a.n_mix), dim3(a.D / 8), 0, s, a, n_tokens,
+        e = launch_pdl(seq_prep_vec_kernel<false>, dim3(static_cast<unsigned>((n_tokens + run - 1) / run), a.n_mix), dim3(a.D / 8), 0, s, a, n_tokens,
                        static_cast<int>(run));
     } else {
         e = launch_pdl(seq_ln_shift_mix_prep_kernel, dim3(static_cast<unsigned>(n_tokens)), dim3(kSeqThreads), 0, s, a);

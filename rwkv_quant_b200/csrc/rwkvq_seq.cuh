@@ -1,6 +1,6 @@
 // Launchers of the sequence-path glue kernels (rwkvq_seq.cu, rwkvq_wkv.cu) for the one-call forward.
 #pragma once
-#include "rwkvq_common.cuh"
+#include "rwkvq_gemm_sb.cuh"
 
 namespace rwkvq {
 
@@ -10,6 +10,8 @@ constexpr int kPrepSplit = 2;       // fp16 pair [hi | lo]
 constexpr int kPrepF32 = 4;
 constexpr int kPrepAmax = 8;        // max|row| into scale[m] (beside kPrepF32: what the small-batch linears read)
 
+constexpr int kPrepPair = 16;       // scaled fp16 pair with block sums into pair[m]: what launch_gemm_sb reads
+
 struct SeqPrepArgs {
     const float *x, *ln_w, *ln_b, *shift_in, *mix;
     float* shift_out;
@@ -17,12 +19,16 @@ struct SeqPrepArgs {
     float* scale[6];       // [N]
     __half* split[6];      // [N, 2 D]
     float* f32[6];         // [N, D]
+    SbRows pair[6];
     int mode[6];
     int T, D, n_mix;
     float* n2;             // optional [N]: squared norm of mix row 0 (unscaled)
     float *zero_a, *zero_b;    // optional [N]: cleared
 };
+// mix == NULL: no shift and no lerp, the normalised row itself (n_mix = 1; shift_in, shift_out NULL).  shift_out may equal
+// shift_in where T = 1 and D is a multiple of 256 (seq_prep_in_place_ok).  kPrepPair needs D % 256 == 0.
 int launch_seq_prep(const SeqPrepArgs& a, long long n_tokens, cudaStream_t s);
+inline bool seq_prep_in_place_ok(int D) { return D % 256 == 0 && D <= 4096; }
 
 int launch_wkv_tail(const float* wkv, const float* r, const float* k, const float* v, const float* r_k, const float* ln_w,
                     const float* ln_b, const float* g, float* out, int N, int H, float eps, float* og_amax, cudaStream_t s);
