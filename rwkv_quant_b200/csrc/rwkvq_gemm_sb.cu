@@ -29,6 +29,7 @@
 
 #include <algorithm>
 #include <cstdlib>
+#include <type_traits>
 
 #include "rwkvq_gemv_mma.cuh"
 #include "rwkvq_tc.cuh"
@@ -210,6 +211,7 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
     __shared__ uint64_t bar_full[G::ST], bar_empty[G::ST], bar_done;
     __shared__ uint32_t s_tmem;
     __shared__ volatile int s_fail;
+    __shared__ float s_un[NT];
     cg::cluster_group cluster = cg::this_cluster();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int ks = a.ks, z = blockIdx.x % ks, first_tile = blockIdx.x / ks, tile_step = gridDim.x / ks;
@@ -295,6 +297,8 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
             const uint64_t b0 = umma_desc(smem_addr(smem));
             const uint64_t ma0 = umma_desc_plain(smem_addr(smem + G::OFF_MA), kGmRows * 16, 128);
             const uint64_t mb0 = umma_desc_plain(smem_addr(smem + G::OFF_MB), 2 * NT * 16, 128);
+            if (ti == 0) pdl_wait();
+            for (int n = lane; n < NT; n += 32) s_un[n] = n < nn ? __ldcg(a.unscale[mat] + n0 + n) : 0.f;   // read behind bar_done
             uint32_t elected;
             asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xFFFFFFFF;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(elected));
             bool ok = true;
@@ -425,70 +429,100 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
         }
         constexpr int TPW = NT / 4;                                  // tokens per warp: four warps share a lane quadrant
         constexpr int TC = TPW < 16 ? TPW : 16;                      // ... in chunks of at most 16
-        const int q = warp & 3, tg = warp >> 2, rl = q * 32 + lane;
-        float* y = a.y[mat] + static_cast<size_t>(n0) * a.ldy;
-        const float* rs = a.resid[mat] ? a.resid[mat] + static_cast<size_t>(n0) * a.ldy : nullptr;
+        const int q = warp & 3, tg = warp >> 2, rl = q * 32 + lane, row = row0 + rl;
+        const bool row_ok = row < t.rows && !s_fail;
+        float* y = a.y[mat] + static_cast<size_t>(n0) * a.ldy + row;
+        const float* rs = a.resid[mat] ? a.resid[mat] + static_cast<size_t>(n0) * a.ldy + row : nullptr;
         float* am_out = a.amax_out[mat] ? a.amax_out[mat] + n0 : nullptr;
-        const float* un = a.unscale[mat] + n0;
-        auto store = [&](float v, int n, int row) {                  // whole warps; the 32 lanes hold 32 consecutive rows
-            const bool in = n < nn && row < t.rows && !s_fail;
-            const size_t o = static_cast<size_t>(n) * a.ldy + row;
-            if (a.epilogue == RWKVQ_EPI_RELU2) { v = fmaxf(v, 0.f); v = v * v; }
-            else if (a.epilogue == RWKVQ_EPI_ADD && in) v = __fadd_rn(v, __ldcg(rs + o));
-            if (in) y[o] = v;
-            if (am_out != nullptr && n < nn) {                       // |v| as bits orders like the float, a NaN above every number
-                const unsigned m = __reduce_max_sync(0xFFFFFFFFu, in ? __float_as_uint(fabsf(v)) : 0u);
-                if (lane == 0 && m != 0u) atomicMax(reinterpret_cast<unsigned*>(am_out) + n, m);
+        const bool add = a.epilogue == RWKVQ_EPI_ADD;
+        // a lane's U values at tokens first + j * step (whole warps; 32 lanes = 32 consecutive rows).  Loads first: behind
+        // a store each would wait for its own L2 round trip (16 of them: 5 us).
+        auto load_resid = [&](auto& r, int first, int step, int end) {
+#pragma unroll
+            for (int j = 0; j < static_cast<int>(sizeof(r) / sizeof(r[0])); ++j) {
+                const int n = first + j * step;
+                r[j] = add && row_ok && n < end ? __ldcg(rs + static_cast<size_t>(n) * a.ldy) : 0.f;
             }
         };
-        float* part = reinterpret_cast<float*>(smem);                // every MMA that read the operands has completed
-        if (warp < kSbTmaWarp) {
+        auto store = [&](const auto& v, const auto& r, int first, int step, int end) {
 #pragma unroll
-            for (int c0 = 0; c0 < TPW; c0 += TC) {
-                float v[TC], lo[TC];
-                const uint32_t base = tmem + (static_cast<uint32_t>(q * 32) << 16) + tg * TPW + c0;
-                sb_tmem_ld<TC>(base, v);
-                sb_tmem_ld<TC>(base + NT, lo);
-#pragma unroll
-                for (int j = 0; j < TC; ++j) {
-                    const int n = tg * TPW + c0 + j;
-                    v[j] = n < nn ? (v[j] + lo[j]) * __ldcg(un + n) : 0.f;
-                    if (ks == 1) store(v[j], n, row0 + rl);
-                    else part[n * kSbPitch + rl] = v[j];
+            for (int j = 0; j < static_cast<int>(sizeof(v) / sizeof(v[0])); ++j) {
+                const int n = first + j * step;
+                float o = v[j];
+                if (a.epilogue == RWKVQ_EPI_RELU2) { o = fmaxf(o, 0.f); o = o * o; }
+                else if (add) o = __fadd_rn(o, r[j]);
+                if (row_ok && n < end) y[static_cast<size_t>(n) * a.ldy] = o;
+                if (am_out != nullptr && n < end) {                  // |o| as bits orders like the float, a NaN above every number
+                    const unsigned m = __reduce_max_sync(0xFFFFFFFFu, row_ok ? __float_as_uint(fabsf(o)) : 0u);
+                    if (lane == 0 && m != 0u) atomicMax(reinterpret_cast<unsigned*>(am_out) + n, m);
                 }
             }
-            tc_fence_before();
-        }
-        if (ks == 1) {                                               // the accumulator is free for the next tile
+        };
+        auto accumulators = [&](float (&v)[TC], int c0) {
+            float lo[TC];
+            const uint32_t base = tmem + (static_cast<uint32_t>(q * 32) << 16) + tg * TPW + c0;
+            sb_tmem_ld<TC>(base, v);
+            sb_tmem_ld<TC>(base + NT, lo);
+#pragma unroll
+            for (int j = 0; j < TC; ++j) v[j] = (v[j] + lo[j]) * s_un[tg * TPW + c0 + j];
+        };
+        if (ks == 1) {
+            if (warp < kSbTmaWarp) {
+#pragma unroll 1
+                for (int c0 = 0; c0 < TPW; c0 += TC) {
+                    float v[TC], r[TC];
+                    load_resid(r, tg * TPW + c0, 1, nn);
+                    accumulators(v, c0);
+                    store(v, r, tg * TPW + c0, 1, nn);
+                }
+                tc_fence_before();
+            }
+            // the accumulator is free for the next tile
             if (warp != kSbTmaWarp) asm volatile("bar.sync 1, %0;" ::"n"(kSbThreads - 32) : "memory");
             tc_fence_after();
         } else {
-            cluster.sync();
-            if (warp < kSbTmaWarp) {                                 // this CTA's share of the tokens, ranks added in order
-                const int per = (NT + ks - 1) / ks, n1 = min(nn, (z + 1) * per);
-                constexpr int UT = 4;                                // tokens whose remote loads are in flight together
-                for (int nb = z * per + tg; nb < n1; nb += 4 * UT) {
-                    float s4[UT];
+            float* part = reinterpret_cast<float*>(smem);            // every MMA that read the operands has completed
+            if (warp < kSbTmaWarp) {
+#pragma unroll 1
+                for (int c0 = 0; c0 < TPW; c0 += TC) {
+                    float v[TC];
+                    accumulators(v, c0);
 #pragma unroll
-                    for (int j = 0; j < UT; ++j) s4[j] = 0.f;
-                    for (int u = 0; u < ks; u += 2) {
-                        const float* p0 = cluster.map_shared_rank(part, u);
-                        const float* p1 = cluster.map_shared_rank(part, u + 1 < ks ? u + 1 : u);
-                        float v0[UT], v1[UT];
+                    for (int j = 0; j < TC; ++j) part[(tg * TPW + c0 + j) * kSbPitch + rl] = v[j];
+                }
+                tc_fence_before();
+            }
+            // this CTA's share of the tokens, ranks added in order; U tokens of K ranks in flight per thread
+            const int per = (NT + ks - 1) / ks, first = z * per + tg, end = min(nn, (z + 1) * per);
+            auto reduce = [&](auto u_tag, auto k_tag) {
+                constexpr int U = decltype(u_tag)::value, K = decltype(k_tag)::value;
+                float r[U];
+                if (warp < kSbTmaWarp) load_resid(r, first, 4, end);
+                cluster.sync();
+                if (warp < kSbTmaWarp) {
+#pragma unroll 1
+                    for (int nb = first; nb < end; nb += 4 * U) {
+                        float pv[K][U], v[U];
+                        if (nb != first) load_resid(r, nb, 4, end);
 #pragma unroll
-                        for (int j = 0; j < UT; ++j) {
-                            const int n = min(nb + 4 * j, NT - 1);
-                            v0[j] = p0[n * kSbPitch + rl];
-                            v1[j] = u + 1 < ks ? p1[n * kSbPitch + rl] : 0.f;
+                        for (int u = 0; u < K; ++u) {
+                            const float* src = cluster.map_shared_rank(part, u < ks ? u : 0);
+#pragma unroll
+                            for (int j = 0; j < U; ++j) pv[u][j] = u < ks ? src[min(nb + 4 * j, NT - 1) * kSbPitch + rl] : 0.f;
                         }
 #pragma unroll
-                        for (int j = 0; j < UT; ++j) s4[j] = (s4[j] + v0[j]) + v1[j];
-                    }
+                        for (int j = 0; j < U; ++j) {
+                            v[j] = pv[0][j];
 #pragma unroll
-                    for (int j = 0; j < UT; ++j)
-                        if (nb + 4 * j < n1) store(s4[j], nb + 4 * j, row0 + rl);
+                            for (int u = 1; u < K; ++u) v[j] += pv[u][j];
+                        }
+                        store(v, r, nb, 4, end);
+                    }
                 }
-            }
+            };
+            if (ks == 2) reduce(std::integral_constant<int, NT >= 64 ? 8 : 4>{}, std::integral_constant<int, 2>{});
+            else if (ks <= 4) reduce(std::integral_constant<int, 4>{}, std::integral_constant<int, 4>{});
+            else reduce(std::integral_constant<int, 4>{}, std::integral_constant<int, 8>{});
             cluster.sync();                                          // nobody leaves while a peer still reads its partial tile
         }
     }
