@@ -674,11 +674,11 @@ bool sb_wanted(int B) {
     return g_tcb_exact == 1 || B >= kSbMinStreams;
 }
 bool sb_model_ok(const rwkvq_model& m) {
-    if (!seq_prep_in_place_ok(m.n_embd) || !gemm_tcb_ok(m.head)) return false;
+    if (!seq_prep_in_place_ok(m.n_embd) || !gemm_sb_ok(m.head)) return false;
     for (int l = 0; l < m.n_layer; ++l) {
         const rwkvq_layer& L = m.layers[l];
         for (const rwkvq_qtensor* t : {&L.Wr, &L.Wk, &L.Wv, &L.Wo, &L.Wfk, &L.Wfv})
-            if (!gemm_tcb_ok(*t)) return false;
+            if (!gemm_sb_ok(*t)) return false;
         for (const rwkvq_qtensor* t : {&L.Wk, &L.Wv})
             if (t->kind != L.Wr.kind || t->bits != L.Wr.bits || t->rows != L.Wr.rows || t->cols != L.Wr.cols) return false;
     }
@@ -948,9 +948,11 @@ int rwkvq_decode_step(const rwkvq_model* m, int B, const int64_t* tokens, float*
         }
         // Up to 16 streams the LoRA pair (two dependent launches) is the longer of the two branches: it then
         // stays on the caller's stream, where its first kernel starts programmatically behind the LayerNorm
-        // and stages its weights while that still runs, and r / k / v take the side stream.
+        // and stages its weights while that still runs, and r / k / v take the side stream.  So it does beside the tcgen05
+        // pipeline at any stream count: that leaves some 50 SMs for the second LoRA launch, but none of its CTAs
+        // shares an SM with the first (64 streams: 17 + 11 + 6 us in the other order, 13 + 16 in this).
         cudaStream_t s_rkv = s;
-        if (lane && B <= 16) { s_rkv = lane->stream; s_lora = s; }
+        if (lane && (B <= 16 || sb)) { s_rkv = lane->stream; s_lora = s; }
         if (B == 1 && ml >= 0 && mma_layout_of(L.Wk) == ml && mma_layout_of(L.Wv) == ml && L.Wk.rows == D &&
             L.Wv.rows == D && L.Wr.rows == D && L.Wk.cols == D && L.Wv.cols == D && L.Wr.cols == D) {
             // r, k, v in one launch: three matrices, three inputs (rows 0, 2, 3 of xs)

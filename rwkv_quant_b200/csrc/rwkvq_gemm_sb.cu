@@ -67,9 +67,9 @@ template <int L>
 struct SbLayout {
     static constexpr bool SB6 = L <= ML_SB6_6;
     static constexpr int CODE_BYTES = L == ML_SYM8 ? 64 : 32;                      // of a row's stage
-    static constexpr int PLANES = L == ML_SB6_5 ? 1 : (L == ML_SB6_6 || L == ML_SYM6) ? 2 : 0;
-    // one stage in shared memory: codes and the scale record as planes of 16 bytes a row, bit planes 8 bytes a row
-    static constexpr int RAW = kGmRows * (CODE_BYTES + 16 + 8 * PLANES);
+    static constexpr int PLANE_BYTES = L == ML_SB6_5 ? 8 : (L == ML_SB6_6 || L == ML_SYM6) ? 16 : 0;
+    // one stage in shared memory: codes, the scale record and planes, each as columns of 16 (8) bytes a row
+    static constexpr int RAW = kGmRows * (CODE_BYTES + 16 + PLANE_BYTES);
 };
 
 template <int L, int NT>
@@ -130,72 +130,45 @@ __device__ __forceinline__ void sb_tmem_ld(uint32_t taddr, float (&v)[NC]) {
     for (int i = 0; i < NC; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// The 32 weights of item `it` of a super-block: codes * scale as product pw and rounding error ew, two per word in
-// column order; returns the block's min (fp16 by the codec's definition; zero for sym).  decode_item with the layout
-// known at compile time.
+// Codes of block b (32 columns) of a stage as bytes in column order; the relayouted planes give the high bits of four
+// codes with one shift and mask.
 template <int L>
-__device__ __forceinline__ __half sb_convert(const Packed& p, bool in_rec, int it, int half, uint32_t (&pw)[16], uint32_t (&ew)[16]) {
-    uint32_t bytes[8];
-    __half2 s2[2], m2 = __float2half2_rn(0.f), bias;
-    const uint32_t w[4] = {p.c0.x, p.c0.y, p.c0.z, p.c0.w};
+__device__ __forceinline__ void sb_codes(const uint4& c0, const uint4& c1, const uint4& pl, int b, uint32_t (&bytes)[8]) {
+    const uint32_t w[4] = {c0.x, c0.y, c0.z, c0.w};
     if constexpr (SbLayout<L>::SB6) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {              // byte k of the block: column k (low), k + 16 (high)
             bytes[i] = w[i] & 0x0F0F0F0Fu;
             bytes[4 + i] = (w[i] >> 4) & 0x0F0F0F0Fu;
-            if (L != ML_SB6_4) {
-                bytes[i] |= spread_nibble<4>((p.h >> (4 * i)) & 0xFu);
-                bytes[4 + i] |= spread_nibble<4>((p.h >> (16 + 4 * i)) & 0xFu);
-            }
-            if (L == ML_SB6_6) {
-                bytes[i] |= spread_nibble<5>((p.h2 >> (4 * i)) & 0xFu);
-                bytes[4 + i] |= spread_nibble<5>((p.h2 >> (16 + 4 * i)) & 0xFu);
+            if (L == ML_SB6_5) {
+                const uint32_t p = b ? pl.y : pl.x;
+                bytes[i] |= (p << (4 - i)) & 0x10101010u;
+                bytes[4 + i] |= (p >> i) & 0x10101010u;
+            } else if (L == ML_SB6_6) {
+                const uint32_t p0 = b ? pl.z : pl.x, p1 = b ? pl.w : pl.y;
+                bytes[i] |= (i < 2 ? (p0 << (4 - 2 * i)) : (p0 >> (2 * i - 4))) & 0x30303030u;
+                bytes[4 + i] |= (i < 2 ? (p1 << (4 - 2 * i)) : (p1 >> (2 * i - 4))) & 0x30303030u;
             }
         }
-        float s, m;
-        if (in_rec) {
-            const int tt = it >> 1;                // record word it / 2: codes of blocks 2 (it / 2), + 1 and one byte of d | dm << 16
-            const uint32_t w4 = (tt & 2) ? ((tt & 1) ? p.rec.w : p.rec.z) : ((tt & 1) ? p.rec.y : p.rec.x);
-            const uint32_t dd = __byte_perm(p.rec.x, p.rec.y, 0x0073) & 0xFFFFu, dm = __byte_perm(p.rec.z, p.rec.w, 0x0073) & 0xFFFFu;
-            s = fmaxf(half_roundtrip(__fmul_rn(static_cast<float>((w4 >> (6 * half)) & 0x3Fu), half_bits_to_float(dd))), 1e-8f);
-            m = half_roundtrip(__fmul_rn(static_cast<float>(static_cast<int>((w4 >> (12 + 6 * half)) & 0x3Fu) - 31), half_bits_to_float(dm)));
-        } else {
-            sb6_scale_min(p.rec.x, p.rec.y, p.rec.z, it, half_bits_to_float(p.rec.w & 0xFFFFu), half_bits_to_float(p.rec.w >> 16), s, m);
-        }
-        s2[0] = s2[1] = __float2half2_rn(s);
-        m2 = __float2half2_rn(m);
-        bias = __float2half2_rn(1024.f);
+    } else if constexpr (L == ML_SYM8) {
+        const uint32_t w8[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) bytes[i] = w8[i] ^ 0x80808080u;          // code + 128
     } else {
-        const float d = half_bits_to_float(p.rec.y);
 #pragma unroll
-        for (int b = 0; b < 2; ++b)
-            s2[b] = __float2half2_rn(half_roundtrip(__fmul_rn(static_cast<float>(static_cast<int8_t>((p.rec.x >> (8 * b)) & 0xFFu)), d)));
-        if constexpr (L == ML_SYM8) {
-            const uint32_t w8[8] = {p.c0.x, p.c0.y, p.c0.z, p.c0.w, p.c1.x, p.c1.y, p.c1.z, p.c1.w};
-#pragma unroll
-            for (int i = 0; i < 8; ++i) bytes[i] = w8[i] ^ 0x80808080u;      // code + 128
-            bias = __float2half2_rn(1152.f);
-        } else {
-#pragma unroll
-            for (int b = 0; b < 2; ++b)            // block b: words 2b, 2b + 1; byte k: column k (low), k + 8 (high)
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    const int cl = 16 * b + 4 * i, ch = cl + 8;
-                    bytes[4 * b + i] = (w[2 * b + i] & 0x0F0F0F0Fu) | spread_nibble<4>((p.h >> cl) & 0xFu) | spread_nibble<5>((p.h2 >> cl) & 0xFu);
-                    bytes[4 * b + 2 + i] =
-                        ((w[2 * b + i] >> 4) & 0x0F0F0F0Fu) | spread_nibble<4>((p.h >> ch) & 0xFu) | spread_nibble<5>((p.h2 >> ch) & 0xFu);
-                }
-            bias = __float2half2_rn(1056.f);       // stored code = value + 32
+        for (int h = 0; h < 2; ++h) {              // block h of 16: words 2h, 2h + 1; byte k: column k (low), k + 8 (high)
+            const uint32_t p = b ? (h ? pl.w : pl.z) : (h ? pl.y : pl.x);
+            bytes[4 * h] = (w[2 * h] & 0x0F0F0F0Fu) | ((p << 4) & 0x30303030u);
+            bytes[4 * h + 1] = (w[2 * h + 1] & 0x0F0F0F0Fu) | ((p << 2) & 0x30303030u);
+            bytes[4 * h + 2] = ((w[2 * h] >> 4) & 0x0F0F0F0Fu) | (p & 0x30303030u);
+            bytes[4 * h + 3] = ((w[2 * h + 1] >> 4) & 0x0F0F0F0Fu) | ((p >> 2) & 0x30303030u);
         }
     }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        uint2 pa, ea;
-        bytes_to_half4_pair(bytes[j], bias, s2[j >> 2], pa, ea);
-        pw[2 * j] = pa.x; pw[2 * j + 1] = pa.y;
-        ew[2 * j] = ea.x; ew[2 * j + 1] = ea.y;
-    }
-    return __low2half(m2);
+}
+// Two bytes of `two` (scale codes) times the fp16 in both halves of dd
+__device__ __forceinline__ __half2 sb_sym_scales(uint32_t two, uint32_t dd) {
+    const uint32_t x = two ^ 0x8080u, u = (x & 0xFFu) | ((x << 8) & 0x00FF0000u) | 0x64006400u;      // 1024 + code + 128
+    return __hmul2(__hsub2(*reinterpret_cast<const __half2*>(&u), __float2half2_rn(1152.f)), *reinterpret_cast<const __half2*>(&dd));
 }
 
 template <int L, int NT>
@@ -235,38 +208,29 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
     // ---- weight threads: group grp takes stage grp of every super-block, thread wrow its row
     const int grp = tid / kGmRows, wrow = tid % kGmRows;
     unsigned char* raw = smem + G::OFF_RAW + (grp % kSbGroups) * G::AHEAD * Y::RAW;
-    constexpr int OFF_R = kGmRows * Y::CODE_BYTES, OFF_H = OFF_R + kGmRows * 16, OFF_H2 = OFF_H + kGmRows * 8;
+    constexpr int OFF_R = kGmRows * Y::CODE_BYTES, OFF_H = OFF_R + kGmRows * 16;
     int c_ti = 0, c_sb = 0, c_slot = 0;                              // copy side: tile of this CTA, super-block, ring slot
-    const uint8_t *c_codes = nullptr, *c_h = nullptr, *c_h2 = nullptr, *c_meta = nullptr;
-    bool c_long = true;                                              // a 16-byte record (else the 12 bytes of the file)
+    const uint8_t *c_codes = nullptr, *c_pl = nullptr, *c_meta = nullptr;
     auto copy_tile = [&]() {                                         // source pointers of tile c_ti
         const int tile = first_tile + c_ti * tile_step;
         const QView& t = a.t[tile / a.row_tiles];
         const size_t R = static_cast<size_t>(min((tile % a.row_tiles) * kGmRows + wrow, t.rows - 1));
         const int col = sb0 * 256 + grp * 64;
         c_codes = t.codes + (L == ML_SYM8 ? R * t.cols + col : R * (t.cols >> 1) + (col >> 1));
-        if (Y::PLANES >= 1) c_h = t.qh + R * (t.cols >> 3) + (col >> 3);
-        if (Y::PLANES == 2) c_h2 = t.qh2 + R * (t.cols >> 3) + (col >> 3);
-        c_long = !Y::SB6 || t.dev_meta != nullptr;
-        if (!Y::SB6) c_meta = reinterpret_cast<const uint8_t*>(t.qs) + R * (t.cols >> 4) + sb0 * 16;
-        else c_meta = c_long ? t.dev_meta + (R * (t.cols >> 8) + sb0) * 16 : t.qsqm + (R * (t.cols >> 8) + sb0) * 12;
+        // planes: 4 bytes per 32 columns (5 bits), 8 per 32 (6 bits; sym as 4 per 16)
+        if (Y::PLANE_BYTES) c_pl = reinterpret_cast<const uint8_t*>(t.dev_planes) + R * (t.cols >> 6) * Y::PLANE_BYTES + (col >> 6) * Y::PLANE_BYTES;
+        c_meta = Y::SB6 ? t.dev_meta + (R * (t.cols >> 8) + sb0) * 16 : reinterpret_cast<const uint8_t*>(t.qs) + R * (t.cols >> 4) + sb0 * 16;
     };
     auto copy_stage = [&]() {
         if (c_ti < n_my) {
             unsigned char* slot = raw + c_slot * Y::RAW;
 #pragma unroll
             for (int k = 0; k < Y::CODE_BYTES / 16; ++k) sb_cp<16>(slot + k * (kGmRows * 16) + wrow * 16, c_codes + 16 * k);
-            if (c_long) sb_cp<16>(slot + OFF_R + wrow * 16, c_meta);
-            else {
-#pragma unroll
-                for (int k = 0; k < 3; ++k) sb_cp<4>(slot + OFF_R + wrow * 16 + 4 * k, c_meta + 4 * k);
-            }
-            if (Y::PLANES >= 1) sb_cp<8>(slot + OFF_H + wrow * 8, c_h);
-            if (Y::PLANES == 2) sb_cp<8>(slot + OFF_H2 + wrow * 8, c_h2);
+            sb_cp<16>(slot + OFF_R + wrow * 16, c_meta);
+            if constexpr (Y::PLANE_BYTES > 0) sb_cp<Y::PLANE_BYTES>(slot + OFF_H + wrow * Y::PLANE_BYTES, c_pl);
             c_codes += L == ML_SYM8 ? 256 : 128;
-            c_meta += c_long ? 16 : 12;
-            if (Y::PLANES >= 1) c_h += 32;
-            if (Y::PLANES == 2) c_h2 += 32;
+            c_meta += 16;
+            c_pl += 4 * Y::PLANE_BYTES;
             c_slot = c_slot == G::AHEAD - 1 ? 0 : c_slot + 1;
             if (++c_sb == n_super) {
                 c_sb = 0;
@@ -350,17 +314,10 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
             }
         } else {
             // ------------------------------------------------------------------ weights
-            // super-scales that are not part of the staged record (sym d; sb6 d | dm without the relayouted record), one
-            // super-block ahead
-            const bool in_rec = Y::SB6 && t.dev_meta != nullptr;
-            const size_t drow = static_cast<size_t>(min(row0 + wrow, t.rows - 1)) * (t.cols >> 8) + sb0;
-            uint32_t dd = 0, dd_next = 0;
-            auto load_d = [&](int sb) {
-                if (in_rec || sb >= n_super) return;
-                dd_next = __half_as_ushort(__ldg(t.d + drow + sb));
-                if (Y::SB6) dd_next |= static_cast<uint32_t>(__half_as_ushort(__ldg(t.dm + drow + sb))) << 16;
-            };
-            load_d(0);
+            // sym: the super-scale is not part of the staged record; one super-block ahead
+            const __half* dp = Y::SB6 ? nullptr : t.d + static_cast<size_t>(min(row0 + wrow, t.rows - 1)) * (t.cols >> 8) + sb0;
+            uint32_t d_next = Y::SB6 ? 0u : __half_as_ushort(__ldg(dp));
+            const __half2 bias = __float2half2_rn(L == ML_SYM8 ? 1152.f : L == ML_SYM6 ? 1056.f : 1024.f);
             const uint32_t lane_base = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + 2 * NT;
 #pragma unroll 1
             for (int sb = 0; sb < n_super; ++sb) {
@@ -368,28 +325,29 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
                 asm volatile("cp.async.wait_group %0;" ::"n"(G::AHEAD - 1) : "memory");
                 const unsigned char* slot = raw + r_slot * Y::RAW;
                 r_slot = r_slot == G::AHEAD - 1 ? 0 : r_slot + 1;
-                Packed p[2];
-                uint2 h = make_uint2(0, 0), h2 = h;
-                if (Y::PLANES >= 1) h = *reinterpret_cast<const uint2*>(slot + OFF_H + wrow * 8);
-                if (Y::PLANES == 2) h2 = *reinterpret_cast<const uint2*>(slot + OFF_H2 + wrow * 8);
-                uint4 rec = *reinterpret_cast<const uint4*>(slot + OFF_R + wrow * 16);
-                dd = dd_next;
-                load_d(sb + 1);
-                if (Y::SB6) {
-                    if (!in_rec) rec.w = dd;
-                } else {                                             // the two scale codes of each block of this stage
-                    const uint32_t w = (grp & 2) ? ((grp & 1) ? rec.w : rec.z) : ((grp & 1) ? rec.y : rec.x);
-                    rec = make_uint4(w, dd, 0, 0);
-                }
+                constexpr int CB = Y::CODE_BYTES / 32;               // 16-byte pieces of a block
+                uint4 code[2 * CB], pl = make_uint4(0, 0, 0, 0);
 #pragma unroll
-                for (int b = 0; b < 2; ++b) {
-                    constexpr int CB = Y::CODE_BYTES / 32;           // 16-byte pieces of an item
-                    p[b].c0 = *reinterpret_cast<const uint4*>(slot + (CB * b) * (kGmRows * 16) + wrow * 16);
-                    if (L == ML_SYM8) p[b].c1 = *reinterpret_cast<const uint4*>(slot + (CB * b + 1) * (kGmRows * 16) + wrow * 16);
-                    p[b].h = b ? h.y : h.x;
-                    p[b].h2 = b ? h2.y : h2.x;
-                    p[b].rec = rec;
-                    if (!Y::SB6 && b) p[b].rec.x = rec.x >> 16;
+                for (int k = 0; k < 2 * CB; ++k) code[k] = *reinterpret_cast<const uint4*>(slot + k * (kGmRows * 16) + wrow * 16);
+                if (Y::PLANE_BYTES == 16) pl = *reinterpret_cast<const uint4*>(slot + OFF_H + wrow * 16);
+                if (Y::PLANE_BYTES == 8) {
+                    const uint2 p2 = *reinterpret_cast<const uint2*>(slot + OFF_H + wrow * 8);
+                    pl.x = p2.x; pl.y = p2.y;
+                }
+                const uint4 rec = *reinterpret_cast<const uint4*>(slot + OFF_R + wrow * 16);
+                // scales of the stage's columns by quarters of 16, and the mins of its two blocks; fp16 values by the codec's
+                // definition: one half-precision multiply of the exact small integer
+                __half2 s4[2], mins = __float2half2_rn(0.f);
+                if (Y::SB6) {
+                    __half2 hs;
+                    sb6_pair_scales_h2(rec, grp, hs, mins);
+                    s4[0] = __low2half2(hs);
+                    s4[1] = __high2half2(hs);
+                } else {
+                    const uint32_t w = (grp & 2) ? ((grp & 1) ? rec.w : rec.z) : ((grp & 1) ? rec.y : rec.x), dd = d_next * 0x00010001u;
+                    if (sb + 1 < n_super) d_next = __half_as_ushort(__ldg(dp + sb + 1));
+                    s4[0] = sb_sym_scales(w & 0xFFFFu, dd);
+                    s4[1] = sb_sym_scales(w >> 16, dd);
                 }
                 if (g >= G::ST) {                                    // the MMAs that read this buffer have completed
                     if (lane == 0 && !s_fail && !mbar_wait_bounded(&bar_empty[st], (g / G::ST - 1) & 1)) s_fail = 1;
@@ -397,17 +355,23 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
                     tc_fence_after();
                 }
                 const uint32_t ta = lane_base + st * kSbACols;
-                __half mn[2];
 #pragma unroll
                 for (int b = 0; b < 2; ++b) {
-                    uint32_t pw[16], ew[16];
-                    mn[b] = sb_convert<L>(p[b], in_rec, 2 * grp + b, b, pw, ew);
+                    uint32_t bytes[8], pw[16], ew[16];
+                    sb_codes<L>(code[CB * b], code[CB * b + CB - 1], pl, b, bytes);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const __half2 s2 = Y::SB6 ? s4[b] : (j < 4 ? __low2half2(s4[b]) : __high2half2(s4[b]));
+                        uint2 pa, ea;
+                        bytes_to_half4_pair(bytes[j], bias, s2, pa, ea);
+                        pw[2 * j] = pa.x; pw[2 * j + 1] = pa.y;
+                        ew[2 * j] = ea.x; ew[2 * j + 1] = ea.y;
+                    }
                     sb_tmem_st16(ta + 16 * b, pw);
                     sb_tmem_st16(ta + kSbACols / 2 + 16 * b, ew);
                 }
                 if (Y::SB6) {
-                    const __half2 m2 = __halves2half2(mn[0], mn[1]);
-                    *reinterpret_cast<__half2*>(smem + G::OFF_MA + ((g >> 2) & 1) * G::MA + wrow * 16 + grp * 4) = m2;
+                    *reinterpret_cast<__half2*>(smem + G::OFF_MA + ((g >> 2) & 1) * G::MA + wrow * 16 + grp * 4) = mins;
                     fence_async_smem();
                 }
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -668,10 +632,13 @@ int launch_sb_nt(SbArgs& a, const SbMaps& maps, int nt, int groups, int force_ks
 
 }  // namespace
 
+bool gemm_sb_ok(const rwkvq_qtensor& t) {
+    return gemm_tcb_ok(t) && (t.kind == RWKVQ_KIND_SB6 || t.kind == RWKVQ_KIND_SYM) && mma_layout_of(t) >= 0;
+}
 // Whether this kernel takes a product the mma.sync kernel serves too.
 bool gemm_sb_pays(const rwkvq_qtensor& t, int N) {
     static const int least = [] { const char* e = getenv("SBMIN"); return e ? atoi(e) : 17; }();
-    return tcb_enabled() && gemm_tcb_ok(t) && N >= least;
+    return tcb_enabled() && gemm_sb_ok(t) && N >= least;
 }
 
 int launch_gemm_sb(const rwkvq_qtensor* ts, int n_mats, const SbRows* rows, int N, float* const* ys, long long ldy, int epilogue,
@@ -681,7 +648,7 @@ int launch_gemm_sb(const rwkvq_qtensor* ts, int n_mats, const SbRows* rows, int 
     SbMaps maps;
     const int nt = N <= 16 ? 16 : N <= 32 ? 32 : N <= 64 ? 64 : 128, groups = (N + nt - 1) / nt;
     for (int k = 0; k < n_mats; ++k) {
-        RWKVQ_REQUIRE(gemm_tcb_ok(ts[k]) && ts[k].kind == ts[0].kind && ts[k].bits == ts[0].bits && ts[k].rows == ts[0].rows &&
+        RWKVQ_REQUIRE(gemm_sb_ok(ts[k]) && ts[k].kind == ts[0].kind && ts[k].bits == ts[0].bits && ts[k].rows == ts[0].rows &&
                           ts[k].cols == ts[0].cols, RWKVQ_E_SHAPE, "gemm_sb: fused matrices must share layout and shape");
         RWKVQ_REQUIRE(rows[k].hi && rows[k].lo && rows[k].sums && rows[k].unscale && ys[k], RWKVQ_E_NULL, "gemm_sb: x pairs or y is null");
         a.t[k] = make_view(ts[k]);

@@ -85,20 +85,6 @@ __device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t a0, uint32_t a1,
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// sb6: (s, m) of blocks 2t, 2t+1 as half2 pairs; the arithmetic of sb6_pair_scales without the
-// widening to fp32.  The codec's floor max(s, 1e-8) is below the fp16 range and is dropped: a
-// block whose scale code or super-scale is zero dequantises to its min alone (|dw| <= 63e-8).
-__device__ __forceinline__ void sb6_pair_scales_h2(const uint4& rec, int t, __half2& hs, __half2& hm) {
-    const uint32_t w = (t & 2) ? ((t & 1) ? rec.w : rec.z) : ((t & 1) ? rec.y : rec.x);
-    const uint32_t dd = __byte_perm(rec.x, rec.y, 0x7373);
-    const uint32_t dmm = __byte_perm(rec.z, rec.w, 0x7373);
-    const uint32_t qs = (w & 0x3Fu) | ((w << 10) & 0x003F0000u) | 0x64006400u;
-    const uint32_t qm = ((w >> 12) & 0x3Fu) | ((w >> 2) & 0x003F0000u) | 0x64006400u;
-    hs = __hmul2(__hsub2(*reinterpret_cast<const __half2*>(&qs), __float2half2_rn(1024.f)),
-                 *reinterpret_cast<const __half2*>(&dd));
-    hm = __hmul2(__hsub2(*reinterpret_cast<const __half2*>(&qm), __float2half2_rn(1055.f)),
-                 *reinterpret_cast<const __half2*>(&dmm));
-}
 __device__ __forceinline__ __half2 sym_pair_scales_h2(uint32_t q_lo, uint32_t q_hi, uint32_t d_bits, int t) {
     const uint32_t w = (t & 2) ? q_hi : q_lo;
     const uint32_t two = (t & 1) ? (w >> 16) : (w & 0xFFFFu);
@@ -770,8 +756,10 @@ extern "C" int rwkvq_gemv_batch(const rwkvq_qtensor* t, const float* x, int N, i
     // default: the two-term mma.sync kernel.  The tcgen05 kernel (single fp16 operands) serves more than
     // 32 rows in fast mode, tensors the mma.sync kernel has no layout for, and the profiling override.
     const bool tcb_ok = tcb_enabled() && gemm_tcb_ok(*t) && t->cols <= kPairCols;
-    const bool tcb = tcb_ok && batch_fast() && ldx % 8 == 0 && (N > 32 || mma_layout_of(*t) < 0 || tcb_forced());
-    const bool sb = tcb_ok && !batch_fast() && (gemm_sb_pays(*t, N) || mma_layout_of(*t) < 0 || tcb_forced());
+    // tensors without the relayouted streams: the tcgen05 kernel that reads the file buffers, in either precision
+    const bool bare = mma_layout_of(*t) < 0;
+    const bool tcb = tcb_ok && ldx % 8 == 0 && (bare || (batch_fast() && (N > 32 || tcb_forced())));
+    const bool sb = tcb_ok && !batch_fast() && gemm_sb_ok(*t) && (gemm_sb_pays(*t, N) || tcb_forced());
     RWKVQ_REQUIRE(tcb || sb || mma_layout_of(*t) >= 0, RWKVQ_E_DTYPE,
                   "rwkvq_gemv_batch: needs an sb6 tensor, a sym tensor or per-row int8 with columns in multiples of 128");
     RWKVQ_REQUIRE(aligned(x, 16) && ldx % 4 == 0, RWKVQ_E_ALIGN, "rwkvq_gemv_batch: x rows must be 16-byte aligned");
@@ -794,7 +782,7 @@ extern "C" int rwkvq_gemv_batch(const rwkvq_qtensor* t, const float* x, int N, i
     if (rc) return rc;
     const void* xs[1] = {x};
     const float* am[1] = {amax};
-    rc = tcb ? launch_gemm_tcb(t, 1, xs, false, am, N, ldx, ys, ldy, epilogue, rs, nullptr, status, s)
+    rc = tcb ? launch_gemm_tcb(t, 1, xs, false, am, N, ldx, ys, ldy, epilogue, rs, nullptr, status, s, !batch_fast())
              : launch_gemv_batch(t, 1, xs, false, am, N, ldx, ys, ldy, epilogue, rs, nullptr, s);
     return rc ? rc : check_launch("rwkvq_gemv_batch");
 }

@@ -110,6 +110,21 @@ __device__ __forceinline__ void sb6_pair_scales(const uint4& rec, int t, float2&
     s.y = fmaxf(s.y, 1e-8f);
 }
 
+// sb6: (s, m) of blocks 2t, 2t+1 as half2 pairs; the arithmetic of sb6_pair_scales without the
+// widening to fp32.  The codec's floor max(s, 1e-8) is below the fp16 range and is dropped: a
+// block whose scale code or super-scale is zero dequantises to its min alone (|dw| <= 63e-8).
+__device__ __forceinline__ void sb6_pair_scales_h2(const uint4& rec, int t, __half2& hs, __half2& hm) {
+    const uint32_t w = (t & 2) ? ((t & 1) ? rec.w : rec.z) : ((t & 1) ? rec.y : rec.x);
+    const uint32_t dd = __byte_perm(rec.x, rec.y, 0x7373);
+    const uint32_t dmm = __byte_perm(rec.z, rec.w, 0x7373);
+    const uint32_t qs = (w & 0x3Fu) | ((w << 10) & 0x003F0000u) | 0x64006400u;
+    const uint32_t qm = ((w >> 12) & 0x3Fu) | ((w >> 2) & 0x003F0000u) | 0x64006400u;
+    hs = __hmul2(__hsub2(*reinterpret_cast<const __half2*>(&qs), __float2half2_rn(1024.f)),
+                 *reinterpret_cast<const __half2*>(&dd));
+    hm = __hmul2(__hsub2(*reinterpret_cast<const __half2*>(&qm), __float2half2_rn(1055.f)),
+                 *reinterpret_cast<const __half2*>(&dmm));
+}
+
 // sym: the two int8 scale codes of blocks 2t, 2t+1 times the fp16 super-scale
 __device__ __forceinline__ float2 sym_pair_scales(uint32_t q_lo, uint32_t q_hi, uint32_t d_bits, int t) {
     const uint32_t w = (t & 2) ? q_hi : q_lo;
