@@ -249,8 +249,7 @@ int validate_qtensor(const rwkvq_qtensor* t, const char* who);
 int mma_layout_of(const rwkvq_qtensor& t);
 int launch_gemv_mma(int layout, const rwkvq_qtensor* ts, int n_mats, const void* x, int x_dtype,
                     long long ldx, float* y, long long ldy, int epilogue, const float* resid,
-                    int fused, cudaStream_t s, const void* const* x_each = nullptr, float* scratch = nullptr);
-size_t gemv_mma_scratch_bytes();
+                    int fused, cudaStream_t s, const void* const* x_each = nullptr, bool split = false);
 // Small-batch tensor-core kernel (rwkvq_gemv_batch.cu): n_mats same-shape matrices, each with its
 // own [N, ldx] input and [N, ldy] output; weights read once for all N right-hand sides.  Inputs are
 // fp32 rows with scales[k] = max|x| of every row (written by the producer of x or by launch_row_amax),

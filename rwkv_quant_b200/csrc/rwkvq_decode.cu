@@ -21,7 +21,7 @@
 #include <mutex>
 #include <utility>
 
-#include "rwkvq_decode_parts.cuh"
+#include "rwkvq_lora_vec.cuh"
 #include "rwkvq_seq.cuh"
 
 namespace rwkvq {
@@ -504,7 +504,10 @@ __device__ __forceinline__ float warp_sum64(const float* v, int lane) {
     return s;
 }
 
-__global__ void __launch_bounds__(256) tmix_core_kernel(const TmixCoreArgs p) {
+// UP (one stream): the LoRA up projections of the head's 64 channels run here, their weights staged before the wait.
+template <bool UP>
+__global__ void __launch_bounds__(256) tmix_core_kernel(const TmixCoreArgs p, const std::conditional_t<UP, LoraVecArgs, int> up) {
+    extern __shared__ __align__(16) unsigned char up_smem[];         // UP: [ranks][64] fp16, [ranks] h, [8][4][64] partial sums
     // per-column operands of the state update, written once by warps 0 and 1 and read as float4 by all:
     // sA = -kk / |kk|, sB = (kk / |kk|) * a_gate, sW decay, sK key, sR receptance
     __shared__ __align__(16) float sA[64], sB[64], sW[64], sK[64], sR[64];
@@ -533,18 +536,43 @@ __global__ void __launch_bounds__(256) tmix_core_kernel(const TmixCoreArgs p) {
         prk0 = __ldg(p.r_k + hi * 64 + lane); prk1 = __ldg(p.r_k + hi * 64 + lane + 32);
         plw = __ldg(p.lnx_w + c); plb = __ldg(p.lnx_b + c);
     }
-    pdl_wait();            // the state above was written a whole token ago
+    float* part_up = nullptr;
+    if constexpr (UP) {
+        const int ranks = up.first[up.n_br];
+        __half* wt = reinterpret_cast<__half*>(up_smem);
+        float* h = reinterpret_cast<float*>(wt + ranks * 64);
+        part_up = h + ranks;
+        lora_up_stage(up, hi * 64, wt);
+        pdl_wait();
+        for (int i = tid; i < ranks; i += 256) h[i] = __ldcg(up.h + i);
+        __syncthreads();
+        lora_up_vec(up, wt, h, part_up);
+        __syncthreads();
+    } else {
+        pdl_wait();            // the state above was written a whole token ago
+    }
+    // LoRA output `br` (decay, rate, gate, value-residual) of the thread's channel
+    auto lora = [&](int br, const float* y) {
+        if constexpr (UP) {
+            float v = 0.f;
+#pragma unroll
+            for (int w = 0; w < 8; ++w) v += part_up[w * 256 + br * 64 + tid];
+            return v;
+        } else {
+            return __ldcg(y + row + tid);
+        }
+    };
     if (tid < 64) {
         const float r = __ldcg(p.r + row + tid), k = __ldcg(p.k + row + tid);
         float v = __ldcg(p.v + row + tid);
-        const float w = expf(-0.606531f * sigmoidf_(__ldcg(p.yw + row + tid) + pw0));
-        const float av = sigmoidf_(__ldcg(p.ya + row + tid) + pa0);
+        const float w = expf(-0.606531f * sigmoidf_(lora(0, p.yw) + pw0));
+        const float av = sigmoidf_(lora(1, p.ya) + pa0);
         const float k2 = k * (1.0f + (av - 1.0f) * pka);
         if (p.layer0) p.v_first[row + tid] = v;
-        else v = v + (__ldcg(p.v_first + row + tid) - v) * sigmoidf_(__ldcg(p.yv + row + tid) + pv0);
+        else v = v + (__ldcg(p.v_first + row + tid) - v) * sigmoidf_(lora(3, p.yv) + pv0);
         const float kk = k * pkk;
         sT[tid] = kk * kk;
-        sW[tid] = w; sK[tid] = k2; sR[tid] = r; sV[tid] = v; sG[tid] = __ldcg(p.g + row + tid);
+        sW[tid] = w; sK[tid] = k2; sR[tid] = r; sV[tid] = v; sG[tid] = lora(2, p.g);
         asm volatile("bar.sync 1, 64;" ::: "memory");        // warps 0 and 1 only: sT is complete
         // both warps reduce the head-wide sum themselves; a = -kk / |kk|, b = -a * a_gate
         const float kn = kk * (1.0f / sqrtf(warp_sum64(sT, lane) + 1e-12f));
@@ -686,7 +714,7 @@ bool sb_model_ok(const rwkvq_model& m) {
 }
 
 struct Workspace {
-    float *x, *xs, *rkv, *part, *yl, *og, *xk, *hffn, *xo, *v_first, *logits, *argv, *gscratch, *gemm_ws;
+    float *x, *xs, *rkv, *part, *yl, *og, *xk, *hffn, *xo, *v_first, *logits, *argv, *gemm_ws;
     int* status;             // first word of the workspace: RWKVQ_E_TIMEOUT if a bounded device-side wait of a step ran out
     float* amax;             // [10][B] per-row scale inverses / maxima for the small-batch linears: 6 mix rows, og, xk, hffn, xo
     __half *xs16, *xk16, *xo16;     // fp16 forms of the mix rows, the channel-mix row and the final row
@@ -726,7 +754,6 @@ Workspace carve(const rwkvq_model& m, int B, void* base) {
         w.d_pair = pair(D);
         w.f_pair = pair(F);
     }
-    w.gscratch = take(gemv_mma_scratch_bytes() / sizeof(float));
     w.gemm_ws = take(rwkvq_gemm_workspace_bytes_for(B, static_cast<int>(F > D ? F : D)) / sizeof(float) + 1);
     w.bytes = off;
     return w;
@@ -734,19 +761,19 @@ Workspace carve(const rwkvq_model& m, int B, void* base) {
 
 // y_br = (act_br(x_br @ W1_br)) @ W2_br for up to 4 branches, B right-hand sides
 // One quantized linear for B right-hand sides; the single-vector tensor-core kernel gets
-// the K-split scratch, everything else goes through the public entry point.
+// the K split, everything else goes through the public entry point.
 // x16 / x_scale: the fp16 form of x with its per-row scale inverses (what the LayerNorm kernels write
 // in fast mode), or null with x_scale = max|x| per row for fp32 rows; y_amax: optional slots max|y| per row is
 // merged into.
 int linear(const rwkvq_qtensor* t, const float* x, int B, int in, float* y, int out, int epi, const float* resid,
-           float* scratch, void* gemm_ws, void* stream, const __half* x16 = nullptr, const float* x_scale = nullptr,
+           void* gemm_ws, void* stream, const __half* x16 = nullptr, const float* x_scale = nullptr,
            float* y_amax = nullptr, int* status = nullptr) {
     const int ml = mma_layout_of(*t);
     if (B == 1 && ml >= 0) {
         int rc = validate_qtensor(t, "rwkvq_decode_step(linear)");
         if (rc) return rc;
         return launch_gemv_mma(ml, t, 1, x, RWKVQ_F32, in, y, out, epi, resid, 0, static_cast<cudaStream_t>(stream),
-                               nullptr, scratch);
+                               nullptr, true);
     }
     if (batch_path(B) && ml >= 0 && x_scale) {            // small batch: weights read once, tokens as MMA columns
         int rc = validate_qtensor(t, "rwkvq_decode_step(linear)");
@@ -795,6 +822,17 @@ SideLane* side_lane(cudaStream_t caller) {
         l = n;
     }
     return &l;
+}
+
+int launch_tmix_core_up(const TmixCoreArgs& tc, const LoraVecArgs& up, int H, cudaStream_t s) {
+    const size_t smem = lora_vec_smem(up.first[up.n_br]);
+    if (smem > 40 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(tmix_core_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLvMaxSmem);
+        if (e != cudaSuccess) return fail(RWKVQ_E_LIMIT, "tmix_core: %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
+    }
+    cudaError_t e = launch_pdl(tmix_core_kernel<true>, dim3(H, 1), dim3(256), smem, s, tc, up);
+    if (e != cudaSuccess) return fail(RWKVQ_E_LAUNCH, "tmix_core: %s", cudaGetErrorString(e));
+    return RWKVQ_OK;
 }
 
 int lora_rep(int B) { return B > kLmMaxN ? 8 : 1; }
@@ -939,6 +977,40 @@ int rwkvq_decode_step(const rwkvq_model* m, int B, const int64_t* tokens, float*
         float *xr = w.xs, *xw = w.xs + BD, *xk = w.xs + 2 * BD, *xv = w.xs + 3 * BD, *xa = w.xs + 4 * BD,
               *xg = w.xs + 5 * BD;
         float *r = w.rkv, *k = w.rkv + BD, *v = w.rkv + 2 * BD;
+        const rwkvq_qtensor* t1[4] = {&L.w1, &L.a1, &L.g1, &L.v1};
+        const rwkvq_qtensor* t2[4] = {&L.w2, &L.a2, &L.g2, &L.v2};
+        const float* x1[4] = {xw, xa, xg, xv};
+        const int act[4] = {1, 0, 2, 0};           // tanh (decay), none, sigmoid (gate), none
+        const int n_br = layer0 ? 3 : 4;
+        float *yw = w.yl, *ya = w.yl + BD, *yv = w.yl + 2 * BD, *yg = w.yl + 3 * BD;
+        TmixCoreArgs tc{r, k, v, yw, ya, layer0 ? nullptr : yv, yg, L.w0, L.a0, L.v0, L.k_k, L.k_a, L.r_k,
+                        L.lnx_w, L.lnx_b, w.v_first, wkv[l], w.og, D, H, layer0 ? 1 : 0, sb ? nullptr : am_og};
+        // One stream: r / k / v and the LoRA down projections in one launch, the up projections inside the time-mix core
+        const bool one = B == 1 && ml >= 0 && rkv_fused && L.Wr.rows == D && L.Wr.cols == D && lora_vec_ok(t1, t2, n_br, D);
+        if (one) {
+            LoraVecArgs down{}, up{};
+            for (const rwkvq_qtensor* t : {&L.Wr, &L.Wk, &L.Wv}) {
+                rc = validate_qtensor(t, "rwkvq_decode_step(r/k/v)");
+                if (rc) return rc;
+            }
+            for (int i = 0; i < n_br; ++i) {
+                rc = validate_qtensor(t1[i], "rwkvq_decode_step(lora down)");
+                if (rc) return rc;
+                rc = validate_qtensor(t2[i], "rwkvq_decode_step(lora up)");
+                if (rc) return rc;
+                down.t[i] = make_view(*t1[i]); up.t[i] = make_view(*t2[i]);
+                down.x[i] = x1[i]; down.act[i] = act[i];
+                down.first[i + 1] = up.first[i + 1] = down.first[i] + t1[i]->cols;
+            }
+            down.h = up.h = w.part;
+            down.n_br = up.n_br = n_br; down.D = up.D = D;
+            const rwkvq_qtensor three[3] = {L.Wr, L.Wk, L.Wv};
+            const void* x_each[3] = {xr, xk, xv};
+            rc = launch_gemv_mma_lora(ml, three, 3, x_each, r, D, down, s);
+            if (rc) return rc;
+            rc = launch_tmix_core_up(tc, up, H, s);
+            if (rc) return rc;
+        } else {
         SideLane* lane = side_lane(s);
         cudaStream_t s_lora = s;
         if (lane) {                                  // fork: the LoRA branches leave the chain here
@@ -962,7 +1034,7 @@ int rwkvq_decode_step(const rwkvq_model* m, int B, const int64_t* tokens, float*
             }
             const rwkvq_qtensor three[3] = {L.Wr, L.Wk, L.Wv};
             const void* x_each[3] = {xr, xk, xv};
-            rc = launch_gemv_mma(ml, three, 3, xr, RWKVQ_F32, D, r, D, RWKVQ_EPI_NONE, nullptr, 1, s_rkv, x_each, w.gscratch);
+            rc = launch_gemv_mma(ml, three, 3, xr, RWKVQ_F32, D, r, D, RWKVQ_EPI_NONE, nullptr, 1, s_rkv, x_each, true);
             if (rc) return rc;
         } else if (sb) {
             const rwkvq_qtensor three[3] = {L.Wr, L.Wk, L.Wv};
@@ -985,32 +1057,26 @@ int rwkvq_decode_step(const rwkvq_model* m, int B, const int64_t* tokens, float*
                 rc = launch_gemv_batch(three, 3, x3, h16, a3, B, D, y3, D, RWKVQ_EPI_NONE, nullptr, nullptr, s_rkv);
             if (rc) return rc;
         } else {
-            rc = linear(&L.Wr, xr, B, D, r, D, RWKVQ_EPI_NONE, nullptr, w.gscratch, w.gemm_ws, s_rkv, h16 ? w.xs16 : nullptr, am, nullptr, w.status);
+            rc = linear(&L.Wr, xr, B, D, r, D, RWKVQ_EPI_NONE, nullptr, w.gemm_ws, s_rkv, h16 ? w.xs16 : nullptr, am, nullptr, w.status);
             if (rc) return rc;
-            rc = linear(&L.Wk, xk, B, D, k, D, RWKVQ_EPI_NONE, nullptr, w.gscratch, w.gemm_ws, s_rkv,
+            rc = linear(&L.Wk, xk, B, D, k, D, RWKVQ_EPI_NONE, nullptr, w.gemm_ws, s_rkv,
                         h16 ? w.xs16 + 2 * BD : nullptr, bp ? am + 2 * B : nullptr, nullptr, w.status);
             if (rc) return rc;
-            rc = linear(&L.Wv, xv, B, D, v, D, RWKVQ_EPI_NONE, nullptr, w.gscratch, w.gemm_ws, s_rkv,
+            rc = linear(&L.Wv, xv, B, D, v, D, RWKVQ_EPI_NONE, nullptr, w.gemm_ws, s_rkv,
                         h16 ? w.xs16 + 3 * BD : nullptr, bp ? am + 3 * B : nullptr, nullptr, w.status);
             if (rc) return rc;
         }
-        float *yw = w.yl, *ya = w.yl + BD, *yv = w.yl + 2 * BD, *yg = w.yl + 3 * BD;
         {
-            const rwkvq_qtensor* t1[4] = {&L.w1, &L.a1, &L.g1, &L.v1};
-            const rwkvq_qtensor* t2[4] = {&L.w2, &L.a2, &L.g2, &L.v2};
-            const float* x1[4] = {xw, xa, xg, xv};
             float* y2[4] = {yw, ya, yg, yv};
-            const int act[4] = {1, 0, 2, 0};       // tanh (decay), none, sigmoid (gate), none
-            rc = lora_pair(t1, t2, x1, y2, act, layer0 ? 3 : 4, B, D, m->max_rank, w.part, w.part_floats, w.n_chunks, s_lora);
+            rc = lora_pair(t1, t2, x1, y2, act, n_br, B, D, m->max_rank, w.part, w.part_floats, w.n_chunks, s_lora);
             if (rc) return rc;
         }
         if (lane) {                                  // join before the time-mix core
             if (cudaEventRecord(lane->join, lane->stream) != cudaSuccess || cudaStreamWaitEvent(s, lane->join, 0) != cudaSuccess)
                 return fail(RWKVQ_E_LAUNCH, "rwkvq_decode_step: join of the side stream failed");
         }
-        TmixCoreArgs tc{r, k, v, yw, ya, layer0 ? nullptr : yv, yg, L.w0, L.a0, L.v0, L.k_k, L.k_a, L.r_k,
-                        L.lnx_w, L.lnx_b, w.v_first, wkv[l], w.og, D, H, layer0 ? 1 : 0, sb ? nullptr : am_og};
-        launch_pdl(tmix_core_kernel, dim3(H, B), dim3(256), 0, s, tc);
+        launch_pdl(tmix_core_kernel<false>, dim3(H, B), dim3(256), 0, s, tc, 0);
+        }
         if (sb) {
             const float* res[1] = {w.x};
             float *yx[1] = {w.x}, *yh[1] = {w.hffn};
@@ -1031,16 +1097,16 @@ int rwkvq_decode_step(const rwkvq_model* m, int B, const int64_t* tokens, float*
             if (rc) return rc;
             continue;
         }
-        rc = linear(&L.Wo, w.og, B, D, w.x, D, RWKVQ_EPI_ADD, w.x, w.gscratch, w.gemm_ws, stream, nullptr, am_og, nullptr, w.status);
+        rc = linear(&L.Wo, w.og, B, D, w.x, D, RWKVQ_EPI_ADD, w.x, w.gemm_ws, stream, nullptr, am_og, nullptr, w.status);
         if (rc) return rc;
         // ---- channel mix
         launch_pdl(D <= 8 * kRowThreads ? ln_shift_mix_kernel<1, 8> : ln_shift_mix_kernel<1, kRowPer>, dim3(B), dim3(kRowThreads), 0, s, w.x, L.ln2_w,
                    L.ln2_b, cshift[l], L.ffn_x_k, w.xk, B, D, h16 ? w.xk16 : static_cast<__half*>(nullptr), am_xk, 1, static_cast<float*>(nullptr),
                    static_cast<float*>(nullptr));
-        rc = linear(&L.Wfk, w.xk, B, D, w.hffn, F, RWKVQ_EPI_RELU2, nullptr, w.gscratch, w.gemm_ws, stream, h16 ? w.xk16 : nullptr, am_xk, am_h,
+        rc = linear(&L.Wfk, w.xk, B, D, w.hffn, F, RWKVQ_EPI_RELU2, nullptr, w.gemm_ws, stream, h16 ? w.xk16 : nullptr, am_xk, am_h,
                     w.status);
         if (rc) return rc;
-        rc = linear(&L.Wfv, w.hffn, B, F, w.x, D, RWKVQ_EPI_ADD, w.x, w.gscratch, w.gemm_ws, stream, nullptr, am_h, nullptr, w.status);
+        rc = linear(&L.Wfv, w.hffn, B, F, w.x, D, RWKVQ_EPI_ADD, w.x, w.gemm_ws, stream, nullptr, am_h, nullptr, w.status);
         if (rc) return rc;
     }
     if (sb) {
@@ -1056,7 +1122,7 @@ int rwkvq_decode_step(const rwkvq_model* m, int B, const int64_t* tokens, float*
         launch_pdl(D <= 8 * kRowThreads ? ln_shift_mix_kernel<0, 8> : ln_shift_mix_kernel<0, kRowPer>, dim3(B), dim3(kRowThreads), 0, s, w.x, m->lnout_w,
                    m->lnout_b, static_cast<float*>(nullptr), static_cast<const float*>(nullptr), w.xo, B, D, xo_h16 ? w.xo16 : static_cast<__half*>(nullptr),
                    am_xo, 1, static_cast<float*>(nullptr), static_cast<float*>(nullptr));
-        rc = linear(&m->head, w.xo, B, D, lg, V, RWKVQ_EPI_NONE, nullptr, w.gscratch, w.gemm_ws, stream, xo_h16 ? w.xo16 : nullptr, am_xo, nullptr,
+        rc = linear(&m->head, w.xo, B, D, lg, V, RWKVQ_EPI_NONE, nullptr, w.gemm_ws, stream, xo_h16 ? w.xo16 : nullptr, am_xo, nullptr,
                     w.status);
         if (rc) return rc;
     }

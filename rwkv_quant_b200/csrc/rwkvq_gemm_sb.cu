@@ -55,6 +55,7 @@ struct SbArgs {
     float* amax_out[kSbMaxMats];
     long long ldy;
     int n_tokens, epilogue;
+    int nt;                                       // tokens of a CTA's tile: 16, 32, 64 or, where NT is 128, any multiple of 16
     int row_tiles;                                // of one matrix
     int n_tiles;                                  // matrices * row_tiles
     int n_sb;                                     // super-blocks of a row
@@ -188,7 +189,7 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
     cg::cluster_group cluster = cg::this_cluster();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int ks = a.ks, z = blockIdx.x % ks, first_tile = blockIdx.x / ks, tile_step = gridDim.x / ks;
-    const int n0 = blockIdx.y * NT, nn = min(NT, a.n_tokens - n0);
+    const int nt = NT > 64 ? a.nt : NT, n0 = blockIdx.y * nt, nn = min(nt, a.n_tokens - n0);
     const int sb0 = a.n_sb * z / ks, n_super = a.n_sb * (z + 1) / ks - sb0, n_stages = n_super * 4;     // this CTA's K slice
     const int n_my = (a.n_tiles - first_tile + tile_step - 1) / tile_step;
 
@@ -257,12 +258,12 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
         const QView& t = a.t[mat];
         if (warp == kSbMmaWarp) {
             // ------------------------------------------------------------------ MMA issuer (whole warp, one lane elected)
-            const uint32_t id2 = umma_idesc(2 * NT), id1 = umma_idesc(NT);
+            const uint32_t id2 = umma_idesc(2 * nt), id1 = umma_idesc(nt);
             const uint64_t b0 = umma_desc(smem_addr(smem));
             const uint64_t ma0 = umma_desc_plain(smem_addr(smem + G::OFF_MA), kGmRows * 16, 128);
-            const uint64_t mb0 = umma_desc_plain(smem_addr(smem + G::OFF_MB), 2 * NT * 16, 128);
+            const uint64_t mb0 = umma_desc_plain(smem_addr(smem + G::OFF_MB), 2 * nt * 16, 128);
             if (ti == 0) pdl_wait();
-            for (int n = lane; n < NT; n += 32) s_un[n] = n < nn ? __ldcg(a.unscale[mat] + n0 + n) : 0.f;   // read behind bar_done
+            for (int n = lane; n < nt; n += 32) s_un[n] = n < nn ? __ldcg(a.unscale[mat] + n0 + n) : 0.f;   // read behind bar_done
             uint32_t elected;
             asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xFFFFFFFF;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(elected));
             bool ok = true;
@@ -297,15 +298,15 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
                     if (g >= G::ST && !mbar_wait_bounded(&bar_empty[st], (g / G::ST - 1) & 1)) { s_fail = 1; break; }
                     unsigned char* b = smem + st * G::BSLAB;
                     const bool with_sums = Y::SB6 && (i & 3) == 0;
-                    mbar_expect_tx(&bar_full[st], G::BSLAB + (with_sums ? 2 * nn * 16 : 0));
+                    mbar_expect_tx(&bar_full[st], 2 * nt * 128 + (with_sums ? 2 * nn * 16 : 0));
                     tma_load_2d(b, &maps.hi[mat], sb0 * 256 + i * 64, n0, &bar_full[st]);
-                    tma_load_2d(b + NT * 128, &maps.lo[mat], sb0 * 256 + i * 64, n0, &bar_full[st]);
+                    tma_load_2d(b + nt * 128, &maps.lo[mat], sb0 * 256 + i * 64, n0, &bar_full[st]);
                     if (with_sums) {
                         unsigned char* m = smem + G::OFF_MB + ((g >> 2) & 1) * G::MB;
 #pragma unroll
                         for (int h = 0; h < 2; ++h)
                             asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                                             smem_addr(m + h * NT * 16)),
+                                             smem_addr(m + h * nt * 16)),
                                          "l"(a.sums[mat] + ((static_cast<size_t>(sb0 + (i >> 2)) * 2 + h) * a.n_tokens + n0) * 8), "r"(nn * 16),
                                          "r"(smem_addr(&bar_full[st]))
                                          : "memory");
@@ -391,8 +392,7 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
             tc_fence_after();
             if (ti == 0) pdl_wait();                                 // token scales, residual, output
         }
-        constexpr int TPW = NT / 4;                                  // tokens per warp: four warps share a lane quadrant
-        constexpr int TC = TPW < 16 ? TPW : 16;                      // ... in chunks of at most 16
+        constexpr int TC = NT < 64 ? NT / 4 : 16;                    // tokens a warp takes at a time; four warps share a lane quadrant
         const int q = warp & 3, tg = warp >> 2, rl = q * 32 + lane, row = row0 + rl;
         const bool row_ok = row < t.rows && !s_fail;
         float* y = a.y[mat] + static_cast<size_t>(n0) * a.ldy + row;
@@ -424,20 +424,22 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
         };
         auto accumulators = [&](float (&v)[TC], int c0) {
             float lo[TC];
-            const uint32_t base = tmem + (static_cast<uint32_t>(q * 32) << 16) + tg * TPW + c0;
+            const uint32_t base = tmem + (static_cast<uint32_t>(q * 32) << 16) + c0;
             sb_tmem_ld<TC>(base, v);
-            sb_tmem_ld<TC>(base + NT, lo);
+            sb_tmem_ld<TC>(base + nt, lo);
 #pragma unroll
-            for (int j = 0; j < TC; ++j) v[j] = (v[j] + lo[j]) * s_un[tg * TPW + c0 + j];
+            for (int j = 0; j < TC; ++j) v[j] = (v[j] + lo[j]) * s_un[c0 + j];
         };
         if (ks == 1) {
             if (warp < kSbTmaWarp) {
 #pragma unroll 1
-                for (int c0 = 0; c0 < TPW; c0 += TC) {
+                for (int c = 0; c < NT; c += 4 * TC) {              // one pass up to 64 tokens
+                    const int c0 = c + tg * TC;
+                    if (c0 >= nt) break;
                     float v[TC], r[TC];
-                    load_resid(r, tg * TPW + c0, 1, nn);
+                    load_resid(r, c0, 1, nn);
                     accumulators(v, c0);
-                    store(v, r, tg * TPW + c0, 1, nn);
+                    store(v, r, c0, 1, nn);
                 }
                 tc_fence_before();
             }
@@ -448,16 +450,18 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
             float* part = reinterpret_cast<float*>(smem);            // every MMA that read the operands has completed
             if (warp < kSbTmaWarp) {
 #pragma unroll 1
-                for (int c0 = 0; c0 < TPW; c0 += TC) {
+                for (int c = 0; c < NT; c += 4 * TC) {              // one pass up to 64 tokens
+                    const int c0 = c + tg * TC;
+                    if (c0 >= nt) break;
                     float v[TC];
                     accumulators(v, c0);
 #pragma unroll
-                    for (int j = 0; j < TC; ++j) part[(tg * TPW + c0 + j) * kSbPitch + rl] = v[j];
+                    for (int j = 0; j < TC; ++j) part[(c0 + j) * kSbPitch + rl] = v[j];
                 }
                 tc_fence_before();
             }
             // this CTA's share of the tokens, ranks added in order; U tokens of K ranks in flight per thread
-            const int per = (NT + ks - 1) / ks, first = z * per + tg, end = min(nn, (z + 1) * per);
+            const int per = (nn + ks - 1) / ks, first = z * per + tg, end = min(nn, (z + 1) * per);
             auto reduce = [&](auto u_tag, auto k_tag) {
                 constexpr int U = decltype(u_tag)::value, K = decltype(k_tag)::value;
                 float r[U];
@@ -472,7 +476,7 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
                         for (int u = 0; u < K; ++u) {
                             const float* src = cluster.map_shared_rank(part, u < ks ? u : 0);
 #pragma unroll
-                            for (int j = 0; j < U; ++j) pv[u][j] = u < ks ? src[min(nb + 4 * j, NT - 1) * kSbPitch + rl] : 0.f;
+                            for (int j = 0; j < U; ++j) pv[u][j] = u < ks ? src[min(nb + 4 * j, nt - 1) * kSbPitch + rl] : 0.f;
                         }
 #pragma unroll
                         for (int j = 0; j < U; ++j) {
@@ -590,9 +594,9 @@ int launch_sb(SbArgs& a, const SbMaps& maps, int groups, int force_ks, cudaStrea
         if (dev < 64) configured[dev] = true;
     }
     // K split into up to 8 slices of whole super-blocks, by a model of the slowest CTA in microseconds fitted to
-    // [2048, 2048] .. [65536, 2048] at 8 to 100 rows: 0.36 to 0.55 a stage, 5 for ramp and store, 3.5 for the cluster
+    // [2048, 2048] .. [65536, 2048] at 8 to 128 rows: 0.37 to 0.55 a stage by the tile's width, 5 for ramp and store, 3.5 for the cluster
     // reduction; without a split the CTAs are persistent and pay the ramp once
-    const double stage = NT > 64 ? 0.55 : NT > 32 ? 0.41 : 0.37;
+    const double stage = std::max(0.37, 0.41 + 0.0022 * (a.nt - 64));
     double best = 1e300;
     a.ks = 1;
     for (int c = 1; c <= 8 && c <= a.n_sb; ++c) {
@@ -622,12 +626,10 @@ int launch_sb(SbArgs& a, const SbMaps& maps, int groups, int force_ks, cudaStrea
 
 template <int L>
 int launch_sb_nt(SbArgs& a, const SbMaps& maps, int nt, int groups, int force_ks, cudaStream_t s) {
-    switch (nt) {
-        case 16: return launch_sb<L, 16>(a, maps, groups, force_ks, s);
-        case 32: return launch_sb<L, 32>(a, maps, groups, force_ks, s);
-        case 64: return launch_sb<L, 64>(a, maps, groups, force_ks, s);
-        default: return launch_sb<L, 128>(a, maps, groups, force_ks, s);
-    }
+    if (nt <= 16) return launch_sb<L, 16>(a, maps, groups, force_ks, s);
+    if (nt <= 32) return launch_sb<L, 32>(a, maps, groups, force_ks, s);
+    if (nt <= 64) return launch_sb<L, 64>(a, maps, groups, force_ks, s);
+    return launch_sb<L, 128>(a, maps, groups, force_ks, s);
 }
 
 }  // namespace
@@ -635,10 +637,12 @@ int launch_sb_nt(SbArgs& a, const SbMaps& maps, int nt, int groups, int force_ks
 bool gemm_sb_ok(const rwkvq_qtensor& t) {
     return gemm_tcb_ok(t) && (t.kind == RWKVQ_KIND_SB6 || t.kind == RWKVQ_KIND_SYM) && mma_layout_of(t) >= 0;
 }
-// Whether this kernel takes a product the mma.sync kernel serves too.
+// Whether this kernel takes a product the mma.sync kernel serves too.  That one stages the activations per row group,
+// which costs it as much as the conversion to tensor memory costs this one up to 16 rows ([2048, 2048] 14.3 against 18 us,
+// [8192, 2048] and [2048, 8192] 17 both); from there its time doubles with every 16 rows and this one's stays.
+constexpr int kSbLeastRows = 17;
 bool gemm_sb_pays(const rwkvq_qtensor& t, int N) {
-    static const int least = [] { const char* e = getenv("SBMIN"); return e ? atoi(e) : 17; }();
-    return tcb_enabled() && gemm_sb_ok(t) && N >= least;
+    return tcb_enabled() && gemm_sb_ok(t) && N >= kSbLeastRows;
 }
 
 int launch_gemm_sb(const rwkvq_qtensor* ts, int n_mats, const SbRows* rows, int N, float* const* ys, long long ldy, int epilogue,
@@ -646,7 +650,11 @@ int launch_gemm_sb(const rwkvq_qtensor* ts, int n_mats, const SbRows* rows, int 
     RWKVQ_REQUIRE(n_mats >= 1 && n_mats <= kSbMaxMats, RWKVQ_E_LIMIT, "gemm_sb: %d matrices", n_mats);
     SbArgs a{};
     SbMaps maps;
-    const int nt = N <= 16 ? 16 : N <= 32 ? 32 : N <= 64 ? 64 : 128, groups = (N + nt - 1) / nt;
+    // token groups of at most 128, tiles as wide as they need (the tensor time of a stage goes with the width: 100 rows
+    // 4.24 -> 4.18 ms per decode step); up to 64 the width is the template's (known to the epilogue: 2.83 against 2.88 ms)
+    const int groups = (N + 127) / 128, per = (N + groups - 1) / groups;
+    const int nt = per <= 16 ? 16 : per <= 32 ? 32 : per <= 64 ? 64 : (per + 15) / 16 * 16;
+    a.nt = nt;
     for (int k = 0; k < n_mats; ++k) {
         RWKVQ_REQUIRE(gemm_sb_ok(ts[k]) && ts[k].kind == ts[0].kind && ts[k].bits == ts[0].bits && ts[k].rows == ts[0].rows &&
                           ts[k].cols == ts[0].cols, RWKVQ_E_SHAPE, "gemm_sb: fused matrices must share layout and shape");

@@ -1,8 +1,15 @@
 // Single-vector decode GEMV on the integer tensor-core path: the stand-alone kernel,
 // its launcher and the relayout kernels.  The arithmetic is described in rwkvq_gemv_mma.cuh.
+#include <cooperative_groups.h>
+
+#include <algorithm>
 #include <cstdlib>
+#include <type_traits>
 
 #include "rwkvq_gemv_mma.cuh"
+#include "rwkvq_lora_vec.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace rwkvq {
 
@@ -14,13 +21,28 @@ namespace rwkvq {
 // before item n is consumed.
 // ZS: the exact zero-group skip (see prepare_x / load_frag), a compile-time variant so that launches
 // without it carry none of its instructions
-template <int L, int WK, bool SPLIT, bool ZS>      // SPLIT: the K loop is also split across gridDim.z CTAs
-__global__ void __launch_bounds__(kMmaWarps * 32, 2) gemv_mma_kernel(const MmaArgs a) {
+// SPLIT: the K loop is also split over a cluster of gridDim.z CTAs.  Bound: latency (the [2048, 8192] product streams 9.4 MB,
+// 1.4 us; its chain is x, block maximum, digits, two iterations, sum).  Hence each CTA prepares its own slice of x only,
+// scaled by the slice's maximum (never coarser than the row's), and the slices meet in distributed shared memory instead
+// of global scratch with an arrival counter: MEASURED_SPLIT.
+// LORA: grid rows from n_mats on are the LoRA down projections of the same layer (rwkvq_lora_vec.cuh).
+template <int L, int WK, bool SPLIT, bool ZS, int LORA>
+__global__ void __launch_bounds__(kMmaWarps * 32, 2) gemv_mma_kernel(const MmaArgs a, const std::conditional_t<LORA != 0, LoraVecArgs, int> lora) {
+    if constexpr (LORA != 0) {
+        if (static_cast<int>(blockIdx.y) >= a.n_mats) {
+            const int cta = (static_cast<int>(blockIdx.y) - a.n_mats) * static_cast<int>(gridDim.x) + static_cast<int>(blockIdx.x);
+            pdl_launch_dependents();
+            if (cta * kLvCols < lora.first[lora.n_br]) lora_down_vec<LORA>(lora, cta);
+            return;
+        }
+    }
     using G = Geo<L>;
     constexpr int WT = kMmaWarps / WK;
     extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ float s_part[2][SPLIT ? WT * 16 : 1];                // row sums of this slice, two tiles
     const QView& q = a.t[blockIdx.y];
-    const int n_in = q.cols;
+    const int KS = SPLIT ? static_cast<int>(gridDim.z) : 1;  // K slices across CTAs
+    const int n_in = q.cols / KS;                           // columns of this CTA's slice
     int8_t* dig = reinterpret_cast<int8_t*>(smem);
     float* xs16 = reinterpret_cast<float*>(dig + 3 * n_in);
     float* red = xs16 + (n_in >> 4);                                     // [2][kMmaWarps * 16]
@@ -29,8 +51,7 @@ __global__ void __launch_bounds__(kMmaWarps * 32, 2) gemv_mma_kernel(const MmaAr
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     const int tl = warp / WK, ks = warp % WK;
-    const int KS = SPLIT ? static_cast<int>(gridDim.z) : 1;  // K slices across CTAs
-    const int n_iters = n_in / G::KI / KS;                  // iterations of this CTA's slice
+    const int n_iters = n_in / G::KI;                       // iterations of this CTA's slice
     const int it0 = SPLIT ? blockIdx.z * n_iters : 0;
     const int n_tiles = (q.rows + 15) >> 4;
     const int step = gridDim.x * WT;
@@ -62,11 +83,11 @@ __global__ void __launch_bounds__(kMmaWarps * 32, 2) gemv_mma_kernel(const MmaAr
     const char* xv = a.xk[blockIdx.y] ? static_cast<const char*>(a.xk[blockIdx.y])
                                       : static_cast<const char*>(a.x) + (a.fused ? blockIdx.y * a.ldx * esz : 0);
     bool finite;
-    const float unscale = prepare_x(xv, a.x_dtype, n_in, x_bits<L>(), dig, xs16, red, finite, ZS ? zflag : nullptr);
+    const float unscale = prepare_x(xv + static_cast<size_t>(it0) * G::KI * esz, a.x_dtype, n_in, x_bits<L>(), dig, xs16, red, finite, ZS ? zflag : nullptr);
     __syncthreads();
     // exact sparsity skip: groups of 32 columns whose activations are all zero (relu(k)^2 in the channel
     // mix) are not read from the second fetch on
-    if (ZS) zf = zflag;
+    if (ZS) zf = zflag - it0 * (G::KI / 32);
 
     int c_n = 0, buf = 0;
     for (int base = blockIdx.x * WT; base < n_tiles; base += step, buf ^= 1) {
@@ -76,9 +97,7 @@ __global__ void __launch_bounds__(kMmaWarps * 32, 2) gemv_mma_kernel(const MmaAr
             const Frag<L> cur = nxt;
             fetch_next();
             if (tile >= n_tiles) continue;
-            const int it = it0 + ks + j * WK;
-
-            consume_frag<L>(cur, it, g, t, dig, n_in, xs16, acc0, acc1);
+            consume_frag<L>(cur, ks + j * WK, g, t, dig, n_in, xs16, acc0, acc1);
         }
         // the 4 lanes of a quad hold the 8 blocks of each iteration
         acc0 += __shfl_xor_sync(0xFFFFFFFFu, acc0, 1); acc0 += __shfl_xor_sync(0xFFFFFFFFu, acc0, 2);
@@ -102,42 +121,31 @@ __global__ void __launch_bounds__(kMmaWarps * 32, 2) gemv_mma_kernel(const MmaAr
                 }
             }
         } else {
-            __shared__ unsigned int s_last;
-            float* part = a.partial + (static_cast<size_t>(blockIdx.z) * gridDim.y + blockIdx.y) * a.rows_padded;
+            // own slice's sums; every rank walks the same tiles, so the barrier is uniform and, with two buffers, the one
+            // of the next tile also says that this one has been read
             if (threadIdx.x < WT * 16) {
                 const int wtl = threadIdx.x >> 4, r = threadIdx.x & 15;
-                const int row = (base + wtl) * 16 + r;
                 float v = 0.f;
 #pragma unroll
                 for (int k = 0; k < WK; ++k) v += rb[(wtl * WK + k) * 16 + r];
-                if (row < a.rows_padded) __stcg(part + row, finite ? v * unscale : NAN);
+                s_part[buf][threadIdx.x] = finite ? v * unscale : NAN;
             }
-            __threadfence();
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                unsigned int* ctr = a.counters + blockIdx.y * ((n_tiles + WT - 1) / WT) + base / WT;
-                const unsigned int old = atomicAdd(ctr, 1u);
-                s_last = (old == static_cast<unsigned int>(KS - 1));
-                if (s_last) *ctr = 0u;                      // ready for the next launch
-            }
-            __syncthreads();
-            if (s_last) {
-                __threadfence();
-                if (threadIdx.x < WT * 16) {
-                    const int row = base * 16 + threadIdx.x;
-                    if (row < q.rows) {
-                        float v = 0.f;
-                        for (int z = 0; z < KS; ++z)
-                            v += __ldcg(a.partial + (static_cast<size_t>(z) * gridDim.y + blockIdx.y) * a.rows_padded + row);
-                        const long long idx = (a.fused ? static_cast<long long>(blockIdx.y) * a.ldy : 0) + row;
-                        if (a.epilogue == RWKVQ_EPI_RELU2) { v = fmaxf(v, 0.f); v = v * v; }
-                        else if (a.epilogue == RWKVQ_EPI_ADD) v = __fadd_rn(v, __ldcg(a.resid + idx));
-                        a.y[idx] = v;
-                    }
+            cg::cluster_group cluster = cg::this_cluster();
+            cluster.sync();
+            if (blockIdx.z == 0 && threadIdx.x < WT * 16) {
+                const int row = base * 16 + threadIdx.x;
+                if (row < q.rows) {
+                    float v = s_part[buf][threadIdx.x];
+                    for (int z = 1; z < KS; ++z) v += cluster.map_shared_rank(&s_part[buf][threadIdx.x], z)[0];
+                    const long long idx = (a.fused ? static_cast<long long>(blockIdx.y) * a.ldy : 0) + row;
+                    if (a.epilogue == RWKVQ_EPI_RELU2) { v = fmaxf(v, 0.f); v = v * v; }
+                    else if (a.epilogue == RWKVQ_EPI_ADD) v = __fadd_rn(v, __ldcg(a.resid + idx));
+                    a.y[idx] = v;
                 }
             }
         }
     }
+    if (SPLIT) cg::this_cluster().sync();                           // nobody leaves while a peer still reads its sums
 }
 
 // ------------------------------------------------------------ relayout kernels
@@ -213,28 +221,48 @@ static bool zero_skip_enabled() {
 }
 
 constexpr int kResidentCtas = 2 * 148;     // 2 CTAs of 256 threads per SM at <= 128 registers
-constexpr int kSplitMaxRows = 4096;        // rows a K-split launch may have (scratch sizing)
-constexpr int kSplitMaxSlices = 4;
+constexpr int kSplitAnyCols = 4096;        // rows from which on the K split does not depend on the caller
+constexpr int kSplitMaxRows = 4096;        // rows a K-split launch may have: above, the row tiles alone fill the chip
 
-// Scratch of a K-split launch: partial sums, then the (self-resetting) arrival counters.
-size_t gemv_mma_scratch_bytes() {
-    return sizeof(float) * kSplitMaxSlices * kMmaMaxFused * kSplitMaxRows + sizeof(unsigned int) * 1024;
-}
-
-template <int L, int WK, bool SPLIT, bool ZS>
-static int launch_one_zs(MmaArgs& a, int rows, int cols, int n_mats, int KS, cudaStream_t s) {
+template <int L, int WK, bool SPLIT, bool ZS, int LORA = 0>
+static int launch_one_zs(MmaArgs& a, int rows, int cols, int n_mats, int KS, cudaStream_t s, const LoraVecArgs* lora = nullptr) {
     constexpr int WT = kMmaWarps / WK;
-    const size_t smem = 3 * static_cast<size_t>(cols) + 4 * (cols / 16) + 2 * kMmaWarps * 16 * 4 + ((cols / 32 + 15) / 16) * 16;
+    const int slice = cols / KS;
+    const size_t smem = 3 * static_cast<size_t>(slice) + 4 * (slice / 16) + 2 * kMmaWarps * 16 * 4 + ((slice / 32 + 15) / 16) * 16;
     if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(gemv_mma_kernel<L, WK, SPLIT, ZS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaError_t e = cudaFuncSetAttribute(gemv_mma_kernel<L, WK, SPLIT, ZS, LORA>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              static_cast<int>(smem));
         if (e != cudaSuccess) return fail(RWKVQ_E_LIMIT, "gemv_mma: %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
     }
     const int units = ((rows + 15) / 16 + WT - 1) / WT;
     const int cap = kResidentCtas / (n_mats * KS) > 0 ? kResidentCtas / (n_mats * KS) : 1;
-    a.rows_padded = ((rows + 15) / 16) * 16;
-    cudaError_t le = launch_pdl(gemv_mma_kernel<L, WK, SPLIT, ZS>, dim3(units < cap ? units : cap, n_mats, KS),
-                                dim3(kMmaWarps * 32), smem, s, a);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(units < cap ? units : cap, n_mats, KS);
+    if constexpr (LORA != 0) {                   // still one wave: the tiles walk what the LoRA CTAs leave
+        const int extra = lora->first[lora->n_br] / kLvCols, room = std::max(1, (kResidentCtas - extra) / n_mats);
+        cfg.gridDim.x = std::min(units, room);
+        cfg.gridDim.y = n_mats + (extra + cfg.gridDim.x - 1) / cfg.gridDim.x;
+    }
+    cfg.blockDim = dim3(kMmaWarps * 32);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    int n_attr = 0;
+    if (SPLIT) {
+        attr[n_attr].id = cudaLaunchAttributeClusterDimension;
+        attr[n_attr].val.clusterDim.x = 1; attr[n_attr].val.clusterDim.y = 1; attr[n_attr].val.clusterDim.z = KS;
+        ++n_attr;
+    }
+    if (pdl_enabled()) {
+        attr[n_attr].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n_attr].val.programmaticStreamSerializationAllowed = 1;
+        ++n_attr;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n_attr;
+    cudaError_t le;
+    if constexpr (LORA != 0) le = cudaLaunchKernelEx(&cfg, gemv_mma_kernel<L, WK, SPLIT, ZS, LORA>, a, *lora);
+    else le = cudaLaunchKernelEx(&cfg, gemv_mma_kernel<L, WK, SPLIT, ZS, LORA>, a, 0);
     if (le != cudaSuccess) return fail(RWKVQ_E_LAUNCH, "gemv_mma: %s", cudaGetErrorString(le));
     return RWKVQ_OK;
 }
@@ -251,25 +279,24 @@ static int launch_one(MmaArgs& a, int rows, int cols, int n_mats, int KS, cudaSt
 }
 
 // Work split: a single wave of co-resident CTAs whenever the matrix allows it.
-//   * few row tiles, long rows  -> K is also split across CTAs (needs scratch)
+//   * few row tiles, long rows  -> K is also split across CTAs (a cluster of 2 or 4; `split`)
 //   * tiles * n_mats <= resident CTAs -> one tile per CTA, its 8 warps split K
 //   * more tiles -> WT tiles per CTA so that the grid still fits one wave
 //   * very many tiles (head) -> persistent CTAs, 8 warps split K of each tile
 template <int L>
-static int launch_wk(MmaArgs& a, int rows, int cols, int n_mats, float* scratch, cudaStream_t s) {
+static int launch_wk(MmaArgs& a, int rows, int cols, int n_mats, bool split, cudaStream_t s) {
     const int n_iters = cols / Geo<L>::KI;
     const int tiles = (rows + 15) / 16;
     int KS = 1;
-    // the kernel gives every slice n_iters / KS iterations: only an exact division covers the row
-    if (scratch && n_iters >= 16 && rows <= kSplitMaxRows) {
-        if (tiles * n_mats * 4 <= kResidentCtas && n_iters >= 32 && n_iters % 4 == 0) KS = 4;
-        else if (tiles * n_mats * 2 <= kResidentCtas && n_iters % 2 == 0) KS = 2;
+    // the kernel gives every slice n_iters / KS iterations: only an exact division covers the row.  Rows of 4096 columns on
+    // split whoever calls and whatever shares the launch (a fused launch then equals its separate ones bit for bit);
+    // shorter ones only where the caller has nothing else to fill the chip with (`split`).
+    const int ctas = tiles * (cols >= kSplitAnyCols ? 1 : n_mats);
+    if ((split || cols >= kSplitAnyCols) && n_iters >= 16 && rows <= kSplitMaxRows) {
+        if (ctas * 4 <= kResidentCtas && n_iters >= 32 && n_iters % 4 == 0) KS = 4;
+        else if (ctas * 2 <= kResidentCtas && n_iters % 2 == 0) KS = 2;
     }
-    if (KS > 1) {
-        a.partial = scratch;
-        a.counters = reinterpret_cast<unsigned int*>(scratch + kSplitMaxSlices * kMmaMaxFused * kSplitMaxRows);
-        return launch_one<L, 8, true>(a, rows, cols, n_mats, KS, s);
-    }
+    if (KS > 1) return launch_one<L, 8, true>(a, rows, cols, n_mats, KS, s);
     int wt = 1;
     if (tiles * n_mats > kResidentCtas) {
         wt = 0;
@@ -288,23 +315,62 @@ static int launch_wk(MmaArgs& a, int rows, int cols, int n_mats, float* scratch,
 }
 
 // Launch the single-vector tensor-core GEMV for `n_mats` same-shape matrices.
-// `scratch` (gemv_mma_scratch_bytes(), zero-initialised once, reusable) enables the
-// K split across CTAs; nullptr disables it.
+// `split` allows the K split across CTAs for rows shorter than kSplitAnyCols too.
 int launch_gemv_mma(int layout, const rwkvq_qtensor* ts, int n_mats, const void* x, int x_dtype,
                     long long ldx, float* y, long long ldy, int epilogue, const float* resid,
-                    int fused, cudaStream_t s, const void* const* x_each, float* scratch) {
+                    int fused, cudaStream_t s, const void* const* x_each, bool split) {
     MmaArgs a{};
     for (int k = 0; k < n_mats; ++k) { a.t[k] = make_view(ts[k]); a.xk[k] = x_each ? x_each[k] : nullptr; }
     a.x = x; a.x_dtype = x_dtype; a.ldx = ldx; a.y = y; a.ldy = ldy;
     a.resid = resid; a.epilogue = epilogue; a.fused = fused;
     const int rows = ts[0].rows, cols = ts[0].cols;
     switch (layout) {
-        case ML_SB6_4: return launch_wk<ML_SB6_4>(a, rows, cols, n_mats, scratch, s);
-        case ML_SB6_5: return launch_wk<ML_SB6_5>(a, rows, cols, n_mats, scratch, s);
-        case ML_SB6_6: return launch_wk<ML_SB6_6>(a, rows, cols, n_mats, scratch, s);
-        case ML_SYM6: return launch_wk<ML_SYM6>(a, rows, cols, n_mats, scratch, s);
-        case ML_RTN8: return launch_wk<ML_RTN8>(a, rows, cols, n_mats, scratch, s);
-        default: return launch_wk<ML_SYM8>(a, rows, cols, n_mats, scratch, s);
+        case ML_SB6_4: return launch_wk<ML_SB6_4>(a, rows, cols, n_mats, split, s);
+        case ML_SB6_5: return launch_wk<ML_SB6_5>(a, rows, cols, n_mats, split, s);
+        case ML_SB6_6: return launch_wk<ML_SB6_6>(a, rows, cols, n_mats, split, s);
+        case ML_SYM6: return launch_wk<ML_SYM6>(a, rows, cols, n_mats, split, s);
+        case ML_RTN8: return launch_wk<ML_RTN8>(a, rows, cols, n_mats, split, s);
+        default: return launch_wk<ML_SYM8>(a, rows, cols, n_mats, split, s);
+    }
+}
+
+template <int L>
+static int launch_rkv_lora(MmaArgs& a, int rows, int cols, int n_mats, const LoraVecArgs& lora, cudaStream_t s) {
+    switch ((lora.D / 4 + 255) / 256) {
+        case 1: return launch_one_zs<L, 4, false, false, 1>(a, rows, cols, n_mats, 1, s, &lora);
+        case 2: return launch_one_zs<L, 4, false, false, 2>(a, rows, cols, n_mats, 1, s, &lora);
+        case 3: return launch_one_zs<L, 4, false, false, 3>(a, rows, cols, n_mats, 1, s, &lora);
+        default: return launch_one_zs<L, 4, false, false, 4>(a, rows, cols, n_mats, 1, s, &lora);
+    }
+}
+
+bool lora_vec_ok(const rwkvq_qtensor* const* t1, const rwkvq_qtensor* const* t2, int n_br, int D) {
+    int ranks = 0;
+    for (int i = 0; i < n_br; ++i) {
+        const int r = t1[i]->cols;
+        if (t1[i]->rows != D || t2[i]->rows != r || t2[i]->cols != D || r % 16 != 0) return false;
+        ranks += r;
+        for (const rwkvq_qtensor* t : {t1[i], t2[i]}) {
+            if (t->kind == RWKVQ_KIND_ASYM ? t->gs % 4 != 0 : !(t->kind == RWKVQ_KIND_RTN && t->bits > 4)) return false;
+            if (!aligned(t->codes, 16)) return false;
+        }
+    }
+    return D % 64 == 0 && D <= kLvMaxD && ranks > 0 && lora_vec_smem(ranks) <= static_cast<size_t>(kLvMaxSmem);
+}
+
+int launch_gemv_mma_lora(int layout, const rwkvq_qtensor* ts, int n_mats, const void* const* x_each, float* y, long long ldy,
+                         const LoraVecArgs& lora, cudaStream_t s) {
+    MmaArgs a{};
+    for (int k = 0; k < n_mats; ++k) { a.t[k] = make_view(ts[k]); a.xk[k] = x_each[k]; }
+    a.x_dtype = RWKVQ_F32; a.ldx = ts[0].cols; a.y = y; a.ldy = ldy; a.epilogue = RWKVQ_EPI_NONE; a.fused = 1; a.n_mats = n_mats;
+    const int rows = ts[0].rows, cols = ts[0].cols;
+    switch (layout) {
+        case ML_SB6_4: return launch_rkv_lora<ML_SB6_4>(a, rows, cols, n_mats, lora, s);
+        case ML_SB6_5: return launch_rkv_lora<ML_SB6_5>(a, rows, cols, n_mats, lora, s);
+        case ML_SB6_6: return launch_rkv_lora<ML_SB6_6>(a, rows, cols, n_mats, lora, s);
+        case ML_SYM6: return launch_rkv_lora<ML_SYM6>(a, rows, cols, n_mats, lora, s);
+        case ML_RTN8: return launch_rkv_lora<ML_RTN8>(a, rows, cols, n_mats, lora, s);
+        default: return launch_rkv_lora<ML_SYM8>(a, rows, cols, n_mats, lora, s);
     }
 }
 
@@ -343,42 +409,10 @@ int rwkvq_relayout_planes(const rwkvq_qtensor* t, void* planes_out, void* stream
 
 }  // extern "C"
 
-// ------------------------------------------------- K-split GEMV, built-in scratch
-// The K-split launch needs room for the slices' partial row sums and for its
-// arrival counters.  This variant keeps that room in the module image, so the call
-// path never asks the CUDA allocator for anything.
+// ------------------------------------------------- K-split GEMV as an entry point
 namespace rwkvq {
-
 constexpr int kStaticMaxRows = kSplitMaxRows;     // largest OUT served
 constexpr int kStaticMaxCols = 16384;             // largest IN served (shared-memory staging of x)
-constexpr size_t kStaticPartialFloats = static_cast<size_t>(kSplitMaxSlices) * kMmaMaxFused * kSplitMaxRows;
-constexpr size_t kStaticCounterWords = 1024;
-constexpr int kStaticMaxDevices = 64;
-
-// 256 KiB of partial sums followed by 4 KiB of counters; zero at module load.
-static __device__ __align__(256) float g_static_scratch[kStaticPartialFloats + kStaticCounterWords];
-
-// Device address of the scratch on the current device, looked up once per device.
-static int static_scratch(float** out) {
-    static float* ptrs[kStaticMaxDevices] = {};
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return fail(RWKVQ_E_LAUNCH, "rwkvq_gemv_static: cudaGetDevice: %s", cudaGetErrorString(e));
-    if (dev < 0 || dev >= kStaticMaxDevices)
-        return fail(RWKVQ_E_LIMIT, "rwkvq_gemv_static: device ordinal %d, at most %d devices", dev, kStaticMaxDevices);
-    float* p = __atomic_load_n(&ptrs[dev], __ATOMIC_ACQUIRE);
-    if (p == nullptr) {
-        void* sym = nullptr;
-        e = cudaGetSymbolAddress(&sym, g_static_scratch);
-        if (e != cudaSuccess || sym == nullptr)
-            return fail(RWKVQ_E_LAUNCH, "rwkvq_gemv_static: cudaGetSymbolAddress: %s", cudaGetErrorString(e));
-        p = static_cast<float*>(sym);
-        __atomic_store_n(&ptrs[dev], p, __ATOMIC_RELEASE);   // racing threads store the same address
-    }
-    *out = p;
-    return RWKVQ_OK;
-}
-
 }  // namespace rwkvq
 
 extern "C" int rwkvq_gemv_static(const rwkvq_qtensor* t, const void* x, int x_dtype, float* y, int epilogue,
@@ -396,15 +430,8 @@ extern "C" int rwkvq_gemv_static(const rwkvq_qtensor* t, const void* x, int x_dt
     RWKVQ_REQUIRE(ml >= 0, RWKVQ_E_DTYPE,
                   "rwkvq_gemv_static: needs an sb6 tensor with relayouted records/planes, a sym tensor or per-row int8");
     RWKVQ_REQUIRE(t->rows <= kStaticMaxRows && t->cols <= kStaticMaxCols, RWKVQ_E_LIMIT,
-                  "rwkvq_gemv_static: [%d, %d] exceeds the built-in scratch, at most [%d, %d]", t->rows, t->cols,
+                  "rwkvq_gemv_static: [%d, %d] is above the served sizes, at most [%d, %d]", t->rows, t->cols,
                   kStaticMaxRows, kStaticMaxCols);
-    float* scratch = nullptr;
-    rc = static_scratch(&scratch);
-    if (rc) return rc;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    // the arrival counters must read zero when the kernel starts
-    cudaError_t e = cudaMemsetAsync(scratch + kStaticPartialFloats, 0, kStaticCounterWords * sizeof(unsigned int), s);
-    if (e != cudaSuccess) return fail(RWKVQ_E_LAUNCH, "rwkvq_gemv_static: cudaMemsetAsync: %s", cudaGetErrorString(e));
-    rc = launch_gemv_mma(ml, t, 1, x, x_dtype, t->cols, y, t->rows, epilogue, resid, 0, s, nullptr, scratch);
+    rc = launch_gemv_mma(ml, t, 1, x, x_dtype, t->cols, y, t->rows, epilogue, resid, 0, static_cast<cudaStream_t>(stream), nullptr, true);
     return rc ? rc : check_launch("rwkvq_gemv_static");
 }

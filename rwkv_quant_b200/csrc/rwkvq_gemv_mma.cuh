@@ -41,12 +41,7 @@ struct MmaArgs {
     const float* resid;
     int epilogue;
     int fused;
-    // split of the K loop over gridDim.z CTAs: partial row sums go to `partial`
-    // [gridDim.z][n_mats][rows_padded] and the last CTA of a tile group to arrive
-    // (counted in `counters`, which it resets) adds them in slice order
-    float* partial;
-    unsigned int* counters;
-    int rows_padded;
+    int n_mats;         // set where the grid has rows beyond the matrices
 };
 
 template <bool A_UNSIGNED>
