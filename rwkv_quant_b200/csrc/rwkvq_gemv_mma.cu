@@ -14,6 +14,10 @@ namespace cg = cooperative_groups;
 namespace rwkvq {
 
 
+// Co-resident CTAs of 256 threads per SM: 2 at 128 registers; 3 at 80 where an iteration is 128 columns (a fragment of 18
+// to 22 registers against 32)
+template <int L> __host__ __device__ constexpr int ctas_per_sm() { return Geo<L>::KI == 128 ? 3 : 2; }
+
 // Persistent kernel: gridDim.x CTAs walk the 16-row tiles of matrix blockIdx.y with
 // stride gridDim.x * WT.  Inside a CTA step the 8 warps form WT tiles x WK slices
 // of the K loop; the activations are prepared once per CTA.  Each warp sees a flat
@@ -27,7 +31,7 @@ namespace rwkvq {
 // of global scratch with an arrival counter: MEASURED_SPLIT.
 // LORA: grid rows from n_mats on are the LoRA down projections of the same layer (rwkvq_lora_vec.cuh).
 template <int L, int WK, bool SPLIT, bool ZS, int LORA>
-__global__ void __launch_bounds__(kMmaWarps * 32, 2) gemv_mma_kernel(const MmaArgs a, const std::conditional_t<LORA != 0, LoraVecArgs, int> lora) {
+__global__ void __launch_bounds__(kMmaWarps * 32, ctas_per_sm<L>()) gemv_mma_kernel(const MmaArgs a, const std::conditional_t<LORA != 0, LoraVecArgs, int> lora) {
     if constexpr (LORA != 0) {
         if (static_cast<int>(blockIdx.y) >= a.n_mats) {
             const int cta = (static_cast<int>(blockIdx.y) - a.n_mats) * static_cast<int>(gridDim.x) + static_cast<int>(blockIdx.x);
@@ -89,15 +93,14 @@ __global__ void __launch_bounds__(kMmaWarps * 32, 2) gemv_mma_kernel(const MmaAr
     // mix) are not read from the second fetch on
     if (ZS) zf = zflag - it0 * (G::KI / 32);
 
-    int c_n = 0, buf = 0;
+    int buf = 0;
     for (int base = blockIdx.x * WT; base < n_tiles; base += step, buf ^= 1) {
         const int tile = base + tl;
         float acc0 = 0.f, acc1 = 0.f;     // rows g, g+8 of this tile
-        for (int j = 0; j < ipt; ++j, ++c_n) {
+        for (int j = 0; j < ipt; ++j) {
             const Frag<L> cur = nxt;
             fetch_next();
-            if (tile >= n_tiles) continue;
-            consume_frag<L>(cur, ks + j * WK, g, t, dig, n_in, xs16, acc0, acc1);
+            if (tile < n_tiles) consume_frag<L>(cur, ks + j * WK, g, t, dig, n_in, xs16, acc0, acc1);
         }
         // the 4 lanes of a quad hold the 8 blocks of each iteration
         acc0 += __shfl_xor_sync(0xFFFFFFFFu, acc0, 1); acc0 += __shfl_xor_sync(0xFFFFFFFFu, acc0, 2);
@@ -220,7 +223,6 @@ static bool zero_skip_enabled() {
     return g_zero_skip == 1;
 }
 
-constexpr int kResidentCtas = 2 * 148;     // 2 CTAs of 256 threads per SM at <= 128 registers
 constexpr int kSplitAnyCols = 4096;        // rows from which on the K split does not depend on the caller
 constexpr int kSplitMaxRows = 4096;        // rows a K-split launch may have: above, the row tiles alone fill the chip
 
@@ -234,12 +236,13 @@ static int launch_one_zs(MmaArgs& a, int rows, int cols, int n_mats, int KS, cud
                                              static_cast<int>(smem));
         if (e != cudaSuccess) return fail(RWKVQ_E_LIMIT, "gemv_mma: %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
     }
+    constexpr int kResident = ctas_per_sm<L>() * 148;
     const int units = ((rows + 15) / 16 + WT - 1) / WT;
-    const int cap = kResidentCtas / (n_mats * KS) > 0 ? kResidentCtas / (n_mats * KS) : 1;
+    const int cap = kResident / (n_mats * KS) > 0 ? kResident / (n_mats * KS) : 1;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(units < cap ? units : cap, n_mats, KS);
     if constexpr (LORA != 0) {                   // still one wave: the tiles walk what the LoRA CTAs leave
-        const int extra = lora->first[lora->n_br] / kLvCols, room = std::max(1, (kResidentCtas - extra) / n_mats);
+        const int extra = lora->first[lora->n_br] / kLvCols, room = std::max(1, (kResident - extra) / n_mats);
         cfg.gridDim.x = std::min(units, room);
         cfg.gridDim.y = n_mats + (extra + cfg.gridDim.x - 1) / cfg.gridDim.x;
     }
@@ -285,6 +288,7 @@ static int launch_one(MmaArgs& a, int rows, int cols, int n_mats, int KS, cudaSt
 //   * very many tiles (head) -> persistent CTAs, 8 warps split K of each tile
 template <int L>
 static int launch_wk(MmaArgs& a, int rows, int cols, int n_mats, bool split, cudaStream_t s) {
+    constexpr int kResident = ctas_per_sm<L>() * 148;
     const int n_iters = cols / Geo<L>::KI;
     const int tiles = (rows + 15) / 16;
     int KS = 1;
@@ -293,15 +297,15 @@ static int launch_wk(MmaArgs& a, int rows, int cols, int n_mats, bool split, cud
     // shorter ones only where the caller has nothing else to fill the chip with (`split`).
     const int ctas = tiles * (cols >= kSplitAnyCols ? 1 : n_mats);
     if ((split || cols >= kSplitAnyCols) && n_iters >= 16 && rows <= kSplitMaxRows) {
-        if (ctas * 4 <= kResidentCtas && n_iters >= 32 && n_iters % 4 == 0) KS = 4;
-        else if (ctas * 2 <= kResidentCtas && n_iters % 2 == 0) KS = 2;
+        if (ctas * 4 <= kResident && n_iters >= 32 && n_iters % 4 == 0) KS = 4;
+        else if (ctas * 2 <= kResident && n_iters % 2 == 0) KS = 2;
     }
     if (KS > 1) return launch_one<L, 8, true>(a, rows, cols, n_mats, KS, s);
     int wt = 1;
-    if (tiles * n_mats > kResidentCtas) {
+    if (tiles * n_mats > kResident) {
         wt = 0;
         for (int c = 2; c <= 8; c <<= 1)
-            if (((tiles + c - 1) / c) * n_mats <= kResidentCtas && 8 / c <= n_iters) { wt = c; break; }
+            if (((tiles + c - 1) / c) * n_mats <= kResident && 8 / c <= n_iters) { wt = c; break; }
         if (wt == 0) wt = 1;                 // persistent loop
     }
     int wk = 8 / wt;
