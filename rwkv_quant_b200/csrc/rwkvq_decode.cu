@@ -51,6 +51,7 @@ __device__ __forceinline__ void layer_norm_row(float (&x)[PER], int D, const flo
 
 constexpr int kRowThreads = 256;
 constexpr int kRowPer = 16;      // D <= 4096
+constexpr int kLnVecThreads = 1024;      // a float4 of the row per thread
 
 // Columns [32 g, 32 g + 32) of row R of an sb6 or sym table as exact fp32 values (the arithmetic of
 // decode_element: separate multiply and add), with every load of the group issued before any use:
@@ -185,18 +186,12 @@ __global__ void __launch_bounds__(kRowThreads) ln_shift_mix_kernel(const float* 
     __shared__ float redm[kRowThreads / 32][NM];
     const int b = blockIdx.x;
     float v[PER], prev[PER], lw[PER], lb[PER];
-    constexpr bool PRE = PER <= 8 && NMIX > 0;              // lerp vectors in registers
-    float mxr[PRE ? NMIX : 1][PRE ? PER : 1];
     pdl_launch_dependents();
 #pragma unroll
     for (int i = 0; i < PER; ++i) {          // parameters do not depend on the previous kernel
         const int d = threadIdx.x + i * kRowThreads;
         lw[i] = d < D ? ln_w[d] : 0.f;
         lb[i] = d < D ? ln_b[d] : 0.f;
-        if (PRE) {
-#pragma unroll
-            for (int m = 0; m < NMIX; ++m) mxr[PRE ? m : 0][PRE ? i : 0] = d < D ? __ldg(mix + m * D + d) : 0.f;
-        }
     }
     pdl_wait();
     if (threadIdx.x == 0) {
@@ -236,7 +231,7 @@ __global__ void __launch_bounds__(kRowThreads) ln_shift_mix_kernel(const float* 
         shift[bd] = xn;
 #pragma unroll
         for (int m = 0; m < NMIX; ++m) {
-            const float o = xn + xx * (PRE ? mxr[PRE ? m : 0][PRE ? i : 0] : __ldg(mix + m * D + d));
+            const float o = xn + xx * __ldg(mix + m * D + d);
             out[(static_cast<size_t>(m) * B) * D + bd] = o;
             mx[m < NM ? m : 0] = fmaxf(mx[m < NM ? m : 0], fabsf(o));
         }
@@ -283,11 +278,110 @@ __global__ void __launch_bounds__(kRowThreads) ln_shift_mix_kernel(const float* 
 #pragma unroll
             for (int m = 0; m < NMIX; ++m) {
                 if (!((x16_mask >> m) & 1)) continue;
-                const float o = xn + xx * (PRE ? mxr[PRE ? m : 0][PRE ? i : 0] : __ldg(mix + m * D + d));
+                const float o = xn + xx * __ldg(mix + m * D + d);
                 emit(m, o * sc_m[m < NM ? m : 0]);
             }
         }
     }
+}
+
+// The same for rows of whole, aligned float4: a thread per float4, every parameter in registers before the wait.
+// Bound: latency (one L2 round trip, two block sums, the stores); at 256 threads of 8 or 16 scalars each the loads and
+// stores alone issue for a microsecond.  MEASURED_LN
+template <int NMIX>
+__global__ void __launch_bounds__(kLnVecThreads) ln_shift_mix_vec_kernel(const float* __restrict__ x, const float* __restrict__ ln_w,
+                                                                         const float* __restrict__ ln_b, float* __restrict__ shift,
+                                                                         const float* __restrict__ mix, float* __restrict__ out, int B, int D,
+                                                                         __half* __restrict__ x16_out, float* __restrict__ unscale_out,
+                                                                         int x16_mask, float* __restrict__ zero_a, float* __restrict__ zero_b) {
+    constexpr int NM = NMIX > 0 ? NMIX : 1;
+    __shared__ float red[2][32];
+    __shared__ float redm[NM][32];
+    const int b = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, warps = blockDim.x >> 5;
+    const bool ok = 4 * tid < D;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const size_t at = static_cast<size_t>(b) * (D >> 2) + tid;         // in float4
+    pdl_launch_dependents();
+    const float4 lw = ok ? __ldg(reinterpret_cast<const float4*>(ln_w) + tid) : zero;
+    const float4 lb = ok ? __ldg(reinterpret_cast<const float4*>(ln_b) + tid) : zero;
+    float4 mx[NM];
+#pragma unroll
+    for (int m = 0; m < NMIX; ++m) mx[m] = ok ? __ldg(reinterpret_cast<const float4*>(mix + static_cast<size_t>(m) * D) + tid) : zero;
+    pdl_wait();
+    if (tid == 0) {
+        if (zero_a) zero_a[b] = 0.f;
+        if (zero_b) zero_b[b] = 0.f;
+    }
+    const float4 v = ok ? __ldcg(reinterpret_cast<const float4*>(x) + at) : zero;
+    const float4 prev = ok && NMIX > 0 ? __ldcg(reinterpret_cast<const float4*>(shift) + at) : zero;
+    auto sum = [&](float s, float* r) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
+        if (lane == 0) r[warp] = s;
+        __syncthreads();
+        s = lane < warps ? r[lane] : 0.f;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
+        return s;
+    };
+    const float mean = sum((v.x + v.y) + (v.z + v.w), red[0]) / D;
+    const float4 c = ok ? make_float4(v.x - mean, v.y - mean, v.z - mean, v.w - mean) : zero;
+    const float inv = 1.0f / sqrtf(sum((c.x * c.x + c.y * c.y) + (c.z * c.z + c.w * c.w), red[1]) / D + 1e-5f);
+    const float4 xn = make_float4(c.x * inv * lw.x + lb.x, c.y * inv * lw.y + lb.y, c.z * inv * lw.z + lb.z, c.w * inv * lw.w + lb.w);
+    const float4 xx = make_float4(prev.x - xn.x, prev.y - xn.y, prev.z - xn.z, prev.w - xn.w);
+    auto mixed = [&](int m) {
+        return NMIX == 0 ? xn : make_float4(xn.x + xx.x * mx[m].x, xn.y + xx.y * mx[m].y, xn.z + xx.z * mx[m].z, xn.w + xx.w * mx[m].w);
+    };
+    const size_t stride = static_cast<size_t>(B) * (D >> 2);
+#pragma unroll
+    for (int m = 0; m < NM; ++m)
+        if (ok) reinterpret_cast<float4*>(out)[m * stride + at] = mixed(m);
+    if (ok && NMIX > 0) reinterpret_cast<float4*>(shift)[at] = xn;
+    if (unscale_out == nullptr) return;
+#pragma unroll
+    for (int m = 0; m < NM; ++m) {
+        const float4 o = mixed(m);
+        float r = ok ? fmaxf(fmaxf(fabsf(o.x), fabsf(o.y)), fmaxf(fabsf(o.z), fabsf(o.w))) : 0.f;
+#pragma unroll
+        for (int s = 16; s > 0; s >>= 1) r = fmaxf(r, __shfl_xor_sync(0xFFFFFFFFu, r, s));
+        if (lane == 0) redm[m][warp] = r;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < NM; ++m) {
+        if (!((x16_mask >> m) & 1)) continue;
+        float r = lane < warps ? redm[m][lane] : 0.f;
+#pragma unroll
+        for (int s = 16; s > 0; s >>= 1) r = fmaxf(r, __shfl_xor_sync(0xFFFFFFFFu, r, s));
+        if (x16_out == nullptr) {
+            if (tid == 0) unscale_out[m * B + b] = r;
+            continue;
+        }
+        float s1 = 1.f, u1 = 1.f;                                      // as in the scalar form
+        if (r > 0.f && r < INFINITY) {
+            int e = 0;
+            frexpf(r, &e);
+            e = max(-100, e);
+            s1 = ldexpf(1.f, 14 - e);
+            u1 = ldexpf(1.f, e - 14);
+        }
+        if (tid == 0) unscale_out[m * B + b] = u1;
+        const float4 o = mixed(m);
+        __half2 h[2] = {__floats2half2_rn(o.x * s1, o.y * s1), __floats2half2_rn(o.z * s1, o.w * s1)};
+        if (ok) reinterpret_cast<uint2*>(x16_out)[m * stride + at] = *reinterpret_cast<uint2*>(h);
+    }
+}
+
+template <int NMIX>
+void launch_ln_shift_mix(int B, cudaStream_t s, const float* x, const float* ln_w, const float* ln_b, float* shift, const float* mix,
+                         float* out, int D, __half* x16_out, float* unscale_out, int x16_mask, float* zero_a, float* zero_b) {
+    if (D % 4 == 0 && D <= 4 * kLnVecThreads && aligned(x, 16) && aligned(ln_w, 16) && aligned(ln_b, 16) && aligned(out, 16) &&
+        (NMIX == 0 || (aligned(shift, 16) && aligned(mix, 16))))
+        launch_pdl(ln_shift_mix_vec_kernel<NMIX>, dim3(B), dim3((D / 4 + 31) / 32 * 32), 0, s, x, ln_w, ln_b, shift, mix, out, B, D, x16_out,
+                   unscale_out, x16_mask, zero_a, zero_b);
+    else
+        launch_pdl(ln_shift_mix_kernel<NMIX, kRowPer>, dim3(B), dim3(kRowThreads), 0, s, x, ln_w, ln_b, shift, mix, out, B, D, x16_out,
+                   unscale_out, x16_mask, zero_a, zero_b);
 }
 
 // ---- batched LoRA products, tensors stored [in, out] (a warp reads 128 contiguous codes)
@@ -903,10 +997,8 @@ int rwkvq_seq_layer_norm(const float* x, const float* ln_w, const float* ln_b, f
     RWKVQ_REQUIRE(x && ln_w && ln_b && out, RWKVQ_E_NULL, "rwkvq_seq_layer_norm: null pointer");
     RWKVQ_REQUIRE(n_rows >= 1 && D >= 1 && D <= kRowThreads * kRowPer, RWKVQ_E_SHAPE, "rwkvq_seq_layer_norm: %lld rows of %d (at most %d)",
                   (long long)n_rows, D, kRowThreads * kRowPer);
-    launch_pdl(D <= 8 * kRowThreads ? ln_shift_mix_kernel<0, 8> : ln_shift_mix_kernel<0, kRowPer>, dim3(static_cast<unsigned>(n_rows)), dim3(kRowThreads), 0, static_cast<cudaStream_t>(stream), x,
-               ln_w, ln_b, static_cast<float*>(nullptr), static_cast<const float*>(nullptr), out, static_cast<int>(n_rows), D,
-               static_cast<__half*>(nullptr), static_cast<float*>(nullptr), 0,
-               static_cast<float*>(nullptr), static_cast<float*>(nullptr));
+    launch_ln_shift_mix<0>(static_cast<int>(n_rows), static_cast<cudaStream_t>(stream), x, ln_w, ln_b, nullptr, nullptr, out, D, nullptr, nullptr,
+                           0, nullptr, nullptr);
     return check_launch("rwkvq_seq_layer_norm");
 }
 
@@ -970,8 +1062,7 @@ int rwkvq_decode_step(const rwkvq_model* m, int B, const int64_t* tokens, float*
             rc = launch_seq_prep(pa, B, s);
             if (rc) return rc;
         } else {
-            launch_pdl(D <= 8 * kRowThreads ? ln_shift_mix_kernel<6, 8> : ln_shift_mix_kernel<6, kRowPer>, dim3(B), dim3(kRowThreads), 0, s, w.x, L.ln1_w,
-                       L.ln1_b, tshift[l], L.x_mix, w.xs, B, D, h16 ? w.xs16 : static_cast<__half*>(nullptr), am, 0b001101, am_og,
+            launch_ln_shift_mix<6>(B, s, w.x, L.ln1_w, L.ln1_b, tshift[l], L.x_mix, w.xs, D, h16 ? w.xs16 : static_cast<__half*>(nullptr), am, 0b001101, am_og,
                        am_h);      // scales of the r, k, v rows
         }
         float *xr = w.xs, *xw = w.xs + BD, *xk = w.xs + 2 * BD, *xv = w.xs + 3 * BD, *xa = w.xs + 4 * BD,
@@ -1100,8 +1191,7 @@ int rwkvq_decode_step(const rwkvq_model* m, int B, const int64_t* tokens, float*
         rc = linear(&L.Wo, w.og, B, D, w.x, D, RWKVQ_EPI_ADD, w.x, w.gemm_ws, stream, nullptr, am_og, nullptr, w.status);
         if (rc) return rc;
         // ---- channel mix
-        launch_pdl(D <= 8 * kRowThreads ? ln_shift_mix_kernel<1, 8> : ln_shift_mix_kernel<1, kRowPer>, dim3(B), dim3(kRowThreads), 0, s, w.x, L.ln2_w,
-                   L.ln2_b, cshift[l], L.ffn_x_k, w.xk, B, D, h16 ? w.xk16 : static_cast<__half*>(nullptr), am_xk, 1, static_cast<float*>(nullptr),
+        launch_ln_shift_mix<1>(B, s, w.x, L.ln2_w, L.ln2_b, cshift[l], L.ffn_x_k, w.xk, D, h16 ? w.xk16 : static_cast<__half*>(nullptr), am_xk, 1, static_cast<float*>(nullptr),
                    static_cast<float*>(nullptr));
         rc = linear(&L.Wfk, w.xk, B, D, w.hffn, F, RWKVQ_EPI_RELU2, nullptr, w.gemm_ws, stream, h16 ? w.xk16 : nullptr, am_xk, am_h,
                     w.status);
@@ -1119,8 +1209,7 @@ int rwkvq_decode_step(const rwkvq_model* m, int B, const int64_t* tokens, float*
     } else {
         float* am_xo = batch_path(B) ? w.amax + 9 * B : nullptr;
         const bool xo_h16 = am_xo && batch_fast();
-        launch_pdl(D <= 8 * kRowThreads ? ln_shift_mix_kernel<0, 8> : ln_shift_mix_kernel<0, kRowPer>, dim3(B), dim3(kRowThreads), 0, s, w.x, m->lnout_w,
-                   m->lnout_b, static_cast<float*>(nullptr), static_cast<const float*>(nullptr), w.xo, B, D, xo_h16 ? w.xo16 : static_cast<__half*>(nullptr),
+        launch_ln_shift_mix<0>(B, s, w.x, m->lnout_w, m->lnout_b, nullptr, nullptr, w.xo, D, xo_h16 ? w.xo16 : static_cast<__half*>(nullptr),
                    am_xo, 1, static_cast<float*>(nullptr), static_cast<float*>(nullptr));
         rc = linear(&m->head, w.xo, B, D, lg, V, RWKVQ_EPI_NONE, nullptr, w.gemm_ws, stream, xo_h16 ? w.xo16 : nullptr, am_xo, nullptr,
                     w.status);
