@@ -287,7 +287,7 @@ __global__ void __launch_bounds__(kRowThreads) ln_shift_mix_kernel(const float* 
 
 // The same for rows of whole, aligned float4: a thread per float4, every parameter in registers before the wait.
 // Bound: latency (one L2 round trip, two block sums, the stores); at 256 threads of 8 or 16 scalars each the loads and
-// stores alone issue for a microsecond.  MEASURED_LN
+// stores alone issue for a microsecond.  One stream: 2560 wide 8.7 -> 3.3 us, 2048 wide 3.9 -> 3.0 us.
 template <int NMIX>
 __global__ void __launch_bounds__(kLnVecThreads) ln_shift_mix_vec_kernel(const float* __restrict__ x, const float* __restrict__ ln_w,
                                                                          const float* __restrict__ ln_b, float* __restrict__ shift,
@@ -376,12 +376,14 @@ template <int NMIX>
 void launch_ln_shift_mix(int B, cudaStream_t s, const float* x, const float* ln_w, const float* ln_b, float* shift, const float* mix,
                          float* out, int D, __half* x16_out, float* unscale_out, int x16_mask, float* zero_a, float* zero_b) {
     if (D % 4 == 0 && D <= 4 * kLnVecThreads && aligned(x, 16) && aligned(ln_w, 16) && aligned(ln_b, 16) && aligned(out, 16) &&
-        (NMIX == 0 || (aligned(shift, 16) && aligned(mix, 16))))
+        (NMIX == 0 || (aligned(shift, 16) && aligned(mix, 16)))) {
+        decode_carveout<ln_shift_mix_vec_kernel<NMIX>>();
         launch_pdl(ln_shift_mix_vec_kernel<NMIX>, dim3(B), dim3((D / 4 + 31) / 32 * 32), 0, s, x, ln_w, ln_b, shift, mix, out, B, D, x16_out,
                    unscale_out, x16_mask, zero_a, zero_b);
-    else
+    } else {
         launch_pdl(ln_shift_mix_kernel<NMIX, kRowPer>, dim3(B), dim3(kRowThreads), 0, s, x, ln_w, ln_b, shift, mix, out, B, D, x16_out,
                    unscale_out, x16_mask, zero_a, zero_b);
+    }
 }
 
 // ---- batched LoRA products, tensors stored [in, out] (a warp reads 128 contiguous codes)
@@ -919,6 +921,7 @@ SideLane* side_lane(cudaStream_t caller) {
 }
 
 int launch_tmix_core_up(const TmixCoreArgs& tc, const LoraVecArgs& up, int H, cudaStream_t s) {
+    decode_carveout<tmix_core_kernel<true>>();
     const size_t smem = lora_vec_smem(up.first[up.n_br]);
     if (smem > 40 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(tmix_core_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLvMaxSmem);
