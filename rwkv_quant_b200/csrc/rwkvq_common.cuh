@@ -39,10 +39,11 @@ static inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 b
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
-// The kernels of a one-stream step ask for one split of an SM's 256 KB, a third of it shared memory.  An SM changes the
+// The GEMV and the time-mix core of a one-stream step ask for one split of an SM's 256 KB, a third of it shared memory.  An SM changes the
 // split only when it is idle, so a CTA that needs more than its predecessors' split waits for all of them to leave instead
 // of staging its weights beside them; and the driver's own choice (as much as full occupancy could use) leaves the weight
-// streams, which take half a sector at a time from records and scales, too little L1.  2.9B one stream: driver's choice
+// streams, which take half a sector at a time from records and scales, too little L1.  (Not the LayerNorms, which the
+// small-batch kernels with 110 KB a CTA share: 13 streams 1.90 -> 2.15 ms.)  2.9B one stream: driver's choice
 // 1.91 ms, 15% 1.69, 29% to 44% 1.65 to 1.68, 58% 1.75, 100% 2.64; 1.5B 0.946, 0.953, 0.926, 0.919, 1.14.
 constexpr int kDecodeCarveout = 36;
 template <auto Kernel>

@@ -377,7 +377,6 @@ void launch_ln_shift_mix(int B, cudaStream_t s, const float* x, const float* ln_
                          float* out, int D, __half* x16_out, float* unscale_out, int x16_mask, float* zero_a, float* zero_b) {
     if (D % 4 == 0 && D <= 4 * kLnVecThreads && aligned(x, 16) && aligned(ln_w, 16) && aligned(ln_b, 16) && aligned(out, 16) &&
         (NMIX == 0 || (aligned(shift, 16) && aligned(mix, 16)))) {
-        decode_carveout<ln_shift_mix_vec_kernel<NMIX>>();
         launch_pdl(ln_shift_mix_vec_kernel<NMIX>, dim3(B), dim3((D / 4 + 31) / 32 * 32), 0, s, x, ln_w, ln_b, shift, mix, out, B, D, x16_out,
                    unscale_out, x16_mask, zero_a, zero_b);
     } else {
