@@ -777,7 +777,8 @@ using namespace rwkvq;
 namespace {
 
 constexpr int kBatchMax = 256;     // streams up to which the small-batch kernel serves the linears of a step
-inline bool batch_path(int B) { return B > 2 && B <= kBatchMax; }
+// (two streams: 1.60 ms per step of the 1.5B model against 1.82 on one single-vector launch per stream, 2.9B 2.79 / 3.81)
+inline bool batch_path(int B) { return B > 1 && B <= kBatchMax; }
 // Which small-batch kernel: measured on B200 (1.5B, whole decode step) the tcgen05 form wins from 33
 // streams on (64 streams: 3.77 against 4.43 ms per step) and loses below (32: 2.87 / 2.68 ms, 8: 2.42 / 2.01 ms):
 // its pass (dependent weight loads -> conversion -> MMA) is longer than a warp-iteration of the mma.sync form
@@ -953,10 +954,8 @@ int lora_pair(const rwkvq_qtensor* const* t1, const rwkvq_qtensor* const* t2, co
         u.act[i] = acts[i];
         if (t2[i]->cols > max_cols) max_cols = t2[i]->cols;
     }
-    if (B != 2 && lora_mma_ok(t1, t2, n_br, D)) {
-        // both products on the tensor cores, matrices read once.  Measured per token: one stream 1.160 ms here
-        // against 1.185 ms on the per-stream kernels below, two streams 1.92 against 1.88 ms: those keep two
-        // streams and odd shapes.  (A row's result does not depend on the batch it is computed in, either way.)
+    if (lora_mma_ok(t1, t2, n_br, D)) {
+        // both products on the tensor cores, matrices read once; the kernels below keep the odd shapes
         const int n_stride = ((B + 63) / 64) * 64;
         if (static_cast<size_t>(4) * n_stride * max_rank <= part_floats)
             return launch_lora_pair_mma(t1, t2, xs, ys, acts, n_br, B, D, max_rank, part, n_stride, s);
@@ -1118,6 +1117,14 @@ int rwkvq_decode_step(const rwkvq_model* m, int B, const int64_t* tokens, float*
         // shares an SM with the first (64 streams: 17 + 11 + 6 us in the other order, 13 + 16 in this).
         cudaStream_t s_rkv = s;
         if (lane && (B <= 16 || sb)) { s_rkv = lane->stream; s_lora = s; }
+        auto lora = [&]() {
+            float* y2[4] = {yw, ya, yg, yv};
+            return lora_pair(t1, t2, x1, y2, act, n_br, B, D, m->max_rank, w.part, w.part_floats, w.n_chunks, s_lora);
+        };
+        if (sb) {                                  // first in the graph too: 64 streams 2.88 -> 2.81 ms (13 on mma.sync lose 1%)
+            rc = lora();
+            if (rc) return rc;
+        }
         if (B == 1 && ml >= 0 && mma_layout_of(L.Wk) == ml && mma_layout_of(L.Wv) == ml && L.Wk.rows == D &&
             L.Wv.rows == D && L.Wr.rows == D && L.Wk.cols == D && L.Wv.cols == D && L.Wr.cols == D) {
             // r, k, v in one launch: three matrices, three inputs (rows 0, 2, 3 of xs)
@@ -1159,9 +1166,8 @@ int rwkvq_decode_step(const rwkvq_model* m, int B, const int64_t* tokens, float*
                         h16 ? w.xs16 + 3 * BD : nullptr, bp ? am + 3 * B : nullptr, nullptr, w.status);
             if (rc) return rc;
         }
-        {
-            float* y2[4] = {yw, ya, yg, yv};
-            rc = lora_pair(t1, t2, x1, y2, act, n_br, B, D, m->max_rank, w.part, w.part_floats, w.n_chunks, s_lora);
+        if (!sb) {
+            rc = lora();
             if (rc) return rc;
         }
         if (lane) {                                  // join before the time-mix core
