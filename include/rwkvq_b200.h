@@ -195,14 +195,16 @@ int rwkvq_quantize_sym6_packed(const float* w, int64_t ldw, int rows, int cols, 
  * to ~1e-6 of max|y| (a column's last bits may depend on the batch it is computed in; two calls on
  * the same input give the same bits).  The K split is reduced across a thread-block cluster through
  * distributed shared memory: no scratch for partial sums.
+ * Up to 16 rows the products run on mma.sync; from 17 rows on sb6 / sym tensors with whole 256-column
+ * super-blocks (up to 16384 columns) run on the tcgen05 tensor cores in the same arithmetic (rows of 128
+ * as the UMMA M, the converted weights as its operand in tensor memory, the batch as its N).
  * With RWKVQ_BATCH_FAST=1 in the environment (read once per process) single fp16 operands are used
- * instead (weights fp16(q*s+m)): ~25 % faster at 32 rows and more, results within ~3e-4 of max|y|
- * per call (the precision of rwkvq_gemm), and sb6 / sym tensors with more than 32 rows run on the
- * tcgen05 tensor cores (rows of 128 as the UMMA M, the batch as its N, accumulator in tensor memory).
+ * instead (weights fp16(q*s+m)): results within ~3e-4 of max|y| per call (the precision of rwkvq_gemm),
+ * and sb6 / sym tensors with more than 32 rows run on a single-term tcgen05 form.
  *   workspace: rwkvq_gemv_batch_workspace_bytes(N) bytes, 16-byte aligned: a status word (first
  *   int32: RWKVQ_E_TIMEOUT if a bounded wait on the tensor-core pipeline ran out; read it after
- *   synchronising the stream, 0 = ok) and one float per row, the max|x| a one-block-per-row
- *   pre-pass writes before the product kernel starts.
+ *   synchronising the stream, 0 = ok), one float per row (max|x|, or the inverse scale of the pairs) and
+ *   the rows as fp16 pairs, which a one-block-per-row pre-pass writes before the product kernel starts.
  */
 size_t rwkvq_gemv_batch_workspace_bytes(int N);
 int rwkvq_gemv_batch(const rwkvq_qtensor* t, const float* x, int N, int64_t ldx, float* y, int64_t ldy,
@@ -285,18 +287,14 @@ int rwkvq_lora_pair(const rwkvq_qtensor* t1_host, const rwkvq_qtensor* t2_host, 
  * thread under a real-time budget, code running where cudaMalloc would
  * synchronise the device).
  *   y[o] = epi( sum_c W[o, c] x[c] ),  x [cols] of x_dtype, y / resid [rows] fp32.
- * The K loop is split across CTAs; the slices' partial sums and arrival counters
- * live in a 260 KiB __device__ array inside the library, whose address is looked
- * up once per device.  The call issues one cudaMemsetAsync (counters) and one
- * kernel on `stream`; it calls no cudaMalloc / cudaFree nor any allocating
- * library routine.
+ * The K loop is split across the CTAs of a cluster, whose partial sums meet in
+ * distributed shared memory.  The call issues one kernel on `stream`; it calls no
+ * cudaMalloc / cudaFree nor any allocating library routine.
  *   limits  rows <= 4096, cols <= 16384 (RWKVQ_E_LIMIT beyond); sb6 tensors need
  *           dev_meta (and dev_planes at 5 / 6 bits), sym@6 needs dev_planes, per-row
  *           int8 needs cols % 128 == 0 (RWKVQ_E_DTYPE otherwise); x 16-byte aligned.
- *   set-up  the first call on a device resolves the array's address (and may load
- *           the module): make it before any stream capture begins.
- *   races   every call on a device uses the same array: two calls that can
- *           overlap (different streams or threads) race on it; serialise them.
+ *   set-up  the first call on a device may load the module: make it before any
+ *           stream capture begins.
  * Results equal rwkvq_gemv's up to fp32 summation order and are bit-identical
  * from call to call.
  */
@@ -384,8 +382,8 @@ typedef struct rwkvq_model {
 } rwkvq_model;
 
 /* Bytes of device scratch rwkvq_decode_step needs for batch B (logits included).
- * The workspace must be zero-filled once before its first use (arrival counters of
- * the K-split GEMV live in it and reset themselves after every launch). */
+ * The workspace must be zero-filled once before its first use (its first word is the
+ * status word of the bounded waits). */
 size_t rwkvq_decode_workspace_bytes(const rwkvq_model* m_host, int B);
 
 /*
@@ -397,11 +395,10 @@ size_t rwkvq_decode_workspace_bytes(const rwkvq_model* m_host, int B);
  * (host arrays of device pointers; a fresh stream starts from zeros).
  * logits [B, vocab] fp32 (NULL: kept in the workspace), next_tokens [B] int64 greedy
  * argmax (NULL: skipped), tokens [B] int64 on the device.
- * Linears: B = 1 the single-vector tensor-core GEMV; 3 <= B <= 256 the weights-once small-batch
- * kernels in two-term precision (see rwkvq_gemv_batch), of which r / k / v, the ffn key and the head
- * take the tcgen05 form at 33-48 streams and r / k / v and the head at 49-64 (RWKVQ_TCB_EXACT=0 / 1 in
- * the environment, read once: none / all three at every B above 32); RWKVQ_BATCH_FAST=1 selects single
- * fp16 operands instead; larger B the prefill GEMM.
+ * Linears: B = 1 the single-vector tensor-core GEMV; 2 <= B <= 256 the weights-once small-batch kernels
+ * in two-term precision (see rwkvq_gemv_batch), on the tcgen05 pipeline from 17 streams on where every
+ * linear of the model has its layout (RWKVQ_TCB_EXACT=0 / 1 in the environment, read once: never / from 3
+ * streams on); RWKVQ_BATCH_FAST=1 selects single fp16 operands instead; larger B the prefill GEMM.
  */
 int rwkvq_decode_step(const rwkvq_model* m_host, int B, const int64_t* tokens,
                       float* const* wkv_host, float* const* tshift_host, float* const* cshift_host,

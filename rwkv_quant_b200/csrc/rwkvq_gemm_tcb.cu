@@ -47,9 +47,6 @@ struct TcbArgs {
     const float* x[kTbMaxMats];           // [N, ldx] fp32, or null when x16 is given
     const float* amax[kTbMaxMats];        // with x:   [N] max|x| per token
     const __half* x16[kTbMaxMats];        // [N, ldx] fp16 rows = x * 2^s
-    const __half* x16lo[kTbMaxMats];      // two-term kernel with x16: fp16(x * 2^s - x16)
-    const __half* xsum[kTbMaxMats];       // ... and [N, cols / 128][8]: the sums of x * 2^s over the four 32-column blocks
-                                          //     of every 128 columns, 4 high halves then 4 low halves
     const float* unscale[kTbMaxMats];     // with x16: [N] 2^-s
     float* y[kTbMaxMats];                 // [N, ldy]
     const float* resid[kTbMaxMats];
@@ -111,7 +108,7 @@ __global__ void __launch_bounds__(kTbThreads, 2) gemm_tcb_kernel(const TcbArgs a
     const int row0 = rt * kGmRows;
     const int n0 = blockIdx.z * NT, nn = min(NT, a.n_tokens - n0);
     const int np = a.passes, pass0 = rank * np;                 // first pass of this CTA, in units of PASSK columns
-    const bool is16 = a.x16[blockIdx.y] != nullptr;
+    const bool is16 = !EX && a.x16[blockIdx.y] != nullptr;
 
     tb_mark(a, 0);
     if (tid == 0) {
@@ -209,17 +206,13 @@ __global__ void __launch_bounds__(kTbThreads, 2) gemm_tcb_kernel(const TcbArgs a
         constexpr int VPT = NT * VROW / kTbProducers;           // ... per thread: 2, 4, 8 (EX: 1, 2, 4)
         auto do_pass = [&](int p, Packed* P) {
             const int kbase = (pass0 + p) * PASSK;
-            uint4 xv[VPT], xl[EX ? VPT : 1], sv = make_uint4(0, 0, 0, 0);
-            if (has_min && is16 && tid < nn)
-                sv = __ldcg(reinterpret_cast<const uint4*>(a.xsum[blockIdx.y] + (static_cast<size_t>(n0 + tid) * (t.cols >> 7) + pass0 + p) * 8));
+            uint4 xv[VPT];
             if (is16) {                                          // requested before the wait and the conversion
                 const __half* xg = a.x16[blockIdx.y] + static_cast<size_t>(n0) * a.ldx + kbase;
-                const __half* xlg = EX ? a.x16lo[blockIdx.y] + static_cast<size_t>(n0) * a.ldx + kbase : nullptr;
 #pragma unroll
                 for (int u = 0; u < VPT; ++u) {
                     const int idx = tid + u * kTbProducers, n = idx / VROW, k8 = idx % VROW;
                     xv[u] = n < nn ? __ldcg(reinterpret_cast<const uint4*>(xg + static_cast<size_t>(n) * a.ldx) + k8) : make_uint4(0, 0, 0, 0);
-                    if (EX) xl[u] = n < nn ? __ldcg(reinterpret_cast<const uint4*>(xlg + static_cast<size_t>(n) * a.ldx) + k8) : make_uint4(0, 0, 0, 0);
                 }
             }
             if (p > 0) {                                         // the MMAs of the previous pass have read the operands
@@ -241,13 +234,11 @@ __global__ void __launch_bounds__(kTbThreads, 2) gemm_tcb_kernel(const TcbArgs a
                         convert_store(P[q], t, RGRP * q + prow, pit, pit & 1, a_slabs + (pit >> 1) * SLAB);
                     }
                 }
-                if (has_min && is16 && tid < NT) *reinterpret_cast<uint4*>(m_b + tid * 16) = sv;
                 if (is16) {
 #pragma unroll
                     for (int u = 0; u < VPT; ++u) {
                         const int idx = tid + u * kTbProducers, n = idx / VROW, k8 = idx % VROW;
                         *reinterpret_cast<uint4*>(b_slabs + (k8 >> 3) * BSLAB + sw128_offset(n, k8 & 7)) = xv[u];
-                        if (EX) *reinterpret_cast<uint4*>(l_slabs + (k8 >> 3) * BSLAB + sw128_offset(n, k8 & 7)) = xl[u];
                     }
                 } else if (EX) {
                     const float* xg = a.x[blockIdx.y] + static_cast<size_t>(n0) * a.ldx + kbase;
@@ -475,13 +466,12 @@ bool gemm_tcb_ok(const rwkvq_qtensor& t) {
 }
 
 // Same contract as launch_gemv_batch (rwkvq_common.cuh), plus the device status word.  `exact`: the
-// two-term kernel; with half_in its rows are scaled to at most 2^9 and it needs xs_lo[k] = fp16(x * 2^s
-// - xs[k]) and xs_sum[k] (TcbArgs::xsum) beside xs[k].
+// two-term kernel (fp32 rows), for tensors without the relayouted streams that rwkvq_gemm_sb.cu reads.
 int launch_gemm_tcb(const rwkvq_qtensor* ts, int n_mats, const void* const* xs, bool half_in, const float* const* scales,
                     int N, long long ldx, float* const* ys, long long ldy, int epilogue, const float* const* resids,
-                    float* const* amax_outs, int* status, cudaStream_t s, bool exact, const void* const* xs_lo,
-                    const void* const* xs_sum) {
+                    float* const* amax_outs, int* status, cudaStream_t s, bool exact) {
     RWKVQ_REQUIRE(n_mats >= 1 && n_mats <= kTbMaxMats, RWKVQ_E_LIMIT, "rwkvq_gemm_tcb: %d matrices", n_mats);
+    RWKVQ_REQUIRE(!(exact && half_in), RWKVQ_E_DTYPE, "rwkvq_gemm_tcb: the two-term kernel takes fp32 rows");
     TcbArgs a{};
     for (int k = 0; k < n_mats; ++k) {
         RWKVQ_REQUIRE(gemm_tcb_ok(ts[k]) && ts[k].kind == ts[0].kind && ts[k].bits == ts[0].bits && ts[k].rows == ts[0].rows &&
@@ -491,12 +481,6 @@ int launch_gemm_tcb(const rwkvq_qtensor* ts, int n_mats, const void* const* xs, 
         a.t[k] = make_view(ts[k]);
         if (half_in) { a.x16[k] = static_cast<const __half*>(xs[k]); a.unscale[k] = scales[k]; }
         else { a.x[k] = static_cast<const float*>(xs[k]); a.amax[k] = scales[k]; }
-        if (half_in && exact) {
-            RWKVQ_REQUIRE(xs_lo && xs_lo[k] && aligned(xs_lo[k], 16) && xs_sum && xs_sum[k] && aligned(xs_sum[k], 16), RWKVQ_E_NULL,
-                          "rwkvq_gemm_tcb: the low halves or the block sums of x are missing");
-            a.x16lo[k] = static_cast<const __half*>(xs_lo[k]);
-            a.xsum[k] = static_cast<const __half*>(xs_sum[k]);
-        }
         a.y[k] = ys[k]; a.resid[k] = resids ? resids[k] : nullptr;
         a.amax_out[k] = amax_outs ? amax_outs[k] : nullptr;
         RWKVQ_REQUIRE(epilogue != RWKVQ_EPI_ADD || a.resid[k], RWKVQ_E_NULL, "rwkvq_gemm_tcb: resid is null");

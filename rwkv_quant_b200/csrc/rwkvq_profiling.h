@@ -18,8 +18,8 @@ void rwkvq_profiling_gemm_acc_mode(int mode);
 void rwkvq_profiling_batch_trace(void* buf8, int force_ks);
 /* The same override for tensors of one shape only (rows = 0: every shape); 0 switches it off. */
 void rwkvq_profiling_batch_force(int force_ks, int rows, int cols);
-/* Small-batch linear on tcgen05: > 0 selects it at every batch size and forces the cluster size where
- * that divides the pass count (1000: every batch size, launcher's cluster size), -1 routes every
+/* Small-batch linear on tcgen05: > 0 selects it at every batch size and forces the cluster size (slices of
+ * whole super-blocks in the default precision; 1000: every batch size, launcher's cluster size), -1 routes every
  * call to the mma.sync kernel instead, 0 restores the launcher's choice. */
 void rwkvq_profiling_tcb_force(int force_ks);
 /* Precision of the small-batch linears: 1 single fp16 operands (what RWKVQ_BATCH_FAST=1 selects),
@@ -28,9 +28,9 @@ void rwkvq_profiling_batch_fast(int fast);
 /* The exact zero-group skip of the single-vector GEMV (what RWKVQ_ZERO_SKIP=1 selects): 1 on, 0 off (the
  * default), -1 read the environment again. */
 void rwkvq_profiling_zero_skip(int on);
-/* Decode step above 32 streams in the default precision: 1 runs r / k / v, the ffn key and the head on the
- * two-term tcgen05 linear at every such batch (what RWKVQ_TCB_EXACT=1 selects), 0 keeps them on mma.sync
- * (RWKVQ_TCB_EXACT=0), -1 reads the environment again (unset: the launcher's measured choice by batch size). */
+/* Decode step in the default precision: 1 runs every linear on the tcgen05 pipeline from 3 streams on (what
+ * RWKVQ_TCB_EXACT=1 selects), 0 keeps them on mma.sync (RWKVQ_TCB_EXACT=0), -1 reads the environment again
+ * (unset: from 17 streams on). */
 void rwkvq_profiling_tcb_exact(int on);
 #ifdef __cplusplus
 }
