@@ -16,7 +16,7 @@ One JSON line is printed by rank 0:
              memory and the argmax read back to the host every step
   roofline   the dominant kernel: the quantized-linear launches of one step (6 per layer + head) replayed
              as a graph; algorithmic bytes = their file-format bytes + activation rows, against the
-             measured HBM copy bandwidth; `traffic` = the DRAM bytes of the same launches under ncu
+             measured HBM copy bandwidth; `traffic` (one stream) = the DRAM bytes of the same launches under ncu
   step_roofline  the whole step of one GPU: (file-format weight bytes + WKV state read and written for
              its streams) / step time
   fast_mode  (N = 1) the same step with RWKVQ_BATCH_FAST=1 arithmetic (single fp16 operands), for comparison
@@ -231,10 +231,12 @@ def linear_phase(model, B, steps, warmup):
 # dram__bytes_read.sum + dram__bytes_write.sum of the quantized-linear launches of one decoded token
 # (1.5B compression, one stream), from the ncu capture summarised under profiles/
 NCU_GEMV_PHASE_DRAM_BYTES_B1 = 828225280 + 342272
-# the same for one step of 64 streams on the default (two-term) small-batch kernels: 24 x 45.60 MB per layer
-# (r/k/v 12.63, output projection 6.11, ffn key 13.19, ffn value 13.68) + 101.84 MB for the head, from a 2-layer
-# capture (profiles/decode_step_b64_b8_launch_list_1p5b_compression.md); traffic grows with the layer count
-NCU_BATCH_PHASE_DRAM_BYTES_B64 = 24 * 45602560 + 101837824
+
+
+def kernel_name(B, fast):
+    if fast:
+        return "row_amax_kernel + " + ("gemm_tcb_kernel" if B > 32 else "gemv_batch_kernel")
+    return "split_rows_kernel + gemm_sb_kernel" if B > 16 else "row_amax_kernel + gemv_batch_kernel"
 
 
 def time_decode(model, B, prompt, steps, warmup, sync_all, clock_index=None, groups=None):
@@ -275,7 +277,7 @@ def time_decode(model, B, prompt, steps, warmup, sync_all, clock_index=None, gro
     sync_all()
     t_e2e = e0.elapsed_time(e1) * 1e-3
     del dec2
-    return t_dev, t_e2e, clk.summary(), (model.launches_per_token + 1) * steps
+    return t_dev, t_e2e, clk.summary(), (model.launches_per_step(B) + 1) * steps
 
 
 def prefill_block(dev, model_name, peaks, peak_kind):
@@ -457,13 +459,11 @@ def run_ours(a, rank, world, local_rank):
                           "bytes_per_step": step_bytes, "us_per_step": sec_step * 1e6},
         "roofline": {"bound": "hbm", "achieved": g_bytes / g_sec / 1e9, "peak": peak, "unit": "GB/s",
                          "frac": g_bytes / g_sec / 1e9 / peak, "peak_kind": peak_kind,
-                         "traffic": NCU_BATCH_PHASE_DRAM_BYTES_B64 if (a.model, a.recipe, B, fast_env) == ("1.5b", "compression", 64, False) else None,
-                         "what": "the dominant kernel (the mma.sync small-batch linear: 72 % of a 64-stream step in the ncu launch list "
-                                 "when every linear runs on it, as timed here; the step itself runs r / k / v and the head on the "
-                                 "tcgen05 form above 48 streams): file-format bytes of the quantized linears + their activation "
-                                 "rows / time of those launches, all through rwkvq_gemv_batch, replayed as one graph",
-                         "kernel": (f"row_amax_kernel + {'gemm_tcb_kernel' if (fast_env and B > 32) else 'gemv_batch_kernel'}, "
-                                    f"the {g_launches} launches of the quantized linears of one step at "
+                         "traffic": None,
+                         "what": "the dominant kernel (the small-batch linear on tcgen05 from 17 streams on, on mma.sync below): "
+                                 "file-format bytes of the quantized linears + their activation rows / time of those "
+                                 "launches, all through rwkvq_gemv_batch, replayed as one graph",
+                         "kernel": (f"{kernel_name(B, fast_env)}, the {g_launches} launches of the quantized linears of one step at "
                                     f"{B} streams" if B > 2 else f"gemv_mma_kernel, {g_launches} launches"),
                          "bytes_per_replay": g_bytes, "us_per_replay": g_sec * 1e6},
     }

@@ -429,17 +429,21 @@ class QuantRWKV7:
         return Decoder(self, batch_size, states, use_graph, self_feed, groups)
 
     def decode_groups(self, batch_size: int) -> int:
-        """Stream groups whose launch chains run side by side (see ``Decoder``).  Measured on B200
-        (1.5B, ms per step, one group / two groups): 64 streams 4.20 / 4.38, 32 streams 3.02 / 3.03,
-        16 streams 2.13 / 2.54 with the default two-term linears (which walk 16-token tiles inside one
-        launch), 3.57 / 3.8 at 64 streams with RWKVQ_BATCH_FAST=1.  One group is the default."""
+        """Stream groups whose launch chains run side by side (see ``Decoder``).  One: every group streams the weights
+        itself, and the chains of two groups that each fill the SMs run one after the other (64 streams on the
+        mma.sync kernels: 4.20 ms per step as one group, 4.38 as two)."""
         return 1
+
+    def launches_per_step(self, batch_size: int = 1) -> int:
+        """Kernels one decoded token of ``batch_size`` streams launches.  Per layer, one stream: 2 norm/shift/lerp, r/k/v
+        with the LoRA down projections, time-mix core with the up projections, 3 GEMV.  2 to 16 streams: the LoRA pair
+        in launches of its own.  More: two passes that make fp16 pairs of fp32 rows besides.  Plus embedding, final norm,
+        head, argmax (2)."""
+        return self.n_layer * (7 if batch_size == 1 else 9 if batch_size <= 16 else 11) + 5
 
     @property
     def launches_per_token(self) -> int:
-        """Kernels one decoded token launches at batch 1: per layer 2 norm/shift/lerp,
-        4 GEMV (r/k/v fused), 2 LoRA, 1 time-mix core; plus embedding, final norm, head, argmax (2)."""
-        return self.n_layer * 9 + 5
+        return self.launches_per_step(1)
 
 
 class Decoder:
