@@ -7,14 +7,16 @@
 //
 // Per layer (backends/metal/quant_model.py:638-728, 803-836):
 //   ln_shift_mix   LN1 + token shift + the six lerps           -> xs[6][B][D]
-//   gemv x3        r, k, v projections (one fused launch)
-//   lora_down      the LoRA down projections w1, a1, v1, g1 as row-chunk partial sums
-//   lora_up        activation (tanh / - / - / sigmoid) and the up projections w2, a2, v2, g2
+//   linear x3      r, k, v projections (one fused launch; one stream: with the LoRA down projections)
+//   lora pair      w1, a1, v1, g1, activation (tanh / - / - / sigmoid), w2, a2, v2, g2 (rwkvq_lora_mma.cu; the SIMT
+//                  kernels of this file for odd shapes; one stream: inside its neighbours, rwkvq_lora_vec.cuh)
 //   tmix_core      decay, gates, kk, k and v updates, WKV-7 step on the 64x64 state,
 //                  group norm, bonus, gate                      -> og[B][D]
-//   gemv + add     output projection and residual
+//   linear + add   output projection and residual
 //   ln_shift_mix   LN2 + token shift + lerp                     -> xk[B][D]
-//   gemv + relu^2  ffn key;  gemv + add  ffn value and residual
+//   linear + relu^2  ffn key;  linear + add  ffn value and residual
+// Linears: one stream rwkvq_gemv_mma.cu, 2 to 16 rwkvq_gemv_batch.cu, from 17 on rwkvq_gemm_sb.cu (LayerNorms by
+// rwkvq_seq.cu, rows as fp16 pairs).
 #include <stdlib.h>
 
 #include <map>

@@ -1,5 +1,5 @@
-// Quantized linear for a small batch of right-hand sides (3..64 decode streams, short verify
-// runs): every packed weight byte is read ONCE for the whole batch.
+// Quantized linear for a small batch of right-hand sides (2 to 16 decode streams, short verify
+// runs; more on tensors without the tcgen05 form or with single-term operands): every packed weight byte is read ONCE for the whole batch.
 //
 //     y[n, o] = epi( sum_c W[o, c] x[n, c] ),   n < N
 //
@@ -753,8 +753,8 @@ extern "C" int rwkvq_gemv_batch(const rwkvq_qtensor* t, const float* x, int N, i
     RWKVQ_REQUIRE(epilogue >= RWKVQ_EPI_NONE && epilogue <= RWKVQ_EPI_ADD, RWKVQ_E_DTYPE, "rwkvq_gemv_batch: epilogue %d", epilogue);
     RWKVQ_REQUIRE(ldx >= t->cols && ldy >= t->rows, RWKVQ_E_SHAPE, "rwkvq_gemv_batch: ldx %lld / ldy %lld", (long long)ldx, (long long)ldy);
     RWKVQ_REQUIRE(x && y, RWKVQ_E_NULL, "rwkvq_gemv_batch: x or y is null");
-    // default: the two-term mma.sync kernel.  The tcgen05 kernel (single fp16 operands) serves more than
-    // 32 rows in fast mode, tensors the mma.sync kernel has no layout for, and the profiling override.
+    // default: the two-term mma.sync kernel below kSbLeastRows rows, the tcgen05 pipeline from there on (gemm_sb_pays);
+    // single-term operands: mma.sync up to 32 rows, the single-buffer tcgen05 kernel above
     const bool tcb_ok = tcb_enabled() && gemm_tcb_ok(*t) && t->cols <= kPairCols;
     // tensors without the relayouted streams: the tcgen05 kernel that reads the file buffers, in either precision
     const bool bare = mma_layout_of(*t) < 0;

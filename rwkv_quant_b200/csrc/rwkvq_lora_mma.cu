@@ -1,8 +1,7 @@
 // The four LoRA branches of the time-mix block for a BATCH of decode streams on the tensor
 // cores (backends/metal/quant_model.py:462-526: y_br = act_br(x_br @ W1_br) @ W2_br with
 // act = tanh / none / sigmoid / none for the decay, in-context rate, gate and value-residual
-// branches).  The per-stream kernels of rwkvq_decode.cu serve up to 8 streams; beyond that
-// they re-read the matrices for every group of 8 streams and run on the SIMT pipes.  Here:
+// branches), and for the rows of short forward calls.
 //
 //   down   grid (8 K slices = one cluster, branch x stream group, 32-column groups of the rank):
 //          a CTA turns its [K/8, 32] slice of W1 (file bytes, stored [in, out]) into fp16 in the

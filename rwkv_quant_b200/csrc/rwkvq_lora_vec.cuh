@@ -2,8 +2,7 @@
 //   down   y-slices of the r / k / v GEMV's grid (rwkvq_gemv_mma.cu): both products read rows the same LayerNorm wrote;
 //   up     the head of the time-mix core (rwkvq_decode.cu): a head's CTA needs its own 64 columns of the four W2 only.
 // The layer's chain loses two dependent launches and the fork and join of a side stream, behind which no kernel starts
-// programmatically (its weight loads then wait for
-// the join).  2048 wide: 18.5 us of chain in four launches -> 14 us in three.
+// programmatically (its weight loads then wait for the join).  2048 wide: 18.5 us of chain in four launches -> 14 in three.
 #pragma once
 #include <type_traits>
 
