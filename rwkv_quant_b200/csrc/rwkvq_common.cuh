@@ -290,6 +290,14 @@ bool lora_mma_ok(const rwkvq_qtensor* const* t1, const rwkvq_qtensor* const* t2,
 int launch_lora_pair_mma(const rwkvq_qtensor* const* t1, const rwkvq_qtensor* const* t2, const float* const* xs,
                          float* const* ys, const int* acts, int n_br, int B, int D, int max_rank, float* h, int n_stride,
                          cudaStream_t s);
+// A second stream beside the caller's for the independent half of a layer's time mix (rwkvq_decode.cu); null: go without
+struct SideLane {
+    cudaStream_t stream = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
+    int start(cudaStream_t caller) const;        // the side stream waits for what the caller has issued
+    int finish(cudaStream_t caller) const;       // the caller waits for the side stream
+};
+SideLane* side_lane(cudaStream_t caller);
 int launch_row_amax(const float* x, long long ldx, int cols, int N, float* amax, int* status, cudaStream_t s);
 
 }  // namespace rwkvq

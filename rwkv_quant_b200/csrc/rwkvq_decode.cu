@@ -772,6 +772,48 @@ __global__ void __launch_bounds__(kArgSlices) argmax_final_kernel(const float* p
     }
 }
 
+// The LoRA branches depend on the normalised row only, not on r/k/v: the two run on two streams between a fork after LN1
+// and a join before the time mix, in a captured graph as parallel branches.  One side stream and two events per (device,
+// caller stream), created on the first call that uses that stream (not during its capture: such a call goes without):
+// sequences issued on different streams, from one or several host threads, never share an event.  Calls on the SAME
+// stream must come from one thread at a time, as for any stream-ordered API.
+// RWKVQ_FORK=0 keeps everything on the caller's stream.
+SideLane* side_lane(cudaStream_t caller) {
+    static const bool enabled = [] { const char* e = getenv("RWKVQ_FORK"); return !(e && e[0] == '0'); }();
+    if (!enabled) return nullptr;
+    static std::mutex mu;
+    static std::map<std::pair<int, cudaStream_t>, SideLane> lanes;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+    std::lock_guard<std::mutex> lock(mu);
+    SideLane& l = lanes[std::make_pair(dev, caller)];
+    if (!l.stream) {
+        cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(caller, &capturing) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+        if (capturing != cudaStreamCaptureStatusNone) return nullptr;
+        SideLane n;
+        if (cudaStreamCreateWithFlags(&n.stream, cudaStreamNonBlocking) != cudaSuccess ||
+            cudaEventCreateWithFlags(&n.fork, cudaEventDisableTiming) != cudaSuccess ||
+            cudaEventCreateWithFlags(&n.join, cudaEventDisableTiming) != cudaSuccess) {
+            if (n.fork) cudaEventDestroy(n.fork);
+            if (n.stream) cudaStreamDestroy(n.stream);
+            return nullptr;
+        }
+        l = n;
+    }
+    return &l;
+}
+int SideLane::start(cudaStream_t caller) const {
+    if (cudaEventRecord(fork, caller) != cudaSuccess || cudaStreamWaitEvent(stream, fork, 0) != cudaSuccess)
+        return fail(RWKVQ_E_LAUNCH, "fork onto the side stream failed");
+    return RWKVQ_OK;
+}
+int SideLane::finish(cudaStream_t caller) const {
+    if (cudaEventRecord(join, stream) != cudaSuccess || cudaStreamWaitEvent(caller, join, 0) != cudaSuccess)
+        return fail(RWKVQ_E_LAUNCH, "join of the side stream failed");
+    return RWKVQ_OK;
+}
+
 }  // namespace rwkvq
 
 using namespace rwkvq;
@@ -888,38 +930,6 @@ int linear(const rwkvq_qtensor* t, const float* x, int B, int in, float* y, int 
     if (B > 2 && (t->kind == RWKVQ_KIND_SB6 || t->kind == RWKVQ_KIND_SYM))     // tcgen05 path for large batches
         return rwkvq_gemm(t, x, B, in, y, out, epi, resid, gemm_ws, rwkvq_gemm_workspace_bytes_for(B, in), stream);
     return rwkvq_gemv(t, x, RWKVQ_F32, B, in, y, out, epi, resid, stream);
-}
-
-// The LoRA branches depend on the normalised row only, not on r/k/v: they run on a side
-// stream between a fork after LN1 and a join before the time-mix core, so that in a captured
-// graph they form a parallel branch beside the r/k/v GEMV instead of two more links of the
-// dependent chain.  One side stream and two events per (device, caller stream), created on the
-// first call that uses that stream (make it outside stream capture): sequences issued on
-// different streams, from one or several host threads, never share an event.  Calls on the SAME
-// stream must come from one thread at a time, as for any stream-ordered API.
-// RWKVQ_FORK=0 keeps everything on the caller's stream.
-struct SideLane { cudaStream_t stream = nullptr; cudaEvent_t fork = nullptr, join = nullptr; };
-SideLane* side_lane(cudaStream_t caller) {
-    static const bool enabled = [] { const char* e = getenv("RWKVQ_FORK"); return !(e && e[0] == '0'); }();
-    if (!enabled) return nullptr;
-    static std::mutex mu;
-    static std::map<std::pair<int, cudaStream_t>, SideLane> lanes;
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
-    std::lock_guard<std::mutex> lock(mu);
-    SideLane& l = lanes[std::make_pair(dev, caller)];
-    if (!l.stream) {
-        SideLane n;
-        if (cudaStreamCreateWithFlags(&n.stream, cudaStreamNonBlocking) != cudaSuccess ||
-            cudaEventCreateWithFlags(&n.fork, cudaEventDisableTiming) != cudaSuccess ||
-            cudaEventCreateWithFlags(&n.join, cudaEventDisableTiming) != cudaSuccess) {
-            if (n.fork) cudaEventDestroy(n.fork);
-            if (n.stream) cudaStreamDestroy(n.stream);
-            return nullptr;
-        }
-        l = n;
-    }
-    return &l;
 }
 
 int launch_tmix_core_up(const TmixCoreArgs& tc, const LoraVecArgs& up, int H, cudaStream_t s) {
@@ -1108,8 +1118,8 @@ int rwkvq_decode_step(const rwkvq_model* m, int B, const int64_t* tokens, float*
         SideLane* lane = side_lane(s);
         cudaStream_t s_lora = s;
         if (lane) {                                  // fork: the LoRA branches leave the chain here
-            if (cudaEventRecord(lane->fork, s) != cudaSuccess || cudaStreamWaitEvent(lane->stream, lane->fork, 0) != cudaSuccess)
-                return fail(RWKVQ_E_LAUNCH, "rwkvq_decode_step: fork onto the side stream failed");
+            rc = lane->start(s);
+            if (rc) return rc;
             s_lora = lane->stream;
         }
         // Up to 16 streams the LoRA pair (two dependent launches) is the longer of the two branches: it then
@@ -1173,8 +1183,8 @@ int rwkvq_decode_step(const rwkvq_model* m, int B, const int64_t* tokens, float*
             if (rc) return rc;
         }
         if (lane) {                                  // join before the time-mix core
-            if (cudaEventRecord(lane->join, lane->stream) != cudaSuccess || cudaStreamWaitEvent(s, lane->join, 0) != cudaSuccess)
-                return fail(RWKVQ_E_LAUNCH, "rwkvq_decode_step: join of the side stream failed");
+            rc = lane->finish(s);
+            if (rc) return rc;
         }
         launch_pdl(tmix_core_kernel<false>, dim3(H, B), dim3(256), 0, s, tc, 0);
         }
