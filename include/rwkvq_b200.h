@@ -411,7 +411,7 @@ int rwkvq_decode_step(const rwkvq_model* m_host, int B, const int64_t* tokens,
  *   tokens [B, T] int64 on the device
  *   *_in   host arrays [n_layer] of device pointers: wkv [B, H, 64, 64], shift rows [B, D] fp32 (not
  *          modified; NULL entries: zeros).  *_out: where the carried states go (an entry may equal its
- *          wkv_in entry; the shift rows of a layer must not alias their inputs)
+ *          wkv_in entry; the shift rows of a layer must not alias their inputs).  All 16-byte aligned.
  *   hidden [B, T, D] the final-LayerNorm rows, or NULL;  logits [B, tail, vocab] of the last `tail`
  *          positions (tail = 0: none)
  * Rows N = B * T up to 64 run on the fp32-grade small-batch linears (rwkvq_gemv_batch), more on fp16

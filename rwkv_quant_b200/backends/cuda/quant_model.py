@@ -347,6 +347,8 @@ class QuantRWKV7:
         idx = idx.contiguous()
         ins = [[None if st[k] is None else st[k].reshape(shape).contiguous().float() for st in states]
                for k, shape in ((0, (B, H, S, S)), (1, (B, D)), (2, (B, D)))]
+        # shift rows may start anywhere; the call reads float4
+        ins[1:] = [[t if t is None or t.data_ptr() % 16 == 0 else t.clone() for t in ts] for ts in ins[1:]]
         f32 = dict(dtype=torch.float32, device=dev)
         outs = [torch.empty((L, B, H, S, S), **f32), torch.empty((L, B, 1, D), **f32), torch.empty((L, B, 1, D), **f32)]
         hidden = torch.empty((B, T, D), **f32) if want_hidden else None

@@ -853,6 +853,17 @@ bool sb_model_ok(const rwkvq_model& m) {
     return true;
 }
 
+// The pipeline's row preparation reads and writes float4 (the LayerNorm kernels of the other forms take any row)
+bool sb_rows_ok(const rwkvq_model& m, float* const* tshift, float* const* cshift) {
+    bool ok = aligned(m.lnout_w, 16) && aligned(m.lnout_b, 16);
+    for (int l = 0; l < m.n_layer && ok; ++l) {
+        const rwkvq_layer& L = m.layers[l];
+        for (const float* p : {L.ln1_w, L.ln1_b, L.ln2_w, L.ln2_b, L.x_mix, L.ffn_x_k, const_cast<const float*>(tshift[l]), const_cast<const float*>(cshift[l])})
+            ok = ok && aligned(p, 16);
+    }
+    return ok;
+}
+
 struct Workspace {
     float *x, *xs, *rkv, *part, *yl, *og, *xk, *hffn, *xo, *v_first, *logits, *argv, *gemm_ws;
     int* status;             // first word of the workspace: RWKVQ_E_TIMEOUT if a bounded device-side wait of a step ran out
@@ -1039,7 +1050,9 @@ int rwkvq_decode_step(const rwkvq_model* m, int B, const int64_t* tokens, float*
     int rc = validate_qtensor(&m->emb, "rwkvq_decode_step(emb)");
     if (rc) return rc;
     float* lg = logits ? logits : w.logits;
-    const bool sb = sb_wanted(B) && sb_model_ok(*m);
+    for (int l = 0; l < m->n_layer; ++l)
+        RWKVQ_REQUIRE(aligned(wkv[l], 16), RWKVQ_E_ALIGN, "rwkvq_decode_step: the WKV state of layer %d must be 16-byte aligned", l);
+    const bool sb = sb_wanted(B) && sb_model_ok(*m) && sb_rows_ok(*m, tshift, cshift);
     if (sb) {
         for (int l = 0; l < m->n_layer; ++l)
             for (const rwkvq_qtensor* t : {&m->layers[l].Wr, &m->layers[l].Wk, &m->layers[l].Wv, &m->layers[l].Wo, &m->layers[l].Wfk, &m->layers[l].Wfv}) {

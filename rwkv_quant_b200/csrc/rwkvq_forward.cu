@@ -217,6 +217,12 @@ int rwkvq_forward_seq(const rwkvq_model* m, int B, int T, const int64_t* tokens,
             if (rc) return rc;
         }
     }
+    for (int l = 0; l < m->n_layer; ++l)
+        RWKVQ_REQUIRE(wkv_out[l] && tshift_out[l] && cshift_out[l], RWKVQ_E_NULL, "rwkvq_forward_seq: a state of layer %d has nowhere to go", l);
+    for (int l = 0; l < m->n_layer; ++l)
+        for (const float* p : {wkv_in[l], tshift_in[l], cshift_in[l], const_cast<const float*>(wkv_out[l]),
+                               const_cast<const float*>(tshift_out[l]), const_cast<const float*>(cshift_out[l])})
+            RWKVQ_REQUIRE(aligned(p, 16), RWKVQ_E_ALIGN, "rwkvq_forward_seq: the states of layer %d must be 16-byte aligned", l);
     const ForwardWs w = carve(*m, B, T, static_cast<size_t>(B) * tail, workspace);
     RWKVQ_REQUIRE(workspace_bytes >= w.bytes && aligned(workspace, 256), RWKVQ_E_LIMIT,
                   "rwkvq_forward_seq: workspace %zu of %zu bytes, 256-byte aligned", workspace_bytes, w.bytes);

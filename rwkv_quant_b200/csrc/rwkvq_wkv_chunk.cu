@@ -553,6 +553,8 @@ int launch_wkv_chunked(const WkvChunkArgs& p, cudaStream_t s) {
     static_assert(sizeof(PreSmem) * kPreUnits <= kPreStage, "operands over the staged rows");
     const long long blocks = static_cast<long long>(p.B) * n_chunks * groups;
     RWKVQ_REQUIRE(blocks < (1ll << 31), RWKVQ_E_LIMIT, "wkv_chunked: too many tokens");
+    RWKVQ_REQUIRE(aligned(p.h_in, 16) && aligned(p.h_out, 16) && aligned(p.ln_w, 8) && aligned(p.ln_b, 8), RWKVQ_E_ALIGN,
+                  "wkv_chunked: states on 16-byte boundaries, group-norm parameters on 8-byte ones");
     cudaError_t e = cudaFuncSetAttribute(wkv_operands_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kPreStage));
     if (e != cudaSuccess) return fail(RWKVQ_E_LIMIT, "wkv_operands: shared memory: %s", cudaGetErrorString(e));
     e = launch_pdl(wkv_operands_kernel, dim3(static_cast<unsigned>(blocks)), dim3(64 * kPreUnits), kPreStage, s, p, n_chunks);

@@ -1,0 +1,49 @@
+"""Inputs at the edges of what the forward calls, the decode step and the linears take: non-finite values, tensors off
+16-byte boundaries, states that share their storage, shapes beyond one kernel's range."""
+import numpy as np
+import pytest
+import torch
+
+from helpers import relmax
+from test_gpu_dequant_gemv import _oracle_w, _synth_linear, _x
+
+pytestmark = pytest.mark.gpu
+
+
+def _model(recipe="compression", n_embd=256, ffn=1024, **kw):
+    from rwkv_quant_b200 import synth
+    from rwkv_quant_b200.backends.cuda import QuantRWKV7
+    return QuantRWKV7(synth.build_checkpoint(dict(n_layer=2, vocab=512, n_embd=n_embd, ffn=ffn), recipe, seed=3, device="cuda"),
+                      device="cuda", **kw)
+
+
+def _states(model, B, offset=0):
+    """States whose shift rows start ``offset`` floats behind a 16-byte boundary."""
+    gen = torch.Generator(device="cuda").manual_seed(B)
+
+    def draw(*shape, off=0):
+        t = torch.empty(int(np.prod(shape)) + off, device="cuda")[off:].view(shape)
+        return t.copy_(0.2 * torch.randn(shape, generator=gen, device="cuda"))
+    D, H = model.n_embd, model.n_head
+    return [(draw(B, H, 64, 64), draw(B, 1, D, off=offset), draw(B, 1, D, off=offset)) for _ in range(model.n_layer)]
+
+
+def _idx(B, T):
+    return torch.randint(1, 512, (B, T), generator=torch.Generator().manual_seed(100 * B + T)).cuda()
+
+
+@pytest.mark.parametrize("B", [3, 20])
+def test_shift_rows_off_16_byte_boundaries(cuda_lib, B):
+    """Both regimes of a decode step and of short and long forward calls; a WKV state there is refused."""
+    model = _model()
+    for T in (1, 2, 17):
+        idx = _idx(B, T)
+        ref, rst = model.forward_stateful(idx, _states(model, B))
+        got, gst = model.forward_stateful(idx, _states(model, B, offset=1))
+        assert relmax(got.cpu().numpy(), ref.cpu().numpy()) <= 1e-4
+        for s, r in zip(gst, rst):
+            for a, b in zip(s, r):
+                assert relmax(a.cpu().numpy(), b.cpu().numpy()) <= 1e-4
+        off = [(torch.zeros(s[0].numel() + 1, device="cuda")[1:].view(s[0].shape), s[1], s[2]) for s in _states(model, B)]
+        with pytest.raises(RuntimeError, match="16-byte"):
+            model.forward_stateful(idx, off)
