@@ -251,7 +251,7 @@ def gemv_direct(dq: "DeviceQT", x: torch.Tensor, epilogue: int = 0, resid: Optio
     single-row call took); a graph being traced gets the registered operator."""
     if torch.compiler.is_compiling():
         return gemv(dq.bufs, dq.meta, x, epilogue, resid)
-    _require_cuda(x, resid)
+    _require_cuda(dq.bufs[0], x, resid)
     n = x.shape[0]
     y = torch.empty((n, dq.rows), dtype=torch.float32, device=x.device)
     _lib.check(_lib.load().rwkvq_gemv(dq.struct_ref, x.data_ptr(), _lib.DTYPE_CODE[x.dtype], n, x.stride(0), y.data_ptr(),
@@ -300,7 +300,7 @@ def gemv_batch(dq: "DeviceQT", x: torch.Tensor, epilogue: int = 0, resid: Option
                check: bool = False) -> torch.Tensor:
     """x [N, IN] -> y [N, OUT] fp32 with the packed weights read once for all N rows (mma.sync
     tensor cores, tokens as the MMA columns, fp16 operands, fp32 accumulation)."""
-    _require_cuda(x, resid)
+    _require_cuda(dq.bufs[0], x, resid)
     lib = _lib.load()
     x = x.float()
     if x.stride(-1) != 1 or x.stride(0) % 4 or x.data_ptr() % 16:
@@ -326,10 +326,10 @@ def lora_pair_ok(pairs, D: int) -> bool:
 def lora_pair(pairs, xs: Sequence[torch.Tensor], acts: Sequence[int]) -> List[torch.Tensor]:
     """y_i = act_i(x_i @ W1_i) @ W2_i for up to four (W1, W2) pairs of tensors stored [in, out], x_i
     [N, D] fp32 -> y_i [N, C]: two tensor-core launches for all branches (act: 0 none, 1 tanh, 2 sigmoid)."""
-    lib = _lib.load()
     n_br = len(pairs)
     xs = [x.float().contiguous() for x in xs]
-    _require_cuda(*xs)
+    _require_cuda(*xs, *(w.bufs[0] for pair in pairs for w in pair))
+    lib = _lib.load()
     N, D = xs[0].shape
     ys = [torch.empty((N, pairs[0][1].cols), dtype=torch.float32, device=xs[0].device) for _ in range(n_br)]
     t1 = (QTensorStruct * n_br)(*[a.struct for a, _ in pairs])
@@ -347,7 +347,7 @@ def gemm(dq: "DeviceQT", x: torch.Tensor, epilogue: int = 0, resid: Optional[tor
     """x [M, IN] fp32 -> y [M, OUT] fp32 on the tcgen05 tensor cores with the dequantisation
     fused into the operand producer (sb6 / sym tensors).  ``check`` synchronises and raises
     if the kernel reported that a bounded pipeline wait ran out."""
-    _require_cuda(x, resid)
+    _require_cuda(dq.bufs[0], x, resid)
     lib = _lib.load()
     x = x.float().contiguous()
     m = x.shape[0]
@@ -377,7 +377,7 @@ PREP_SCALED, PREP_SPLIT, PREP_F32 = 1, 2, 4
 
 def gemm_x16(dq: "DeviceQT", rows: PreparedRows, epilogue: int = 0, resid: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``gemm`` on rows already scaled and rounded to fp16 (no pre-pass over the activations)."""
-    _require_cuda(rows.x16, resid)
+    _require_cuda(dq.bufs[0], rows.x16, resid)
     lib = _lib.load()
     m = rows.n
     nws = lib.rwkvq_gemm_workspace_bytes_for(m, 0)
@@ -429,7 +429,7 @@ def seq_ln_shift_mix_prep(x: torch.Tensor, ln_w, ln_b, shift_in: Optional[torch.
 
 def gemv_fused(dqts: Sequence[DeviceQT], xstack: torch.Tensor) -> torch.Tensor:
     """K same-shape matrices, K inputs [K, IN] -> [K, OUT], one launch."""
-    _require_cuda(xstack)
+    _require_cuda(xstack, *(d.bufs[0] for d in dqts))
     lib = _lib.load()
     k = len(dqts)
     arr = (QTensorStruct * k)(*[d.struct for d in dqts])
@@ -456,7 +456,7 @@ def seq_ln_shift_mix(x: torch.Tensor, ln_w, ln_b, shift_in: Optional[torch.Tenso
 
 def seq_embed_ln0(emb: "DeviceQT", idx: torch.Tensor, ln_w: torch.Tensor, ln_b: torch.Tensor) -> torch.Tensor:
     """idx [...] int64 -> LayerNorm0(rows of the packed embedding table) [..., D] fp32, one kernel."""
-    _require_cuda(idx, ln_w)
+    _require_cuda(idx, ln_w, emb.bufs[0])
     flat = idx.reshape(-1).contiguous().long()
     out = torch.empty((flat.numel(), emb.cols), dtype=torch.float32, device=idx.device)
     _lib.check(_lib.load().rwkvq_seq_embed_ln0(C.byref(emb.struct), flat.data_ptr(), ln_w.data_ptr(), ln_b.data_ptr(),

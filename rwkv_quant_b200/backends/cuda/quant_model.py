@@ -166,6 +166,7 @@ class QuantRWKV7:
     def _materialize(self, states, B):
         out = []
         for wkv, ts, cs in states:
+            ops._require_cuda(wkv, ts, cs)
             z = lambda t: (torch.zeros((B, 1, self.n_embd), device=self.device) if t is None
                            else t.reshape(B, 1, self.n_embd).contiguous().float())
             out.append((wkv.contiguous().float(), z(ts), z(cs)))
@@ -343,6 +344,8 @@ class QuantRWKV7:
         launch of the pass issued by one library call."""
         B, T = idx.shape
         L, H, S, D, dev = self.n_layer, self.n_head, self.head_size, self.n_embd, self.device
+        for st in states:
+            ops._require_cuda(*st)
         lib = _lib.load()
         idx = idx.contiguous()
         ins = [[None if st[k] is None else st[k].reshape(shape).contiguous().float() for st in states]

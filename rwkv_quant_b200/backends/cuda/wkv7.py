@@ -21,6 +21,8 @@ def wkv7_infer(r, w, k, v, a, b, state):
         if not t.is_cuda or t.shape != (B, T, H, S):
             raise RuntimeError("wkv7_infer: CUDA tensors of one shape [B, T, H, 64] are required")
     h_in = state.contiguous().float()
+    if not h_in.is_cuda:
+        raise RuntimeError("wkv7_infer: the state must be a CUDA tensor")
     out = torch.empty((B, T, H, S), dtype=torch.float32, device=r.device)
     h_out = torch.empty_like(h_in)
     lib = _lib.load()
