@@ -418,7 +418,7 @@ int rwkvq_decode_step(const rwkvq_model* m_host, int B, const int64_t* tokens,
  * tensor-core operands (the arithmetic of rwkvq_gemm; LoRA products with x as an fp16 pair).
  * rwkvq_forward_seq_ok: 1 if every tensor of the model has a layout this serves at n_rows rows (sb6 / sym
  * linears with their relayouted streams; per-row int8 up to 64 rows; LoRA shapes of rwkvq_lora_pair;
- * n_embd a multiple of 128 up to 4096).  workspace: rwkvq_forward_seq_workspace_bytes, 256-byte
+ * n_embd a multiple of 128 up to 4096) and the shape the model's dimensions give it.  workspace: rwkvq_forward_seq_workspace_bytes, 256-byte
  * aligned; its first int32 is a status word (RWKVQ_E_TIMEOUT if a bounded device-side wait ran out).
  */
 int rwkvq_forward_seq_ok(const rwkvq_model* m_host, int64_t n_rows);

@@ -842,13 +842,16 @@ bool sb_wanted(int B) {
     return g_tcb_exact == 1 || B >= kSbMinStreams;
 }
 bool sb_model_ok(const rwkvq_model& m) {
-    if (!seq_prep_in_place_ok(m.n_embd) || !gemm_sb_ok(m.head)) return false;
+    const int D = m.n_embd, F = m.ffn_dim;
+    auto ok = [](const rwkvq_qtensor& t, int rows, int cols) { return gemm_sb_ok(t) && t.rows == rows && t.cols == cols; };
+    if (!seq_prep_in_place_ok(D) || !ok(m.head, m.vocab_size, D)) return false;
     for (int l = 0; l < m.n_layer; ++l) {
         const rwkvq_layer& L = m.layers[l];
-        for (const rwkvq_qtensor* t : {&L.Wr, &L.Wk, &L.Wv, &L.Wo, &L.Wfk, &L.Wfv})
-            if (!gemm_sb_ok(*t)) return false;
+        for (const rwkvq_qtensor* t : {&L.Wr, &L.Wk, &L.Wv, &L.Wo})
+            if (!ok(*t, D, D)) return false;
+        if (!ok(L.Wfk, F, D) || !ok(L.Wfv, D, F)) return false;
         for (const rwkvq_qtensor* t : {&L.Wk, &L.Wv})
-            if (t->kind != L.Wr.kind || t->bits != L.Wr.bits || t->rows != L.Wr.rows || t->cols != L.Wr.cols) return false;
+            if (t->kind != L.Wr.kind || t->bits != L.Wr.bits) return false;
     }
     return true;
 }

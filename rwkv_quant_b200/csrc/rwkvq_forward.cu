@@ -183,16 +183,23 @@ int rwkvq_forward_seq_ok(const rwkvq_model* m, int64_t n_rows) {
     if (!m || !m->layers || n_rows < 2 || n_rows >= (1ll << 31) / 64) return 0;
     if (m->head_size != 64 || m->n_embd % 128 != 0 || m->n_embd > 4096 || m->ffn_dim % 256 != 0 || m->ffn_dim > 32768) return 0;
     const bool small = n_rows <= kSmallRows;
-    auto linear_ok = [&](const rwkvq_qtensor& t) { return mma_layout_of(t) >= 0 && (small || fp16_gemm_ok(t)); };
+    const int D = m->n_embd, F = m->ffn_dim;
+    // sizes of the scratch and of every launch follow from the model's dimensions: the tensors must have them too
+    auto linear_ok = [&](const rwkvq_qtensor& t, int rows, int cols) {
+        return t.rows == rows && t.cols == cols && mma_layout_of(t) >= 0 && (small || fp16_gemm_ok(t));
+    };
     for (int l = 0; l < m->n_layer; ++l) {
         const rwkvq_layer& L = m->layers[l];
-        for (const rwkvq_qtensor* t : {&L.Wr, &L.Wk, &L.Wv, &L.Wo, &L.Wfk, &L.Wfv})
-            if (!linear_ok(*t)) return 0;
+        for (const rwkvq_qtensor* t : {&L.Wr, &L.Wk, &L.Wv, &L.Wo})
+            if (!linear_ok(*t, D, D)) return 0;
+        if (!linear_ok(L.Wfk, F, D) || !linear_ok(L.Wfv, D, F)) return 0;
         const rwkvq_qtensor* t1[4] = {&L.w1, &L.a1, &L.g1, &L.v1};
         const rwkvq_qtensor* t2[4] = {&L.w2, &L.a2, &L.g2, &L.v2};
-        if (!lora_mma_ok(t1, t2, l == 0 ? 3 : 4, m->n_embd) || t2[0]->cols != m->n_embd) return 0;
+        if (!lora_mma_ok(t1, t2, l == 0 ? 3 : 4, D) || t2[0]->cols != D) return 0;
+        for (int i = 0; i < (l == 0 ? 3 : 4); ++i)
+            if (t1[i]->cols > m->max_rank) return 0;
     }
-    return mma_layout_of(m->head) >= 0 && fp16_gemm_ok(m->head) ? 1 : 0;
+    return m->emb.cols == D && m->head.rows == m->vocab_size && m->head.cols == D && mma_layout_of(m->head) >= 0 && fp16_gemm_ok(m->head) ? 1 : 0;
 }
 
 size_t rwkvq_forward_seq_workspace_bytes(const rwkvq_model* m, int B, int T, int tail) {
@@ -214,6 +221,10 @@ int rwkvq_forward_seq(const rwkvq_model* m, int B, int T, const int64_t* tokens,
         const rwkvq_layer& L = m->layers[l];
         for (const rwkvq_qtensor* t : {&L.Wr, &L.Wk, &L.Wv, &L.Wo, &L.Wfk, &L.Wfv, &L.w1, &L.w2, &L.a1, &L.a2, &L.g1, &L.g2}) {
             int rc = validate_qtensor(t, "rwkvq_forward_seq");
+            if (rc) return rc;
+        }
+        for (const rwkvq_qtensor* t : {&L.v1, &L.v2}) {
+            int rc = l == 0 ? RWKVQ_OK : validate_qtensor(t, "rwkvq_forward_seq");
             if (rc) return rc;
         }
     }
