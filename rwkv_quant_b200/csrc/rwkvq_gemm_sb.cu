@@ -635,7 +635,9 @@ int launch_sb_nt(SbArgs& a, const SbMaps& maps, int nt, int groups, int force_ks
 }  // namespace
 
 bool gemm_sb_ok(const rwkvq_qtensor& t) {
-    return gemm_tcb_ok(t) && (t.kind == RWKVQ_KIND_SB6 || t.kind == RWKVQ_KIND_SYM) && mma_layout_of(t) >= 0;
+    // 16-byte copies of codes, records (sym: block scales) and planes; the mma.sync form reads block scales by 8 bytes
+    return gemm_tcb_ok(t) && (t.kind == RWKVQ_KIND_SB6 || t.kind == RWKVQ_KIND_SYM) && mma_layout_of(t) >= 0 && aligned(t.codes, 16) &&
+           aligned(t.kind == RWKVQ_KIND_SB6 ? static_cast<const void*>(t.dev_meta) : static_cast<const void*>(t.qs), 16) && aligned(t.dev_planes, 16);
 }
 // Whether this kernel takes a product the mma.sync kernel serves too.  That one stages the activations per row group,
 // which costs it as much as the conversion to tensor memory costs this one up to 16 rows ([2048, 2048] 14.3 against 18 us,

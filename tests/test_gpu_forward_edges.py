@@ -47,3 +47,21 @@ def test_shift_rows_off_16_byte_boundaries(cuda_lib, B):
         off = [(torch.zeros(s[0].numel() + 1, device="cuda")[1:].view(s[0].shape), s[1], s[2]) for s in _states(model, B)]
         with pytest.raises(RuntimeError, match="16-byte"):
             model.forward_stateful(idx, off)
+
+
+@pytest.mark.parametrize("bits", [6, 8])
+@pytest.mark.parametrize("N", [16, 17, 64])
+def test_block_scales_on_an_8_byte_boundary(cuda_lib, bits, N):
+    """The int8 scale codes of a sym tensor may start on any boundary that suits the mma.sync kernel (8 bytes)."""
+    from rwkv_quant_b200.backends.cuda import ops
+    dq = ops.DeviceQT(_synth_linear("sym", bits, 256, 512, seed=bits))
+    x = _x(N, 512, N)
+    want = ops.gemv_batch(dq, x, check=True)
+    i = ops._BUF_ORDER.index("qs")
+    qs = dq.bufs[i]
+    room = torch.empty(qs.numel() + 8, dtype=qs.dtype, device="cuda")
+    assert room.data_ptr() % 16 == 0
+    dq.bufs[i] = room[8:].view(qs.shape).copy_(qs)
+    dq.struct = ops._descr(dq.bufs, dq.meta)
+    got = ops.gemv_batch(dq, x, check=True)
+    assert relmax(got.cpu().numpy(), want.cpu().numpy()) <= 4e-6       # another kernel from 17 rows on
