@@ -218,7 +218,7 @@ int rwkvq_gemv_batch(const rwkvq_qtensor* t, const float* x, int N, int64_t ldx,
  * fp16, then a dense matmul).  The weights are converted into scratch in row chunks that stay in L2
  * and read back by TMA.  Operands are fp16 (weights: fp16(q*s+m); tokens:
  * scaled per row by a power of two), accumulation fp32 in tensor memory.
- *   x [M, ldx] fp32, y [M, ldy] fp32, sb6 / sym tensors of at most 32768 columns.
+ *   x [M, ldx] fp32, y [M, ldy] fp32, sb6 / sym tensors only.
  *   workspace: rwkvq_gemm_workspace_bytes_for(M, IN) bytes, 256-byte aligned (or
  *   rwkvq_gemm_workspace_bytes(M), which covers IN <= 16384); it holds the fp16 copy of x and of a
  *   chunk of the weights.  Its first int32 is a status word the

@@ -23,6 +23,8 @@
 
 #include <cooperative_groups.h>
 
+#include <algorithm>
+
 #include "rwkvq_decode_parts.cuh"
 #include "rwkvq_tc.cuh"
 
@@ -92,8 +94,8 @@ __global__ void __launch_bounds__(256) dequant_f16_kernel(const QView t, int row
 }
 
 int launch_dequant_f16(const rwkvq_qtensor& t, int row0, int rows, __half* out, float* n2, cudaStream_t s) {
-    RWKVQ_REQUIRE((t.kind == RWKVQ_KIND_SB6 || t.kind == RWKVQ_KIND_SYM) && t.cols % 256 == 0 && t.cols <= 32768, RWKVQ_E_DTYPE,
-                  "dequant_f16: sb6 / sym tensors of at most 32768 columns");
+    RWKVQ_REQUIRE((t.kind == RWKVQ_KIND_SB6 || t.kind == RWKVQ_KIND_SYM) && t.cols % 256 == 0 && (n2 == nullptr || t.cols <= 32768), RWKVQ_E_DTYPE,
+                  "dequant_f16: sb6 / sym tensors (with norms of at most 32768 columns)");
     const long long items = static_cast<long long>(rows) * (t.cols >> 5);
     const long long want = (items + 255) / 256;
     const unsigned grid = static_cast<unsigned>(want < 148 * 6 ? want : 148 * 6);
@@ -793,15 +795,21 @@ namespace {
 // Row pitch of the fp16 activation copy: 128 bytes more than the row, so that the rows of a TMA box do
 // not all map to the same L2 slice (a power-of-two pitch does).
 inline size_t x16_pitch(int cols) { return static_cast<size_t>(cols) + 64; }
-// Weights are converted in chunks of rows that fit this scratch, half of L2: it is read back at once.
+// Weights are converted in chunks of rows that fit this scratch, half of L2: it is read back at once.  Whole tiles of
+// 256 rows up to 131072 columns, at least one row beyond.
 constexpr size_t kGemmScratch = 64u << 20;
+inline int gemm_chunk_rows(int cols) {
+    const size_t n = kGemmScratch / sizeof(__half) / cols;
+    return n >= 256 ? static_cast<int>(n / 256 * 256) : n > 0 ? static_cast<int>(n) : 1;
+}
+inline size_t gemm_scratch(int cols) { return std::max(kGemmScratch, sizeof(__half) * cols); }
 inline size_t up256(size_t n) { return (n + 255) / 256 * 256; }
 inline size_t ws_x16_off(size_t m) { return 256 + up256(sizeof(float) * m); }
 inline size_t ws_w_off(size_t m, int x_cols) { return ws_x16_off(m) + (x_cols > 0 ? up256(sizeof(__half) * m * x16_pitch(x_cols)) : 0); }
 
 int gemm_chunks(const rwkvq_qtensor* t, const __half* x16, const float* row_scale, int M, float* y, int64_t ldy, int epilogue,
                 const float* resid, __half* scratch, int* status, cudaStream_t s) {
-    const int chunk = static_cast<int>(kGemmScratch / sizeof(__half) / t->cols / 256) * 256;
+    const int chunk = gemm_chunk_rows(t->cols);
     for (int r0 = 0; r0 < t->rows; r0 += chunk) {
         const int rows = t->rows - r0 < chunk ? t->rows - r0 : chunk;
         int rc = launch_dequant_f16(*t, r0, rows, scratch, nullptr, s);
@@ -823,7 +831,7 @@ void rwkvq_profiling_gemm_acc_mode(int mode) { g_gemm_acc_mode = mode; }      //
 
 size_t rwkvq_gemm_x16_pitch(int cols) { return x16_pitch(cols); }
 size_t rwkvq_gemm_workspace_bytes_for(int M, int max_cols) {
-    return ws_w_off(static_cast<size_t>(M < 1 ? 1 : M), max_cols) + kGemmScratch;
+    return ws_w_off(static_cast<size_t>(M < 1 ? 1 : M), max_cols) + gemm_scratch(max_cols);
 }
 size_t rwkvq_gemm_workspace_bytes(int M) { return rwkvq_gemm_workspace_bytes_for(M, 16384); }
 
@@ -832,7 +840,6 @@ static int gemm_check(const rwkvq_qtensor* t, const char* who, int M, int64_t ld
     if (rc) return rc;
     RWKVQ_REQUIRE(t->kind == RWKVQ_KIND_SB6 || t->kind == RWKVQ_KIND_SYM, RWKVQ_E_DTYPE,
                   "%s: only sb6 and sym tensors have a tensor-core path (kind %d)", who, t->kind);
-    RWKVQ_REQUIRE(t->cols <= 32768, RWKVQ_E_LIMIT, "%s: %d columns, at most 32768", who, t->cols);
     RWKVQ_REQUIRE(M >= 1 && ldy >= t->rows, RWKVQ_E_SHAPE, "%s: M=%d ldy=%lld", who, M, (long long)ldy);
     RWKVQ_REQUIRE(epilogue >= RWKVQ_EPI_NONE && epilogue <= RWKVQ_EPI_ADD, RWKVQ_E_DTYPE, "%s: epilogue %d", who, epilogue);
     RWKVQ_REQUIRE(epilogue != RWKVQ_EPI_ADD || resid, RWKVQ_E_NULL, "%s: resid is null", who);

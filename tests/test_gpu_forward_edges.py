@@ -65,3 +65,14 @@ def test_block_scales_on_an_8_byte_boundary(cuda_lib, bits, N):
     dq.struct = ops._descr(dq.bufs, dq.meta)
     got = ops.gemv_batch(dq, x, check=True)
     assert relmax(got.cpu().numpy(), want.cpu().numpy()) <= 4e-6       # another kernel from 17 rows on
+
+
+@pytest.mark.parametrize("layout,bits,cols", [("sb6", 4, 33024), ("sym", 8, 33024), ("sb6", 5, 131328)])
+def test_many_rows_through_a_wide_tensor(cuda_lib, layout, bits, cols):
+    """More columns than a chunk of 256 converted rows leaves room for, and more than the norm table of the channel mix."""
+    from rwkv_quant_b200.backends.cuda import ops
+    qt = _synth_linear(layout, bits, 300, cols, seed=bits)
+    x = _x(130, cols, bits)
+    y = ops.gemm(ops.DeviceQT(qt), x, check=True)
+    want = x.cpu().numpy().astype(np.float64) @ _oracle_w(qt).astype(np.float64).T
+    assert relmax(y.cpu().numpy(), want) <= 1e-3
