@@ -755,11 +755,11 @@ extern "C" int rwkvq_gemv_batch(const rwkvq_qtensor* t, const float* x, int N, i
     RWKVQ_REQUIRE(x && y, RWKVQ_E_NULL, "rwkvq_gemv_batch: x or y is null");
     // default: the two-term mma.sync kernel below kSbLeastRows rows, the tcgen05 pipeline from there on (gemm_sb_pays);
     // single-term operands: mma.sync up to 32 rows, the single-buffer tcgen05 kernel above
-    const bool tcb_ok = tcb_enabled() && gemm_tcb_ok(*t) && t->cols <= kPairCols;
+    const bool tcb_ok = tcb_enabled() && gemm_tcb_ok(*t);
     // tensors without the relayouted streams: the tcgen05 kernel that reads the file buffers, in either precision
     const bool bare = mma_layout_of(*t) < 0;
     const bool tcb = tcb_ok && ldx % 8 == 0 && (bare || (batch_fast() && (N > 32 || tcb_forced())));
-    const bool sb = tcb_ok && !batch_fast() && gemm_sb_ok(*t) && (gemm_sb_pays(*t, N) || tcb_forced());
+    const bool sb = tcb_ok && t->cols <= kPairCols && !batch_fast() && gemm_sb_ok(*t) && (gemm_sb_pays(*t, N) || tcb_forced());
     RWKVQ_REQUIRE(tcb || sb || mma_layout_of(*t) >= 0, RWKVQ_E_DTYPE,
                   "rwkvq_gemv_batch: needs an sb6 tensor, a sym tensor or per-row int8 with columns in multiples of 128");
     RWKVQ_REQUIRE(aligned(x, 16) && ldx % 4 == 0, RWKVQ_E_ALIGN, "rwkvq_gemv_batch: x rows must be 16-byte aligned");

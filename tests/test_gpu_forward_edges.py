@@ -76,3 +76,16 @@ def test_many_rows_through_a_wide_tensor(cuda_lib, layout, bits, cols):
     y = ops.gemm(ops.DeviceQT(qt), x, check=True)
     want = x.cpu().numpy().astype(np.float64) @ _oracle_w(qt).astype(np.float64).T
     assert relmax(y.cpu().numpy(), want) <= 1e-3
+
+
+@pytest.mark.parametrize("layout,bits", [("sb6", 4), ("sb6", 6), ("sym", 6)])
+@pytest.mark.parametrize("N", [3, 20, 70])
+def test_wide_tensor_without_relayouted_streams(cuda_lib, layout, bits, N):
+    """More columns than the pipeline's operand scratch holds: the kernel that reads the file buffers serves them."""
+    from rwkv_quant_b200.backends.cuda import ops
+    qt = _synth_linear(layout, bits, 160, 16640, seed=bits + N)
+    x = _x(N, 16640, N)
+    want = x.cpu().numpy().astype(np.float64) @ _oracle_w(qt).astype(np.float64).T
+    for relayout in (False, True):
+        y = ops.gemv_batch(ops.DeviceQT(qt, relayout=relayout), x, check=True)
+        assert relmax(y.cpu().numpy(), want) <= 2e-5, relayout
