@@ -342,7 +342,8 @@ int rwkvq_seq_ln_shift_mix(const float* x, const float* ln_w, const float* ln_b,
  * per mix by modes[m] (host array; bit 0: scaled fp16 copy + scale for rwkvq_gemm_x16 into
  * out_x16[m] [N, D + 64] / out_scale[m] [N]; bit 1: fp16 hi/lo split as rwkvq_split_fp16 into
  * out_split[m] [N, 2 D]; bit 2: fp32 row into out_f32[m] [N, D]).  Pointer tables are host arrays
- * of n_mix device pointers (entries of unselected forms are ignored).  D even. */
+ * of n_mix device pointers (entries of unselected forms are ignored).  D even.  shift_out may be
+ * shift_in where T = 1. */
 int rwkvq_seq_ln_shift_mix_prep(const float* x, const float* ln_w, const float* ln_b, const float* shift_in,
                                 const float* mix, int n_mix, const int* modes, void* const* out_x16,
                                 float* const* out_scale, void* const* out_split, float* const* out_f32,

@@ -536,10 +536,11 @@ int launch_seq_prep(const SeqPrepArgs& a, long long n_tokens, cudaStream_t s) {
     bool pair = a.mix == nullptr;
     for (int m = 0; m < a.n_mix; ++m) pair = pair || (a.mode[m] & kPrepPair) != 0;
     const bool in_place = a.shift_out != nullptr && a.shift_in == a.shift_out;
-    RWKVQ_REQUIRE(vec || !(pair || in_place), RWKVQ_E_ALIGN, "seq_ln_shift_mix_prep: D %d, rows on 16-byte boundaries", a.D);
+    RWKVQ_REQUIRE(vec || !pair, RWKVQ_E_ALIGN, "seq_ln_shift_mix_prep: D %d, rows on 16-byte boundaries", a.D);
     RWKVQ_REQUIRE(aligned(a.x, 8) && aligned(a.ln_w, 8) && aligned(a.ln_b, 8) && aligned(a.mix, 8) && aligned(a.shift_in, 8) && aligned(a.shift_out, 8),
                   RWKVQ_E_ALIGN, "seq_ln_shift_mix_prep: 8-byte aligned rows required");       // the scalar form reads pairs
     RWKVQ_REQUIRE(!in_place || a.T == 1, RWKVQ_E_SHAPE, "seq_ln_shift_mix_prep: the shift state in place needs T = 1");
+    // (in place: the scalar form has a token's mixes in one CTA, the vector form in one cluster)
     // up to one wave of CTAs (two per SM) with a token and mix each, then groups of 64 threads per token
     const bool few = n_tokens * a.n_mix <= 2 * 148 || pair || in_place;
     if (vec && !few && a.D == 2048) e = launch_prep_group<4>(a, n_tokens, s);

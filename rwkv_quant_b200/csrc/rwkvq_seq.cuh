@@ -26,7 +26,7 @@ struct SeqPrepArgs {
     float *zero_a, *zero_b;    // optional [N]: cleared
 };
 // mix == NULL: no shift and no lerp, the normalised row itself (n_mix = 1; shift_in, shift_out NULL).  shift_out may equal
-// shift_in where T = 1 and D is a multiple of 256 (seq_prep_in_place_ok).  kPrepPair needs D % 256 == 0.
+// shift_in where T = 1 (kPrepPair: seq_prep_in_place_ok).  kPrepPair needs D % 256 == 0.
 int launch_seq_prep(const SeqPrepArgs& a, long long n_tokens, cudaStream_t s);
 inline bool seq_prep_in_place_ok(int D) { return D % 256 == 0 && D <= 4096; }
 

@@ -89,3 +89,23 @@ def test_wide_tensor_without_relayouted_streams(cuda_lib, layout, bits, N):
     for relayout in (False, True):
         y = ops.gemv_batch(ops.DeviceQT(qt, relayout=relayout), x, check=True)
         assert relmax(y.cpu().numpy(), want) <= 2e-5, relayout
+
+
+@pytest.mark.parametrize("D", [256, 384, 2048])
+def test_shift_state_updated_in_place(cuda_lib, D):
+    """One token a sequence: the row preparation may write the shift state over its input, whatever the width."""
+    import ctypes as C
+    from rwkv_quant_b200 import _lib
+    B, gen = 70, torch.Generator(device="cuda").manual_seed(D)
+    draw = lambda *s: torch.randn(s, generator=gen, device="cuda")
+    x, w, b, mix, shift = draw(B, D), draw(D), draw(D), draw(6, D), draw(B, D)
+    xn = torch.nn.functional.layer_norm(x.double(), (D,), w.double(), b.double())
+    want = torch.stack([xn + (shift.double() - xn) * m.double() for m in mix])
+    out = torch.empty(6, B, D, device="cuda")
+    tab = (C.c_void_p * 6)(*[out[m].data_ptr() for m in range(6)])
+    none = (C.c_void_p * 6)()
+    _lib.check(cuda_lib.rwkvq_seq_ln_shift_mix_prep(x.data_ptr(), w.data_ptr(), b.data_ptr(), shift.data_ptr(), mix.data_ptr(), 6,
+                                                    (C.c_int * 6)(*[4] * 6), none, none, none, tab, shift.data_ptr(), B, 1, D,
+                                                    _lib.stream_ptr()), "prep")
+    assert relmax(out.cpu().numpy(), want.cpu().numpy()) <= 1e-5
+    assert relmax(shift.cpu().numpy(), xn.cpu().numpy()) <= 1e-5
