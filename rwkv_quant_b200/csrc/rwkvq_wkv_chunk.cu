@@ -44,19 +44,7 @@ struct PreSmem {
     float red[2][2 * kC];
 };
 
-// 1 / x and 1 / sqrt(x) for normal x: the hardware estimate and one Newton step (within one unit of the last
-// place, a sixth of the instructions of the rounded division: half of this kernel's issue slots were divisions)
-__device__ __forceinline__ float newton_rcp(float x) {
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return fmaf(r, fmaf(-x, r, 1.0f), r);
-}
-__device__ __forceinline__ float newton_rsqrt(float x) {
-    float r;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return fmaf(0.5f * r, fmaf(-x * r, r, 1.0f), r);
-}
-__device__ __forceinline__ float fast_sigmoid(float x) { return newton_rcp(1.0f + expf(fminf(-x, 80.0f))); }
+__device__ __forceinline__ float gate_sigmoid(float x) { return __frcp_rn(1.0f + expf(-x)); }      // a NaN stays one, +-inf give 1 and 0
 
 __global__ void __launch_bounds__(64 * kPreUnits, 3) wkv_operands_kernel(const WkvChunkArgs p, int n_chunks) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -114,9 +102,9 @@ __global__ void __launch_bounds__(64 * kPreUnits, 3) wkv_operands_kernel(const W
     float q[2 * kC];                                   // sums over the head: |k k_k|^2 and r k' r_k of every step
 #pragma unroll
     for (int t = 0; t < kC; ++t) {
-        yw[t] = t < n ? expf(-0.606531f * fast_sigmoid(yw[t] + w0)) : 1.f;        // the decay
-        ya[t] = fast_sigmoid(ya[t] + a0);                                        // the gate
-        if (p.yv) v[t] = t < n ? v[t] + (vf[t] - v[t]) * fast_sigmoid(yv[t] + v0) : 0.f;
+        yw[t] = t < n ? expf(-0.606531f * gate_sigmoid(yw[t] + w0)) : 1.f;        // the decay
+        ya[t] = gate_sigmoid(ya[t] + a0);                                        // the gate
+        if (p.yv) v[t] = t < n ? v[t] + (vf[t] - v[t]) * gate_sigmoid(yv[t] + v0) : 0.f;
         vf[t] = k[t] * kkw;                                                    // un-normalised removal key
         k[t] = k[t] * (1.0f + (ya[t] - 1.0f) * kaw);
         q[t] = vf[t] * vf[t];
@@ -143,13 +131,15 @@ __global__ void __launch_bounds__(64 * kPreUnits, 3) wkv_operands_kernel(const W
     if (lane < 16) s.red[wp][(lane & 1) * 8 + (lane & 2) * 2 + ((lane & 4) >> 1) + ((lane & 8) >> 3)] = q[0];
     sync();
     float P = 1.f, at_[kC];
+    // 1 / |k k_k| of the 8 steps, a step per lane: the rounded root is some 15 instructions
+    const float inv_mine = __frsqrt_rn(s.red[0][lane & (kC - 1)] + s.red[1][lane & (kC - 1)] + 1e-12f);
 #pragma unroll
     for (int t = 0; t < kC; ++t) {
-        const float inv = newton_rsqrt(s.red[0][t] + s.red[1][t] + 1e-12f);
+        const float inv = __shfl_sync(0xFFFFFFFFu, inv_mine, t);
         const float kk = vf[t] * inv, a = -kk, bb = kk * ya[t];
         at_[t] = P * a;                                                        // P_{t-1} a_t
         P *= yw[t];
-        const float ip = newton_rcp(P);
+        const float ip = __frcp_rn(P);
         s.a[t][d] = at_[t];
         r[t] *= P;
         s.r[t][d] = r[t];

@@ -109,3 +109,24 @@ def test_shift_state_updated_in_place(cuda_lib, D):
                                                     _lib.stream_ptr()), "prep")
     assert relmax(out.cpu().numpy(), want.cpu().numpy()) <= 1e-5
     assert relmax(shift.cpu().numpy(), xn.cpu().numpy()) <= 1e-5
+
+
+@pytest.mark.parametrize("name", ["w0", "a0", "v0"])
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), -float("inf")])
+@pytest.mark.parametrize("T", [15, 17])
+def test_a_non_finite_gate_input_reaches_the_outputs(cuda_lib, name, value, T):
+    """Both time-mix forms of calls of more than 64 rows (T on each side of the shortest chunked one) against the
+    per-operator path: a NaN in front of a sigmoid stays a NaN, an infinity saturates it."""
+    model = _model()
+    getattr(model.blocks[1], name)[70] = value
+    idx, st = _idx(5, T), _states(model, 5)
+    got, gst = model.forward_stateful(idx, st)
+    model.fused_prep = False
+    ref, rst = model.forward_stateful(idx, st)
+    for a, b in [(got, ref)] + [(x, y) for s, r in zip(gst, rst) for x, y in zip(s, r)]:
+        assert torch.equal(a.isnan(), b.isnan())
+        assert torch.equal(a.isnan(), torch.zeros_like(a.isnan())) or value != value
+        ok = ~a.isnan()
+        if ok.any():
+            assert relmax(a[ok].cpu().numpy(), b[ok].cpu().numpy()) <= 1e-3
+    assert value == value or got.isnan().any()
