@@ -393,10 +393,12 @@ __global__ void __launch_bounds__(ScanGeo<R, SPLIT>::THREADS) wkv_scan_kernel(co
         for (int j = 0; j < kC; ++j) {
             float v[R];
             rows_of(blk + kOffV + j * kS + dv0, v);
+            if (j <= my_t) {                                        // not only zero factors: a NaN of a later step stays there
 #pragma unroll
-            for (int i = 0; i < R; ++i) {
-                uy[2 * i] = fmaf(nv[j], v[i], uy[2 * i]);
-                uy[2 * i + 1] = fmaf(gv[j], v[i], uy[2 * i + 1]);
+                for (int i = 0; i < R; ++i) {
+                    uy[2 * i] = fmaf(nv[j], v[i], uy[2 * i]);
+                    uy[2 * i + 1] = fmaf(gv[j], v[i], uy[2 * i + 1]);
+                }
             }
         }
 #pragma unroll

@@ -130,3 +130,19 @@ def test_a_non_finite_gate_input_reaches_the_outputs(cuda_lib, name, value, T):
         if ok.any():
             assert relmax(a[ok].cpu().numpy(), b[ok].cpu().numpy()) <= 1e-3
     assert value == value or got.isnan().any()
+
+
+@pytest.mark.parametrize("B,t", [(3, 0), (3, 3), (3, 7), (3, 8), (3, 21), (30, 5), (40, 5)])      # one form of the scan each
+def test_a_nan_token_leaves_earlier_positions_alone(cuda_lib, B, t):
+    from rwkv_quant_b200.backends.cuda.ops import _BUF_ORDER
+    model = _model()
+    idx, st = _idx(B, 24), _states(model, B)
+    idx[idx == 500] = 501
+    idx[1, t] = 500
+    clean, _ = model.forward_stateful(idx, st)
+    model.emb.bufs[_BUF_ORDER.index("dm")][500] = float("nan")
+    got, _ = model.forward_stateful(idx, st)
+    assert got[1, t:].isnan().all()
+    assert torch.equal(got[1, :t], clean[1, :t])
+    others = [b for b in range(B) if b != 1]
+    assert torch.equal(got[others], clean[others])
