@@ -330,11 +330,13 @@ class QuantRWKV7:
         return rows.half().float()[inv].reshape(*idx.shape, self.n_embd)
 
     def _one_call_ok(self, n_rows: int) -> bool:
-        """Whether ``rwkvq_forward_seq`` serves calls of this many rows (layouts, shapes); the answer
-        depends on the regime only."""
-        if self._model_c is None or not self.fused_prep:
+        """Whether ``rwkvq_forward_seq`` serves calls of this many rows: layouts and shapes, whose answer
+        depends on the regime only, and a choice of kernels by row count that is the library's own."""
+        if self._model_c is None or not self.fused_prep or n_rows < 2:
             return False
-        small = n_rows <= self.batch_max
+        small = n_rows <= 64
+        if (n_rows <= self.gemv_max_batch) != (n_rows <= 2) or (n_rows <= self.batch_max) != small:
+            return False
         if small not in self._seq_ok:
             self._seq_ok[small] = bool(_lib.load().rwkvq_forward_seq_ok(C.byref(self._model_c), n_rows))
         return self._seq_ok[small]
