@@ -396,7 +396,7 @@ class QuantRWKV7:
             logits = self._decode(idx.reshape(B).contiguous(), st)
             return logits.reshape(B, 1, self.vocab_size), st
         if self._one_call_ok(B * T):
-            tail = 1 if last_only else tail_only if tail_only and T > tail_only else T
+            tail = 1 if last_only else len(range(T)[-tail_only:]) if tail_only and T > tail_only else T
             _, logits, new_states = self._forward_one_call(idx, states, tail, False)
             return logits, new_states
         x, new_states = self.forward_hidden(idx, states)

@@ -146,3 +146,13 @@ def test_a_nan_token_leaves_earlier_positions_alone(cuda_lib, B, t):
     assert torch.equal(got[1, :t], clean[1, :t])
     others = [b for b in range(B) if b != 1]
     assert torch.equal(got[others], clean[others])
+
+
+@pytest.mark.parametrize("tail", [1, 3, 5, 9, -2])
+def test_tail_only_selects_as_a_slice_does(cuda_lib, tail):
+    model = _model()
+    idx, st = _idx(2, 5), _states(model, 2)
+    full, _ = model.forward_stateful(idx, st)
+    got, _ = model.forward_stateful(idx, st, tail_only=tail)
+    want = full[:, -tail:] if 5 > tail else full
+    assert got.shape == want.shape and relmax(got.cpu().numpy(), want.cpu().numpy()) <= 1e-5
