@@ -370,7 +370,8 @@ class QuantRWKV7:
     def forward_hidden(self, idx, states):
         idx = torch.as_tensor(idx, device=self.device).long()
         B, T = idx.shape
-        if B * T > 1 and self._one_call_ok(B * T):
+        states = list(states)
+        if len(states) == self.n_layer and self._one_call_ok(B * T):
             hidden, _, new_states = self._forward_one_call(idx, states, 0, True)
             return hidden, new_states
         states = self._materialize(states, B)
@@ -395,7 +396,8 @@ class QuantRWKV7:
             st = self._materialize(states, B)
             logits = self._decode(idx.reshape(B).contiguous(), st)
             return logits.reshape(B, 1, self.vocab_size), st
-        if self._one_call_ok(B * T):
+        states = list(states)
+        if len(states) == self.n_layer and self._one_call_ok(B * T):
             tail = 1 if last_only else len(range(T)[-tail_only:]) if tail_only and T > tail_only else T
             _, logits, new_states = self._forward_one_call(idx, states, tail, False)
             return logits, new_states

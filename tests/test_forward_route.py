@@ -37,3 +37,20 @@ def test_row_limits_of_the_model_are_kept(monkeypatch, kw, served, refused):
     m = _model(monkeypatch, **kw)
     assert [n for n in served if not m._one_call_ok(n)] == []
     assert [n for n in refused if m._one_call_ok(n)] == []
+
+
+@pytest.mark.parametrize("n,given", [(2, iter), (3, list), (1, list)])
+def test_states_of_another_count_take_the_layers_they_name(monkeypatch, n, given):
+    """Any iterable, one entry a layer; with another count the layers and the states are paired up as far as both go."""
+    import torch
+    calls = []
+    m = _model(monkeypatch, n_layer=2, blocks=["a", "b"], device=torch.device("cpu"), n_embd=8192, vocab_size=5, head="h")
+    m._forward_one_call = lambda idx, states, tail, hidden: calls.append(("one", len(states))) or (None, 0, 0)
+    m._materialize = lambda states, B: list(states)
+    m._embed = lambda idx: torch.zeros(*idx.shape, 8192)
+    m.ln0 = m.ln_out = (torch.ones(8192), torch.zeros(8192))
+    m.emb = type("E", (), {"outliers": None})
+    m._block_seq = lambda i, L, x, v, st: calls.append((L, st)) or (x, v, st)
+    m._linear = lambda dq, x: torch.zeros(x.shape[0], 5)
+    m.forward_stateful(torch.zeros(1, 5, dtype=torch.long), given(["s0", "s1", "s2"][:n]))
+    assert calls == ([("one", 2)] if n == 2 else [("a", "s0"), ("b", "s1")][:n])
