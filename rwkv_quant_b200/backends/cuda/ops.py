@@ -12,6 +12,7 @@ import os
 from typing import List, Optional, Sequence
 
 import torch
+from torch.autograd import forward_ad
 
 from ... import _lib
 from ..._lib import QTensorStruct
@@ -246,12 +247,18 @@ def _(bufs, meta, x, epilogue, resid):
     return torch.empty((x.shape[0], meta[2]), dtype=torch.float32, device=x.device)
 
 
+_n_modes, _transforms, _trace = torch._C._len_torch_dispatch_stack, torch._C._functorch.peek_interpreter_stack, torch._C._get_tracing_state
+
+
 def gemv_direct(dq: "DeviceQT", x: torch.Tensor, epilogue: int = 0, resid: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``gemv`` on the tensor's own descriptor, past the operator dispatcher (40 us of the 50 us a
-    single-row call took); a graph being traced gets the registered operator."""
-    if torch.compiler.is_compiling():
+    single-row call took) where nothing hangs on that: a tensor subclass, autograd (no gradient is defined: the
+    registered operator says so, a plain call would drop the graph), a tracer, a dispatch mode or a transform."""
+    if (torch.compiler.is_compiling() or type(x) is not torch.Tensor or x.requires_grad or (resid is not None and resid.requires_grad)
+            or _n_modes() or _trace() is not None or _transforms() is not None or forward_ad._current_level >= 0):
         return gemv(dq.bufs, dq.meta, x, epilogue, resid)
-    _require_cuda(dq.bufs[0], x, resid)
+    if resid is not None or not (x.is_cuda and dq.bufs[0].is_cuda):
+        _require_cuda(dq.bufs[0], x, resid)
     n = x.shape[0]
     y = torch.empty((n, dq.rows), dtype=torch.float32, device=x.device)
     _lib.check(_lib.load().rwkvq_gemv(dq.struct_ref, x.data_ptr(), _lib.DTYPE_CODE[x.dtype], n, x.stride(0), y.data_ptr(),

@@ -156,3 +156,33 @@ def test_tail_only_selects_as_a_slice_does(cuda_lib, tail):
     got, _ = model.forward_stateful(idx, st, tail_only=tail)
     want = full[:, -tail:] if 5 > tail else full
     assert got.shape == want.shape and relmax(got.cpu().numpy(), want.cpu().numpy()) <= 1e-5
+
+
+@pytest.mark.parametrize("rows", [1, 2])
+def test_an_operator_call_that_autograd_or_a_tracer_sees_is_not_bypassed(cuda_lib, rows):
+    from torch.fx.experimental.proxy_tensor import make_fx
+    from rwkv_quant_b200.backends.cuda import linear_for
+    op = linear_for(_synth_linear("sb6", 4, 128, 256, seed=1))
+    x = _x(rows, 256, 1)
+    want = op(x)
+    y = op(x.clone().requires_grad_())
+    assert y.requires_grad and torch.equal(y.detach(), want)
+    with pytest.raises(RuntimeError):                    # no gradient is defined: not a silent zero
+        y.sum().backward()
+    with torch.no_grad():
+        assert not op(x.clone().requires_grad_()).requires_grad
+    g = make_fx(lambda t: op(t))(x)
+    assert any("rwkvq.gemv" in str(n.target) for n in g.graph.nodes)
+    assert torch.equal(g(x), want)
+    other = _x(rows, 256, 2)
+    assert torch.equal(g(other), op(other))
+    with pytest.raises(Exception):
+        torch.func.jvp(op, (x,), (x,))
+
+
+@pytest.mark.parametrize("rows", [1, 3, 200])
+def test_cuda_rows_on_host_weights_are_refused(cuda_lib, rows):
+    from rwkv_quant_b200.backends.cuda import linear_for
+    op = linear_for(_synth_linear("sb6", 4, 128, 256, seed=1), "cpu")
+    with pytest.raises(RuntimeError, match="CUDA tensors only"):
+        op(_x(rows, 256, 1))
