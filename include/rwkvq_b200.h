@@ -201,12 +201,14 @@ int rwkvq_quantize_sym6_packed(const float* w, int64_t ldw, int rows, int cols, 
  * With RWKVQ_BATCH_FAST=1 in the environment (read once per process) single fp16 operands are used
  * instead (weights fp16(q*s+m)): results within ~3e-4 of max|y| per call (the precision of rwkvq_gemm),
  * and sb6 / sym tensors with more than 32 rows run on a single-term tcgen05 form.
- *   workspace: rwkvq_gemv_batch_workspace_bytes(N) bytes, 16-byte aligned: a status word (first
+ *   workspace: rwkvq_gemv_batch_workspace_bytes_of(t, N) bytes (rwkvq_gemv_batch_workspace_bytes(N): whatever
+ *   the tensor), 16-byte aligned: a status word (first
  *   int32: RWKVQ_E_TIMEOUT if a bounded wait on the tensor-core pipeline ran out; read it after
  *   synchronising the stream, 0 = ok), one float per row (max|x|, or the inverse scale of the pairs) and
  *   the rows as fp16 pairs, which a one-block-per-row pre-pass writes before the product kernel starts.
  */
 size_t rwkvq_gemv_batch_workspace_bytes(int N);
+size_t rwkvq_gemv_batch_workspace_bytes_of(const rwkvq_qtensor* t, int N);
 int rwkvq_gemv_batch(const rwkvq_qtensor* t, const float* x, int N, int64_t ldx, float* y, int64_t ldy,
                      int epilogue, const float* resid, void* workspace, size_t workspace_bytes, void* stream);
 
@@ -219,20 +221,21 @@ int rwkvq_gemv_batch(const rwkvq_qtensor* t, const float* x, int N, int64_t ldx,
  * and read back by TMA.  Operands are fp16 (weights: fp16(q*s+m); tokens:
  * scaled per row by a power of two), accumulation fp32 in tensor memory.
  *   x [M, ldx] fp32, y [M, ldy] fp32, sb6 / sym tensors only.
- *   workspace: rwkvq_gemm_workspace_bytes_for(M, IN) bytes, 256-byte aligned (or
- *   rwkvq_gemm_workspace_bytes(M), which covers IN <= 16384); it holds the fp16 copy of x and of a
- *   chunk of the weights.  Its first int32 is a status word the
+ *   workspace: rwkvq_gemm_workspace_bytes_of(t, M, 1) bytes, 256-byte aligned (whatever the rows of the
+ *   tensor: rwkvq_gemm_workspace_bytes_for(M, IN), or rwkvq_gemm_workspace_bytes(M) for IN <= 16384); it
+ *   holds the fp16 copy of x and of the weights, a chunk of at most 64 MB of them.  Its first int32 is a status word the
  *   kernel sets to RWKVQ_E_TIMEOUT if a bounded wait on the tensor-core pipeline ran out
  *   (read it after synchronising the stream; 0 = ok).
  */
 size_t rwkvq_gemm_workspace_bytes(int M);
 size_t rwkvq_gemm_workspace_bytes_for(int M, int max_cols);
+size_t rwkvq_gemm_workspace_bytes_of(const rwkvq_qtensor* t, int M, int with_rows);   /* with_rows = 0: rwkvq_gemm_x16 */
 int rwkvq_gemm(const rwkvq_qtensor* t, const float* x, int M, int64_t ldx, float* y, int64_t ldy,
                int epilogue, const float* resid, void* workspace, size_t workspace_bytes, void* stream);
 /* The same product on activations the caller has already brought into the form the kernel reads
  * (rwkvq_seq_ln_shift_mix_prep writes it): x16 fp16 [M, rwkvq_gemm_x16_pitch(IN)] = x * row_scale[m],
- * row_scale [M] fp32 powers of two.  The workspace (rwkvq_gemm_workspace_bytes_for(M, 0)) then only
- * carries the status word and the weights. */
+ * row_scale [M] fp32 powers of two.  The workspace (rwkvq_gemm_workspace_bytes_of(t, M, 0), or
+ * rwkvq_gemm_workspace_bytes_for(M, 0)) then only carries the status word and the weights. */
 size_t rwkvq_gemm_x16_pitch(int cols);
 int rwkvq_gemm_x16(const rwkvq_qtensor* t, const void* x16, const float* row_scale, int M, float* y, int64_t ldy,
                    int epilogue, const float* resid, void* workspace, size_t workspace_bytes, void* stream);

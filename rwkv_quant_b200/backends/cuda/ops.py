@@ -314,7 +314,7 @@ def gemv_batch(dq: "DeviceQT", x: torch.Tensor, epilogue: int = 0, resid: Option
         x = x.contiguous()
     n = x.shape[0]
     y = torch.empty((n, dq.rows), dtype=torch.float32, device=x.device)
-    nws = lib.rwkvq_gemv_batch_workspace_bytes(n)
+    nws = lib.rwkvq_gemv_batch_workspace_bytes_of(dq.struct_ref, n)
     ws = torch.empty(nws, dtype=torch.uint8, device=x.device)
     _lib.check(lib.rwkvq_gemv_batch(dq.struct_ref, x.data_ptr(), n, x.stride(0), y.data_ptr(), y.stride(0),
                                     epilogue, _lib.ptr(resid), ws.data_ptr(), nws, _lib.stream_ptr()), "rwkvq_gemv_batch")
@@ -358,7 +358,7 @@ def gemm(dq: "DeviceQT", x: torch.Tensor, epilogue: int = 0, resid: Optional[tor
     lib = _lib.load()
     x = x.float().contiguous()
     m = x.shape[0]
-    nws = lib.rwkvq_gemm_workspace_bytes_for(m, dq.cols)
+    nws = lib.rwkvq_gemm_workspace_bytes_of(dq.struct_ref, m, 1)
     ws = torch.empty(nws, dtype=torch.uint8, device=x.device)
     y = torch.empty((m, dq.rows), dtype=torch.float32, device=x.device)
     _lib.check(lib.rwkvq_gemm(dq.struct_ref, x.data_ptr(), m, x.stride(0), y.data_ptr(), y.stride(0),
@@ -387,7 +387,7 @@ def gemm_x16(dq: "DeviceQT", rows: PreparedRows, epilogue: int = 0, resid: Optio
     _require_cuda(dq.bufs[0], rows.x16, resid)
     lib = _lib.load()
     m = rows.n
-    nws = lib.rwkvq_gemm_workspace_bytes_for(m, 0)
+    nws = lib.rwkvq_gemm_workspace_bytes_of(dq.struct_ref, m, 0)
     ws = torch.empty(nws, dtype=torch.uint8, device=rows.x16.device)
     y = torch.empty((m, dq.rows), dtype=torch.float32, device=rows.x16.device)
     _lib.check(lib.rwkvq_gemm_x16(dq.struct_ref, rows.x16.data_ptr(), rows.scale.data_ptr(), m, y.data_ptr(),

@@ -19,6 +19,7 @@
 // rwkvq_seq.cu, rows as fp16 pairs).
 #include <stdlib.h>
 
+#include <algorithm>
 #include <map>
 #include <mutex>
 #include <utility>
@@ -867,6 +868,11 @@ bool sb_rows_ok(const rwkvq_model& m, float* const* tshift, float* const* cshift
     return ok;
 }
 
+// linears of a step that go to rwkvq_gemm: more streams than the small-batch kernels take, or a tensor without their layout
+bool linear_on_gemm(const rwkvq_qtensor& t, int B) {
+    return B > 2 && (t.kind == RWKVQ_KIND_SB6 || t.kind == RWKVQ_KIND_SYM) && !(batch_path(B) && mma_layout_of(t) >= 0);
+}
+
 struct Workspace {
     float *x, *xs, *rkv, *part, *yl, *og, *xk, *hffn, *xo, *v_first, *logits, *argv, *gemm_ws;
     int* status;             // first word of the workspace: RWKVQ_E_TIMEOUT if a bounded device-side wait of a step ran out
@@ -908,7 +914,14 @@ Workspace carve(const rwkvq_model& m, int B, void* base) {
         w.d_pair = pair(D);
         w.f_pair = pair(F);
     }
-    w.gemm_ws = take(rwkvq_gemm_workspace_bytes_for(B, static_cast<int>(F > D ? F : D)) / sizeof(float) + 1);
+    size_t gemm_bytes = 0;                  // only for the linears that reach rwkvq_gemm
+    auto with_gemm = [&](const rwkvq_qtensor& t) {
+        if (linear_on_gemm(t, B)) gemm_bytes = std::max(gemm_bytes, rwkvq_gemm_workspace_bytes_of(&t, B, 1));
+    };
+    for (int l = 0; l < m.n_layer && m.layers; ++l)
+        for (const rwkvq_qtensor* t : {&m.layers[l].Wr, &m.layers[l].Wk, &m.layers[l].Wv, &m.layers[l].Wo, &m.layers[l].Wfk, &m.layers[l].Wfv}) with_gemm(*t);
+    with_gemm(m.head);
+    w.gemm_ws = take((gemm_bytes + sizeof(float) - 1) / sizeof(float));
     w.bytes = off;
     return w;
 }
@@ -941,8 +954,8 @@ int linear(const rwkvq_qtensor* t, const float* x, int B, int in, float* y, int 
             return launch_gemm_tcb(t, 1, xs, x16 != nullptr, sc, B, in, ys, out, epi, rs, ao, status, static_cast<cudaStream_t>(stream));
         return launch_gemv_batch(t, 1, xs, x16 != nullptr, sc, B, in, ys, out, epi, rs, ao, static_cast<cudaStream_t>(stream));
     }
-    if (B > 2 && (t->kind == RWKVQ_KIND_SB6 || t->kind == RWKVQ_KIND_SYM))     // tcgen05 path for large batches
-        return rwkvq_gemm(t, x, B, in, y, out, epi, resid, gemm_ws, rwkvq_gemm_workspace_bytes_for(B, in), stream);
+    if (linear_on_gemm(*t, B))                              // tcgen05 path for large batches
+        return rwkvq_gemm(t, x, B, in, y, out, epi, resid, gemm_ws, rwkvq_gemm_workspace_bytes_of(t, B, 1), stream);
     return rwkvq_gemv(t, x, RWKVQ_F32, B, in, y, out, epi, resid, stream);
 }
 

@@ -78,8 +78,8 @@ ForwardWs carve(const rwkvq_model& m, int B, int T, size_t n_tail, void* base) {
     }
     if (n_tail > 0) {
         w.tailx = f32(n_tail * D); w.taily = f32(n_tail * D);
-        w.head_ws_bytes = std::max(rwkvq_gemv_batch_workspace_bytes(static_cast<int>(n_tail)),
-                                   n_tail > kSmallRows ? rwkvq_gemm_workspace_bytes_for(static_cast<int>(n_tail), static_cast<int>(D)) : 0);
+        w.head_ws_bytes = n_tail <= 2 ? 0 : n_tail <= kSmallRows ? rwkvq_gemv_batch_workspace_bytes_of(&m.head, static_cast<int>(n_tail))
+                                                                : rwkvq_gemm_workspace_bytes_of(&m.head, static_cast<int>(n_tail), 1);
         w.head_ws = take(w.head_ws_bytes);
     }
     w.bytes = off;

@@ -795,6 +795,7 @@ namespace {
 // Row pitch of the fp16 activation copy: 128 bytes more than the row, so that the rows of a TMA box do
 // not all map to the same L2 slice (a power-of-two pitch does).
 inline size_t x16_pitch(int cols) { return static_cast<size_t>(cols) + 64; }
+inline size_t up256(size_t n) { return (n + 255) / 256 * 256; }
 // Weights are converted in chunks of rows that fit this scratch, half of L2: it is read back at once.  Whole tiles of
 // 256 rows up to 131072 columns, at least one row beyond.
 constexpr size_t kGemmScratch = 64u << 20;
@@ -802,8 +803,10 @@ inline int gemm_chunk_rows(int cols) {
     const size_t n = kGemmScratch / sizeof(__half) / cols;
     return n >= 256 ? static_cast<int>(n / 256 * 256) : n > 0 ? static_cast<int>(n) : 1;
 }
-inline size_t gemm_scratch(int cols) { return std::max(kGemmScratch, sizeof(__half) * cols); }
-inline size_t up256(size_t n) { return (n + 255) / 256 * 256; }
+// converted weights of a tensor, a chunk of it where it is larger
+inline size_t gemm_scratch(int rows, int cols) {
+    return up256(sizeof(__half) * cols * static_cast<size_t>(std::min(rows, gemm_chunk_rows(cols))));
+}
 inline size_t ws_x16_off(size_t m) { return 256 + up256(sizeof(float) * m); }
 inline size_t ws_w_off(size_t m, int x_cols) { return ws_x16_off(m) + (x_cols > 0 ? up256(sizeof(__half) * m * x16_pitch(x_cols)) : 0); }
 
@@ -831,7 +834,11 @@ void rwkvq_profiling_gemm_acc_mode(int mode) { g_gemm_acc_mode = mode; }      //
 
 size_t rwkvq_gemm_x16_pitch(int cols) { return x16_pitch(cols); }
 size_t rwkvq_gemm_workspace_bytes_for(int M, int max_cols) {
-    return ws_w_off(static_cast<size_t>(M < 1 ? 1 : M), max_cols) + gemm_scratch(max_cols);
+    return ws_w_off(static_cast<size_t>(M < 1 ? 1 : M), max_cols) + std::max(kGemmScratch, sizeof(__half) * static_cast<size_t>(max_cols));
+}
+size_t rwkvq_gemm_workspace_bytes_of(const rwkvq_qtensor* t, int M, int with_rows) {
+    if (!t || M < 1 || t->rows < 1 || t->cols < 1) return 0;
+    return ws_w_off(M, with_rows ? t->cols : 0) + gemm_scratch(t->rows, t->cols);
 }
 size_t rwkvq_gemm_workspace_bytes(int M) { return rwkvq_gemm_workspace_bytes_for(M, 16384); }
 
@@ -854,8 +861,8 @@ int rwkvq_gemm(const rwkvq_qtensor* t, const float* x, int M, int64_t ldx, float
     RWKVQ_REQUIRE(ldx >= t->cols, RWKVQ_E_SHAPE, "rwkvq_gemm: ldx=%lld", (long long)ldx);
     RWKVQ_REQUIRE(aligned(x, 16) && ldx % 4 == 0 && aligned(workspace, 256), RWKVQ_E_ALIGN,
                   "rwkvq_gemm: x and its row stride must be 16-byte aligned, the workspace 256-byte aligned");
-    RWKVQ_REQUIRE(workspace_bytes >= rwkvq_gemm_workspace_bytes_for(M, t->cols), RWKVQ_E_LIMIT,
-                  "rwkvq_gemm: workspace %zu < %zu bytes", workspace_bytes, rwkvq_gemm_workspace_bytes_for(M, t->cols));
+    RWKVQ_REQUIRE(workspace_bytes >= rwkvq_gemm_workspace_bytes_of(t, M, 1), RWKVQ_E_LIMIT,
+                  "rwkvq_gemm: workspace %zu < %zu bytes", workspace_bytes, rwkvq_gemm_workspace_bytes_of(t, M, 1));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     char* ws = static_cast<char*>(workspace);
     int* status = reinterpret_cast<int*>(ws);
@@ -874,8 +881,8 @@ int rwkvq_gemm_x16(const rwkvq_qtensor* t, const void* x16, const float* row_sca
     if (rc) return rc;
     RWKVQ_REQUIRE(aligned(x16, 16) && aligned(workspace, 256), RWKVQ_E_ALIGN,
                   "rwkvq_gemm_x16: x16 must be 16-byte aligned, the workspace 256-byte aligned");
-    RWKVQ_REQUIRE(workspace_bytes >= rwkvq_gemm_workspace_bytes_for(M, 0), RWKVQ_E_LIMIT, "rwkvq_gemm_x16: workspace %zu < %zu bytes",
-                  workspace_bytes, rwkvq_gemm_workspace_bytes_for(M, 0));
+    RWKVQ_REQUIRE(workspace_bytes >= rwkvq_gemm_workspace_bytes_of(t, M, 0), RWKVQ_E_LIMIT, "rwkvq_gemm_x16: workspace %zu < %zu bytes",
+                  workspace_bytes, rwkvq_gemm_workspace_bytes_of(t, M, 0));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     char* ws = static_cast<char*>(workspace);
     int* status = reinterpret_cast<int*>(ws);

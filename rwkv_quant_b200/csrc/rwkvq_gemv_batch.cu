@@ -743,7 +743,17 @@ namespace {
 constexpr int kPairCols = 16384;
 inline size_t batch_ws_pairs(int N) { return 256 + ((static_cast<size_t>(N) * sizeof(float) + 255) / 256) * 256; }
 }
+// whether the product runs on the tcgen05 pipeline, which reads the rows as pairs
+namespace {
+bool batch_on_pipeline(const rwkvq_qtensor& t, int N) {
+    return tcb_enabled() && t.cols <= kPairCols && !batch_fast() && gemm_sb_ok(t) && (gemm_sb_pays(t, N) || tcb_forced());
+}
+}
 extern "C" size_t rwkvq_gemv_batch_workspace_bytes(int N) { return N > 0 ? batch_ws_pairs(N) + sb_halves(N, kPairCols) * sizeof(__half) : 0; }
+extern "C" size_t rwkvq_gemv_batch_workspace_bytes_of(const rwkvq_qtensor* t, int N) {
+    if (!t || N < 1) return 0;
+    return batch_ws_pairs(N) + (batch_on_pipeline(*t, N) ? sb_halves(N, t->cols) * sizeof(__half) : 0);
+}
 
 extern "C" int rwkvq_gemv_batch(const rwkvq_qtensor* t, const float* x, int N, int64_t ldx, float* y, int64_t ldy,
                                 int epilogue, const float* resid, void* workspace, size_t workspace_bytes, void* stream) {
@@ -759,13 +769,13 @@ extern "C" int rwkvq_gemv_batch(const rwkvq_qtensor* t, const float* x, int N, i
     // tensors without the relayouted streams: the tcgen05 kernel that reads the file buffers, in either precision
     const bool bare = mma_layout_of(*t) < 0;
     const bool tcb = tcb_ok && ldx % 8 == 0 && (bare || (batch_fast() && (N > 32 || tcb_forced())));
-    const bool sb = tcb_ok && t->cols <= kPairCols && !batch_fast() && gemm_sb_ok(*t) && (gemm_sb_pays(*t, N) || tcb_forced());
+    const bool sb = batch_on_pipeline(*t, N);
     RWKVQ_REQUIRE(tcb || sb || mma_layout_of(*t) >= 0, RWKVQ_E_DTYPE,
                   "rwkvq_gemv_batch: needs an sb6 tensor, a sym tensor or per-row int8 with columns in multiples of 128");
     RWKVQ_REQUIRE(aligned(x, 16) && ldx % 4 == 0, RWKVQ_E_ALIGN, "rwkvq_gemv_batch: x rows must be 16-byte aligned");
     RWKVQ_REQUIRE(aligned(workspace, 16), RWKVQ_E_ALIGN, "rwkvq_gemv_batch: workspace must be 16-byte aligned");
-    RWKVQ_REQUIRE(workspace && workspace_bytes >= rwkvq_gemv_batch_workspace_bytes(N), RWKVQ_E_LIMIT,
-                  "rwkvq_gemv_batch: workspace of %zu bytes, %zu needed", workspace_bytes, rwkvq_gemv_batch_workspace_bytes(N));
+    RWKVQ_REQUIRE(workspace && workspace_bytes >= rwkvq_gemv_batch_workspace_bytes_of(t, N), RWKVQ_E_LIMIT,
+                  "rwkvq_gemv_batch: workspace of %zu bytes, %zu needed", workspace_bytes, rwkvq_gemv_batch_workspace_bytes_of(t, N));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     int* status = static_cast<int*>(workspace);
     float* amax = reinterpret_cast<float*>(static_cast<char*>(workspace) + 256);
