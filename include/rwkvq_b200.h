@@ -431,6 +431,12 @@ int rwkvq_forward_seq(const rwkvq_model* m_host, int B, int T, const int64_t* to
                       const float* const* wkv_in, const float* const* tshift_in, const float* const* cshift_in,
                       float* const* wkv_out, float* const* tshift_out, float* const* cshift_out,
                       int tail, float* hidden, float* logits, void* workspace, size_t workspace_bytes, void* stream);
+/* The same with the status word in memory of the caller's (device int32, zero before its first use): set by
+ * compare-and-swap where a wait ran out and never cleared, so calls on several streams may share one. */
+int rwkvq_forward_seq_status(const rwkvq_model* m_host, int B, int T, const int64_t* tokens,
+                             const float* const* wkv_in, const float* const* tshift_in, const float* const* cshift_in,
+                             float* const* wkv_out, float* const* tshift_out, float* const* cshift_out,
+                             int tail, float* hidden, float* logits, int32_t* status, void* workspace, size_t workspace_bytes, void* stream);
 
 /*
  * Load-time relayout of the side streams of an sb6 / sym tensor for the decode

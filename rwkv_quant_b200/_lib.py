@@ -96,6 +96,8 @@ _PROTOS = {
     "rwkvq_forward_seq_workspace_bytes": (C.c_size_t, [C.POINTER(ModelStruct), C.c_int, C.c_int, C.c_int]),
     "rwkvq_forward_seq": (C.c_int, [C.POINTER(ModelStruct), C.c_int, C.c_int, C.c_void_p] + [C.POINTER(C.c_void_p)] * 6
                           + [C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p]),
+    "rwkvq_forward_seq_status": (C.c_int, [C.POINTER(ModelStruct), C.c_int, C.c_int, C.c_void_p] + [C.POINTER(C.c_void_p)] * 6
+                                 + [C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p]),
     "rwkvq_relayout_meta": (C.c_int, [C.POINTER(QTensorStruct), C.c_void_p, C.c_void_p]),
     "rwkvq_relayout_planes": (C.c_int, [C.POINTER(QTensorStruct), C.c_void_p, C.c_void_p]),
     "rwkvq_gemv_t": (C.c_int, [C.POINTER(QTensorStruct), C.c_void_p, C.c_int, C.c_int64,

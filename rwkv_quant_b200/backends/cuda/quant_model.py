@@ -112,6 +112,7 @@ class QuantRWKV7:
         self._build_struct()
         self._ws = {}
         self._seq_ok = {}
+        self._status = torch.zeros(1, dtype=torch.int32, device=dev)      # of the forward calls, on any stream
         self._lora_dense = {}
         self.fused_prep = True       # sequence path: LN/shift/lerp rows written in their consumers' forms
         torch.cuda.synchronize(dev)
@@ -363,9 +364,21 @@ class QuantRWKV7:
         table = C.c_void_p * L
         arr_in = [table(*[None if t is None else t.data_ptr() for t in ts]) for ts in ins]
         arr_out = [table(*[o.data_ptr() + i * o.stride(0) * 4 for i in range(L)]) for o in outs]
-        _lib.check(lib.rwkvq_forward_seq(C.byref(self._model_c), B, T, idx.data_ptr(), *arr_in, *arr_out, tail, _lib.ptr(hidden),
-                                         _lib.ptr(logits), ws.data_ptr(), nws, _lib.stream_ptr()), "rwkvq_forward_seq")
+        _lib.check(lib.rwkvq_forward_seq_status(C.byref(self._model_c), B, T, idx.data_ptr(), *arr_in, *arr_out, tail, _lib.ptr(hidden),
+                                                _lib.ptr(logits), self._status.data_ptr(), ws.data_ptr(), nws, _lib.stream_ptr()),
+                   "rwkvq_forward_seq")
         return hidden, logits, list(zip(*(o.unbind(0) for o in outs)))
+
+    def check(self):
+        """Synchronise and raise if a bounded device-side wait of a forward call ran out since the last check (its
+        outputs are then not to be used); ``Decoder.check`` does the same for decode steps."""
+        torch.cuda.synchronize(self.device)
+        words = [self._status] + [ws[:4].view(torch.int32) for ws in self._ws.values()]     # T > 1; T = 1
+        codes = [int(w.item()) for w in words]
+        for w in words:
+            w.zero_()
+        for code in codes:
+            _lib.check(code, "forward_stateful(kernel status)")
 
     def forward_hidden(self, idx, states):
         idx = torch.as_tensor(idx, device=self.device).long()

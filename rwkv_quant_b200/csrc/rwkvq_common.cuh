@@ -298,6 +298,13 @@ struct SideLane {
     int finish(cudaStream_t caller) const;       // the caller waits for the side stream
 };
 SideLane* side_lane(cudaStream_t caller);
+// rwkvq_gemv_batch / rwkvq_gemm with the scratch and the status word apart: the word is only set, `clear` (optional) is zeroed
+size_t gemv_batch_rows_bytes(const rwkvq_qtensor& t, int N);
+int launch_gemv_batch_rows(const rwkvq_qtensor& t, const float* x, int N, long long ldx, float* y, long long ldy, int epilogue,
+                           const float* resid, void* scratch, int* status, int* clear, cudaStream_t s);
+size_t gemm_rows_bytes(const rwkvq_qtensor& t, int M);
+int launch_gemm_rows(const rwkvq_qtensor& t, const float* x, int M, long long ldx, float* y, long long ldy, int epilogue,
+                     const float* resid, void* scratch, int* status, int* clear, cudaStream_t s);
 int launch_row_amax(const float* x, long long ldx, int cols, int N, float* amax, int* status, cudaStream_t s);
 
 }  // namespace rwkvq

@@ -916,7 +916,7 @@ Workspace carve(const rwkvq_model& m, int B, void* base) {
     }
     size_t gemm_bytes = 0;                  // only for the linears that reach rwkvq_gemm
     auto with_gemm = [&](const rwkvq_qtensor& t) {
-        if (linear_on_gemm(t, B)) gemm_bytes = std::max(gemm_bytes, rwkvq_gemm_workspace_bytes_of(&t, B, 1));
+        if (linear_on_gemm(t, B)) gemm_bytes = std::max(gemm_bytes, gemm_rows_bytes(t, B));
     };
     for (int l = 0; l < m.n_layer && m.layers; ++l)
         for (const rwkvq_qtensor* t : {&m.layers[l].Wr, &m.layers[l].Wk, &m.layers[l].Wv, &m.layers[l].Wo, &m.layers[l].Wfk, &m.layers[l].Wfv}) with_gemm(*t);
@@ -954,8 +954,11 @@ int linear(const rwkvq_qtensor* t, const float* x, int B, int in, float* y, int 
             return launch_gemm_tcb(t, 1, xs, x16 != nullptr, sc, B, in, ys, out, epi, rs, ao, status, static_cast<cudaStream_t>(stream));
         return launch_gemv_batch(t, 1, xs, x16 != nullptr, sc, B, in, ys, out, epi, rs, ao, static_cast<cudaStream_t>(stream));
     }
-    if (linear_on_gemm(*t, B))                              // tcgen05 path for large batches
-        return rwkvq_gemm(t, x, B, in, y, out, epi, resid, gemm_ws, rwkvq_gemm_workspace_bytes_of(t, B, 1), stream);
+    if (linear_on_gemm(*t, B)) {                            // tcgen05 path for large batches
+        int rc = validate_qtensor(t, "rwkvq_decode_step(linear)");
+        if (rc) return rc;
+        return launch_gemm_rows(*t, x, B, in, y, out, epi, resid, gemm_ws, status, nullptr, static_cast<cudaStream_t>(stream));
+    }
     return rwkvq_gemv(t, x, RWKVQ_F32, B, in, y, out, epi, resid, stream);
 }
 

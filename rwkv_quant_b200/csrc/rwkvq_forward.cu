@@ -78,8 +78,8 @@ ForwardWs carve(const rwkvq_model& m, int B, int T, size_t n_tail, void* base) {
     }
     if (n_tail > 0) {
         w.tailx = f32(n_tail * D); w.taily = f32(n_tail * D);
-        w.head_ws_bytes = n_tail <= 2 ? 0 : n_tail <= kSmallRows ? rwkvq_gemv_batch_workspace_bytes_of(&m.head, static_cast<int>(n_tail))
-                                                                : rwkvq_gemm_workspace_bytes_of(&m.head, static_cast<int>(n_tail), 1);
+        w.head_ws_bytes = n_tail <= 2 ? 0 : n_tail <= kSmallRows ? gemv_batch_rows_bytes(m.head, static_cast<int>(n_tail))
+                                                                : gemm_rows_bytes(m.head, static_cast<int>(n_tail));
         w.head_ws = take(w.head_ws_bytes);
     }
     w.bytes = off;
@@ -210,6 +210,13 @@ size_t rwkvq_forward_seq_workspace_bytes(const rwkvq_model* m, int B, int T, int
 int rwkvq_forward_seq(const rwkvq_model* m, int B, int T, const int64_t* tokens, const float* const* wkv_in, const float* const* tshift_in,
                       const float* const* cshift_in, float* const* wkv_out, float* const* tshift_out, float* const* cshift_out, int tail,
                       float* hidden, float* logits, void* workspace, size_t workspace_bytes, void* stream) {
+    return rwkvq_forward_seq_status(m, B, T, tokens, wkv_in, tshift_in, cshift_in, wkv_out, tshift_out, cshift_out, tail, hidden, logits, nullptr,
+                                    workspace, workspace_bytes, stream);
+}
+
+int rwkvq_forward_seq_status(const rwkvq_model* m, int B, int T, const int64_t* tokens, const float* const* wkv_in, const float* const* tshift_in,
+                      const float* const* cshift_in, float* const* wkv_out, float* const* tshift_out, float* const* cshift_out, int tail,
+                      float* hidden, float* logits, int32_t* status, void* workspace, size_t workspace_bytes, void* stream) {
     RWKVQ_REQUIRE(m && m->layers && tokens && wkv_in && tshift_in && cshift_in && wkv_out && tshift_out && cshift_out && workspace,
                   RWKVQ_E_NULL, "rwkvq_forward_seq: null pointer");
     RWKVQ_REQUIRE(B >= 1 && T >= 1 && tail >= 0 && tail <= T, RWKVQ_E_SHAPE, "rwkvq_forward_seq: B=%d T=%d tail=%d", B, T, tail);
@@ -234,7 +241,9 @@ int rwkvq_forward_seq(const rwkvq_model* m, int B, int T, const int64_t* tokens,
         for (const float* p : {wkv_in[l], tshift_in[l], cshift_in[l], const_cast<const float*>(wkv_out[l]),
                                const_cast<const float*>(tshift_out[l]), const_cast<const float*>(cshift_out[l])})
             RWKVQ_REQUIRE(aligned(p, 16), RWKVQ_E_ALIGN, "rwkvq_forward_seq: the states of layer %d must be 16-byte aligned", l);
-    const ForwardWs w = carve(*m, B, T, static_cast<size_t>(B) * tail, workspace);
+    int head_rc = validate_qtensor(&m->head, "rwkvq_forward_seq");
+    if (head_rc) return head_rc;
+    ForwardWs w = carve(*m, B, T, static_cast<size_t>(B) * tail, workspace);
     RWKVQ_REQUIRE(workspace_bytes >= w.bytes && aligned(workspace, 256), RWKVQ_E_LIMIT,
                   "rwkvq_forward_seq: workspace %zu of %zu bytes, 256-byte aligned", workspace_bytes, w.bytes);
     const int N = static_cast<int>(rows64), D = m->n_embd, F = m->ffn_dim, H = D / 64;
@@ -244,6 +253,7 @@ int rwkvq_forward_seq(const rwkvq_model* m, int B, int T, const int64_t* tokens,
     Pass ps{*m, w, B, T, N, D, F, H, s};
     // the status word and every layer's norm bounds (merged by atomic max)
     if (cudaMemsetAsync(w.status, 0, 256 + sizeof(float) * 128 * m->n_layer, s) != cudaSuccess) return check_launch("rwkvq_forward_seq(memset)");
+    if (status) w.status = status;
     int rc = rwkvq_seq_embed_ln0(&m->emb, tokens, m->ln0_w, m->ln0_b, w.x, N, D, stream);
     if (rc) return rc;
     // r / k / v beside the LoRA branches while neither fills the chip (5 rows 2.07 -> 2.00 ms, 231 rows 4.46 -> 4.30,
@@ -408,8 +418,8 @@ int rwkvq_forward_seq(const rwkvq_model* m, int B, int T, const int64_t* tokens,
         rc = rwkvq_seq_layer_norm(w.tailx, m->lnout_w, m->lnout_b, w.taily, n, D, stream);
         if (rc) return rc;
         if (n <= 2) rc = rwkvq_gemv(&m->head, w.taily, RWKVQ_F32, n, D, logits, V, RWKVQ_EPI_NONE, nullptr, stream);
-        else if (n <= kSmallRows) rc = rwkvq_gemv_batch(&m->head, w.taily, n, D, logits, V, RWKVQ_EPI_NONE, nullptr, w.head_ws, w.head_ws_bytes, stream);
-        else rc = rwkvq_gemm(&m->head, w.taily, n, D, logits, V, RWKVQ_EPI_NONE, nullptr, w.head_ws, w.head_ws_bytes, stream);
+        else if (n <= kSmallRows) rc = launch_gemv_batch_rows(m->head, w.taily, n, D, logits, V, RWKVQ_EPI_NONE, nullptr, w.head_ws, w.status, nullptr, s);
+        else rc = launch_gemm_rows(m->head, w.taily, n, D, logits, V, RWKVQ_EPI_NONE, nullptr, w.head_ws, w.status, nullptr, s);
         if (rc) return rc;
     }
     return check_launch("rwkvq_forward_seq");

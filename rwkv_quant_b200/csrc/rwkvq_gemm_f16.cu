@@ -828,6 +828,17 @@ int gemm_chunks(const rwkvq_qtensor* t, const __half* x16, const float* row_scal
 }
 }  // namespace
 
+size_t rwkvq::gemm_rows_bytes(const rwkvq_qtensor& t, int M) { return ws_w_off(M, t.cols) - 256 + gemm_scratch(t.rows, t.cols); }
+int rwkvq::launch_gemm_rows(const rwkvq_qtensor& t, const float* x, int M, long long ldx, float* y, long long ldy, int epilogue,
+                            const float* resid, void* scratch, int* status, int* clear, cudaStream_t s) {
+    char* ws = static_cast<char*>(scratch) - 256;        // the offsets are those of the workspace, whose head is the status word
+    float* scale = reinterpret_cast<float*>(ws + 256);
+    __half* x16 = reinterpret_cast<__half*>(ws + ws_x16_off(M));
+    int rc = launch_row_scale(x, ldx, t.cols, M, scale, x16, static_cast<long long>(x16_pitch(t.cols)), clear, s);
+    if (rc) return rc;
+    return gemm_chunks(&t, x16, scale, M, y, ldy, epilogue, resid, reinterpret_cast<__half*>(ws + ws_w_off(M, t.cols)), status, s);
+}
+
 extern "C" {
 
 void rwkvq_profiling_gemm_acc_mode(int mode) { g_gemm_acc_mode = mode; }      // rwkvq_profiling.h
@@ -863,14 +874,9 @@ int rwkvq_gemm(const rwkvq_qtensor* t, const float* x, int M, int64_t ldx, float
                   "rwkvq_gemm: x and its row stride must be 16-byte aligned, the workspace 256-byte aligned");
     RWKVQ_REQUIRE(workspace_bytes >= rwkvq_gemm_workspace_bytes_of(t, M, 1), RWKVQ_E_LIMIT,
                   "rwkvq_gemm: workspace %zu < %zu bytes", workspace_bytes, rwkvq_gemm_workspace_bytes_of(t, M, 1));
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    char* ws = static_cast<char*>(workspace);
-    int* status = reinterpret_cast<int*>(ws);
-    float* scale = reinterpret_cast<float*>(ws + 256);
-    __half* x16 = reinterpret_cast<__half*>(ws + ws_x16_off(M));
-    rc = launch_row_scale(x, ldx, t->cols, M, scale, x16, static_cast<long long>(x16_pitch(t->cols)), status, s);
-    if (rc) return rc;
-    rc = gemm_chunks(t, x16, scale, M, y, ldy, epilogue, resid, reinterpret_cast<__half*>(ws + ws_w_off(M, t->cols)), status, s);
+    int* status = static_cast<int*>(workspace);
+    rc = launch_gemm_rows(*t, x, M, ldx, y, ldy, epilogue, resid, static_cast<char*>(workspace) + 256, status, status,
+                          static_cast<cudaStream_t>(stream));
     return rc ? rc : check_launch("rwkvq_gemm");
 }
 

@@ -752,7 +752,40 @@ bool batch_on_pipeline(const rwkvq_qtensor& t, int N) {
 extern "C" size_t rwkvq_gemv_batch_workspace_bytes(int N) { return N > 0 ? batch_ws_pairs(N) + sb_halves(N, kPairCols) * sizeof(__half) : 0; }
 extern "C" size_t rwkvq_gemv_batch_workspace_bytes_of(const rwkvq_qtensor* t, int N) {
     if (!t || N < 1) return 0;
-    return batch_ws_pairs(N) + (batch_on_pipeline(*t, N) ? sb_halves(N, t->cols) * sizeof(__half) : 0);
+    return 256 + gemv_batch_rows_bytes(*t, N);
+}
+size_t rwkvq::gemv_batch_rows_bytes(const rwkvq_qtensor& t, int N) {
+    return batch_ws_pairs(N) - 256 + (batch_on_pipeline(t, N) ? sb_halves(N, t.cols) * sizeof(__half) : 0);
+}
+
+// The product on rows whose scale is not known: a pass that measures (or splits) them, then the kernel that pays
+// (scratch: gemv_batch_rows_bytes, 16-byte aligned; clear, optional: a status word of the product's own).
+int rwkvq::launch_gemv_batch_rows(const rwkvq_qtensor& t, const float* x, int N, long long ldx, float* y, long long ldy, int epilogue,
+                                  const float* resid, void* scratch, int* status, int* clear, cudaStream_t s) {
+    // default: the two-term mma.sync kernel below kSbLeastRows rows, the tcgen05 pipeline from there on (gemm_sb_pays);
+    // single-term operands: mma.sync up to 32 rows, the single-buffer tcgen05 kernel above
+    const bool tcb_ok = tcb_enabled() && gemm_tcb_ok(t);
+    // tensors without the relayouted streams: the tcgen05 kernel that reads the file buffers, in either precision
+    const bool bare = mma_layout_of(t) < 0;
+    const bool tcb = tcb_ok && ldx % 8 == 0 && (bare || (batch_fast() && (N > 32 || tcb_forced())));
+    const bool sb = batch_on_pipeline(t, N);
+    RWKVQ_REQUIRE(tcb || sb || mma_layout_of(t) >= 0, RWKVQ_E_DTYPE,
+                  "rwkvq_gemv_batch: needs an sb6 tensor, a sym tensor or per-row int8 with columns in multiples of 128");
+    float* amax = static_cast<float*>(scratch);
+    float* ys[1] = {y};
+    const float* rs[1] = {resid};
+    if (sb) {
+        const SbRows rows = sb_rows(reinterpret_cast<__half*>(static_cast<char*>(scratch) + batch_ws_pairs(N) - 256), amax, N, t.cols);
+        int rc = launch_split_rows(x, ldx, t.cols, N, rows, clear, s);
+        if (rc) return rc;
+        return launch_gemm_sb(&t, 1, &rows, N, ys, ldy, epilogue, rs, nullptr, status, tcb_forced_ks(), s);
+    }
+    int rc = launch_row_amax(x, ldx, t.cols, N, amax, clear, s);
+    if (rc) return rc;
+    const void* xs[1] = {x};
+    const float* am[1] = {amax};
+    return tcb ? launch_gemm_tcb(&t, 1, xs, false, am, N, ldx, ys, ldy, epilogue, rs, nullptr, status, s, !batch_fast())
+               : launch_gemv_batch(&t, 1, xs, false, am, N, ldx, ys, ldy, epilogue, rs, nullptr, s);
 }
 
 extern "C" int rwkvq_gemv_batch(const rwkvq_qtensor* t, const float* x, int N, int64_t ldx, float* y, int64_t ldy,
@@ -763,36 +796,12 @@ extern "C" int rwkvq_gemv_batch(const rwkvq_qtensor* t, const float* x, int N, i
     RWKVQ_REQUIRE(epilogue >= RWKVQ_EPI_NONE && epilogue <= RWKVQ_EPI_ADD, RWKVQ_E_DTYPE, "rwkvq_gemv_batch: epilogue %d", epilogue);
     RWKVQ_REQUIRE(ldx >= t->cols && ldy >= t->rows, RWKVQ_E_SHAPE, "rwkvq_gemv_batch: ldx %lld / ldy %lld", (long long)ldx, (long long)ldy);
     RWKVQ_REQUIRE(x && y, RWKVQ_E_NULL, "rwkvq_gemv_batch: x or y is null");
-    // default: the two-term mma.sync kernel below kSbLeastRows rows, the tcgen05 pipeline from there on (gemm_sb_pays);
-    // single-term operands: mma.sync up to 32 rows, the single-buffer tcgen05 kernel above
-    const bool tcb_ok = tcb_enabled() && gemm_tcb_ok(*t);
-    // tensors without the relayouted streams: the tcgen05 kernel that reads the file buffers, in either precision
-    const bool bare = mma_layout_of(*t) < 0;
-    const bool tcb = tcb_ok && ldx % 8 == 0 && (bare || (batch_fast() && (N > 32 || tcb_forced())));
-    const bool sb = batch_on_pipeline(*t, N);
-    RWKVQ_REQUIRE(tcb || sb || mma_layout_of(*t) >= 0, RWKVQ_E_DTYPE,
-                  "rwkvq_gemv_batch: needs an sb6 tensor, a sym tensor or per-row int8 with columns in multiples of 128");
     RWKVQ_REQUIRE(aligned(x, 16) && ldx % 4 == 0, RWKVQ_E_ALIGN, "rwkvq_gemv_batch: x rows must be 16-byte aligned");
     RWKVQ_REQUIRE(aligned(workspace, 16), RWKVQ_E_ALIGN, "rwkvq_gemv_batch: workspace must be 16-byte aligned");
     RWKVQ_REQUIRE(workspace && workspace_bytes >= rwkvq_gemv_batch_workspace_bytes_of(t, N), RWKVQ_E_LIMIT,
                   "rwkvq_gemv_batch: workspace of %zu bytes, %zu needed", workspace_bytes, rwkvq_gemv_batch_workspace_bytes_of(t, N));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    int* status = static_cast<int*>(workspace);
-    float* amax = reinterpret_cast<float*>(static_cast<char*>(workspace) + 256);
-    float* ys[1] = {y};
-    const float* rs[1] = {resid};
-    if (sb) {
-        const SbRows rows = sb_rows(reinterpret_cast<__half*>(static_cast<char*>(workspace) + batch_ws_pairs(N)), amax, N, t->cols);
-        rc = launch_split_rows(x, ldx, t->cols, N, rows, status, s);
-        if (rc) return rc;
-        rc = launch_gemm_sb(t, 1, &rows, N, ys, ldy, epilogue, rs, nullptr, status, tcb_forced_ks(), s);
-        return rc ? rc : check_launch("rwkvq_gemv_batch");
-    }
-    rc = launch_row_amax(x, ldx, t->cols, N, amax, status, s);
-    if (rc) return rc;
-    const void* xs[1] = {x};
-    const float* am[1] = {amax};
-    rc = tcb ? launch_gemm_tcb(t, 1, xs, false, am, N, ldx, ys, ldy, epilogue, rs, nullptr, status, s, !batch_fast())
-             : launch_gemv_batch(t, 1, xs, false, am, N, ldx, ys, ldy, epilogue, rs, nullptr, s);
+    rc = launch_gemv_batch_rows(*t, x, N, ldx, y, ldy, epilogue, resid, static_cast<char*>(workspace) + 256, static_cast<int*>(workspace),
+                                static_cast<int*>(workspace), s);
     return rc ? rc : check_launch("rwkvq_gemv_batch");
 }

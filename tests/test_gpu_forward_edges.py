@@ -186,3 +186,29 @@ def test_cuda_rows_on_host_weights_are_refused(cuda_lib, rows):
     op = linear_for(_synth_linear("sb6", 4, 128, 256, seed=1), "cpu")
     with pytest.raises(RuntimeError, match="CUDA tensors only"):
         op(_x(rows, 256, 1))
+
+
+@pytest.mark.parametrize("B,T", [(1, 2), (1, 5), (1, 40), (5, 20)])      # every kind of head and of layer linear
+def test_a_time_out_is_kept_until_it_is_asked_for(cuda_lib, B, T):
+    """The kernels set one word of the model's by compare-and-swap; no later launch or call clears it."""
+    from rwkv_quant_b200 import _lib
+    model = _model()
+    idx, st = _idx(B, T), _states(model, B)
+    model.forward_stateful(idx, st)
+    model.check()
+    model._status.fill_(-9)                                       # as a kernel whose wait ran out leaves it
+    model.forward_stateful(idx, st)
+    with pytest.raises(_lib.RwkvqError, match="kernel status"):
+        model.check()
+    model.check()
+
+
+def test_a_time_out_of_a_large_step_is_kept(cuda_lib):
+    """More streams than the small-batch kernels take: the linears report to the step's own word."""
+    from rwkv_quant_b200 import _lib
+    model = _model()
+    dec = model.decoder(260, use_graph=False)
+    dec._ws[0][:4].view(torch.int32).fill_(-9)
+    dec.step(torch.ones(260, dtype=torch.long, device="cuda"))
+    with pytest.raises(_lib.RwkvqError, match="kernel status"):
+        dec.check()
