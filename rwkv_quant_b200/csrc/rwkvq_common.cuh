@@ -298,6 +298,23 @@ struct SideLane {
     int finish(cudaStream_t caller) const;       // the caller waits for the side stream
 };
 SideLane* side_lane(cudaStream_t caller);
+// A fork onto a lane (or none): joined on every way out, so that what ran beside is ordered before the caller's next work
+struct Fork {
+    const SideLane* lane;
+    cudaStream_t caller;
+    bool open = false;
+    int start() {
+        if (!lane) return RWKVQ_OK;
+        open = true;
+        return lane->start(caller);
+    }
+    int join() {
+        if (!open) return RWKVQ_OK;
+        open = false;
+        return lane->finish(caller);
+    }
+    ~Fork() { if (open) lane->finish(caller); }
+};
 // rwkvq_gemv_batch / rwkvq_gemm with the scratch and the status word apart: the word is only set, `clear` (optional) is zeroed
 size_t gemv_batch_rows_bytes(const rwkvq_qtensor& t, int N);
 int launch_gemv_batch_rows(const rwkvq_qtensor& t, const float* x, int N, long long ldx, float* y, long long ldy, int epilogue,

@@ -1148,9 +1148,10 @@ int rwkvq_decode_step(const rwkvq_model* m, int B, const int64_t* tokens, float*
             if (rc) return rc;
         } else {
         SideLane* lane = side_lane(s);
+        Fork fork{lane, s};
         cudaStream_t s_lora = s;
         if (lane) {                                  // fork: the LoRA branches leave the chain here
-            rc = lane->start(s);
+            rc = fork.start();
             if (rc) return rc;
             s_lora = lane->stream;
         }
@@ -1214,10 +1215,8 @@ int rwkvq_decode_step(const rwkvq_model* m, int B, const int64_t* tokens, float*
             rc = lora();
             if (rc) return rc;
         }
-        if (lane) {                                  // join before the time-mix core
-            rc = lane->finish(s);
-            if (rc) return rc;
-        }
+        rc = fork.join();                            // before the time-mix core
+        if (rc) return rc;
         launch_pdl(tmix_core_kernel<false>, dim3(H, B), dim3(256), 0, s, tc, 0);
         }
         if (sb) {

@@ -274,6 +274,7 @@ int rwkvq_forward_seq_status(const rwkvq_model* m, int B, int T, const int64_t* 
         // mix rows: r, w, k, v, a, g
         const bool sb = small && D % 256 == 0 && same_shape(L.Wr, L.Wk) && same_shape(L.Wr, L.Wv) && gemm_sb_pays(L.Wr, N) &&
                         gemm_sb_pays(L.Wo, N) && gemm_sb_pays(L.Wfk, N) && gemm_sb_pays(L.Wfv, N);
+        Fork fork{lane, s};
         if (small) {
             for (int q = 0; q < 6; ++q) {
                 a.f32[q] = w.xs + q * ND; a.scale[q] = w.amax + q * N;
@@ -288,7 +289,7 @@ int rwkvq_forward_seq_status(const rwkvq_model* m, int B, int T, const int64_t* 
             }
             rc = launch_seq_prep(a, N, s);
             if (rc) return rc;
-            if (lane && (rc = lane->start(s)) != 0) return rc;
+            if ((rc = fork.start()) != 0) return rc;
             const rwkvq_qtensor* t3[3] = {&L.Wr, &L.Wk, &L.Wv};
             const float* x3[3] = {w.xs, w.xs + 2 * ND, w.xs + 3 * ND};
             const float* a3[3] = {w.amax, w.amax + 2 * N, w.amax + 3 * N};
@@ -319,11 +320,11 @@ int rwkvq_forward_seq_status(const rwkvq_model* m, int B, int T, const int64_t* 
             }
             rc = launch_seq_prep(a, N, s);
             if (rc) return rc;
-            if (lane && (rc = lane->start(s)) != 0) return rc;
+            if ((rc = fork.start()) != 0) return rc;
             rc = ps.mix_large(L, layer0, y3, s_rkv);
         }
         if (rc) return rc;
-        if (lane && (rc = lane->finish(s)) != 0) return rc;
+        if ((rc = fork.join()) != 0) return rc;
         if (!small && T >= kChunkedT) {
             WkvChunkArgs q{};
             q.r = r; q.k = k; q.v = v; q.yw = yw; q.ya = ya; q.yv = layer0 ? nullptr : yv; q.v_first = layer0 ? nullptr : w.v_first; q.g = yg;

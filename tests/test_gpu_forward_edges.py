@@ -212,3 +212,34 @@ def test_a_time_out_of_a_large_step_is_kept(cuda_lib):
     dec.step(torch.ones(260, dtype=torch.long, device="cuda"))
     with pytest.raises(_lib.RwkvqError, match="kernel status"):
         dec.check()
+
+
+@pytest.mark.parametrize("B", [2, 13])
+def test_an_error_behind_the_fork_joins_the_side_stream(cuda_lib, B):
+    """A tensor of the last layer is refused when that layer is reached: what ran on the side stream until then must be
+    ordered before the caller's later work (memory goes back to the allocator in that order).  Under capture an open
+    side stream is an error of its own."""
+    from rwkv_quant_b200 import _lib
+    model = _model()
+    dec = model.decoder(B, use_graph=False)
+    dec.step(torch.ones(B, dtype=torch.long, device="cuda"))
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        dec.step(torch.ones(B, dtype=torch.long, device="cuda"))          # the stream has its side stream now
+        torch.cuda.synchronize()
+        layer = model._layers_c[1]
+        codes = layer.w2.codes                                             # looked at behind the launch of r / k / v beside it
+        graph = torch.cuda.CUDAGraph()
+        graph.capture_begin()
+        try:
+            layer.w2.codes = None
+            with pytest.raises(_lib.RwkvqError, match="null"):
+                dec._run()
+        finally:
+            layer.w2.codes = codes
+            graph.capture_end()
+    torch.cuda.synchronize()
+    ref = model.decoder(B, use_graph=False)
+    dec = model.decoder(B)
+    tok = torch.arange(1, B + 1, device="cuda")
+    assert torch.equal(ref.step(tok), dec.step(tok))
