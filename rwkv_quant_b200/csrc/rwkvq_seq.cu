@@ -541,12 +541,28 @@ int launch_seq_prep(const SeqPrepArgs& a, long long n_tokens, cudaStream_t s) {
                   RWKVQ_E_ALIGN, "seq_ln_shift_mix_prep: 8-byte aligned rows required");       // the scalar form reads pairs
     RWKVQ_REQUIRE(!in_place || a.T == 1, RWKVQ_E_SHAPE, "seq_ln_shift_mix_prep: the shift state in place needs T = 1");
     // (in place: the scalar form has a token's mixes in one CTA, the vector form in one cluster)
-    // up to one wave of CTAs (two per SM) with a token and mix each, then groups of 64 threads per token
-    const bool few = n_tokens * a.n_mix <= 2 * 148 || pair || in_place;
-    if (vec && !few && a.D == 2048) e = launch_prep_group<4>(a, n_tokens, s);
-    else if (vec && !few && a.D == 2560) e = launch_prep_group<5>(a, n_tokens, s);
-    else if (vec && !few && a.D == 1024) e = launch_prep_group<2>(a, n_tokens, s);
-    else if (vec && in_place && a.n_mix > 1) {
+    // Which form (us, scalar / vector / groups, six mixes and one):
+    //   few      the vector form while its CTAs, one per token and mix, are one wave: two an SM up to 2048 columns, one above (six
+    //            mixes: still ahead at two a slot).  2048 columns, 49 tokens: 7.6 / 4.1, one mix 296: 4.8 / 4.2; 2304, 231: 4.9 / 7.1
+    //   many     groups where D is a multiple of 512 up to 3072 (above, two rows a thread no longer fit its registers: 4096 columns,
+    //            8192 tokens 245 / 711 / 319), from where one wave of the scalar form (3 CTAs an SM) ends.  8192 tokens, six
+    //            mixes: 1536 163 / 240 / 74, 2048 174 / 276 / 102, 2560 186 / 542 / 132; 512 tokens: 16.7 / 23.7 / 12.1, 17.9 / 26.8 / 13.1,
+    //            19.4 / 49 / 18.9, one mix 7.4 / 6.7 / 6.4, 8.0 / 7.7 / 7.2, 8.5 / 13.8 / 9.7
+    //   other widths: the vector form where it is narrow (768: 139 / 91, one mix 60 / 20; 1280, one mix 63 / 41), else the scalar one
+    //            (2304, 8192 tokens: 177 / 521; 1792: 166 / 260)
+    const int wave = a.n_mix == 1 && a.D > 2048 ? 148 : 2 * 148;
+    const bool few = n_tokens * a.n_mix <= wave || pair || in_place;
+    const long long groups_from = a.D <= 1536 ? 0 : a.D > 2048 ? 1024 : a.n_mix > 1 ? 200 : 445;
+    if (vec && !few && a.D % 512 == 0 && a.D <= 3072 && n_tokens >= groups_from) {
+        switch (a.D / 512) {
+            case 1: e = launch_prep_group<1>(a, n_tokens, s); break;
+            case 2: e = launch_prep_group<2>(a, n_tokens, s); break;
+            case 3: e = launch_prep_group<3>(a, n_tokens, s); break;
+            case 4: e = launch_prep_group<4>(a, n_tokens, s); break;
+            case 5: e = launch_prep_group<5>(a, n_tokens, s); break;
+            default: e = launch_prep_group<6>(a, n_tokens, s); break;
+        }
+    } else if (vec && in_place && a.n_mix > 1) {
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(static_cast<unsigned>(n_tokens), a.n_mix);
         cfg.blockDim = dim3(a.D / 8);
@@ -559,7 +575,7 @@ int launch_seq_prep(const SeqPrepArgs& a, long long n_tokens, cudaStream_t s) {
         cfg.attrs = attr;
         cfg.numAttrs = pdl_enabled() ? 2 : 1;
         e = cudaLaunchKernelEx(&cfg, seq_prep_vec_kernel<true>, a, n_tokens, 1);
-    } else if (vec) {
+    } else if (vec && (few || a.D <= (a.n_mix == 1 ? 1280 : 1024))) {
         long long run = in_place ? 1 : n_tokens * a.n_mix / (148 * 8);
         run = run < 1 ? 1 : run > 16 ? 16 : run;
         e = launch_pdl(seq_prep_vec_kernel<false>, dim3(static_cast<unsigned>((n_tokens + run - 1) / run), a.n_mix), dim3(a.D / 8), 0, s, a, n_tokens,

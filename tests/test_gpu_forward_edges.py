@@ -243,3 +243,31 @@ def test_an_error_behind_the_fork_joins_the_side_stream(cuda_lib, B):
     dec = model.decoder(B)
     tok = torch.arange(1, B + 1, device="cuda")
     assert torch.equal(ref.step(tok), dec.step(tok))
+
+
+@pytest.mark.parametrize("D", [128, 512, 768, 1024, 1280, 1536, 2048, 2304, 2560, 3072, 3584, 4096])
+@pytest.mark.parametrize("N", [24, 49, 50, 199, 444, 1024])
+def test_row_preparation_in_every_form(cuda_lib, D, N):
+    """Widths and token counts on each side of the lines between the scalar, vector and group forms; the three row forms of a
+    mix agree with the fp64 LayerNorm, shift and lerp: fp32 rows to rounding, pairs to 2^-20, scaled fp16 to half an ulp of 2^-10."""
+    from rwkv_quant_b200.backends.cuda import ops
+    gen = torch.Generator(device="cuda").manual_seed(D + N)
+    draw = lambda *s: torch.randn(s, generator=gen, device="cuda")
+    x, w, b, shift = draw(2, N // 2, D), draw(D), draw(D), draw(2, 1, D)
+    xn = torch.nn.functional.layer_norm(x.double(), (D,), w.double(), b.double())
+    prev = torch.cat([shift.double(), xn[:, :-1]], 1)
+    for modes in ([1, 2, 4, 7, 2, 2], [7]):
+        mix = draw(len(modes), D)
+        rows, new = ops.seq_ln_shift_mix_prep(x, w, b, shift, mix, modes)
+        assert relmax(new.cpu().numpy(), xn[:, -1:].cpu().numpy()) <= 2e-6
+        for m, r in enumerate(rows):
+            want = (xn + (prev - xn) * mix[m].double()).reshape(-1, D)
+            top = want.abs().amax(1, keepdim=True)
+            if r.f32 is not None:
+                assert relmax(r.f32.cpu().numpy(), want.cpu().numpy()) <= 2e-6
+            if r.split is not None:
+                assert ((r.split[:, :D].double() + r.split[:, D:].double() - want).abs() <= top * 2.0 ** -20).all()
+            if r.x16 is not None:
+                got = r.x16[:, :D].double() / r.scale[:, None].double()
+                assert ((got - want).abs() <= want.abs() * 2.0 ** -11 + top * 2.0 ** -20).all()
+                assert (r.scale[:, None] * top <= 2.0 ** 14).all()
