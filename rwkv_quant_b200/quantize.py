@@ -23,13 +23,13 @@ SYM_MODES = ("sym", "sym_aw", "sym_plain")
 def sym_factors() -> torch.Tensor:
     """The scale factors the reference's symmetric search visits: the float32 nodes of
     torch.linspace(0.7, 1.15, 19) (calibration/groupwise.py:305)."""
-    return torch.linspace(0.7, 1.15, 19)
+    return torch.linspace(0.7, 1.15, 19, dtype=torch.float32, device="cpu")
 
 
 @functools.lru_cache(maxsize=16)
 def _factors(search: bool, device: torch.device) -> torch.Tensor:
     """The search's scale factors on a device (19 constants: uploaded once)."""
-    return (sym_factors() if search else torch.ones(1)).to(device)
+    return (sym_factors() if search else torch.ones(1, dtype=torch.float32, device="cpu")).to(device)
 
 
 def _prepared(who: str, w: torch.Tensor, ex2: Optional[torch.Tensor]):
@@ -74,8 +74,6 @@ def quantize_sb6(key: str, group: str, w: torch.Tensor, bits: int, mode: str = "
         raise ValueError(f"quantize_sb6: mode {mode!r}")
     if (mode == "asym_sb6_aw") != (ex2 is not None):
         raise ValueError("quantize_sb6: ex2 goes with mode asym_sb6_aw, and only with it")
-    if not 4 <= bits <= 6:
-        raise ValueError(f"quantize_sb6: {bits} bits (4, 5 or 6)")
     w32, e = _prepared("quantize_sb6", w, ex2)
     (o, n), dev = w32.shape, w32.device
     u8 = dict(dtype=torch.uint8, device=dev)
@@ -118,11 +116,9 @@ def quantize_sym(key: str, group: str, w: torch.Tensor, bits: int, mode: str = "
         raise ValueError(f"quantize_sym: mode {mode!r}")
     if (mode == "sym_aw") != (ex2 is not None):
         raise ValueError("quantize_sym: ex2 goes with mode sym_aw, and only with it")
-    if bits == 8:
+    if bits != 6:                                        # 8; the library refuses others
         q, qs, d = quantize_sym_parts(w, bits, mode != "sym_plain", ex2)
-        return QuantizedTensor(key=key, group=group, bits=8, shape=tuple(w.shape), gw_mode="sym", gw_gs=16, gw_sb=16, gw_qs=qs, gw_d=d, codes=q)
-    if bits != 6:
-        raise ValueError(f"quantize_sym: {bits} bits (6 or 8)")
+        return QuantizedTensor(key=key, group=group, bits=bits, shape=tuple(w.shape), gw_mode="sym", gw_gs=16, gw_sb=16, gw_qs=qs, gw_d=d, codes=q)
     w32, e = _prepared("quantize_sym", w, ex2)
     (o, n), dev = w32.shape, w32.device
     f = _factors(mode != "sym_plain", dev)
