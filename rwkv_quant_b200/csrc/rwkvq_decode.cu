@@ -823,7 +823,8 @@ namespace {
 
 constexpr int kBatchMax = 256;     // streams up to which the small-batch kernel serves the linears of a step
 // (two streams: 1.60 ms per step of the 1.5B model against 1.82 on one single-vector launch per stream, 2.9B 2.79 / 3.81)
-inline bool batch_path(int B) { return B > 1 && B <= kBatchMax; }
+// with single-term operands from three on: two streams keep the single-vector kernels' precision in every mode
+inline bool batch_path(int B) { return B > (batch_fast() ? 2 : 1) && B <= kBatchMax; }
 // Which small-batch kernel: measured on B200 (1.5B, whole decode step) the tcgen05 form wins from 33
 // streams on (64 streams: 3.77 against 4.43 ms per step) and loses below (32: 2.87 / 2.68 ms, 8: 2.42 / 2.01 ms):
 // its pass (dependent weight loads -> conversion -> MMA) is longer than a warp-iteration of the mma.sync form

@@ -271,3 +271,23 @@ def test_row_preparation_in_every_form(cuda_lib, D, N):
                 got = r.x16[:, :D].double() / r.scale[:, None].double()
                 assert ((got - want).abs() <= want.abs() * 2.0 ** -11 + top * 2.0 ** -20).all()
                 assert (r.scale[:, None] * top <= 2.0 ** 14).all()
+
+
+def test_two_streams_keep_their_precision_with_single_term_operands(cuda_lib):
+    """RWKVQ_BATCH_FAST=1 (here by the library's profiling switch) selects single fp16 operands from three streams on."""
+    import ctypes as C
+    model = _model(n_embd=512, ffn=2048)
+    hook = cuda_lib.rwkvq_profiling_batch_fast
+    hook.restype, hook.argtypes = None, [C.c_int]
+    out = {}
+    try:
+        for fast in (0, 1):
+            hook(fast)
+            for B in (2, 3):
+                dec = model.decoder(B, states=_states(model, B), use_graph=False)
+                dec.step(torch.arange(1, B + 1, device="cuda"))
+                out[fast, B] = dec.logits.cpu().numpy()
+    finally:
+        hook(-1)
+    assert relmax(out[1, 2], out[0, 2]) <= 2e-5
+    assert relmax(out[1, 3], out[0, 3]) > 5e-5                    # the switch was on
