@@ -4,8 +4,8 @@ The reference-written toy files pin the model at D = 256; here the same comparis
 2-layer builds with the real width, heads, LoRA ranks, channel-mix width and vocabulary of
 RWKV-7 1.5B (D 2048, 32 heads, FFN 8192, ranks 96/96/64/256) and 2.9B (D 2560, 40 heads,
 FFN 10240, ranks 96/96/64/320), vocabulary 65536, in both recipes, so that every launch
-geometry of the benchmark (K-split GEMVs, the persistent 296-CTA head launch, the 65536-row
-argmax, 32/40-head time-mix core, 256-token GEMM tiles, 8192-token glue) runs inside a model
+geometry of the benchmark (K-split GEMVs, the persistent head launch, the 65536-row argmax,
+32/40-head time-mix core, CTA-pair GEMM tiles, 8192-token glue) runs inside a model
 and is compared with the CPU oracle (the reference's model gate is tests/test_quant_parity.py:129-138).
 
   decode   8 teacher-forced tokens at batch 1 and batch 64, eager launches and CUDA-graph
@@ -139,12 +139,11 @@ def test_prefill_then_decode_full_width(build):
 
 @pytest.mark.parametrize("B", [40, 64])
 def test_decode_two_term_tcgen05_linears(build, cuda_lib, B):
-    """Batched decode above 32 streams runs some linears on the two-term tcgen05 kernel, fed with fp16
-    pairs and block sums by the LayerNorm kernels: r / k / v, the ffn key and the head up to 48 streams,
-    the head alone up to 64 (RWKVQ_TCB_EXACT=1 / 0 force all three / none; here through the library's
-    profiling switch, not part of the C ABI).  With all three forced: the tolerance of the default path
-    against the oracle (streams 0 and B - 1) and fp32-grade agreement with the all-mma.sync step; at 40
-    streams the launcher's own choice must be exactly the forced one."""
+    """Batched decode from 17 streams on runs every linear on the tcgen05 pipeline, fed with fp16 pairs and block sums by the
+    LayerNorm kernels and by a pass over the other rows (RWKVQ_TCB_EXACT=1 / 0: from three streams on / never; here through
+    the library's profiling switch, not part of the C ABI).  Forced: the tolerance of the default path against the oracle
+    (streams 0 and B - 1) and fp32-grade agreement with the all-mma.sync step; the launcher's own choice must be exactly
+    the forced one."""
     import ctypes as C
     model, oracle, name = build
     hook = cuda_lib.rwkvq_profiling_tcb_exact
@@ -175,13 +174,12 @@ def test_decode_two_term_tcgen05_linears(build, cuda_lib, B):
     err = relmax(got[1][rows], ref)
     both = relmax(got[1], got[0])
     own = relmax(got[-1][rows], ref)
-    print(f"{name} decode B={B}, two-term tcgen05 linears: logits relmax {err:.2e} vs oracle, {both:.2e} vs the mma.sync form; "
+    print(f"{name} decode B={B}, tcgen05 pipeline: logits relmax {err:.2e} vs oracle, {both:.2e} vs the mma.sync form; "
           f"launcher's choice {own:.2e} vs oracle")
     assert np.isfinite(got[1]).all() and err <= TOL, err
     assert both <= 2e-4, both
     assert np.isfinite(got[-1]).all() and own <= TOL, own
-    if B == 40:
-        assert np.array_equal(got[-1], got[1])
+    assert np.array_equal(got[-1], got[1])
 
 
 def test_full_depth_decode_and_prefill(tmp_path, cuda_lib):

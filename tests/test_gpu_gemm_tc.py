@@ -1,4 +1,4 @@
-"""Dequant-fused tcgen05 GEMM (rwkvq_gemm) against the oracle.
+"""Many-row tcgen05 GEMM (rwkvq_gemm: weights to fp16 once, then TMA + tcgen05) against the oracle.
 
 Operands are fp16 (weights fp16(q*s+m), tokens scaled per row by a power of two) with
 fp32 accumulation in tensor memory, so the bar is the reference's own GEMM-path gate:
@@ -55,9 +55,9 @@ def test_gemm_tc_epilogues_and_determinism(cuda_lib):
 
 
 @pytest.fixture
-def two_accumulators(cuda_lib):
-    """256-row tiles (two accumulators per activation slab) wherever the shape allows: the
-    launcher takes them by itself only once they fill the SMs (row tiles x token tiles >= 148)."""
+def pair_tiles(cuda_lib):
+    """CTA pairs (256 x 256 tiles) whatever the shape; the launcher takes them by itself once they fill the chip.  They are
+    legal where K has at most 4096 columns or 16 tiles share the work."""
     import ctypes as C
     f = cuda_lib.rwkvq_profiling_gemm_acc_mode          # rwkvq_profiling.h: not part of the C ABI
     f.restype, f.argtypes = None, [C.c_int]
@@ -67,11 +67,10 @@ def two_accumulators(cuda_lib):
 
 
 @pytest.mark.parametrize("layout,bits", [("sb6", 4), ("sb6", 5), ("sb6", 6), ("sym", 6), ("sym", 8)])
-@pytest.mark.parametrize("rows,cols,M", [(256, 256, 129), (512, 1024, 300), (2048, 2048, 520), (256, 8192, 256)])
-def test_gemm_tc_two_accumulator_tiles(cuda_lib, two_accumulators, layout, bits, rows, cols, M):
-    """Same bar as the one-accumulator form, bit-equal to it (the same MMAs in the same order per
-    output element), on shapes with one CTA, a K split (few tiles, long K) and a ragged token tile;
-    the epilogues go through both accumulators."""
+@pytest.mark.parametrize("rows,cols,M", [(256, 256, 129), (512, 1024, 300), (2048, 2048, 520), (256, 4096, 256), (1100, 8192, 1000)])
+def test_gemm_tc_cta_pairs(cuda_lib, pair_tiles, layout, bits, rows, cols, M):
+    """Same bar as the single-CTA tiles and equal to them up to the order of a K split, on shapes with one tile, several waves'
+    worth of K, ragged rows and a ragged token tile; every epilogue."""
     from rwkv_quant_b200.backends.cuda import ops
     qt = _synth_linear(layout, bits, rows, cols, seed=rows + cols + M + 1)
     dq = ops.DeviceQT(qt)
@@ -86,9 +85,10 @@ def test_gemm_tc_two_accumulator_tiles(cuda_lib, two_accumulators, layout, bits,
     resid = torch.randn(M, rows, device="cuda")
     r2 = ops.gemm(dq, xt, 2, resid, check=True)
     q2 = ops.gemm(dq, xt, 1, None, check=True)
-    two_accumulators(1)                                  # the same call on 128-row tiles
+    pair_tiles(1)                                        # the same call on single-CTA tiles
     y1 = ops.gemm(dq, xt, 0, None, check=True)
-    two_accumulators(2)
+    pair_tiles(2)
     assert torch.equal(r2, y2 + resid) and torch.equal(q2, torch.relu(y2) ** 2)
-    assert relmax(y2.cpu().numpy(), y1.cpu().numpy()) <= 1e-6
-    print(f"{layout}{bits} [{rows},{cols}] M={M} (256-row tiles): worst row relmax {per_row.max():.2e}")
+    # one tile's chain is K / 16 accumulations, each rounded to 2^-24 of its partial sum; a split shortens it
+    assert relmax(y2.cpu().numpy(), y1.cpu().numpy()) <= max(1e-6, cols / 16 * 2.0 ** -24)
+    print(f"{layout}{bits} [{rows},{cols}] M={M} (CTA pairs): worst row relmax {per_row.max():.2e}")

@@ -1,7 +1,11 @@
 """The one-call sequence forward and the one-stream decode step where their splits can go wrong: rows on each side of the
-small-batch, tcgen05 and fp16-GEMM ranges, tokens on each side of a chunk of 16, heads on each side of a half and a whole
-wave, and widths with a ragged last group of the LoRA and LayerNorm threads.  Reference: the package's own per-operator
-sequence path, which the oracle tests cover."""
+small-batch, tcgen05 and fp16-GEMM ranges, tokens on each side of the shortest chunked call and of a chunk of 8, heads on
+each side of a half and a whole wave (one form of the scan each), and widths with a ragged last group of the LoRA and
+LayerNorm threads.  Reference: the CPU oracle for the calls, the package's per-operator path for the steps.
+
+Tolerances (of the largest value): calls of up to 64 rows and single steps are fp32 grade, some 1e-6 a linear and 2e-5
+through two layers: 1e-4, a third of what one dropped half of an operand pair costs; longer calls have fp16 operands,
+2^-11 a value and some 5e-4 through two layers: 1e-3."""
 import pytest
 import torch
 
@@ -10,10 +14,14 @@ from helpers import relmax
 pytestmark = pytest.mark.gpu
 
 
-def _model(recipe, **dims):
+def _checkpoint(recipe, **dims):
     from rwkv_quant_b200 import synth
+    return synth.build_checkpoint(dict(n_layer=2, vocab=512, **dims), recipe, seed=3, device="cuda", keep_on_device=False)
+
+
+def _model(recipe, **dims):
     from rwkv_quant_b200.backends.cuda import QuantRWKV7
-    return QuantRWKV7(synth.build_checkpoint(dict(n_layer=2, vocab=512, **dims), recipe, seed=3, device="cuda"), device="cuda")
+    return QuantRWKV7(_checkpoint(recipe, **dims), device="cuda")
 
 
 def _states(model, B):
@@ -23,22 +31,50 @@ def _states(model, B):
     return [(draw(B, H, 64, 64), draw(B, 1, D), draw(B, 1, D)) for _ in range(model.n_layer)]
 
 
-def _same(a, b):
-    assert relmax(a[0].cpu().numpy(), b[0].cpu().numpy()) <= 1e-3
+def _same(a, b, tol):
+    n = lambda t: t.cpu().numpy() if isinstance(t, torch.Tensor) else t
+    assert relmax(n(a[0]), n(b[0])) <= tol
     for sa, sb in zip(a[1], b[1]):
         for x, y in zip(sa, sb):
-            assert relmax(x.cpu().numpy(), y.cpu().numpy()) <= 1e-3
+            assert relmax(n(x), n(y).reshape(tuple(x.shape))) <= tol
 
 
 @pytest.mark.parametrize("recipe", ["compression", "reduction"])
-@pytest.mark.parametrize("B,T", [(1, 16), (1, 17), (2, 32), (1, 65), (5, 16), (4, 17), (3, 31), (19, 15), (37, 33)])
-def test_forward_call_matches_separate_passes(cuda_lib, recipe, B, T):
-    model = _model(recipe, n_embd=256, ffn=1024)
-    idx = torch.randint(1, 512, (B, T), generator=torch.Generator().manual_seed(B * 100 + T)).cuda()
-    st = _states(model, B)
-    one = model.forward_stateful(idx, st)
+def test_forward_calls_match_the_oracle(cuda_lib, tmp_path, recipe):
+    from oracle import codec_np as oc
+    from oracle.model_np import OracleRWKV7
+    from rwkv_quant_b200.backends.cuda import QuantRWKV7
+    from rwkv_quant_b200.formats import save_rwkvq
+    ck = _checkpoint(recipe, n_embd=256, ffn=1024)
+    save_rwkvq(ck, str(tmp_path / "m.rwkvq"))
+    model, oracle = QuantRWKV7(ck, device="cuda"), OracleRWKV7(*oc.open_rwkvq(str(tmp_path / "m.rwkvq")))
+    for B, T in [(1, 2), (1, 16), (1, 17), (2, 32), (1, 65), (5, 15), (5, 16), (4, 17), (3, 23), (3, 24), (3, 25), (3, 31), (19, 15),
+                 (18, 17), (19, 17), (37, 33), (38, 33)]:
+        idx = torch.randint(1, 512, (B, T), generator=torch.Generator().manual_seed(B * 100 + T))
+        st = _states(model, B)
+        got = model.forward_stateful(idx.cuda(), st)
+        model.check()
+        ref = oracle.forward_stateful(idx.numpy(), [tuple(t.cpu().numpy() for t in s) for s in st])
+        _same(got, ref, 1e-4 if B * T <= 64 else 1e-3)
+
+
+def test_hidden_rows_far_below_their_bound(cuda_lib):
+    """The channel mix of long calls scales its fp16 hidden rows by a bound on |W||x| instead of by their own maximum.  One row
+    of W 2^9 times the others: tokens whose product with it is negative keep hidden rows some 2^11 below the bound (2^22
+    squared), and lose nothing against the per-operator path, which scales by the maximum."""
+    ck = _checkpoint("compression", n_embd=256, ffn=1024)
+    for layer in (0, 1):
+        t = ck.tensors[f"blocks.{layer}.ffn.key.weight"]
+        t.gw_d[7] *= 2.0 ** 9
+        t.gw_dm[7] *= 2.0 ** 9
+    from rwkv_quant_b200.backends.cuda import QuantRWKV7
+    model = QuantRWKV7(ck, device="cuda")
+    idx = torch.randint(1, 512, (3, 40), generator=torch.Generator().manual_seed(1)).cuda()
+    got, _ = model.forward_stateful(idx, _states(model, 3))
     model.fused_prep = False
-    _same(one, model.forward_stateful(idx, st))
+    ref, _ = model.forward_stateful(idx, _states(model, 3))
+    err = (got - ref).abs().amax(-1) / ref.abs().amax(-1)
+    assert err.max() <= 2e-3 and err.median() <= 1e-3, (err.max(), err.median())
 
 
 @pytest.mark.parametrize("recipe,D,F", [("compression", 256, 1024), ("reduction", 1280, 8192), ("compression_eh8", 2560, 10240),
@@ -54,4 +90,4 @@ def test_one_stream_steps_match_the_sequence(cuda_lib, recipe, D, F):
         steps.append(dec.logits.clone())
     model.fused_prep = False
     ref, _ = model.forward_stateful(idx, st)
-    assert relmax(torch.stack(steps, 1).cpu().numpy(), ref.cpu().numpy()) <= 1e-3
+    assert relmax(torch.stack(steps, 1).cpu().numpy(), ref.cpu().numpy()) <= 1e-4
