@@ -318,7 +318,12 @@ __global__ void __launch_bounds__(kBtThreads, 2) gemv_batch_kernel(const BatchAr
                         (resid == nullptr || (reinterpret_cast<uintptr_t>(resid) & 15) == 0);
 
     // the staged iterations [0, cits) of one tile: c += W x
-    auto run_its = [&](int tile, int cits, float (&c)[NT][4]) {
+    // d: the terms with a low half, up to 8 tokens.  The tensor cores truncate an accumulator at every step, so a sum that
+    // shares its chain with them loses three units in place of one: c gets one step per 16 columns (two streams, error of the
+    // logits against 64 bits 1.22e-5 -> 5.6e-6; the single-vector kernels 6.8e-6).  With two tiles the accumulators spill: 13
+    // streams 1.90 -> 1.94 ms.
+    constexpr bool LOW = EX && NT == 1;
+    auto run_its = [&](int tile, int cits, float (&c)[NT][4], float (&d)[4]) {
         for (int il = 0; il < cits; ++il) {
             const Frag<L> cur = nxt;
             fetch_next();
@@ -354,8 +359,8 @@ __global__ void __launch_bounds__(kBtThreads, 2) gemv_batch_kernel(const BatchAr
 #pragma unroll
                             for (int nt = 0; nt < NT; ++nt) {
                                 const uint4 b = *reinterpret_cast<const uint4*>(xp + nt * 512);     // hi (x, y), lo (z, w)
-                                mma_f16(c[nt], e0, e1, e2, e3, b.x, b.y);       // small terms first
-                                mma_f16(c[nt], a0, a1, a2, a3, b.z, b.w);
+                                mma_f16(LOW ? d : c[nt], e0, e1, e2, e3, b.x, b.y);
+                                mma_f16(LOW ? d : c[nt], a0, a1, a2, a3, b.z, b.w);
                                 mma_f16(c[nt], a0, a1, a2, a3, b.x, b.y);
                             }
                         }
@@ -368,7 +373,7 @@ __global__ void __launch_bounds__(kBtThreads, 2) gemv_batch_kernel(const BatchAr
                     for (int nt = 0; nt < NT; ++nt) {
                         const uint32_t bh = *reinterpret_cast<const uint32_t*>(sp + nt * 256);
                         const uint32_t bl = *reinterpret_cast<const uint32_t*>(sp + nt * 256 + 16);
-                        mma_f16(c[nt], m0, m1, 0u, 0u, bl, 0u);
+                        mma_f16(LOW ? d : c[nt], m0, m1, 0u, 0u, bl, 0u);
                         mma_f16(c[nt], m0, m1, 0u, 0u, bh, 0u);
                     }
                 }
@@ -411,9 +416,18 @@ __global__ void __launch_bounds__(kBtThreads, 2) gemv_batch_kernel(const BatchAr
             }
         }
     };
+    auto clear = [](float (&c)[NT][4], float (&d)[4]) {
+#pragma unroll
+        for (int i = 0; i < NT; ++i) c[i][0] = c[i][1] = c[i][2] = c[i][3] = 0.f;
+        d[0] = d[1] = d[2] = d[3] = 0.f;
+    };
     // undo the token scales and leave the tile for the reduction
-    auto put_part = [&](int ti, const float (&c)[NT][4]) {
+    auto put_part = [&](int ti, float (&c)[NT][4], const float (&d)[4]) {
         const int r = (warp + ti * kBtWarps) * 16 + g;
+        if (LOW) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) c[0][k] += d[k];
+        }
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
             const int n = nt * 8 + 2 * t;
@@ -428,23 +442,21 @@ __global__ void __launch_bounds__(kBtThreads, 2) gemv_batch_kernel(const BatchAr
     for (int rg = cid; rg < n_rg; rg += n_clusters) {
         if (n_chunks == 1) {
             for (int ti = 0; ti < my_tiles; ++ti) {
-                float c[NT][4];
-#pragma unroll
-                for (int i = 0; i < NT; ++i) c[i][0] = c[i][1] = c[i][2] = c[i][3] = 0.f;
-                run_its(rg * tpc + warp + ti * kBtWarps, a.its_per_cta, c);
-                put_part(ti, c);
+                float c[NT][4], d[4];
+                clear(c, d);
+                run_its(rg * tpc + warp + ti * kBtWarps, a.its_per_cta, c, d);
+                put_part(ti, c, d);
             }
         } else {
-            float c[NT][4];
-#pragma unroll
-            for (int i = 0; i < NT; ++i) c[i][0] = c[i][1] = c[i][2] = c[i][3] = 0.f;
+            float c[NT][4], d[4];
+            clear(c, d);
             for (int ch = 0; ch < n_chunks; ++ch) {
                 __syncthreads();                   // everyone is done with the chunk staged before
                 stage(ch);
                 __syncthreads();
-                run_its(rg * tpc + warp, min(a.chunk_its, a.its_per_cta - ch * a.chunk_its), c);
+                run_its(rg * tpc + warp, min(a.chunk_its, a.its_per_cta - ch * a.chunk_its), c, d);
             }
-            put_part(0, c);
+            put_part(0, c, d);
         }
         if (rg == cid) bt_mark(a, 3);
         cluster.sync();

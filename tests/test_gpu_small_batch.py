@@ -40,3 +40,18 @@ def test_token_tiles_and_k_splits(cuda_lib, layout, bits, rows, cols, ks):
                     y.fill_(float("nan"))
     finally:
         force(0)
+
+
+@pytest.mark.parametrize("N", [2, 8, 17, 64, 128])
+def test_error_of_a_long_chain(cuda_lib, N):
+    """Rows without a K split: 2048 columns are 128 steps of an accumulator that the tensor cores truncate, 2^-24 of the
+    partial sum on average at the end of the chain and half of that over it.  The terms with a low half stay out of that chain
+    (with them in it there are two to three times the steps)."""
+    from rwkv_quant_b200 import synth
+    from rwkv_quant_b200.backends.cuda import ops
+    gen = torch.Generator(device="cuda").manual_seed(N)
+    dq = ops.DeviceQT(synth.quant_sym("w", "proj", 0.02 * torch.randn(65536, 2048, generator=gen, device="cuda"), 8))
+    x = torch.randn(N, 2048, generator=gen, device="cuda")
+    want = x.double() @ dq.dequant().double().t()
+    err = (ops.gemv_batch(dq, x, check=True).double() - want).norm() / want.norm()
+    assert err <= 128 * 2.0 ** -25, float(err)
