@@ -305,8 +305,8 @@ def has_batch_layout(dq: "DeviceQT") -> bool:
 
 def gemv_batch(dq: "DeviceQT", x: torch.Tensor, epilogue: int = 0, resid: Optional[torch.Tensor] = None,
                check: bool = False) -> torch.Tensor:
-    """x [N, IN] -> y [N, OUT] fp32 with the packed weights read once for all N rows (mma.sync
-    tensor cores, tokens as the MMA columns, fp16 operands, fp32 accumulation)."""
+    """x [N, IN] -> y [N, OUT] fp32 with the packed weights read once for up to 128 rows: tokens as the MMA columns, both
+    operands as fp16 pairs, fp32 accumulation (mma.sync up to 16 rows, the tcgen05 pipeline above)."""
     _require_cuda(dq.bufs[0], x, resid)
     lib = _lib.load()
     x = x.float()
@@ -351,8 +351,8 @@ def lora_pair(pairs, xs: Sequence[torch.Tensor], acts: Sequence[int]) -> List[to
 
 def gemm(dq: "DeviceQT", x: torch.Tensor, epilogue: int = 0, resid: Optional[torch.Tensor] = None,
          check: bool = False) -> torch.Tensor:
-    """x [M, IN] fp32 -> y [M, OUT] fp32 on the tcgen05 tensor cores with the dequantisation
-    fused into the operand producer (sb6 / sym tensors).  ``check`` synchronises and raises
+    """x [M, IN] fp32 -> y [M, OUT] fp32 on the tcgen05 tensor cores, the weights converted to fp16
+    once per call in chunks that stay in L2 (sb6 / sym tensors).  ``check`` synchronises and raises
     if the kernel reported that a bounded pipeline wait ran out."""
     _require_cuda(dq.bufs[0], x, resid)
     lib = _lib.load()

@@ -203,7 +203,7 @@ class QuantRWKV7:
     # ------------------------------------------------------------------ T > 1
     def _linear(self, dq, x, epilogue=_lib.EPI_NONE, resid=None):
         """x [N, IN] fp32 -> [N, OUT].  Up to ``gemv_max_batch`` rows: the exact
-        weight-streaming GEMV per row; more rows: the dequant-fused tensor-core GEMM
+        weight-streaming GEMV per row; more rows: the fp16 tensor-core GEMM
         (sb6 / sym); other layouts at large N: dequantise once + dense fp32 GEMM."""
         if x.shape[0] <= self.gemv_max_batch:
             return ops.gemv(dq.bufs, dq.meta, x, epilogue, resid)
@@ -259,7 +259,7 @@ class QuantRWKV7:
 
     def _prep_modes(self, N, lins):
         """Which form each mix row is written in: the scaled fp16 copy when its linear runs on
-        the dequant-fused GEMM, else fp32."""
+        the fp16 GEMM, else fp32."""
         gemm = lambda dq: dq.kind in ("sb6", "sym") and N > max(self.gemv_max_batch, self.batch_max)
         return [ops.PREP_SCALED if gemm(dq) else ops.PREP_F32 for dq in lins]
 

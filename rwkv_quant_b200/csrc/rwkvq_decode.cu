@@ -165,9 +165,8 @@ __global__ void __launch_bounds__(kRowThreads) embed_ln0_kernel(QView emb, const
 
 // xn = LN(x[b]); prev = shift[b] (zeros for a fresh stream); shift[b] = xn;
 // out[m][b] = xn + (prev - xn) * mix[m]   for m < n_mix   (n_mix = 0: out[0][b] = xn)
-// All loads are issued before the reductions so that their latencies overlap.  PER: elements per
-// thread (8 serves D <= 2048 and leaves registers for the lerp vectors, which are then loaded with the
-// LayerNorm parameters before the launch wait; 16 serves D <= 4096 and reads them where they are used).
+// All loads are issued before the reductions so that their latencies overlap.  PER: elements per thread (16: D <= 4096).
+// For rows the vector form below cannot read: odd widths, rows off a 16-byte boundary.
 template <int NMIX, int PER>
 __global__ void __launch_bounds__(kRowThreads) ln_shift_mix_kernel(const float* __restrict__ x,
                                                                   const float* __restrict__ ln_w,
@@ -825,13 +824,16 @@ constexpr int kBatchMax = 256;     // streams up to which the small-batch kernel
 // (two streams: 1.60 ms per step of the 1.5B model against 1.82 on one single-vector launch per stream, 2.9B 2.79 / 3.81)
 // with single-term operands from three on: two streams keep the single-vector kernels' precision in every mode
 inline bool batch_path(int B) { return B > (batch_fast() ? 2 : 1) && B <= kBatchMax; }
-// Which small-batch kernel: measured on B200 (1.5B, whole decode step) the tcgen05 form wins from 33
-// streams on (64 streams: 3.77 against 4.43 ms per step) and loses below (32: 2.87 / 2.68 ms, 8: 2.42 / 2.01 ms):
-// its pass (dependent weight loads -> conversion -> MMA) is longer than a warp-iteration of the mma.sync form
+// Single-term operands (RWKVQ_BATCH_FAST=1): the tcgen05 form wins over the mma.sync one from 33 streams on (1.5B, whole
+// step, 64 streams: 3.77 against 4.43 ms) and loses below (32: 2.87 / 2.68 ms, 8: 2.42 / 2.01): its pass (dependent weight
+// loads -> conversion -> MMA) is longer than a warp-iteration.  The default precision is faster from 17 streams on (64: 2.80
+// ms); the mode pays below.
 inline bool tcb_pays(int B) { return batch_fast() && tcb_enabled() && B > 32; }
 // Default (two-term) precision: from kSbMinStreams streams on every linear of the step runs on the tcgen05 pipeline
 // (rwkvq_gemm_sb.cu), fed with fp16 pairs and block sums by the LayerNorm kernels and, for the output projection and the
-// ffn value, by a pass over the fp32 rows.  Below, the mma.sync form: few tokens give its 3 MMAs per step little to do.
+// ffn value, by a pass over the fp32 rows.  Below, the mma.sync form: few tokens give its 3 MMAs per step little to do.  The
+// line is the mma.sync kernel's second tile of 16 tokens, which doubles its time; at 16 the two are within a few per cent (ms,
+// mma.sync / pipeline: 1.5B sb6 1.92 / 1.90, sym 1.92 / 2.10, 2.9B 3.63 / 3.63 and 3.45 / 3.32), at 4 mma.sync is ahead (1.63 / 1.80).
 // RWKVQ_TCB_EXACT in the environment (read once) overrides: 0 never, 1 at every batch.
 constexpr int kSbMinStreams = 17;
 int g_tcb_exact = -2;          // -2 environment not read yet, -1 by stream count, 0 never, 1 always
@@ -927,7 +929,6 @@ Workspace carve(const rwkvq_model& m, int B, void* base) {
     return w;
 }
 
-// y_br = (act_br(x_br @ W1_br)) @ W2_br for up to 4 branches, B right-hand sides
 // One quantized linear for B right-hand sides; the single-vector tensor-core kernel gets
 // the K split, everything else goes through the public entry point.
 // x16 / x_scale: the fp16 form of x with its per-row scale inverses (what the LayerNorm kernels write
@@ -977,6 +978,7 @@ int launch_tmix_core_up(const TmixCoreArgs& tc, const LoraVecArgs& up, int H, cu
 
 int lora_rep(int B) { return B > kLmMaxN ? 8 : 1; }
 
+// y_br = (act_br(x_br @ W1_br)) @ W2_br for up to 4 branches, B right-hand sides
 int lora_pair(const rwkvq_qtensor* const* t1, const rwkvq_qtensor* const* t2, const float* const* xs,
               float* const* ys, const int* acts, int n_br, int B, int D, int max_rank, float* part,
               size_t part_floats, int n_chunks, cudaStream_t s) {
@@ -1148,77 +1150,77 @@ int rwkvq_decode_step(const rwkvq_model* m, int B, const int64_t* tokens, float*
             rc = launch_tmix_core_up(tc, up, H, s);
             if (rc) return rc;
         } else {
-        SideLane* lane = side_lane(s);
-        Fork fork{lane, s};
-        cudaStream_t s_lora = s;
-        if (lane) {                                  // fork: the LoRA branches leave the chain here
-            rc = fork.start();
-            if (rc) return rc;
-            s_lora = lane->stream;
-        }
-        // Up to 16 streams the LoRA pair (two dependent launches) is the longer of the two branches: it then
-        // stays on the caller's stream, where its first kernel starts programmatically behind the LayerNorm
-        // and stages its weights while that still runs, and r / k / v take the side stream.  So it does beside the tcgen05
-        // pipeline at any stream count: that leaves some 50 SMs for the second LoRA launch, but none of its CTAs
-        // shares an SM with the first (64 streams: 17 + 11 + 6 us in the other order, 13 + 16 in this).
-        cudaStream_t s_rkv = s;
-        if (lane && (B <= 16 || sb)) { s_rkv = lane->stream; s_lora = s; }
-        auto lora = [&]() {
-            float* y2[4] = {yw, ya, yg, yv};
-            return lora_pair(t1, t2, x1, y2, act, n_br, B, D, m->max_rank, w.part, w.part_floats, w.n_chunks, s_lora);
-        };
-        if (sb) {                                  // first in the graph too: 64 streams 2.88 -> 2.81 ms (13 on mma.sync lose 1%)
-            rc = lora();
-            if (rc) return rc;
-        }
-        if (B == 1 && ml >= 0 && mma_layout_of(L.Wk) == ml && mma_layout_of(L.Wv) == ml && L.Wk.rows == D &&
-            L.Wv.rows == D && L.Wr.rows == D && L.Wk.cols == D && L.Wv.cols == D && L.Wr.cols == D) {
-            // r, k, v in one launch: three matrices, three inputs (rows 0, 2, 3 of xs)
-            for (const rwkvq_qtensor* t : {&L.Wr, &L.Wk, &L.Wv}) {
-                rc = validate_qtensor(t, "rwkvq_decode_step(r/k/v)");
+            SideLane* lane = side_lane(s);
+            Fork fork{lane, s};
+            cudaStream_t s_lora = s;
+            if (lane) {                                  // fork: the LoRA branches leave the chain here
+                rc = fork.start();
+                if (rc) return rc;
+                s_lora = lane->stream;
+            }
+            // Up to 16 streams the LoRA pair (two dependent launches) is the longer of the two branches: it then
+            // stays on the caller's stream, where its first kernel starts programmatically behind the LayerNorm
+            // and stages its weights while that still runs, and r / k / v take the side stream.  So it does beside the tcgen05
+            // pipeline at any stream count: that leaves some 50 SMs for the second LoRA launch, but none of its CTAs
+            // shares an SM with the first (64 streams: 17 + 11 + 6 us in the other order, 13 + 16 in this).
+            cudaStream_t s_rkv = s;
+            if (lane && (B <= 16 || sb)) { s_rkv = lane->stream; s_lora = s; }
+            auto lora = [&]() {
+                float* y2[4] = {yw, ya, yg, yv};
+                return lora_pair(t1, t2, x1, y2, act, n_br, B, D, m->max_rank, w.part, w.part_floats, w.n_chunks, s_lora);
+            };
+            if (sb) {                                  // first in the graph too: 64 streams 2.88 -> 2.81 ms (13 on mma.sync lose 1%)
+                rc = lora();
                 if (rc) return rc;
             }
-            const rwkvq_qtensor three[3] = {L.Wr, L.Wk, L.Wv};
-            const void* x_each[3] = {xr, xk, xv};
-            rc = launch_gemv_mma(ml, three, 3, xr, RWKVQ_F32, D, r, D, RWKVQ_EPI_NONE, nullptr, 1, s_rkv, x_each, true);
-            if (rc) return rc;
-        } else if (sb) {
-            const rwkvq_qtensor three[3] = {L.Wr, L.Wk, L.Wv};
-            float* y3[3] = {r, k, v};
-            rc = launch_gemm_sb(three, 3, w.rkv_pair, B, y3, D, RWKVQ_EPI_NONE, nullptr, nullptr, w.status, 0, s_rkv);
-            if (rc) return rc;
-        } else if (bp && rkv_fused) {
-            for (const rwkvq_qtensor* t : {&L.Wr, &L.Wk, &L.Wv}) {
-                rc = validate_qtensor(t, "rwkvq_decode_step(r/k/v)");
+            if (B == 1 && ml >= 0 && mma_layout_of(L.Wk) == ml && mma_layout_of(L.Wv) == ml && L.Wk.rows == D &&
+                L.Wv.rows == D && L.Wr.rows == D && L.Wk.cols == D && L.Wv.cols == D && L.Wr.cols == D) {
+                // r, k, v in one launch: three matrices, three inputs (rows 0, 2, 3 of xs)
+                for (const rwkvq_qtensor* t : {&L.Wr, &L.Wk, &L.Wv}) {
+                    rc = validate_qtensor(t, "rwkvq_decode_step(r/k/v)");
+                    if (rc) return rc;
+                }
+                const rwkvq_qtensor three[3] = {L.Wr, L.Wk, L.Wv};
+                const void* x_each[3] = {xr, xk, xv};
+                rc = launch_gemv_mma(ml, three, 3, xr, RWKVQ_F32, D, r, D, RWKVQ_EPI_NONE, nullptr, 1, s_rkv, x_each, true);
+                if (rc) return rc;
+            } else if (sb) {
+                const rwkvq_qtensor three[3] = {L.Wr, L.Wk, L.Wv};
+                float* y3[3] = {r, k, v};
+                rc = launch_gemm_sb(three, 3, w.rkv_pair, B, y3, D, RWKVQ_EPI_NONE, nullptr, nullptr, w.status, 0, s_rkv);
+                if (rc) return rc;
+            } else if (bp && rkv_fused) {
+                for (const rwkvq_qtensor* t : {&L.Wr, &L.Wk, &L.Wv}) {
+                    rc = validate_qtensor(t, "rwkvq_decode_step(r/k/v)");
+                    if (rc) return rc;
+                }
+                const rwkvq_qtensor three[3] = {L.Wr, L.Wk, L.Wv};
+                const void* x3[3] = {w.xs16, w.xs16 + 2 * BD, w.xs16 + 3 * BD};
+                if (!h16) { x3[0] = xr; x3[1] = xk; x3[2] = xv; }
+                const float* a3[3] = {am, am + 2 * B, am + 3 * B};
+                float* y3[3] = {r, k, v};
+                if (tcb_pays(B) && gemm_tcb_ok(L.Wr))
+                    rc = launch_gemm_tcb(three, 3, x3, h16, a3, B, D, y3, D, RWKVQ_EPI_NONE, nullptr, nullptr, w.status, s_rkv);
+                else
+                    rc = launch_gemv_batch(three, 3, x3, h16, a3, B, D, y3, D, RWKVQ_EPI_NONE, nullptr, nullptr, s_rkv);
+                if (rc) return rc;
+            } else {
+                rc = linear(&L.Wr, xr, B, D, r, D, RWKVQ_EPI_NONE, nullptr, w.gemm_ws, s_rkv, h16 ? w.xs16 : nullptr, am, nullptr, w.status);
+                if (rc) return rc;
+                rc = linear(&L.Wk, xk, B, D, k, D, RWKVQ_EPI_NONE, nullptr, w.gemm_ws, s_rkv,
+                            h16 ? w.xs16 + 2 * BD : nullptr, bp ? am + 2 * B : nullptr, nullptr, w.status);
+                if (rc) return rc;
+                rc = linear(&L.Wv, xv, B, D, v, D, RWKVQ_EPI_NONE, nullptr, w.gemm_ws, s_rkv,
+                            h16 ? w.xs16 + 3 * BD : nullptr, bp ? am + 3 * B : nullptr, nullptr, w.status);
                 if (rc) return rc;
             }
-            const rwkvq_qtensor three[3] = {L.Wr, L.Wk, L.Wv};
-            const void* x3[3] = {w.xs16, w.xs16 + 2 * BD, w.xs16 + 3 * BD};
-            if (!h16) { x3[0] = xr; x3[1] = xk; x3[2] = xv; }
-            const float* a3[3] = {am, am + 2 * B, am + 3 * B};
-            float* y3[3] = {r, k, v};
-            if (tcb_pays(B) && gemm_tcb_ok(L.Wr))
-                rc = launch_gemm_tcb(three, 3, x3, h16, a3, B, D, y3, D, RWKVQ_EPI_NONE, nullptr, nullptr, w.status, s_rkv);
-            else
-                rc = launch_gemv_batch(three, 3, x3, h16, a3, B, D, y3, D, RWKVQ_EPI_NONE, nullptr, nullptr, s_rkv);
+            if (!sb) {
+                rc = lora();
+                if (rc) return rc;
+            }
+            rc = fork.join();                            // before the time-mix core
             if (rc) return rc;
-        } else {
-            rc = linear(&L.Wr, xr, B, D, r, D, RWKVQ_EPI_NONE, nullptr, w.gemm_ws, s_rkv, h16 ? w.xs16 : nullptr, am, nullptr, w.status);
-            if (rc) return rc;
-            rc = linear(&L.Wk, xk, B, D, k, D, RWKVQ_EPI_NONE, nullptr, w.gemm_ws, s_rkv,
-                        h16 ? w.xs16 + 2 * BD : nullptr, bp ? am + 2 * B : nullptr, nullptr, w.status);
-            if (rc) return rc;
-            rc = linear(&L.Wv, xv, B, D, v, D, RWKVQ_EPI_NONE, nullptr, w.gemm_ws, s_rkv,
-                        h16 ? w.xs16 + 3 * BD : nullptr, bp ? am + 3 * B : nullptr, nullptr, w.status);
-            if (rc) return rc;
-        }
-        if (!sb) {
-            rc = lora();
-            if (rc) return rc;
-        }
-        rc = fork.join();                            // before the time-mix core
-        if (rc) return rc;
-        launch_pdl(tmix_core_kernel<false>, dim3(H, B), dim3(256), 0, s, tc, 0);
+            launch_pdl(tmix_core_kernel<false>, dim3(H, B), dim3(256), 0, s, tc, 0);
         }
         if (sb) {
             const float* res[1] = {w.x};

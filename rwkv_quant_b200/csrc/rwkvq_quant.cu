@@ -16,8 +16,8 @@
 //   per super-block  d = fp16(max s / 63), qs = clamp(rint(s / d), 1, 63), dm = fp16(max|m| / 31),
 //                  qm = clamp(rint(m / dm), -31, 31); s' = max(fp16(qs d), 1e-8), m' = fp16(qm dm)
 //   per weight     q = clamp(rint((w - m') / s'), 0, qmax)
-// All in fp32 with IEEE division and round-half-to-even, like the torch code.  The sums run as
-// shuffle trees, torch's in its own order: (s, m) agree to their last bits, so a code can differ
+// All in fp32 with IEEE division and round-half-to-even, like the torch code.  The sums run in the
+// order above, torch's in its own: (s, m) agree to their last bits, so a code can differ
 // where a quotient sits within an ulp of a rounding boundary or two factors tie (measured: 3 codes
 // per million against tensors packed by the reference).
 #include <cuda_fp16.h>

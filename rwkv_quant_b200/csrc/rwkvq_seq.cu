@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(kSeqThreads) seq_ln_shift_mix_kernel(const flo
 }
 
 // ---- the same, emitting what the consumers of each mix read ---------------------------------
-// A mix row feeds either the dequant-fused GEMM (which reads a per-token power-of-two-scaled
+// A mix row feeds either the fp16 GEMM (which reads a per-token power-of-two-scaled
 // fp16 copy, pitch D + 64 halves, plus the scale) or the LoRA GEMM (which reads the fp16 hi/lo
 // split [hi | lo]), or both; writing those forms here saves the fp32 round trip through HBM and
 // one launch per consumer.  The conversions are those of the GEMM's own pre-pass (scale =
