@@ -229,8 +229,9 @@ def linear_phase(model, B, steps, warmup):
 
 
 # dram__bytes_read.sum + dram__bytes_write.sum of the quantized-linear launches of one decoded token
-# (1.5B compression, one stream), from the ncu capture summarised under profiles/
-NCU_GEMV_PHASE_DRAM_BYTES_B1 = 828225280 + 342272
+# (1.5B compression, one stream), from the ncu capture summarised under profiles/; 26.6 MB of them are the LoRA down
+# matrices, which share the r / k / v launch of a step and are not part of the launches timed here
+NCU_GEMV_PHASE_DRAM_BYTES_B1 = 856284928 + 68864 - 26591232
 
 
 def kernel_name(B, fast):
