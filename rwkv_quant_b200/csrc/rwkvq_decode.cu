@@ -780,7 +780,7 @@ __global__ void __launch_bounds__(kArgSlices) argmax_final_kernel(const float* p
 // RWKVQ_FORK=0 keeps everything on the caller's stream.
 SideLane* side_lane(cudaStream_t caller) {
     static const bool enabled = [] { const char* e = getenv("RWKVQ_FORK"); return !(e && e[0] == '0'); }();
-    if (!enabled) return nullptr;
+    if (!enabled || caller == cudaStreamPerThread) return nullptr;      // one handle for a stream of every thread: their forks would mix
     static std::mutex mu;
     static std::map<std::pair<int, cudaStream_t>, SideLane> lanes;
     int dev = 0;
