@@ -35,11 +35,14 @@ class _QuantLinearBase:
         x2, lead = ops.as_rows(x, self.in_features)
         if resid is not None:
             resid = resid.reshape(-1, self.out_features).contiguous()
-        if x2.shape[0] >= GEMM_MIN_BATCH_NB and self.dq.kind in ("sb6", "sym"):
+        n = x2.shape[0]
+        if n <= GEMV_MAX_BATCH:
+            y = self.dq.gemv(x2, epilogue, resid)
+        elif n >= GEMM_MIN_BATCH_NB and self.dq.kind in ("sb6", "sym"):
             # the reference's crossover (quant_linear_gw.py:846-849, quant_linear_sym.py:481-484):
             # its dequant + fp16 matmul; here chunk by chunk inside one call
             y = ops.gemm(self.dq, x2, epilogue, resid)
-        elif x2.shape[0] > GEMV_MAX_BATCH and ops.has_batch_layout(self.dq):
+        elif ops.has_batch_layout(self.dq):
             # the reference decodes each weight once per chunk of 4 columns (_gemv_nb,
             # quant_linear_gw.py:850-905); here once per 16 columns, from 17 on per 128
             y = ops.gemv_batch(self.dq, x2, epilogue, resid)
