@@ -122,3 +122,28 @@ def test_quantize_sym_matches_oracle(cuda_lib, bits, mode):
     y = ops.gemv(dq.bufs, dq.meta, x, 0, None).cpu().numpy()
     yr = x.cpu().numpy().astype(np.float64) @ deq.astype(np.float64).T
     assert np.abs(y - yr).max() <= 1e-3 * np.abs(yr).max()
+
+
+@pytest.mark.parametrize("bits", [4, 5, 6, 8])
+@pytest.mark.parametrize("kind", ["halves", "offset", "far", "heavy"])
+def test_codes_are_those_of_the_rounded_division(cuda_lib, bits, kind):
+    """Without the search nothing is summed, so every code, scale and min equals numpy's: quotients on and beside halves, blocks whose
+    values lie far from zero against their range (the multiply-add in front of the rounding then decides nothing), values past the clamp."""
+    from rwkv_quant_b200 import quantize
+    g = torch.Generator().manual_seed(bits)
+    n = 64 * 1024
+    w = {"halves": lambda: torch.randint(0, 2 * 2 ** bits, (n,), generator=g) * 0.5 * 0.013,
+         "offset": lambda: torch.randn(n, generator=g) * 1e-3 + 5.0,
+         "far": lambda: torch.randn(n, generator=g) * 1e-5 - 300.0,
+         "heavy": lambda: torch.randn(n, generator=g) ** 5}[kind]().reshape(64, 1024).float()
+    w = w * (1 + torch.randint(-2, 3, w.shape, generator=g) * 2.0 ** -23)         # an ulp or two to either side
+    if bits != 8:
+        ref = qn.quant_sb6(w.numpy(), bits, False)
+        got = dict(zip(("q", "qs", "qm", "d", "dm"), quantize.quantize_sb6_parts(w.cuda(), bits, False)))
+        for k, v in got.items():
+            assert np.array_equal(v.cpu().numpy().reshape(ref[k].shape), ref[k]), k
+    if bits in (6, 8):
+        ref = qn.quant_sym(w.numpy(), bits, (1.0,))
+        got = dict(zip(("q", "qs", "d"), quantize.quantize_sym_parts(w.cuda(), bits, False)))
+        for k, v in got.items():
+            assert np.array_equal(v.cpu().numpy().reshape(ref[k].shape), ref[k]), k
