@@ -12,6 +12,7 @@
 
 #include "rwkvq_gemm_f16.cuh"
 #include "rwkvq_seq.cuh"
+#include "rwkvq_tmix_seq.cuh"
 #include "rwkvq_wkv_chunk.cuh"
 
 namespace rwkvq {
@@ -19,6 +20,8 @@ namespace {
 
 constexpr int kSmallRows = 64;
 constexpr int kChunkedT = 16;        // tokens per sequence from which long calls take the chunked scan (two chunks)
+
+bool chunked(size_t rows, int T) { return rows > kSmallRows && T >= kChunkedT; }
 
 struct ForwardWs {
     size_t bytes = 0;
@@ -56,8 +59,8 @@ ForwardWs carve(const rwkvq_model& m, int B, int T, size_t n_tail, void* base) {
     w.status = reinterpret_cast<int*>(take(256));
     w.wn2 = f32(static_cast<size_t>(m.n_layer) * 128);
     w.x = f32(N * D); w.rkv = f32(3 * N * D); w.yl = f32(4 * N * D);
-    w.wkv = f32(std::max(5 * N * D, wkv_chunk_floats(B, T, static_cast<int>(D / 64)))); w.dp = f32(N * D / 64);
-    w.out = f32(N * D); w.og = f32(N * D); w.v_first = f32(N * D);
+    if (chunked(N, T)) { w.wkv = f32(wkv_chunk_floats(B, T, static_cast<int>(D / 64))); w.dp = f32(N * D / 64); w.out = f32(N * D); }
+    w.og = f32(N * D); w.v_first = f32(N * D);
     if (N <= kSmallRows) {
         w.xs = f32(6 * N * D); w.hffn = f32(N * F); w.amax = f32(8 * N);
         w.lora_h = f32(4 * static_cast<size_t>(kSmallRows) * m.max_rank);
@@ -325,7 +328,7 @@ int rwkvq_forward_seq_status(const rwkvq_model* m, int B, int T, const int64_t* 
         }
         if (rc) return rc;
         if ((rc = fork.join()) != 0) return rc;
-        if (!small && T >= kChunkedT) {
+        if (chunked(N, T)) {
             WkvChunkArgs q{};
             q.r = r; q.k = k; q.v = v; q.yw = yw; q.ya = ya; q.yv = layer0 ? nullptr : yv; q.v_first = layer0 ? nullptr : w.v_first; q.g = yg;
             q.w0 = L.w0; q.a0 = L.a0; q.v0 = L.v0; q.k_k = L.k_k; q.k_a = L.k_a; q.r_k = L.r_k; q.ln_w = L.lnx_w; q.ln_b = L.lnx_b;
@@ -334,13 +337,12 @@ int rwkvq_forward_seq_status(const rwkvq_model* m, int B, int T, const int64_t* 
             rc = launch_wkv_chunked(q, s);
             if (rc) return rc;
         } else {
-            float *dw = w.wkv, *k2 = w.wkv + ND, *v2 = w.wkv + 2 * ND, *na = w.wkv + 3 * ND, *nb = w.wkv + 4 * ND;
-            rc = rwkvq_seq_tmix_pre(k, v, yw, ya, layer0 ? nullptr : yv, layer0 ? nullptr : w.v_first, L.w0, L.a0, L.v0, L.k_k, L.k_a, dw,
-                                    k2, v2, na, nb, N, H, stream);
-            if (rc) return rc;
-            rc = rwkvq_wkv7(r, dw, k2, v2, na, nb, wkv_in[l], w.out, wkv_out[l], B, T, H, 64, stream);
-            if (rc) return rc;
-            rc = launch_wkv_tail(w.out, r, k2, v2, L.r_k, L.lnx_w, L.lnx_b, yg, w.og, N, H, 64e-5f, sb ? nullptr : am_og, s);
+            TmixSeqArgs q{};
+            q.r = r; q.k = k; q.v = v; q.yw = yw; q.ya = ya; q.yv = layer0 ? nullptr : yv; q.v_first = layer0 ? nullptr : w.v_first; q.g = yg;
+            q.w0 = L.w0; q.a0 = L.a0; q.v0 = L.v0; q.k_k = L.k_k; q.k_a = L.k_a; q.r_k = L.r_k; q.ln_w = L.lnx_w; q.ln_b = L.lnx_b;
+            q.h_in = wkv_in[l]; q.h_out = wkv_out[l]; q.og = w.og; q.og_amax = sb ? nullptr : am_og;
+            q.B = B; q.T = T; q.H = H;
+            rc = launch_tmix_seq(q, s);
             if (rc) return rc;
         }
         // ---- output projection, channel mix

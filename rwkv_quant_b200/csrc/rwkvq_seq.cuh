@@ -30,7 +30,4 @@ struct SeqPrepArgs {
 int launch_seq_prep(const SeqPrepArgs& a, long long n_tokens, cudaStream_t s);
 inline bool seq_prep_in_place_ok(int D) { return D % 256 == 0 && D <= 4096; }
 
-int launch_wkv_tail(const float* wkv, const float* r, const float* k, const float* v, const float* r_k, const float* ln_w,
-                    const float* ln_b, const float* g, float* out, int N, int H, float eps, float* og_amax, cudaStream_t s);
-
 }  // namespace rwkvq

@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(512 / R / SPLIT, 4) wkv7_kernel(const WkvArgs 
 __global__ void __launch_bounds__(128) wkv_tail_kernel(const float* wkv, const float* r, const float* k,
                                                        const float* v, const float* r_k, const float* ln_w,
                                                        const float* ln_b, const float* g, float* out,
-                                                       int n_pairs, int H, float eps, float* og_amax) {
+                                                       int n_pairs, int H, float eps) {
     const int pair = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     pdl_launch_dependents();
     pdl_wait();
@@ -252,21 +252,6 @@ __global__ void __launch_bounds__(128) wkv_tail_kernel(const float* wkv, const f
     const float o1 = (d1 * inv * ln_w[hb + lane + 32] + ln_b[hb + lane + 32] + dp * v[base + lane + 32]) * g[base + lane + 32];
     out[base + lane] = o0;
     out[base + lane + 32] = o1;
-    if (og_amax != nullptr) {                 // |o| as int bits orders like the float, a NaN above every number
-        int m = max(__float_as_int(fabsf(o0)), __float_as_int(fabsf(o1)));
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
-        if (lane == 0) atomicMax(reinterpret_cast<int*>(og_amax) + pair / H, m);
-    }
-}
-
-int launch_wkv_tail(const float* wkv, const float* r, const float* k, const float* v, const float* r_k, const float* ln_w,
-                    const float* ln_b, const float* g, float* out, int N, int H, float eps, float* og_amax, cudaStream_t s) {
-    const int pairs = N * H;
-    cudaError_t e = launch_pdl(wkv_tail_kernel, dim3((pairs + 3) / 4), dim3(128), 0, s, wkv, r, k, v, r_k, ln_w, ln_b, g, out, pairs, H,
-                               eps, og_amax);
-    if (e != cudaSuccess) return fail(RWKVQ_E_LAUNCH, "wkv_tail: %s", cudaGetErrorString(e));
-    return RWKVQ_OK;
 }
 
 }  // namespace rwkvq
@@ -303,8 +288,10 @@ int rwkvq_wkv_tail(const float* wkv, const float* r, const float* k, const float
     RWKVQ_REQUIRE(wkv && r && k && v && r_k && ln_w && ln_b && g && out, RWKVQ_E_NULL, "rwkvq_wkv_tail: null pointer");
     RWKVQ_REQUIRE(head_size == kS, RWKVQ_E_SHAPE, "rwkvq_wkv_tail: head size %d, only 64 is built", head_size);
     RWKVQ_REQUIRE(N >= 1 && H >= 1, RWKVQ_E_SHAPE, "rwkvq_wkv_tail: N=%d H=%d", N, H);
-    int rc = launch_wkv_tail(wkv, r, k, v, r_k, ln_w, ln_b, g, out, N, H, eps, nullptr, static_cast<cudaStream_t>(stream));
-    if (rc) return rc;
+    const int pairs = N * H;
+    cudaError_t e = launch_pdl(wkv_tail_kernel, dim3((pairs + 3) / 4), dim3(128), 0, static_cast<cudaStream_t>(stream), wkv, r, k, v, r_k, ln_w,
+                               ln_b, g, out, pairs, H, eps);
+    if (e != cudaSuccess) return fail(RWKVQ_E_LAUNCH, "wkv_tail: %s", cudaGetErrorString(e));
     return check_launch("rwkvq_wkv_tail");
 }
 

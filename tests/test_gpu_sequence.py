@@ -91,3 +91,17 @@ def test_one_stream_steps_match_the_sequence(cuda_lib, recipe, D, F):
     model.fused_prep = False
     ref, _ = model.forward_stateful(idx, st)
     assert relmax(torch.stack(steps, 1).cpu().numpy(), ref.cpu().numpy()) <= 1e-4
+
+
+@pytest.mark.parametrize("B,T", [(1, 31), (1, 33), (1, 48), (1, 49), (1, 64), (2, 32), (20, 3)])
+def test_time_mix_of_short_sequences_matches_its_steps(cuda_lib, B, T):
+    """Chunks of 16 tokens, whole and ragged, against the step's kernel token by token; fresh and carried states."""
+    model = _model("reduction", n_embd=256, ffn=1024)
+    idx = torch.randint(1, 512, (B, T), generator=torch.Generator().manual_seed(T)).cuda()
+    for st in (_states(model, B), model.init_state(B)):
+        got = model.forward_stateful(idx, [tuple(t.clone() for t in s) for s in st])
+        rows = []
+        for t in range(T):
+            lo, st = model.forward_stateful(idx[:, t:t + 1], st)
+            rows.append(lo)
+        _same(got, (torch.cat(rows, 1), st), 1e-4)
