@@ -263,9 +263,10 @@ int validate_qtensor(const rwkvq_qtensor* t, const char* who);
 // Single-vector tensor-core GEMV (rwkvq_gemv_mma.cu): layout id >= 0 when the
 // tensor carries what that kernel needs, and its launcher.
 int mma_layout_of(const rwkvq_qtensor& t);
+struct Ahead;             // memory to bring into L2 for later launches (rwkvq_ahead.cuh), null: none
 int launch_gemv_mma(int layout, const rwkvq_qtensor* ts, int n_mats, const void* x, int x_dtype,
                     long long ldx, float* y, long long ldy, int epilogue, const float* resid,
-                    int fused, cudaStream_t s, const void* const* x_each = nullptr, bool split = false);
+                    int fused, cudaStream_t s, const void* const* x_each = nullptr, bool split = false, const Ahead* ahead = nullptr);
 // Small-batch tensor-core kernel (rwkvq_gemv_batch.cu): n_mats same-shape matrices, each with its
 // own [N, ldx] input and [N, ldy] output; weights read once for all N right-hand sides.  Inputs are
 // fp32 rows with scales[k] = max|x| of every row (written by the producer of x or by launch_row_amax),
@@ -274,7 +275,7 @@ int launch_gemv_mma(int layout, const rwkvq_qtensor* ts, int n_mats, const void*
 // the bit pattern; zero them before the launch).
 int launch_gemv_batch(const rwkvq_qtensor* ts, int n_mats, const void* const* xs, bool half_in, const float* const* scales,
                       int N, long long ldx, float* const* ys, long long ldy, int epilogue, const float* const* resids,
-                      float* const* amax_outs, cudaStream_t s);
+                      float* const* amax_outs, cudaStream_t s, const Ahead* ahead = nullptr);
 // The same product on the tcgen05 tensor cores (rwkvq_gemm_tcb.cu; sb6 / sym tensors, gemm_tcb_ok);
 // status: device word that receives RWKVQ_E_TIMEOUT if a bounded pipeline wait ran out.
 bool gemm_tcb_ok(const rwkvq_qtensor& t);

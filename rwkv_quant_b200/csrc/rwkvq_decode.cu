@@ -24,6 +24,7 @@
 #include <mutex>
 #include <utility>
 
+#include "rwkvq_ahead.cuh"
 #include "rwkvq_lora_vec.cuh"
 #include "rwkvq_seq.cuh"
 
@@ -936,13 +937,13 @@ Workspace carve(const rwkvq_model& m, int B, void* base) {
 // merged into.
 int linear(const rwkvq_qtensor* t, const float* x, int B, int in, float* y, int out, int epi, const float* resid,
            void* gemm_ws, void* stream, const __half* x16 = nullptr, const float* x_scale = nullptr,
-           float* y_amax = nullptr, int* status = nullptr) {
+           float* y_amax = nullptr, int* status = nullptr, const Ahead* ahead = nullptr) {
     const int ml = mma_layout_of(*t);
     if (B == 1 && ml >= 0) {
         int rc = validate_qtensor(t, "rwkvq_decode_step(linear)");
         if (rc) return rc;
         return launch_gemv_mma(ml, t, 1, x, RWKVQ_F32, in, y, out, epi, resid, 0, static_cast<cudaStream_t>(stream),
-                               nullptr, true);
+                               nullptr, true, ahead);
     }
     if (batch_path(B) && ml >= 0 && x_scale) {            // small batch: weights read once, tokens as MMA columns
         int rc = validate_qtensor(t, "rwkvq_decode_step(linear)");
@@ -954,7 +955,7 @@ int linear(const rwkvq_qtensor* t, const float* x, int B, int in, float* y, int 
         float* ao[1] = {y_amax};
         if (tcb_pays(B) && gemm_tcb_ok(*t))
             return launch_gemm_tcb(t, 1, xs, x16 != nullptr, sc, B, in, ys, out, epi, rs, ao, status, static_cast<cudaStream_t>(stream));
-        return launch_gemv_batch(t, 1, xs, x16 != nullptr, sc, B, in, ys, out, epi, rs, ao, static_cast<cudaStream_t>(stream));
+        return launch_gemv_batch(t, 1, xs, x16 != nullptr, sc, B, in, ys, out, epi, rs, ao, static_cast<cudaStream_t>(stream), ahead);
     }
     if (linear_on_gemm(*t, B)) {                            // tcgen05 path for large batches
         int rc = validate_qtensor(t, "rwkvq_decode_step(linear)");
@@ -1121,6 +1122,7 @@ int rwkvq_decode_step(const rwkvq_model* m, int B, const int64_t* tokens, float*
         const float* x1[4] = {xw, xa, xg, xv};
         const int act[4] = {1, 0, 2, 0};           // tanh (decay), none, sigmoid (gate), none
         const int n_br = layer0 ? 3 : 4;
+        const LayerAhead ahead(L, l + 1 < m->n_layer ? &L + 1 : nullptr, layer0, wkv[l], BD * 64 * sizeof(float));
         float *yw = w.yl, *ya = w.yl + BD, *yv = w.yl + 2 * BD, *yg = w.yl + 3 * BD;
         TmixCoreArgs tc{r, k, v, yw, ya, layer0 ? nullptr : yv, yg, L.w0, L.a0, L.v0, L.k_k, L.k_a, L.r_k,
                         L.lnx_w, L.lnx_b, w.v_first, wkv[l], w.og, D, H, layer0 ? 1 : 0, sb ? nullptr : am_og};
@@ -1145,7 +1147,7 @@ int rwkvq_decode_step(const rwkvq_model* m, int B, const int64_t* tokens, float*
             down.n_br = up.n_br = n_br; down.D = up.D = D;
             const rwkvq_qtensor three[3] = {L.Wr, L.Wk, L.Wv};
             const void* x_each[3] = {xr, xk, xv};
-            rc = launch_gemv_mma_lora(ml, three, 3, x_each, r, D, down, s);
+            rc = launch_gemv_mma_lora(ml, three, 3, x_each, r, D, down, ahead.rkv, s);
             if (rc) return rc;
             rc = launch_tmix_core_up(tc, up, H, s);
             if (rc) return rc;
@@ -1182,12 +1184,12 @@ int rwkvq_decode_step(const rwkvq_model* m, int B, const int64_t* tokens, float*
                 }
                 const rwkvq_qtensor three[3] = {L.Wr, L.Wk, L.Wv};
                 const void* x_each[3] = {xr, xk, xv};
-                rc = launch_gemv_mma(ml, three, 3, xr, RWKVQ_F32, D, r, D, RWKVQ_EPI_NONE, nullptr, 1, s_rkv, x_each, true);
+                rc = launch_gemv_mma(ml, three, 3, xr, RWKVQ_F32, D, r, D, RWKVQ_EPI_NONE, nullptr, 1, s_rkv, x_each, true, &ahead.rkv);
                 if (rc) return rc;
             } else if (sb) {
                 const rwkvq_qtensor three[3] = {L.Wr, L.Wk, L.Wv};
                 float* y3[3] = {r, k, v};
-                rc = launch_gemm_sb(three, 3, w.rkv_pair, B, y3, D, RWKVQ_EPI_NONE, nullptr, nullptr, w.status, 0, s_rkv);
+                rc = launch_gemm_sb(three, 3, w.rkv_pair, B, y3, D, RWKVQ_EPI_NONE, nullptr, nullptr, w.status, 0, s_rkv, &ahead.rkv);
                 if (rc) return rc;
             } else if (bp && rkv_fused) {
                 for (const rwkvq_qtensor* t : {&L.Wr, &L.Wk, &L.Wv}) {
@@ -1202,7 +1204,7 @@ int rwkvq_decode_step(const rwkvq_model* m, int B, const int64_t* tokens, float*
                 if (tcb_pays(B) && gemm_tcb_ok(L.Wr))
                     rc = launch_gemm_tcb(three, 3, x3, h16, a3, B, D, y3, D, RWKVQ_EPI_NONE, nullptr, nullptr, w.status, s_rkv);
                 else
-                    rc = launch_gemv_batch(three, 3, x3, h16, a3, B, D, y3, D, RWKVQ_EPI_NONE, nullptr, nullptr, s_rkv);
+                    rc = launch_gemv_batch(three, 3, x3, h16, a3, B, D, y3, D, RWKVQ_EPI_NONE, nullptr, nullptr, s_rkv, &ahead.rkv);
                 if (rc) return rc;
             } else {
                 rc = linear(&L.Wr, xr, B, D, r, D, RWKVQ_EPI_NONE, nullptr, w.gemm_ws, s_rkv, h16 ? w.xs16 : nullptr, am, nullptr, w.status);
@@ -1234,7 +1236,7 @@ int rwkvq_decode_step(const rwkvq_model* m, int B, const int64_t* tokens, float*
             pc.T = 1; pc.D = D; pc.n_mix = 1; pc.mode[0] = kPrepPair; pc.pair[0] = w.d_pair;
             rc = launch_seq_prep(pc, B, s);
             if (rc) return rc;
-            rc = launch_gemm_sb(&L.Wfk, 1, &w.d_pair, B, yh, F, RWKVQ_EPI_RELU2, nullptr, nullptr, w.status, 0, s);
+            rc = launch_gemm_sb(&L.Wfk, 1, &w.d_pair, B, yh, F, RWKVQ_EPI_RELU2, nullptr, nullptr, w.status, 0, s, &ahead.key);
             if (rc) return rc;
             rc = launch_split_rows(w.hffn, F, F, B, w.f_pair, nullptr, s);
             if (rc) return rc;
@@ -1248,7 +1250,7 @@ int rwkvq_decode_step(const rwkvq_model* m, int B, const int64_t* tokens, float*
         launch_ln_shift_mix<1>(B, s, w.x, L.ln2_w, L.ln2_b, cshift[l], L.ffn_x_k, w.xk, D, h16 ? w.xk16 : static_cast<__half*>(nullptr), am_xk, 1, static_cast<float*>(nullptr),
                    static_cast<float*>(nullptr));
         rc = linear(&L.Wfk, w.xk, B, D, w.hffn, F, RWKVQ_EPI_RELU2, nullptr, w.gemm_ws, stream, h16 ? w.xk16 : nullptr, am_xk, am_h,
-                    w.status);
+                    w.status, &ahead.key);
         if (rc) return rc;
         rc = linear(&L.Wfv, w.hffn, B, F, w.x, D, RWKVQ_EPI_ADD, w.x, w.gemm_ws, stream, nullptr, am_h, nullptr, w.status);
         if (rc) return rc;

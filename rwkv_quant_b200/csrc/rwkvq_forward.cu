@@ -10,6 +10,7 @@
 //             made, weights and LoRA matrices converted into scratch layer by layer
 #include <algorithm>
 
+#include "rwkvq_ahead.cuh"
 #include "rwkvq_gemm_f16.cuh"
 #include "rwkvq_seq.cuh"
 #include "rwkvq_tmix_seq.cuh"
@@ -93,7 +94,7 @@ bool fp16_gemm_ok(const rwkvq_qtensor& t) { return t.kind == RWKVQ_KIND_SB6 || t
 
 // One linear of the small regime; scale: max|x| per row (null: measured by a pre-pass into amax_scratch)
 int small_linear(const rwkvq_qtensor* const* ts, int n_mats, const float* const* xs, const float* const* amax, int N, int in, float* const* ys,
-                 int out, int epi, const float* resid, float* amax_out, cudaStream_t s) {
+                 int out, int epi, const float* resid, float* amax_out, cudaStream_t s, const Ahead* ahead = nullptr) {
     if (N <= 2) {
         for (int k = 0; k < n_mats; ++k) {
             int rc = rwkvq_gemv(ts[k], xs[k], RWKVQ_F32, N, in, ys[k], out, epi, resid, s);
@@ -106,7 +107,7 @@ int small_linear(const rwkvq_qtensor* const* ts, int n_mats, const float* const*
     const float* rs[kHgMaxProbs];
     float* ao[kHgMaxProbs];
     for (int k = 0; k < n_mats; ++k) { t[k] = *ts[k]; xv[k] = xs[k]; rs[k] = resid; ao[k] = amax_out; }
-    return launch_gemv_batch(t, n_mats, xv, false, amax, N, in, ys, out, epi, rs, ao, s);
+    return launch_gemv_batch(t, n_mats, xv, false, amax, N, in, ys, out, epi, rs, ao, s, ahead);
 }
 
 bool same_shape(const rwkvq_qtensor& a, const rwkvq_qtensor& b) {
@@ -278,6 +279,7 @@ int rwkvq_forward_seq_status(const rwkvq_model* m, int B, int T, const int64_t* 
         const bool sb = small && D % 256 == 0 && same_shape(L.Wr, L.Wk) && same_shape(L.Wr, L.Wv) && gemm_sb_pays(L.Wr, N) &&
                         gemm_sb_pays(L.Wo, N) && gemm_sb_pays(L.Wfk, N) && gemm_sb_pays(L.Wfv, N);
         Fork fork{lane, s};
+        const LayerAhead ahead(L, l + 1 < m->n_layer ? &L + 1 : nullptr, layer0, wkv_in[l], static_cast<size_t>(B) * D * 64 * sizeof(float));
         if (small) {
             for (int q = 0; q < 6; ++q) {
                 a.f32[q] = w.xs + q * ND; a.scale[q] = w.amax + q * N;
@@ -298,9 +300,9 @@ int rwkvq_forward_seq_status(const rwkvq_model* m, int B, int T, const int64_t* 
             const float* a3[3] = {w.amax, w.amax + 2 * N, w.amax + 3 * N};
             if (sb) {
                 const rwkvq_qtensor three[3] = {L.Wr, L.Wk, L.Wv};
-                rc = launch_gemm_sb(three, 3, w.rkv_pair, N, y3, D, RWKVQ_EPI_NONE, nullptr, nullptr, w.status, 0, s_rkv);
+                rc = launch_gemm_sb(three, 3, w.rkv_pair, N, y3, D, RWKVQ_EPI_NONE, nullptr, nullptr, w.status, 0, s_rkv, &ahead.rkv);
             } else if (same_shape(L.Wr, L.Wk) && same_shape(L.Wr, L.Wv)) {
-                rc = small_linear(t3, 3, x3, a3, N, D, y3, D, RWKVQ_EPI_NONE, nullptr, nullptr, s_rkv);
+                rc = small_linear(t3, 3, x3, a3, N, D, y3, D, RWKVQ_EPI_NONE, nullptr, nullptr, s_rkv, &ahead.rkv);
             } else {
                 for (int q = 0; q < 3 && !rc; ++q) rc = small_linear(t3 + q, 1, x3 + q, a3 + q, N, D, y3 + q, D, RWKVQ_EPI_NONE, nullptr, nullptr, s_rkv);
             }
@@ -359,7 +361,7 @@ int rwkvq_forward_seq_status(const rwkvq_model* m, int B, int T, const int64_t* 
             c.mode[0] = kPrepPair; c.pair[0] = w.d_pair;
             rc = launch_seq_prep(c, N, s);
             if (rc) return rc;
-            rc = launch_gemm_sb(&L.Wfk, 1, &w.d_pair, N, yh, F, RWKVQ_EPI_RELU2, nullptr, nullptr, w.status, 0, s);
+            rc = launch_gemm_sb(&L.Wfk, 1, &w.d_pair, N, yh, F, RWKVQ_EPI_RELU2, nullptr, nullptr, w.status, 0, s, &ahead.key);
             if (rc) return rc;
             rc = launch_split_rows(w.hffn, F, F, N, w.f_pair, nullptr, s);
             if (rc) return rc;
@@ -376,7 +378,7 @@ int rwkvq_forward_seq_status(const rwkvq_model* m, int B, int T, const int64_t* 
             c.mode[0] = kPrepF32 | kPrepAmax; c.f32[0] = w.xs; c.scale[0] = w.amax;
             rc = launch_seq_prep(c, N, s);
             if (rc) return rc;
-            rc = small_linear(tk, 1, xk, ak, N, D, yh, F, RWKVQ_EPI_RELU2, nullptr, am_h, s);
+            rc = small_linear(tk, 1, xk, ak, N, D, yh, F, RWKVQ_EPI_RELU2, nullptr, am_h, s, &ahead.key);
             if (rc) return rc;
             rc = small_linear(tv, 1, xv, av, N, F, yx, D, RWKVQ_EPI_ADD, w.x, nullptr, s);
             if (rc) return rc;

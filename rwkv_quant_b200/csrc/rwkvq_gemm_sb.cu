@@ -32,7 +32,7 @@
 #include <cstdlib>
 #include <type_traits>
 
-#include "rwkvq_gemv_mma.cuh"
+#include "rwkvq_ahead.cuh"
 #include "rwkvq_tc.cuh"
 
 namespace cg = cooperative_groups;
@@ -174,7 +174,7 @@ __device__ __forceinline__ __half2 sb_sym_scales(uint32_t two, uint32_t dd) {
 }
 
 template <int L, int NT>
-__global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_constant__ SbArgs a, const __grid_constant__ SbMaps maps) {
+__global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_constant__ SbArgs a, const __grid_constant__ SbMaps maps, const __grid_constant__ Ahead ahead) {
     using G = SbGeo<L, NT>;
     using Y = SbLayout<L>;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -245,6 +245,7 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
         copy_tile();
         for (int i = 0; i < G::AHEAD; ++i) copy_stage();
     }
+    if (warp == kSbTmaWarp) ahead_prefetch(ahead, blockIdx.x + gridDim.x * blockIdx.y, gridDim.x * gridDim.y);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -584,7 +585,7 @@ int resident_clusters(int dev, int c) {
 }
 
 template <int L, int NT>
-int launch_sb(SbArgs& a, const SbMaps& maps, int groups, int force_ks, cudaStream_t s) {
+int launch_sb(SbArgs& a, const SbMaps& maps, int groups, int force_ks, const Ahead& ahead, cudaStream_t s) {
     static bool configured[64] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) dev = 0;
@@ -620,17 +621,17 @@ int launch_sb(SbArgs& a, const SbMaps& maps, int groups, int force_ks, cudaStrea
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 2 : 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_sb_kernel<L, NT>, a, maps);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_sb_kernel<L, NT>, a, maps, ahead);
     if (e != cudaSuccess) return fail(RWKVQ_E_LAUNCH, "gemm_sb: %s", cudaGetErrorString(e));
     return RWKVQ_OK;
 }
 
 template <int L>
-int launch_sb_nt(SbArgs& a, const SbMaps& maps, int nt, int groups, int force_ks, cudaStream_t s) {
-    if (nt <= 16) return launch_sb<L, 16>(a, maps, groups, force_ks, s);
-    if (nt <= 32) return launch_sb<L, 32>(a, maps, groups, force_ks, s);
-    if (nt <= 64) return launch_sb<L, 64>(a, maps, groups, force_ks, s);
-    return launch_sb<L, 128>(a, maps, groups, force_ks, s);
+int launch_sb_nt(SbArgs& a, const SbMaps& maps, int nt, int groups, int force_ks, const Ahead& ahead, cudaStream_t s) {
+    if (nt <= 16) return launch_sb<L, 16>(a, maps, groups, force_ks, ahead, s);
+    if (nt <= 32) return launch_sb<L, 32>(a, maps, groups, force_ks, ahead, s);
+    if (nt <= 64) return launch_sb<L, 64>(a, maps, groups, force_ks, ahead, s);
+    return launch_sb<L, 128>(a, maps, groups, force_ks, ahead, s);
 }
 
 }  // namespace
@@ -649,7 +650,8 @@ bool gemm_sb_pays(const rwkvq_qtensor& t, int N) {
 }
 
 int launch_gemm_sb(const rwkvq_qtensor* ts, int n_mats, const SbRows* rows, int N, float* const* ys, long long ldy, int epilogue,
-                   const float* const* resids, float* const* amax_outs, int* status, int force_ks, cudaStream_t s) {
+                   const float* const* resids, float* const* amax_outs, int* status, int force_ks, cudaStream_t s, const Ahead* ahead_or_null) {
+    const Ahead none{}, &ahead = ahead_or_null ? *ahead_or_null : none;
     RWKVQ_REQUIRE(n_mats >= 1 && n_mats <= kSbMaxMats, RWKVQ_E_LIMIT, "gemm_sb: %d matrices", n_mats);
     SbArgs a{};
     SbMaps maps;
@@ -677,11 +679,11 @@ int launch_gemm_sb(const rwkvq_qtensor* ts, int n_mats, const SbRows* rows, int 
     a.n_tiles = a.row_tiles * n_mats;
     a.n_sb = ts[0].cols / 256;
     switch (sb_layout_of(ts[0])) {
-        case ML_SB6_4: return launch_sb_nt<ML_SB6_4>(a, maps, nt, groups, force_ks, s);
-        case ML_SB6_5: return launch_sb_nt<ML_SB6_5>(a, maps, nt, groups, force_ks, s);
-        case ML_SB6_6: return launch_sb_nt<ML_SB6_6>(a, maps, nt, groups, force_ks, s);
-        case ML_SYM6: return launch_sb_nt<ML_SYM6>(a, maps, nt, groups, force_ks, s);
-        default: return launch_sb_nt<ML_SYM8>(a, maps, nt, groups, force_ks, s);
+        case ML_SB6_4: return launch_sb_nt<ML_SB6_4>(a, maps, nt, groups, force_ks, ahead, s);
+        case ML_SB6_5: return launch_sb_nt<ML_SB6_5>(a, maps, nt, groups, force_ks, ahead, s);
+        case ML_SB6_6: return launch_sb_nt<ML_SB6_6>(a, maps, nt, groups, force_ks, ahead, s);
+        case ML_SYM6: return launch_sb_nt<ML_SYM6>(a, maps, nt, groups, force_ks, ahead, s);
+        default: return launch_sb_nt<ML_SYM8>(a, maps, nt, groups, force_ks, ahead, s);
     }
 }
 

@@ -66,7 +66,7 @@ int launch_split_rows(const float* x, long long ldx, int cols, int N, const SbRo
 // y[k] = epi(W_k x_k) for tensors gemm_sb_ok accepts, one shape and layout; rows[k]: the pairs of x_k;
 // amax_outs (optional, per matrix): [N] slots merged with max|y| per token
 int launch_gemm_sb(const rwkvq_qtensor* ts, int n_mats, const SbRows* rows, int N, float* const* ys, long long ldy, int epilogue,
-                   const float* const* resids, float* const* amax_outs, int* status, int force_ks, cudaStream_t s);
+                   const float* const* resids, float* const* amax_outs, int* status, int force_ks, cudaStream_t s, const Ahead* ahead = nullptr);
 bool gemm_sb_ok(const rwkvq_qtensor& t);                  // sb6 / sym with the relayouted records and planes, 16-byte aligned streams
 bool gemm_sb_pays(const rwkvq_qtensor& t, int N);
 // tensor map of an fp16 matrix: boxes of 64 columns x box_rows, 128-byte swizzle, zero fill (rwkvq_gemm_f16.cu)

@@ -38,8 +38,8 @@
 #include <algorithm>
 #include <cstdlib>
 
+#include "rwkvq_ahead.cuh"
 #include "rwkvq_gemm_sb.cuh"
-#include "rwkvq_gemv_mma.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -145,7 +145,7 @@ template <int L> struct BtGeo {
 // with their max, scaled to at most 2^9 so that a block sum stays inside the fp16 range; the hi and
 // lo halves of a lane's four activations sit side by side (one 128-bit load per MMA triple).
 template <int L, int NT, bool EX>      // NT: 8-token tiles of the MMA N dimension
-__global__ void __launch_bounds__(kBtThreads, 2) gemv_batch_kernel(const BatchArgs a) {
+__global__ void __launch_bounds__(kBtThreads, 2) gemv_batch_kernel(const BatchArgs a, const __grid_constant__ Ahead ahead) {
     using G = Geo<L>;
     using BG = BtGeo<L>;
     constexpr int N8 = NT * 8;
@@ -195,6 +195,7 @@ __global__ void __launch_bounds__(kBtThreads, 2) gemv_batch_kernel(const BatchAr
     bt_mark(a, 0);
     pdl_launch_dependents();
     fetch_next();                          // weights do not depend on the producer of x
+    if (warp == kBtWarps - 1) ahead_prefetch(ahead, blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z), gridDim.x * gridDim.y * gridDim.z);
     pdl_wait();
     bt_mark(a, 1);
 
@@ -572,7 +573,7 @@ int g_batch_force_rows = 0, g_batch_force_cols = 0;   // ... for tensors of this
 namespace {
 
 template <int L, int NT, bool EX>
-int launch_bt(BatchArgs& a, int n_mats, int n_groups, int n_clusters, size_t smem, cudaStream_t s) {
+int launch_bt(BatchArgs& a, int n_mats, int n_groups, int n_clusters, size_t smem, const Ahead& ahead, cudaStream_t s) {
     static bool configured[64] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) dev = 0;
@@ -593,13 +594,13 @@ int launch_bt(BatchArgs& a, int n_mats, int n_groups, int n_clusters, size_t sme
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 2 : 1;
-    cudaError_t le = cudaLaunchKernelEx(&cfg, gemv_batch_kernel<L, NT, EX>, a);
+    cudaError_t le = cudaLaunchKernelEx(&cfg, gemv_batch_kernel<L, NT, EX>, a, ahead);
     if (le != cudaSuccess) return fail(RWKVQ_E_LAUNCH, "rwkvq_gemv_batch: %s", cudaGetErrorString(le));
     return RWKVQ_OK;
 }
 
 template <int L>
-int launch_bt_l(BatchArgs& a, int n_mats, int rows, int cols, int N, bool exact, cudaStream_t s) {
+int launch_bt_l(BatchArgs& a, int n_mats, int rows, int cols, int N, bool exact, const Ahead& ahead, cudaStream_t s) {
     using G = Geo<L>;
     const int n_iters = cols / G::KI;
     // The two-term kernel works on 16 tokens at a time (grid.z walks the groups of a larger batch): measured
@@ -674,16 +675,16 @@ int launch_bt_l(BatchArgs& a, int n_mats, int rows, int cols, int N, bool exact,
     const size_t smem = fixed_bytes(tpc) + static_cast<size_t>(a.chunk_its) * it_bytes;
     if (exact) {
         switch (nt) {
-            case 1: return launch_bt<L, 1, true>(a, n_mats, n_groups, n_clusters, smem, s);
-            case 2: return launch_bt<L, 2, true>(a, n_mats, n_groups, n_clusters, smem, s);
-            default: return launch_bt<L, 4, true>(a, n_mats, n_groups, n_clusters, smem, s);
+            case 1: return launch_bt<L, 1, true>(a, n_mats, n_groups, n_clusters, smem, ahead, s);
+            case 2: return launch_bt<L, 2, true>(a, n_mats, n_groups, n_clusters, smem, ahead, s);
+            default: return launch_bt<L, 4, true>(a, n_mats, n_groups, n_clusters, smem, ahead, s);
         }
     }
     switch (nt) {
-        case 1: return launch_bt<L, 1, false>(a, n_mats, n_groups, n_clusters, smem, s);
-        case 2: return launch_bt<L, 2, false>(a, n_mats, n_groups, n_clusters, smem, s);
-        case 4: return launch_bt<L, 4, false>(a, n_mats, n_groups, n_clusters, smem, s);
-        default: return launch_bt<L, 8, false>(a, n_mats, n_groups, n_clusters, smem, s);
+        case 1: return launch_bt<L, 1, false>(a, n_mats, n_groups, n_clusters, smem, ahead, s);
+        case 2: return launch_bt<L, 2, false>(a, n_mats, n_groups, n_clusters, smem, ahead, s);
+        case 4: return launch_bt<L, 4, false>(a, n_mats, n_groups, n_clusters, smem, ahead, s);
+        default: return launch_bt<L, 8, false>(a, n_mats, n_groups, n_clusters, smem, ahead, s);
     }
 }
 
@@ -695,7 +696,8 @@ int launch_bt_l(BatchArgs& a, int n_mats, int rows, int cols, int N, bool exact,
 // (optional): [N] per matrix, merged with max|y| per token.
 int launch_gemv_batch(const rwkvq_qtensor* ts, int n_mats, const void* const* xs, bool half_in, const float* const* scales,
                       int N, long long ldx, float* const* ys, long long ldy, int epilogue, const float* const* resids,
-                      float* const* amax_outs, cudaStream_t s) {
+                      float* const* amax_outs, cudaStream_t s, const Ahead* ahead_or_null) {
+    const Ahead none{}, &ahead = ahead_or_null ? *ahead_or_null : none;
     const int ml = mma_layout_of(ts[0]);
     RWKVQ_REQUIRE(ml >= 0, RWKVQ_E_DTYPE,
                   "rwkvq_gemv_batch: needs an sb6 tensor with relayouted records / planes, a sym tensor or per-row int8");
@@ -719,12 +721,12 @@ int launch_gemv_batch(const rwkvq_qtensor* ts, int n_mats, const void* const* xs
     const int rows = ts[0].rows, cols = ts[0].cols;
     const bool exact = !half_in && !batch_fast();
     switch (ml) {
-        case ML_SB6_4: return launch_bt_l<ML_SB6_4>(a, n_mats, rows, cols, N, exact, s);
-        case ML_SB6_5: return launch_bt_l<ML_SB6_5>(a, n_mats, rows, cols, N, exact, s);
-        case ML_SB6_6: return launch_bt_l<ML_SB6_6>(a, n_mats, rows, cols, N, exact, s);
-        case ML_SYM6: return launch_bt_l<ML_SYM6>(a, n_mats, rows, cols, N, exact, s);
-        case ML_RTN8: return launch_bt_l<ML_RTN8>(a, n_mats, rows, cols, N, exact, s);
-        default: return launch_bt_l<ML_SYM8>(a, n_mats, rows, cols, N, exact, s);
+        case ML_SB6_4: return launch_bt_l<ML_SB6_4>(a, n_mats, rows, cols, N, exact, ahead, s);
+        case ML_SB6_5: return launch_bt_l<ML_SB6_5>(a, n_mats, rows, cols, N, exact, ahead, s);
+        case ML_SB6_6: return launch_bt_l<ML_SB6_6>(a, n_mats, rows, cols, N, exact, ahead, s);
+        case ML_SYM6: return launch_bt_l<ML_SYM6>(a, n_mats, rows, cols, N, exact, ahead, s);
+        case ML_RTN8: return launch_bt_l<ML_RTN8>(a, n_mats, rows, cols, N, exact, ahead, s);
+        default: return launch_bt_l<ML_SYM8>(a, n_mats, rows, cols, N, exact, ahead, s);
     }
 }
 

@@ -6,7 +6,7 @@
 #include <cstdlib>
 #include <type_traits>
 
-#include "rwkvq_gemv_mma.cuh"
+#include "rwkvq_ahead.cuh"
 #include "rwkvq_lora_vec.cuh"
 
 namespace cg = cooperative_groups;
@@ -31,11 +31,13 @@ template <int L> __host__ __device__ constexpr int ctas_per_sm() { return Geo<L>
 // of global scratch with an arrival counter: 9.6 to 7.9 us.
 // LORA: grid rows from n_mats on are the LoRA down projections of the same layer (rwkvq_lora_vec.cuh).
 template <int L, int WK, bool SPLIT, bool ZS, int LORA>
-__global__ void __launch_bounds__(kMmaWarps * 32, ctas_per_sm<L>()) gemv_mma_kernel(const MmaArgs a, const std::conditional_t<LORA != 0, LoraVecArgs, int> lora) {
+__global__ void __launch_bounds__(kMmaWarps * 32, ctas_per_sm<L>()) gemv_mma_kernel(const MmaArgs a, const std::conditional_t<LORA != 0, LoraVecArgs, int> lora, const __grid_constant__ Ahead ahead) {
+    const unsigned cta_id = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
     if constexpr (LORA != 0) {
         if (static_cast<int>(blockIdx.y) >= a.n_mats) {
             const int cta = (static_cast<int>(blockIdx.y) - a.n_mats) * static_cast<int>(gridDim.x) + static_cast<int>(blockIdx.x);
             pdl_launch_dependents();
+            if (threadIdx.x >= (kMmaWarps - 1) * 32) ahead_prefetch(ahead, cta_id, gridDim.x * gridDim.y);
             if (cta * kLvCols < lora.first[lora.n_br]) lora_down_vec<LORA>(lora, cta);
             return;
         }
@@ -81,6 +83,7 @@ __global__ void __launch_bounds__(kMmaWarps * 32, ctas_per_sm<L>()) gemv_mma_ker
     // producer of the activations has finished, when launched programmatically)
     pdl_launch_dependents();
     fetch_next();
+    if (warp == kMmaWarps - 1) ahead_prefetch(ahead, cta_id, gridDim.x * gridDim.y * gridDim.z);
     pdl_wait();
 
     const size_t esz = (a.x_dtype == RWKVQ_F32) ? 4 : 2;
@@ -227,7 +230,7 @@ constexpr int kSplitAnyCols = 4096;        // rows from which on the K split doe
 constexpr int kSplitMaxRows = 4096;        // rows a K-split launch may have: above, the row tiles alone fill the chip
 
 template <int L, int WK, bool SPLIT, bool ZS, int LORA = 0>
-static int launch_one_zs(MmaArgs& a, int rows, int cols, int n_mats, int KS, cudaStream_t s, const LoraVecArgs* lora = nullptr) {
+static int launch_one_zs(MmaArgs& a, int rows, int cols, int n_mats, int KS, cudaStream_t s, const Ahead& ahead, const LoraVecArgs* lora = nullptr) {
     constexpr int WT = kMmaWarps / WK;
     const int slice = cols / KS;
     const size_t smem = 3 * static_cast<size_t>(slice) + 4 * (slice / 16) + 2 * kMmaWarps * 16 * 4 + ((slice / 32 + 15) / 16) * 16;
@@ -265,21 +268,21 @@ static int launch_one_zs(MmaArgs& a, int rows, int cols, int n_mats, int KS, cud
     cfg.attrs = attr;
     cfg.numAttrs = n_attr;
     cudaError_t le;
-    if constexpr (LORA != 0) le = cudaLaunchKernelEx(&cfg, gemv_mma_kernel<L, WK, SPLIT, ZS, LORA>, a, *lora);
-    else le = cudaLaunchKernelEx(&cfg, gemv_mma_kernel<L, WK, SPLIT, ZS, LORA>, a, 0);
+    if constexpr (LORA != 0) le = cudaLaunchKernelEx(&cfg, gemv_mma_kernel<L, WK, SPLIT, ZS, LORA>, a, *lora, ahead);
+    else le = cudaLaunchKernelEx(&cfg, gemv_mma_kernel<L, WK, SPLIT, ZS, LORA>, a, 0, ahead);
     if (le != cudaSuccess) return fail(RWKVQ_E_LAUNCH, "gemv_mma: %s", cudaGetErrorString(le));
     return RWKVQ_OK;
 }
 
 template <int L, int WK, bool SPLIT = false>
-static int launch_one(MmaArgs& a, int rows, int cols, int n_mats, int KS, cudaStream_t s) {
+static int launch_one(MmaArgs& a, int rows, int cols, int n_mats, int KS, cudaStream_t s, const Ahead& ahead) {
     // The zero-group skip is opt-in (RWKVQ_ZERO_SKIP=1): on this part a 16-byte hole saves no DRAM traffic
     // (whole 64-128-byte lines are fetched) and the variant costs ~0.2 us per launch.  When on: rows as long as
     // the channel-mix hidden vector, the one input with exact zeros, and the layouts whose loader can leave a
     // group unread.
     if (zero_skip_enabled() && cols >= 4096 && (L <= ML_SB6_6 || L == ML_SYM6))
-        return launch_one_zs<L, WK, SPLIT, true>(a, rows, cols, n_mats, KS, s);
-    return launch_one_zs<L, WK, SPLIT, false>(a, rows, cols, n_mats, KS, s);
+        return launch_one_zs<L, WK, SPLIT, true>(a, rows, cols, n_mats, KS, s, ahead);
+    return launch_one_zs<L, WK, SPLIT, false>(a, rows, cols, n_mats, KS, s, ahead);
 }
 
 // Work split: a single wave of co-resident CTAs whenever the matrix allows it.
@@ -288,7 +291,7 @@ static int launch_one(MmaArgs& a, int rows, int cols, int n_mats, int KS, cudaSt
 //   * more tiles -> WT tiles per CTA so that the grid still fits one wave
 //   * very many tiles (head) -> persistent CTAs, 8 warps split K of each tile
 template <int L>
-static int launch_wk(MmaArgs& a, int rows, int cols, int n_mats, bool split, cudaStream_t s) {
+static int launch_wk(MmaArgs& a, int rows, int cols, int n_mats, bool split, const Ahead& ahead, cudaStream_t s) {
     constexpr int kResident = ctas_per_sm<L>() * 148;
     const int n_iters = cols / Geo<L>::KI;
     const int tiles = (rows + 15) / 16;
@@ -301,7 +304,7 @@ static int launch_wk(MmaArgs& a, int rows, int cols, int n_mats, bool split, cud
         if (ctas * 4 <= kResident && n_iters >= 32 && n_iters % 4 == 0) KS = 4;
         else if (ctas * 2 <= kResident && n_iters % 2 == 0) KS = 2;
     }
-    if (KS > 1) return launch_one<L, 8, true>(a, rows, cols, n_mats, KS, s);
+    if (KS > 1) return launch_one<L, 8, true>(a, rows, cols, n_mats, KS, s, ahead);
     int wt = 1;
     if (tiles * n_mats > kResident) {
         wt = 0;
@@ -312,10 +315,10 @@ static int launch_wk(MmaArgs& a, int rows, int cols, int n_mats, bool split, cud
     int wk = 8 / wt;
     while (wk > n_iters) wk >>= 1;           // short rows: fewer K slices, more tiles per CTA
     switch (wk) {
-        case 8: return launch_one<L, 8>(a, rows, cols, n_mats, 1, s);
-        case 4: return launch_one<L, 4>(a, rows, cols, n_mats, 1, s);
-        case 2: return launch_one<L, 2>(a, rows, cols, n_mats, 1, s);
-        default: return launch_one<L, 1>(a, rows, cols, n_mats, 1, s);
+        case 8: return launch_one<L, 8>(a, rows, cols, n_mats, 1, s, ahead);
+        case 4: return launch_one<L, 4>(a, rows, cols, n_mats, 1, s, ahead);
+        case 2: return launch_one<L, 2>(a, rows, cols, n_mats, 1, s, ahead);
+        default: return launch_one<L, 1>(a, rows, cols, n_mats, 1, s, ahead);
     }
 }
 
@@ -323,29 +326,30 @@ static int launch_wk(MmaArgs& a, int rows, int cols, int n_mats, bool split, cud
 // `split` allows the K split across CTAs for rows shorter than kSplitAnyCols too.
 int launch_gemv_mma(int layout, const rwkvq_qtensor* ts, int n_mats, const void* x, int x_dtype,
                     long long ldx, float* y, long long ldy, int epilogue, const float* resid,
-                    int fused, cudaStream_t s, const void* const* x_each, bool split) {
+                    int fused, cudaStream_t s, const void* const* x_each, bool split, const Ahead* ahead_or_null) {
+    const Ahead none{}, &ahead = ahead_or_null ? *ahead_or_null : none;
     MmaArgs a{};
     for (int k = 0; k < n_mats; ++k) { a.t[k] = make_view(ts[k]); a.xk[k] = x_each ? x_each[k] : nullptr; }
     a.x = x; a.x_dtype = x_dtype; a.ldx = ldx; a.y = y; a.ldy = ldy;
     a.resid = resid; a.epilogue = epilogue; a.fused = fused;
     const int rows = ts[0].rows, cols = ts[0].cols;
     switch (layout) {
-        case ML_SB6_4: return launch_wk<ML_SB6_4>(a, rows, cols, n_mats, split, s);
-        case ML_SB6_5: return launch_wk<ML_SB6_5>(a, rows, cols, n_mats, split, s);
-        case ML_SB6_6: return launch_wk<ML_SB6_6>(a, rows, cols, n_mats, split, s);
-        case ML_SYM6: return launch_wk<ML_SYM6>(a, rows, cols, n_mats, split, s);
-        case ML_RTN8: return launch_wk<ML_RTN8>(a, rows, cols, n_mats, split, s);
-        default: return launch_wk<ML_SYM8>(a, rows, cols, n_mats, split, s);
+        case ML_SB6_4: return launch_wk<ML_SB6_4>(a, rows, cols, n_mats, split, ahead, s);
+        case ML_SB6_5: return launch_wk<ML_SB6_5>(a, rows, cols, n_mats, split, ahead, s);
+        case ML_SB6_6: return launch_wk<ML_SB6_6>(a, rows, cols, n_mats, split, ahead, s);
+        case ML_SYM6: return launch_wk<ML_SYM6>(a, rows, cols, n_mats, split, ahead, s);
+        case ML_RTN8: return launch_wk<ML_RTN8>(a, rows, cols, n_mats, split, ahead, s);
+        default: return launch_wk<ML_SYM8>(a, rows, cols, n_mats, split, ahead, s);
     }
 }
 
 template <int L>
-static int launch_rkv_lora(MmaArgs& a, int rows, int cols, int n_mats, const LoraVecArgs& lora, cudaStream_t s) {
+static int launch_rkv_lora(MmaArgs& a, int rows, int cols, int n_mats, const LoraVecArgs& lora, const Ahead& ahead, cudaStream_t s) {
     switch ((lora.D / 4 + 255) / 256) {
-        case 1: return launch_one_zs<L, 4, false, false, 1>(a, rows, cols, n_mats, 1, s, &lora);
-        case 2: return launch_one_zs<L, 4, false, false, 2>(a, rows, cols, n_mats, 1, s, &lora);
-        case 3: return launch_one_zs<L, 4, false, false, 3>(a, rows, cols, n_mats, 1, s, &lora);
-        default: return launch_one_zs<L, 4, false, false, 4>(a, rows, cols, n_mats, 1, s, &lora);
+        case 1: return launch_one_zs<L, 4, false, false, 1>(a, rows, cols, n_mats, 1, s, ahead, &lora);
+        case 2: return launch_one_zs<L, 4, false, false, 2>(a, rows, cols, n_mats, 1, s, ahead, &lora);
+        case 3: return launch_one_zs<L, 4, false, false, 3>(a, rows, cols, n_mats, 1, s, ahead, &lora);
+        default: return launch_one_zs<L, 4, false, false, 4>(a, rows, cols, n_mats, 1, s, ahead, &lora);
     }
 }
 
@@ -364,18 +368,18 @@ bool lora_vec_ok(const rwkvq_qtensor* const* t1, const rwkvq_qtensor* const* t2,
 }
 
 int launch_gemv_mma_lora(int layout, const rwkvq_qtensor* ts, int n_mats, const void* const* x_each, float* y, long long ldy,
-                         const LoraVecArgs& lora, cudaStream_t s) {
+                         const LoraVecArgs& lora, const Ahead& ahead, cudaStream_t s) {
     MmaArgs a{};
     for (int k = 0; k < n_mats; ++k) { a.t[k] = make_view(ts[k]); a.xk[k] = x_each[k]; }
     a.x_dtype = RWKVQ_F32; a.ldx = ts[0].cols; a.y = y; a.ldy = ldy; a.epilogue = RWKVQ_EPI_NONE; a.fused = 1; a.n_mats = n_mats;
     const int rows = ts[0].rows, cols = ts[0].cols;
     switch (layout) {
-        case ML_SB6_4: return launch_rkv_lora<ML_SB6_4>(a, rows, cols, n_mats, lora, s);
-        case ML_SB6_5: return launch_rkv_lora<ML_SB6_5>(a, rows, cols, n_mats, lora, s);
-        case ML_SB6_6: return launch_rkv_lora<ML_SB6_6>(a, rows, cols, n_mats, lora, s);
-        case ML_SYM6: return launch_rkv_lora<ML_SYM6>(a, rows, cols, n_mats, lora, s);
-        case ML_RTN8: return launch_rkv_lora<ML_RTN8>(a, rows, cols, n_mats, lora, s);
-        default: return launch_rkv_lora<ML_SYM8>(a, rows, cols, n_mats, lora, s);
+        case ML_SB6_4: return launch_rkv_lora<ML_SB6_4>(a, rows, cols, n_mats, lora, ahead, s);
+        case ML_SB6_5: return launch_rkv_lora<ML_SB6_5>(a, rows, cols, n_mats, lora, ahead, s);
+        case ML_SB6_6: return launch_rkv_lora<ML_SB6_6>(a, rows, cols, n_mats, lora, ahead, s);
+        case ML_SYM6: return launch_rkv_lora<ML_SYM6>(a, rows, cols, n_mats, lora, ahead, s);
+        case ML_RTN8: return launch_rkv_lora<ML_RTN8>(a, rows, cols, n_mats, lora, ahead, s);
+        default: return launch_rkv_lora<ML_SYM8>(a, rows, cols, n_mats, lora, ahead, s);
     }
 }
 

@@ -31,7 +31,7 @@ inline size_t lora_vec_smem(int ranks) { return static_cast<size_t>(ranks) * (64
 bool lora_vec_ok(const rwkvq_qtensor* const* t1, const rwkvq_qtensor* const* t2, int n_br, int D);
 // The three projections of one stream (fp32 rows x_each) and the LoRA down projections in one launch.
 int launch_gemv_mma_lora(int layout, const rwkvq_qtensor* ts, int n_mats, const void* const* x_each, float* y, long long ldy,
-                         const LoraVecArgs& lora, cudaStream_t s);
+                         const LoraVecArgs& lora, const Ahead& ahead, cudaStream_t s);
 
 // h[8 columns] = act(x @ W1): thread i owns rows 4 (i + 256 k) + e.  The weights are in registers as fp16 (exact, the
 // loader's precision) before x is awaited; behind it there is one L2 round trip, 64 multiply-adds and one reduction.
