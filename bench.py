@@ -461,7 +461,7 @@ def run_ours(a, rank, world, local_rank):
         "roofline": {"bound": "hbm", "achieved": g_bytes / g_sec / 1e9, "peak": peak, "unit": "GB/s",
                          "frac": g_bytes / g_sec / 1e9 / peak, "peak_kind": peak_kind,
                          "traffic": None,
-                         "what": "the dominant kernel (the small-batch linear on tcgen05 from 17 streams on, on mma.sync below): "
+                         "what": "the dominant kernel (the small-batch linear on tcgen05 from 9 streams on, on mma.sync below): "
                                  "file-format bytes of the quantized linears + their activation rows / time of those "
                                  "launches, all through rwkvq_gemv_batch, replayed as one graph",
                          "kernel": (f"{kernel_name(B, fast_env)}, the {g_launches} launches of the quantized linears of one step at "

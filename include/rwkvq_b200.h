@@ -195,9 +195,10 @@ int rwkvq_quantize_sym6_packed(const float* w, int64_t ldw, int rows, int cols, 
  * to ~1e-6 of max|y| (a column's last bits may depend on the batch it is computed in; two calls on
  * the same input give the same bits).  The K split is reduced across a thread-block cluster through
  * distributed shared memory: no scratch for partial sums.
- * Up to 16 rows the products run on mma.sync; from 17 rows on sb6 / sym tensors with whole 256-column
+ * Up to 8 rows the products run on mma.sync; from 9 rows on sb6 / sym tensors with whole 256-column
  * super-blocks (up to 16384 columns) run on the tcgen05 tensor cores in the same arithmetic (rows of 128
- * as the UMMA M, the converted weights as its operand in tensor memory, the batch as its N).
+ * as the UMMA M, the converted weights as its operand in tensor memory, the batch as its N); 9 to 16 rows
+ * where the workspace is that of rwkvq_gemv_batch_workspace_bytes(N) or has as much room, else on mma.sync.
  * With RWKVQ_BATCH_FAST=1 in the environment (read once per process) single fp16 operands are used
  * instead (weights fp16(q*s+m)): results within ~3e-4 of max|y| per call (the precision of rwkvq_gemm),
  * and sb6 / sym tensors with more than 32 rows run on a single-term tcgen05 form.
@@ -400,7 +401,7 @@ size_t rwkvq_decode_workspace_bytes(const rwkvq_model* m_host, int B);
  * logits [B, vocab] fp32 (NULL: kept in the workspace), next_tokens [B] int64 greedy
  * argmax (NULL: skipped), tokens [B] int64 on the device.
  * Linears: B = 1 the single-vector tensor-core GEMV; 2 <= B <= 256 the weights-once small-batch kernels
- * in two-term precision (see rwkvq_gemv_batch), on the tcgen05 pipeline from 17 streams on where every
+ * in two-term precision (see rwkvq_gemv_batch), on the tcgen05 pipeline from 9 streams on where every
  * linear of the model has its layout (RWKVQ_TCB_EXACT=0 / 1 in the environment, read once: never / from 3
  * streams on); RWKVQ_BATCH_FAST=1 selects single fp16 operands instead; larger B the prefill GEMM.
  */

@@ -314,7 +314,8 @@ def gemv_batch(dq: "DeviceQT", x: torch.Tensor, epilogue: int = 0, resid: Option
         x = x.contiguous()
     n = x.shape[0]
     y = torch.empty((n, dq.rows), dtype=torch.float32, device=x.device)
-    nws = lib.rwkvq_gemv_batch_workspace_bytes_of(dq.struct_ref, n)
+    # 9 to 16 rows: with room for operand pairs the product takes the tcgen05 pipeline
+    nws = lib.rwkvq_gemv_batch_workspace_bytes(n) if 9 <= n <= 16 else lib.rwkvq_gemv_batch_workspace_bytes_of(dq.struct_ref, n)
     ws = torch.empty(nws, dtype=torch.uint8, device=x.device)
     _lib.check(lib.rwkvq_gemv_batch(dq.struct_ref, x.data_ptr(), n, x.stride(0), y.data_ptr(), y.stride(0),
                                     epilogue, _lib.ptr(resid), ws.data_ptr(), nws, _lib.stream_ptr()), "rwkvq_gemv_batch")

@@ -44,7 +44,7 @@ class _QuantLinearBase:
             y = ops.gemm(self.dq, x2, epilogue, resid)
         elif ops.has_batch_layout(self.dq):
             # the reference decodes each weight once per chunk of 4 columns (_gemv_nb,
-            # quant_linear_gw.py:850-905); here once per 16 columns, from 17 on per 128
+            # quant_linear_gw.py:850-905); here once per 8 columns, from 9 on per 128
             y = ops.gemv_batch(self.dq, x2, epilogue, resid)
         else:
             y = self.dq.gemv(x2, epilogue, resid)

@@ -458,10 +458,10 @@ class QuantRWKV7:
 
     def launches_per_step(self, batch_size: int = 1) -> int:
         """Kernels one decoded token of ``batch_size`` streams launches.  Per layer, one stream: 2 norm/shift/lerp, r/k/v
-        with the LoRA down projections, time-mix core with the up projections, 3 GEMV.  2 to 16 streams: the LoRA pair
+        with the LoRA down projections, time-mix core with the up projections, 3 GEMV.  2 to 8 streams: the LoRA pair
         in launches of its own.  More: two passes that make fp16 pairs of fp32 rows besides.  Plus embedding, final norm,
         head, argmax (2)."""
-        return self.n_layer * (7 if batch_size == 1 else 9 if batch_size <= 16 else 11) + 5
+        return self.n_layer * (7 if batch_size == 1 else 9 if batch_size <= 8 else 11) + 5
 
     @property
     def launches_per_token(self) -> int:

@@ -317,9 +317,10 @@ struct Fork {
     ~Fork() { if (open) lane->finish(caller); }
 };
 // rwkvq_gemv_batch / rwkvq_gemm with the scratch and the status word apart: the word is only set, `clear` (optional) is zeroed
+// (scratch of gemv_batch_rows_bytes; `pairs` false: it holds the row maxima only)
 size_t gemv_batch_rows_bytes(const rwkvq_qtensor& t, int N);
 int launch_gemv_batch_rows(const rwkvq_qtensor& t, const float* x, int N, long long ldx, float* y, long long ldy, int epilogue,
-                           const float* resid, void* scratch, int* status, int* clear, cudaStream_t s);
+                           const float* resid, void* scratch, int* status, int* clear, cudaStream_t s, bool pairs = true);
 size_t gemm_rows_bytes(const rwkvq_qtensor& t, int M);
 int launch_gemm_rows(const rwkvq_qtensor& t, const float* x, int M, long long ldx, float* y, long long ldy, int epilogue,
                      const float* resid, void* scratch, int* status, int* clear, cudaStream_t s);

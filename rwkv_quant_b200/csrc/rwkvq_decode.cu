@@ -15,7 +15,7 @@
 //   linear + add   output projection and residual
 //   ln_shift_mix   LN2 + token shift + lerp                     -> xk[B][D]
 //   linear + relu^2  ffn key;  linear + add  ffn value and residual
-// Linears: one stream rwkvq_gemv_mma.cu, 2 to 16 rwkvq_gemv_batch.cu, from 17 on rwkvq_gemm_sb.cu (LayerNorms by
+// Linears: one stream rwkvq_gemv_mma.cu, 2 to 8 rwkvq_gemv_batch.cu, from 9 on rwkvq_gemm_sb.cu (LayerNorms by
 // rwkvq_seq.cu, rows as fp16 pairs).
 #include <stdlib.h>
 
@@ -827,16 +827,17 @@ constexpr int kBatchMax = 256;     // streams up to which the small-batch kernel
 inline bool batch_path(int B) { return B > (batch_fast() ? 2 : 1) && B <= kBatchMax; }
 // Single-term operands (RWKVQ_BATCH_FAST=1): the tcgen05 form wins over the mma.sync one from 33 streams on (1.5B, whole
 // step, 64 streams: 3.77 against 4.43 ms) and loses below (32: 2.87 / 2.68 ms, 8: 2.42 / 2.01): its pass (dependent weight
-// loads -> conversion -> MMA) is longer than a warp-iteration.  The default precision is faster from 17 streams on (64: 2.80
-// ms); the mode pays below.
+// loads -> conversion -> MMA) is longer than a warp-iteration.  The default precision is faster from 9 streams on (64: 2.60
+// ms).
 inline bool tcb_pays(int B) { return batch_fast() && tcb_enabled() && B > 32; }
 // Default (two-term) precision: from kSbMinStreams streams on every linear of the step runs on the tcgen05 pipeline
 // (rwkvq_gemm_sb.cu), fed with fp16 pairs and block sums by the LayerNorm kernels and, for the output projection and the
 // ffn value, by a pass over the fp32 rows.  Below, the mma.sync form: few tokens give its 3 MMAs per step little to do.  The
-// line is the mma.sync kernel's second tile of 16 tokens, which doubles its time; at 16 the two are within a few per cent (ms,
-// mma.sync / pipeline: 1.5B sb6 1.92 / 1.90, sym 1.92 / 2.10, 2.9B 3.63 / 3.63 and 3.45 / 3.32), at 4 mma.sync is ahead (1.63 / 1.80).
+// line is that kernel's second tile of 8 tokens (ms, mma.sync / pipeline: 1.5B sb6 at 8 1.67 / 1.71, at 10 1.88 / 1.73, sym 1.71 / 1.66
+// and 1.90 / 1.67, 2.9B sb6 2.77 / 2.88 and 3.35 / 2.90), which also costs it the accumulator of its own that its main sum has
+// up to 8 (error of the logits against 64 bits, sym: 3.2e-6 at 8, 5.2e-6 from 9 on, pipeline 4.1e-6).
 // RWKVQ_TCB_EXACT in the environment (read once) overrides: 0 never, 1 at every batch.
-constexpr int kSbMinStreams = 17;
+constexpr int kSbMinStreams = 9;
 int g_tcb_exact = -2;          // -2 environment not read yet, -1 by stream count, 0 never, 1 always
 bool sb_wanted(int B) {
     if (g_tcb_exact == -2) {

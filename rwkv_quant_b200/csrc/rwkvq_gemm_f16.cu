@@ -717,6 +717,23 @@ int make_half_map(CUtensorMap* map, const __half* base, long long rows, long lon
     return RWKVQ_OK;
 }
 
+int make_byte_map(CUtensorMap* map, const void* base, long long rows, long long row_bytes, int box_bytes, int box_rows) {
+    EncodeTiledFn enc = encode_tiled();
+    RWKVQ_REQUIRE(enc != nullptr, RWKVQ_E_ARCH, "gemm_f16: cuTensorMapEncodeTiled is not available");
+    const cuuint64_t dims[2] = {static_cast<cuuint64_t>(row_bytes), static_cast<cuuint64_t>(rows)};
+    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(row_bytes)};
+    const cuuint32_t box[2] = {static_cast<cuuint32_t>(box_bytes), static_cast<cuuint32_t>(box_rows)};
+    const cuuint32_t estr[2] = {1, 1};
+    const CUtensorMapSwizzle swizzle = box_bytes == 128  ? CU_TENSOR_MAP_SWIZZLE_128B
+                                       : box_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                       : box_bytes == 32 ? CU_TENSOR_MAP_SWIZZLE_32B
+                                                         : CU_TENSOR_MAP_SWIZZLE_NONE;
+    const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    RWKVQ_REQUIRE(r == CUDA_SUCCESS, RWKVQ_E_LAUNCH, "gemm_sb: cuTensorMapEncodeTiled failed (%d)", static_cast<int>(r));
+    return RWKVQ_OK;
+}
+
 // Which kernel and tile: the smallest modelled time of the slowest SM in tensor cycles.  A stage of 64
 // columns costs four MMAs: 512 cycles for the pair's 256-token tile, 200 / 300 for one CTA's 64- / 128-token
 // tile (bound by its shared-memory reads); a launch adds its ramp and the epilogue, a K split the

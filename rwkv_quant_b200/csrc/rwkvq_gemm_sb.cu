@@ -1,4 +1,4 @@
-// Quantized linear for small batches (some 17 to 256 right-hand sides) on the tcgen05 tensor cores at fp32 grade:
+// Quantized linear for small batches (9 to 256 right-hand sides) on the tcgen05 tensor cores at fp32 grade:
 // packed weights converted on the way into the operands, every byte read once per 128 tokens.
 //
 //     y[n, o] = epi( sum_c W[o, c] x[n, c] )
@@ -11,19 +11,22 @@
 // block mins (fp16 by definition) times the block sums of x (as a pair too) are one more MMA of 16 columns per super-block.
 //
 // A CTA owns 128 rows and a K slice (cluster of ks CTAs along K, reduced through distributed shared memory in rank
-// order) and is a pipeline over stages of 64 columns:
-//   warps 0-15   weights, four groups of 128 threads: group g takes stage g of every super-block, a thread one row's 64
-//                columns.  Packed bytes arrive by cp.async in per-thread slots, 8 to 12 stages ahead, so that the HBM
-//                latency of a dependent launch is paid once; p and e go to tensor memory (the A operand of the MMA:
-//                lane = row), so that shared memory carries the activations only (with p and e in shared memory
-//                their stores and the MMAs' reads bound a stage at 0.52 us for 16 tokens, 0.58 for 64, 0.80 for 128)
-//   warp 16      TMA of the activation pairs, which split_rows_kernel or the LayerNorm kernels have made once (converting
-//                in every CTA cost 8 more warps and 0.8 us a stage at 64 tokens)
-//   warp 17      MMAs, the loop run by the whole warp so that descriptors stay in uniform registers (one lane
-//                under a branch: 0.65 us for the nine MMAs of a stage)
+// order) and is a pipeline over units of 128 columns, two of them in flight:
+//   warps 0-15   weights, four groups of 128 threads: group g turns block g (32 columns) of every unit into p and e, a thread
+//                its own row, into tensor memory (the A operand of the MMA: lane = row), so that shared memory carries the
+//                activations only (with p and e there their stores and the MMAs' reads bound 64 columns at 0.52 us)
+//   warp 16      TMA of the activation pairs, which split_rows_kernel or the LayerNorm kernels have made once
+//   warp 17      MMAs, the loop run by the whole warp so that descriptors stay in uniform registers
+//   warp 18      TMA of the packed weights, super-blocks of 256 columns, two ahead; they do not depend on the producer of x
+// Bound: the turn of the MMA warp.  With conversion, stores and MMAs all switched off, a super-block of four units still took 1.6 of its
+// 1.7 us: a wait and a commit are some 400 cycles whatever lies between them.  Hence units of 128 columns with one barrier for
+// all of their weights and activations, and waits that poll: 1.5B step of 64 streams 2.76 -> 2.60 ms, of 100 4.19 -> 3.59 (128 tokens a tile:
+// its MMAs are next, 1.4 us a super-block).  Weights by per-thread cp.async cost the load pipe a line per lane: 2.4 us until
+// the first bytes were asked for, 0.5 by TMA.
 // The mma.sync form of the same product (rwkvq_gemv_batch.cu) issues 3 MMAs of 16 x 8 x 16 per warp and step and tops out
 // at 0.92 G MMA/s per SM.
-// Every mbarrier wait is bounded; on expiry the status word is set and all roles run to the common end.
+// Every mbarrier wait is bounded; a warp whose wait ran out waits no more, the status word is set and all roles run to the
+// common end.
 #include "rwkvq_gemm_sb.cuh"
 
 #include <cooperative_groups.h>
@@ -39,10 +42,10 @@ namespace cg = cooperative_groups;
 
 namespace rwkvq {
 
-constexpr int kSbGroups = 4;                      // = stages of a super-block
-constexpr int kSbWeightThreads = kSbGroups * kGmRows, kSbThreads = kSbWeightThreads + 64;
-constexpr int kSbTmaWarp = kSbWeightThreads / 32, kSbMmaWarp = kSbTmaWarp + 1;
-constexpr int kSbACols = 64;                      // tensor-memory columns of a stage: p 32, e 32
+constexpr int kSbGroups = 4;                      // = blocks of 32 columns in a unit
+constexpr int kSbWeightThreads = kSbGroups * kGmRows, kSbThreads = kSbWeightThreads + 96;
+constexpr int kSbTmaWarp = kSbWeightThreads / 32, kSbMmaWarp = kSbTmaWarp + 1, kSbRawWarp = kSbTmaWarp + 2;
+constexpr int kSbACols = 128;                     // tensor-memory columns of a unit: p 64, e 64
 constexpr uint32_t kSbTmemCols = 512;
 constexpr int kSbPitch = kGmRows + 4;             // partial tile [NT][kSbPitch]
 constexpr int kSbMaxMats = 4;
@@ -63,40 +66,35 @@ struct SbArgs {
     int ks;
     int* status;
 };
-struct SbMaps { CUtensorMap hi[kSbMaxMats], lo[kSbMaxMats]; };
+struct SbMaps { CUtensorMap hi[kSbMaxMats], lo[kSbMaxMats], codes[kSbMaxMats], rec[kSbMaxMats], planes[kSbMaxMats]; };
 
+// A super-block of 128 packed rows in shared memory, as TMA leaves it: codes in boxes of 128 bytes a row and planes, swizzled by
+// the width of their rows so that a thread's 16-byte pieces of its own row meet no bank conflict, and the scale records.
 template <int L>
 struct SbLayout {
     static constexpr bool SB6 = L <= ML_SB6_6;
-    static constexpr int CODE_BYTES = L == ML_SYM8 ? 64 : 32;                      // of a row's stage
-    static constexpr int PLANE_BYTES = L == ML_SB6_5 ? 8 : (L == ML_SB6_6 || L == ML_SYM6) ? 16 : 0;
-    // one stage in shared memory: codes, the scale record and planes, each as columns of 16 (8) bytes a row
-    static constexpr int RAW = kGmRows * (CODE_BYTES + 16 + PLANE_BYTES);
+    static constexpr int CODE_ROW = L == ML_SYM8 ? 256 : 128, PLANE_ROW = L == ML_SB6_5 ? 32 : (L == ML_SB6_6 || L == ML_SYM6) ? 64 : 0;
+    static constexpr int OFF_P = kGmRows * CODE_ROW, OFF_R = OFF_P + kGmRows * PLANE_ROW, RAW = OFF_R + kGmRows * 16;
+    static_assert(RAW % 1024 == 0, "swizzle");
 };
 
 template <int L, int NT>
 struct SbGeo {
-    // Operand buffers: as many as groups, so that a group waits for a buffer it filled itself.  (With three, a group that
-    // ran ahead waited for a phase two ahead of the barrier's, which a parity wait takes for the one just past.)
-    static constexpr int ST = kSbGroups;
-    static constexpr int AHEAD = NT > 64 ? 2 : 3;                    // stages of packed weights a group has in flight
-    static constexpr int BSLAB = 2 * NT * 128;
+    static constexpr int U = 2;                                      // units of operands in flight (three: no gain at 3 to 100 streams)
+    static constexpr int AHEAD = 2;                                  // super-blocks of packed weights in flight (three: no gain either)
+    static constexpr int BATOM = 2 * NT * 128, BSLAB = 2 * BATOM;     // activation pairs of 64 columns, of a unit
     static constexpr int MA = SbLayout<L>::SB6 ? kGmRows * 32 : 0, MB = SbLayout<L>::SB6 ? 2 * NT * 32 : 0;     // min operands of a super-block
     static constexpr int PART = NT * kSbPitch * 4;                   // partial tile of a K slice, over the operands
-    static constexpr int OFF_MA = ST * BSLAB, OFF_MB = OFF_MA + 2 * MA, OFF_RAW = OFF_MB + 2 * MB,
-                         SMEM = OFF_RAW + kSbGroups * AHEAD * SbLayout<L>::RAW;
+    static constexpr int OFF_MA = U * BSLAB, OFF_MB = OFF_MA + 2 * MA, OFF_RAW = OFF_MB + 2 * MB,
+                         SMEM = OFF_RAW + AHEAD * SbLayout<L>::RAW;
     // one CTA per SM: two could wait for each other's tensor memory inside a cluster
     static constexpr size_t BYTES = (SMEM > 119 * 1024 ? SMEM : 119 * 1024) + 1024;
     static_assert(PART <= SMEM, "partial tile");
-    static_assert(2 * NT + ST * kSbACols <= static_cast<int>(kSbTmemCols), "tensor memory");
+    static_assert(2 * NT + U * kSbACols <= static_cast<int>(kSbTmemCols), "tensor memory");
     static_assert(BYTES <= 226 * 1024, "shared memory");
+    static_assert(OFF_RAW % 1024 == 0, "swizzle");
 };
 
-// through L1: the groups read different parts of the same sectors
-template <int BYTES>
-__device__ __forceinline__ void sb_cp(void* dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_addr(dst)), "l"(src), "n"(BYTES) : "memory");
-}
 __device__ __forceinline__ void sb_tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
                  "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
@@ -132,10 +130,10 @@ __device__ __forceinline__ void sb_tmem_ld(uint32_t taddr, float (&v)[NC]) {
     for (int i = 0; i < NC; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// Codes of block b (32 columns) of a stage as bytes in column order; the relayouted planes give the high bits of four
-// codes with one shift and mask.
+// Codes of a block of 32 columns as bytes in column order; its relayouted planes (pl, pl2) give the high bits of four codes with
+// one shift and mask.
 template <int L>
-__device__ __forceinline__ void sb_codes(const uint4& c0, const uint4& c1, const uint4& pl, int b, uint32_t (&bytes)[8]) {
+__device__ __forceinline__ void sb_codes(const uint4& c0, const uint4& c1, uint32_t pl, uint32_t pl2, uint32_t (&bytes)[8]) {
     const uint32_t w[4] = {c0.x, c0.y, c0.z, c0.w};
     if constexpr (SbLayout<L>::SB6) {
 #pragma unroll
@@ -143,13 +141,11 @@ __device__ __forceinline__ void sb_codes(const uint4& c0, const uint4& c1, const
             bytes[i] = w[i] & 0x0F0F0F0Fu;
             bytes[4 + i] = (w[i] >> 4) & 0x0F0F0F0Fu;
             if (L == ML_SB6_5) {
-                const uint32_t p = b ? pl.y : pl.x;
-                bytes[i] |= (p << (4 - i)) & 0x10101010u;
-                bytes[4 + i] |= (p >> i) & 0x10101010u;
+                bytes[i] |= (pl << (4 - i)) & 0x10101010u;
+                bytes[4 + i] |= (pl >> i) & 0x10101010u;
             } else if (L == ML_SB6_6) {
-                const uint32_t p0 = b ? pl.z : pl.x, p1 = b ? pl.w : pl.y;
-                bytes[i] |= (i < 2 ? (p0 << (4 - 2 * i)) : (p0 >> (2 * i - 4))) & 0x30303030u;
-                bytes[4 + i] |= (i < 2 ? (p1 << (4 - 2 * i)) : (p1 >> (2 * i - 4))) & 0x30303030u;
+                bytes[i] |= (i < 2 ? (pl << (4 - 2 * i)) : (pl >> (2 * i - 4))) & 0x30303030u;
+                bytes[4 + i] |= (i < 2 ? (pl2 << (4 - 2 * i)) : (pl2 >> (2 * i - 4))) & 0x30303030u;
             }
         }
     } else if constexpr (L == ML_SYM8) {
@@ -158,8 +154,8 @@ __device__ __forceinline__ void sb_codes(const uint4& c0, const uint4& c1, const
         for (int i = 0; i < 8; ++i) bytes[i] = w8[i] ^ 0x80808080u;          // code + 128
     } else {
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {              // block h of 16: words 2h, 2h + 1; byte k: column k (low), k + 8 (high)
-            const uint32_t p = b ? (h ? pl.w : pl.z) : (h ? pl.y : pl.x);
+        for (int h = 0; h < 2; ++h) {              // block h of 16: words 2h, 2h + 1; byte k: column k (low), column k + 8 (high)
+            const uint32_t p = h ? pl2 : pl;
             bytes[4 * h] = (w[2 * h] & 0x0F0F0F0Fu) | ((p << 4) & 0x30303030u);
             bytes[4 * h + 1] = (w[2 * h + 1] & 0x0F0F0F0Fu) | ((p << 2) & 0x30303030u);
             bytes[4 * h + 2] = ((w[2 * h] >> 4) & 0x0F0F0F0Fu) | (p & 0x30303030u);
@@ -173,17 +169,21 @@ __device__ __forceinline__ __half2 sb_sym_scales(uint32_t two, uint32_t dd) {
     return __hmul2(__hsub2(*reinterpret_cast<const __half2*>(&u), __float2half2_rn(1152.f)), *reinterpret_cast<const __half2*>(&dd));
 }
 
+// a whole warp: one answer, and together again behind it
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity) { return __all_sync(0xFFFFFFFFu, mbar_poll_bounded(bar, parity)); }
+
 template <int L, int NT>
 __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_constant__ SbArgs a, const __grid_constant__ SbMaps maps, const __grid_constant__ Ahead ahead) {
     using G = SbGeo<L, NT>;
     using Y = SbLayout<L>;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    // the operands of a stage are complete (4 weight warps + the TMA bytes) / have been multiplied.  A super-block's min
-    // operands are part of its stages: mins with the weights of each, block sums with the activations of the first.
-    // Two buffers of them need no barrier of their own: the stage that writes buffer s % 2 again has waited for a stage
-    // behind the MMA that read it.
-    __shared__ uint64_t bar_full[G::ST], bar_empty[G::ST], bar_done;
+    // the operands of a unit are complete (16 weight warps + the TMA bytes) / have been multiplied.  A super-block's min
+    // operands are part of its units: mins with the weights of each, block sums with the activations of the first.
+    // Two buffers of them need no barrier of their own: the unit that writes buffer s % 2 again has waited for the MMA that
+    // read it, or for one behind (unit 2 s + 4 - U, U <= 3).
+    __shared__ uint64_t bar_full[G::U], bar_empty[G::U], bar_done;
+    __shared__ uint64_t raw_full[G::AHEAD], raw_empty[G::AHEAD];      // packed weights have arrived / are in registers (16 warps)
     __shared__ uint32_t s_tmem;
     __shared__ volatile int s_fail;
     __shared__ float s_un[NT];
@@ -191,11 +191,12 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int ks = a.ks, z = blockIdx.x % ks, first_tile = blockIdx.x / ks, tile_step = gridDim.x / ks;
     const int nt = NT > 64 ? a.nt : NT, n0 = blockIdx.y * nt, nn = min(nt, a.n_tokens - n0);
-    const int sb0 = a.n_sb * z / ks, n_super = a.n_sb * (z + 1) / ks - sb0, n_stages = n_super * 4;     // this CTA's K slice
+    const int sb0 = a.n_sb * z / ks, n_super = a.n_sb * (z + 1) / ks - sb0;     // this CTA's K slice
     const int n_my = (a.n_tiles - first_tile + tile_step - 1) / tile_step;
 
     if (tid == 0) {
-        for (int s = 0; s < G::ST; ++s) { mbar_init(&bar_full[s], kGmRows / 32 + 1); mbar_init(&bar_empty[s], 1); }
+        for (int s = 0; s < G::U; ++s) { mbar_init(&bar_full[s], kSbWeightThreads / 32 + 1); mbar_init(&bar_empty[s], 1); }
+        for (int s = 0; s < G::AHEAD; ++s) { mbar_init(&raw_full[s], 1); mbar_init(&raw_empty[s], kSbWeightThreads / 32); }
         mbar_init(&bar_done, 1);
         s_fail = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -207,44 +208,8 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
         fence_async_smem();
     }
 
-    // ---- weight threads: group grp takes stage grp of every super-block, thread wrow its row
+    // weight threads: group grp takes block grp of every unit, thread wrow its row
     const int grp = tid / kGmRows, wrow = tid % kGmRows;
-    unsigned char* raw = smem + G::OFF_RAW + (grp % kSbGroups) * G::AHEAD * Y::RAW;
-    constexpr int OFF_R = kGmRows * Y::CODE_BYTES, OFF_H = OFF_R + kGmRows * 16;
-    int c_ti = 0, c_sb = 0, c_slot = 0;                              // copy side: tile of this CTA, super-block, ring slot
-    const uint8_t *c_codes = nullptr, *c_pl = nullptr, *c_meta = nullptr;
-    auto copy_tile = [&]() {                                         // source pointers of tile c_ti
-        const int tile = first_tile + c_ti * tile_step;
-        const QView& t = a.t[tile / a.row_tiles];
-        const size_t R = static_cast<size_t>(min((tile % a.row_tiles) * kGmRows + wrow, t.rows - 1));
-        const int col = sb0 * 256 + grp * 64;
-        c_codes = t.codes + (L == ML_SYM8 ? R * t.cols + col : R * (t.cols >> 1) + (col >> 1));
-        // planes: 4 bytes per 32 columns (5 bits), 8 per 32 (6 bits; sym as 4 per 16)
-        if (Y::PLANE_BYTES) c_pl = reinterpret_cast<const uint8_t*>(t.dev_planes) + R * (t.cols >> 6) * Y::PLANE_BYTES + (col >> 6) * Y::PLANE_BYTES;
-        c_meta = Y::SB6 ? t.dev_meta + (R * (t.cols >> 8) + sb0) * 16 : reinterpret_cast<const uint8_t*>(t.qs) + R * (t.cols >> 4) + sb0 * 16;
-    };
-    auto copy_stage = [&]() {
-        if (c_ti < n_my) {
-            unsigned char* slot = raw + c_slot * Y::RAW;
-#pragma unroll
-            for (int k = 0; k < Y::CODE_BYTES / 16; ++k) sb_cp<16>(slot + k * (kGmRows * 16) + wrow * 16, c_codes + 16 * k);
-            sb_cp<16>(slot + OFF_R + wrow * 16, c_meta);
-            if constexpr (Y::PLANE_BYTES > 0) sb_cp<Y::PLANE_BYTES>(slot + OFF_H + wrow * Y::PLANE_BYTES, c_pl);
-            c_codes += L == ML_SYM8 ? 256 : 128;
-            c_meta += 16;
-            c_pl += 4 * Y::PLANE_BYTES;
-            c_slot = c_slot == G::AHEAD - 1 ? 0 : c_slot + 1;
-            if (++c_sb == n_super) {
-                c_sb = 0;
-                if (++c_ti < n_my) copy_tile();
-            }
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");         // empty groups keep the count uniform
-    };
-    if (tid < kSbWeightThreads) {                                    // weights do not depend on the producer of x
-        copy_tile();
-        for (int i = 0; i < G::AHEAD; ++i) copy_stage();
-    }
     if (warp == kSbTmaWarp) ahead_prefetch(ahead, blockIdx.x + gridDim.x * blockIdx.y, gridDim.x * gridDim.y);
     tc_fence_before();
     __syncthreads();
@@ -252,8 +217,9 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
     const uint32_t tmem = s_tmem;
     if (warp == kSbTmaWarp) pdl_wait();                              // the activations; the others wait before they read or store
 
-    int r_slot = 0;                                                  // read side of the weight ring
-    int it = 0;                                                      // stages of the tiles before
+    int sb_before = 0;                                               // super-blocks of the tiles before
+    bool alive = true;                                               // no wait of this warp has run out
+    int raw_issued = 0;                                              // super-blocks asked for (the thread that does)
     uint32_t done_phase = 0;
     for (int ti = 0; ti < n_my; ++ti) {
         const int tile = first_tile + ti * tile_step, mat = tile / a.row_tiles, row0 = (tile % a.row_tiles) * kGmRows;
@@ -268,49 +234,71 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
             for (int n = lane; n < nt; n += 32) s_un[n] = n < nn ? __ldcg(a.unscale[mat] + n0 + n) : 0.f;   // read behind bar_done
             uint32_t elected;
             asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xFFFFFFFF;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(elected));
-            bool ok = true;
-            int st = it % G::ST, ph = (it / G::ST) & 1;
-            for (int i = 0; i < n_stages; ++i) {
-                if (!mbar_wait_bounded(&bar_full[st], ph)) { ok = false; break; }
+            int buf = (2 * sb_before) % G::U, ph = (2 * sb_before / G::U) & 1;
+            for (int u = 0; u < 2 * n_super; ++u) {
+                alive = alive && warp_wait(&bar_full[buf], ph);
+                if (!alive) break;
                 tc_fence_after();
-                const uint32_t pa = tmem + 2 * NT + st * kSbACols, ea = pa + kSbACols / 2;
-                const uint64_t bd = b0 + (static_cast<uint64_t>(st * G::BSLAB) >> 4);
+                const uint32_t pa = tmem + 2 * NT + buf * kSbACols, ea = pa + kSbACols / 2;
+                const uint64_t bd = b0 + (static_cast<uint64_t>(buf * G::BSLAB) >> 4);
                 if (elected) {
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {                    // e meets the high halves only (e lo is below 2^-22), beside p lo
-                        umma_f16_ta(tmem, pa + 8 * k, bd + 2 * k, id2, (i | k) ? 1u : 0u);
-                        umma_f16_ta(tmem + nt, ea + 8 * k, bd + 2 * k, id1, 1u);
+                    for (int k = 0; k < 8; ++k) {                    // e meets the high halves only (e lo is below 2^-22), beside p lo
+                        const uint64_t bk = bd + (static_cast<uint64_t>((k >> 2) * G::BATOM) >> 4) + 2 * (k & 3);
+                        umma_f16_ta(tmem, pa + 8 * k, bk, id2, (u | k) ? 1u : 0u);
+                        umma_f16_ta(tmem + nt, ea + 8 * k, bk, id1, 1u);
                     }
-                    if (Y::SB6 && (i & 3) == 3) {                    // the super-block's mins are complete with its last stage
-                        const int ms = ((it + i) >> 2) & 1;
+                    if (Y::SB6 && (u & 1)) {                         // the super-block's mins are complete with its second unit
+                        const int ms = (sb_before + (u >> 1)) & 1;
                         umma_f16(tmem, ma0 + (static_cast<uint64_t>(ms * G::MA) >> 4), mb0 + (static_cast<uint64_t>(ms * G::MB) >> 4), id2, 1u);
                     }
-                    umma_commit(&bar_empty[st]);
+                    umma_commit(&bar_empty[buf]);
                 }
                 __syncwarp();
-                if (++st == G::ST) { st = 0; ph ^= 1; }
+                if (++buf == G::U) { buf = 0; ph ^= 1; }
             }
-            if (ok && elected) umma_commit(&bar_done);
-            if (!ok) s_fail = 1;
+            if (alive && elected) umma_commit(&bar_done);
+        } else if (warp == kSbRawWarp) {
+            // ------------------------------------------------------------------ packed weights: do not depend on the producer of x
+            if (lane == 0) {
+                for (int sb = 0; sb < n_super; ++sb) {
+                    const int qi = sb_before + sb, slot = qi % G::AHEAD;
+                    alive = alive && (qi < G::AHEAD || mbar_poll_bounded(&raw_empty[slot], (qi / G::AHEAD - 1) & 1));
+                    if (!alive) break;
+                    unsigned char* w = smem + G::OFF_RAW + slot * Y::RAW;
+                    mbar_expect_tx(&raw_full[slot], Y::RAW);
+#pragma unroll
+                    for (int c = 0; c < Y::CODE_ROW / 128; ++c)
+                        tma_load_2d(w + c * (kGmRows * 128), &maps.codes[mat], (sb0 + sb) * Y::CODE_ROW + c * 128, row0, &raw_full[slot]);
+                    if (Y::PLANE_ROW > 0) tma_load_2d(w + Y::OFF_P, &maps.planes[mat], (sb0 + sb) * Y::PLANE_ROW, row0, &raw_full[slot]);
+                    tma_load_2d(w + Y::OFF_R, &maps.rec[mat], (sb0 + sb) * 16, row0, &raw_full[slot]);
+                    raw_issued = qi + 1;
+                }
+            }
         } else if (warp == kSbTmaWarp) {
             // ------------------------------------------------------------------ activation pairs
             if (lane == 0) {
-                for (int i = 0; i < n_stages; ++i) {
-                    const int g = it + i, st = g % G::ST;
-                    if (g >= G::ST && !mbar_wait_bounded(&bar_empty[st], (g / G::ST - 1) & 1)) { s_fail = 1; break; }
-                    unsigned char* b = smem + st * G::BSLAB;
-                    const bool with_sums = Y::SB6 && (i & 3) == 0;
-                    mbar_expect_tx(&bar_full[st], 2 * nt * 128 + (with_sums ? 2 * nn * 16 : 0));
-                    tma_load_2d(b, &maps.hi[mat], sb0 * 256 + i * 64, n0, &bar_full[st]);
-                    tma_load_2d(b + nt * 128, &maps.lo[mat], sb0 * 256 + i * 64, n0, &bar_full[st]);
+                for (int u = 0; u < 2 * n_super; ++u) {
+                    const int g = 2 * sb_before + u, buf = g % G::U;
+                    alive = alive && (g < G::U || mbar_poll_bounded(&bar_empty[buf], (g / G::U - 1) & 1));
+                    if (!alive) break;
+                    unsigned char* b = smem + buf * G::BSLAB;
+                    const bool with_sums = Y::SB6 && (u & 1) == 0;
+                    mbar_expect_tx(&bar_full[buf], 4 * nt * 128 + (with_sums ? 2 * nn * 16 : 0));
+#pragma unroll
+                    for (int c = 0; c < 2; ++c) {
+                        const int x = sb0 * 256 + u * 128 + c * 64;
+                        tma_load_2d(b + c * G::BATOM, &maps.hi[mat], x, n0, &bar_full[buf]);
+                        tma_load_2d(b + c * G::BATOM + nt * 128, &maps.lo[mat], x, n0, &bar_full[buf]);
+                    }
                     if (with_sums) {
-                        unsigned char* m = smem + G::OFF_MB + ((g >> 2) & 1) * G::MB;
+                        unsigned char* m = smem + G::OFF_MB + ((g >> 1) & 1) * G::MB;
 #pragma unroll
                         for (int h = 0; h < 2; ++h)
                             asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                                              smem_addr(m + h * nt * 16)),
-                                         "l"(a.sums[mat] + ((static_cast<size_t>(sb0 + (i >> 2)) * 2 + h) * a.n_tokens + n0) * 8), "r"(nn * 16),
-                                         "r"(smem_addr(&bar_full[st]))
+                                         "l"(a.sums[mat] + ((static_cast<size_t>(sb0 + (u >> 1)) * 2 + h) * a.n_tokens + n0) * 8), "r"(nn * 16),
+                                         "r"(smem_addr(&bar_full[buf]))
                                          : "memory");
                     }
                 }
@@ -324,79 +312,93 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
             const uint32_t lane_base = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + 2 * NT;
 #pragma unroll 1
             for (int sb = 0; sb < n_super; ++sb) {
-                const int g = it + 4 * sb + grp, st = g % G::ST;
-                asm volatile("cp.async.wait_group %0;" ::"n"(G::AHEAD - 1) : "memory");
-                const unsigned char* slot = raw + r_slot * Y::RAW;
-                r_slot = r_slot == G::AHEAD - 1 ? 0 : r_slot + 1;
-                constexpr int CB = Y::CODE_BYTES / 32;               // 16-byte pieces of a block
-                uint4 code[2 * CB], pl = make_uint4(0, 0, 0, 0);
+                const int qi = sb_before + sb, slot = qi % G::AHEAD;
+                alive = alive && warp_wait(&raw_full[slot], (qi / G::AHEAD) & 1);
+                const unsigned char* raw = smem + G::OFF_RAW + slot * Y::RAW;
+                // blocks grp and 4 + grp of the super-block
+                uint4 code[2], code2[2];
+                uint32_t pl[2] = {0u, 0u}, pl2[2] = {0u, 0u};
 #pragma unroll
-                for (int k = 0; k < 2 * CB; ++k) code[k] = *reinterpret_cast<const uint4*>(slot + k * (kGmRows * 16) + wrow * 16);
-                if (Y::PLANE_BYTES == 16) pl = *reinterpret_cast<const uint4*>(slot + OFF_H + wrow * 16);
-                if (Y::PLANE_BYTES == 8) {
-                    const uint2 p2 = *reinterpret_cast<const uint2*>(slot + OFF_H + wrow * 8);
-                    pl.x = p2.x; pl.y = p2.y;
+                for (int h = 0; h < 2; ++h) {
+                    if (Y::CODE_ROW == 128) {
+                        code[h] = code2[h] = *reinterpret_cast<const uint4*>(raw + wrow * 128 + (((4 * h + grp) ^ (wrow & 7)) << 4));
+                    } else {                                         // 32 bytes a block, four blocks a box
+                        const unsigned char* crow = raw + h * (kGmRows * 128) + wrow * 128;
+                        code[h] = *reinterpret_cast<const uint4*>(crow + (((2 * grp) ^ (wrow & 7)) << 4));
+                        code2[h] = *reinterpret_cast<const uint4*>(crow + (((2 * grp + 1) ^ (wrow & 7)) << 4));
+                    }
+                    if (Y::PLANE_ROW == 64) {                        // 8 bytes a block
+                        const uint4 p4 = *reinterpret_cast<const uint4*>(raw + Y::OFF_P + wrow * 64 + (((2 * h + (grp >> 1)) ^ ((wrow >> 1) & 3)) << 4));
+                        pl[h] = grp & 1 ? p4.z : p4.x;
+                        pl2[h] = grp & 1 ? p4.w : p4.y;
+                    }
+                    if (Y::PLANE_ROW == 32) {                        // 4 bytes a block
+                        const uint4 p4 = *reinterpret_cast<const uint4*>(raw + Y::OFF_P + wrow * 32 + ((h ^ ((wrow >> 2) & 1)) << 4));
+                        pl[h] = word_of(p4, grp);
+                    }
                 }
-                const uint4 rec = *reinterpret_cast<const uint4*>(slot + OFF_R + wrow * 16);
-                // scales of the stage's columns by quarters of 16, and the mins of its two blocks; fp16 values by the codec's
-                // definition: one half-precision multiply of the exact small integer
-                __half2 s4[2], mins = __float2half2_rn(0.f);
-                if (Y::SB6) {
-                    __half2 hs;
-                    sb6_pair_scales_h2(rec, grp, hs, mins);
-                    s4[0] = __low2half2(hs);
-                    s4[1] = __high2half2(hs);
-                } else {
-                    const uint32_t w = (grp & 2) ? ((grp & 1) ? rec.w : rec.z) : ((grp & 1) ? rec.y : rec.x), dd = d_next * 0x00010001u;
-                    if (sb + 1 < n_super) d_next = __half_as_ushort(__ldg(dp + sb + 1));
-                    s4[0] = sb_sym_scales(w & 0xFFFFu, dd);
-                    s4[1] = sb_sym_scales(w >> 16, dd);
-                }
-                if (g >= G::ST) {                                    // the MMAs that read this buffer have completed
-                    if (lane == 0 && !s_fail && !mbar_wait_bounded(&bar_empty[st], (g / G::ST - 1) & 1)) s_fail = 1;
-                    __syncwarp();
-                    tc_fence_after();
-                }
-                const uint32_t ta = lane_base + st * kSbACols;
+                const uint4 rec = *reinterpret_cast<const uint4*>(raw + Y::OFF_R + wrow * 16);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&raw_empty[slot]);        // the super-block is in registers
+                const uint32_t dd = d_next * 0x00010001u;
+                if (!Y::SB6 && sb + 1 < n_super) d_next = __half_as_ushort(__ldg(dp + sb + 1));
 #pragma unroll
-                for (int b = 0; b < 2; ++b) {
+                for (int h = 0; h < 2; ++h) {
+                    const int g = 2 * qi + h, buf = g % G::U;
+                    // scales of the block's halves of 16 columns and its min; fp16 values by the codec's definition: one half-precision
+                    // multiply of the exact small integer
+                    __half2 s_lo, s_hi, mins = __float2half2_rn(0.f);
+                    if (Y::SB6) {
+                        __half2 hs;
+                        sb6_pair_scales_h2(rec, 2 * h + (grp >> 1), hs, mins);
+                        s_lo = s_hi = grp & 1 ? __high2half2(hs) : __low2half2(hs);
+                    } else {
+                        const uint32_t w = h ? (grp & 2 ? rec.w : rec.z) : (grp & 2 ? rec.y : rec.x);
+                        const __half2 s4 = sb_sym_scales(grp & 1 ? w >> 16 : w & 0xFFFFu, dd);
+                        s_lo = __low2half2(s4);
+                        s_hi = __high2half2(s4);
+                    }
                     uint32_t bytes[8], pw[16], ew[16];
-                    sb_codes<L>(code[CB * b], code[CB * b + CB - 1], pl, b, bytes);
+                    sb_codes<L>(code[h], code2[h], pl[h], pl2[h], bytes);
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
-                        const __half2 s2 = Y::SB6 ? s4[b] : (j < 4 ? __low2half2(s4[b]) : __high2half2(s4[b]));
                         uint2 pa, ea;
-                        bytes_to_half4_pair(bytes[j], bias, s2, pa, ea);
+                        bytes_to_half4_pair(bytes[j], bias, j < 4 ? s_lo : s_hi, pa, ea);
                         pw[2 * j] = pa.x; pw[2 * j + 1] = pa.y;
                         ew[2 * j] = ea.x; ew[2 * j + 1] = ea.y;
                     }
-                    sb_tmem_st16(ta + 16 * b, pw);
-                    sb_tmem_st16(ta + kSbACols / 2 + 16 * b, ew);
+                    if (g >= G::U) {                                 // the MMAs that read this buffer have completed
+                        alive = alive && warp_wait(&bar_empty[buf], (g / G::U - 1) & 1);
+                        tc_fence_after();
+                    }
+                    const uint32_t ta = lane_base + buf * kSbACols + 16 * grp;
+                    sb_tmem_st16(ta, pw);
+                    sb_tmem_st16(ta + kSbACols / 2, ew);
+                    if (Y::SB6) {
+                        *reinterpret_cast<__half*>(smem + G::OFF_MA + (qi & 1) * G::MA + wrow * 16 + (4 * h + grp) * 2) =
+                            grp & 1 ? __high2half(mins) : __low2half(mins);
+                        fence_async_smem();
+                    }
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&bar_full[buf]);
                 }
-                if (Y::SB6) {
-                    *reinterpret_cast<__half2*>(smem + G::OFF_MA + ((g >> 2) & 1) * G::MA + wrow * 16 + grp * 4) = mins;
-                    fence_async_smem();
-                }
-                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&bar_full[st]);
-                copy_stage();
             }
         }
-        it += n_stages;
+        sb_before += n_super;
         // ---------------------------------------------------------------------- epilogue of the tile
         __syncwarp();
-        if (warp != kSbTmaWarp) {
-            if (lane == 0 && !s_fail && !mbar_wait_bounded(&bar_done, done_phase)) s_fail = 1;
-            __syncwarp();
+        if (warp != kSbTmaWarp && warp != kSbRawWarp) {
+            alive = alive && warp_wait(&bar_done, done_phase);
             done_phase ^= 1;
             tc_fence_after();
             if (ti == 0) pdl_wait();                                 // token scales, residual, output
         }
         constexpr int TC = NT < 64 ? NT / 4 : 16;                    // tokens a warp takes at a time; four warps share a lane quadrant
         const int q = warp & 3, tg = warp >> 2, rl = q * 32 + lane, row = row0 + rl;
-        const bool row_ok = row < t.rows && !s_fail;
+        if (!alive) s_fail = 1;
+        const bool row_ok = row < t.rows && alive && !s_fail;
         float* y = a.y[mat] + static_cast<size_t>(n0) * a.ldy + row;
         const float* rs = a.resid[mat] ? a.resid[mat] + static_cast<size_t>(n0) * a.ldy + row : nullptr;
         float* am_out = a.amax_out[mat] ? a.amax_out[mat] + n0 : nullptr;
@@ -446,7 +448,7 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
                 tc_fence_before();
             }
             // the accumulator is free for the next tile
-            if (warp != kSbTmaWarp) asm volatile("bar.sync 1, %0;" ::"n"(kSbThreads - 32) : "memory");
+            if (warp != kSbTmaWarp && warp != kSbRawWarp) asm volatile("bar.sync 1, %0;" ::"n"(kSbThreads - 64) : "memory");
             tc_fence_after();
         } else {
             float* part = reinterpret_cast<float*>(smem);            // every MMA that read the operands has completed
@@ -496,7 +498,9 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
             cluster.sync();                                          // nobody leaves while a peer still reads its partial tile
         }
     }
-    if (tid < kSbWeightThreads) asm volatile("cp.async.wait_all;" ::: "memory");
+    // where a wait ran out, copies may still be on their way
+    if (s_fail && warp == kSbRawWarp && lane == 0)
+        for (int qi = max(0, raw_issued - G::AHEAD); qi < raw_issued; ++qi) mbar_poll_bounded(&raw_full[qi % G::AHEAD], (qi / G::AHEAD) & 1);
     __syncthreads();
     if (tid == 0 && s_fail) atomicCAS(a.status, 0, RWKVQ_E_TIMEOUT);
     tc_fence_after();
@@ -641,10 +645,11 @@ bool gemm_sb_ok(const rwkvq_qtensor& t) {
     return gemm_tcb_ok(t) && (t.kind == RWKVQ_KIND_SB6 || t.kind == RWKVQ_KIND_SYM) && mma_layout_of(t) >= 0 && aligned(t.codes, 16) &&
            aligned(t.kind == RWKVQ_KIND_SB6 ? static_cast<const void*>(t.dev_meta) : static_cast<const void*>(t.qs), 16) && aligned(t.dev_planes, 16);
 }
-// Whether this kernel takes a product the mma.sync kernel serves too.  That one stages the activations per row group,
-// which costs it as much as the conversion to tensor memory costs this one up to 16 rows ([2048, 2048] 14.3 against 18 us,
-// [8192, 2048] and [2048, 8192] 17 both); from there its time doubles with every 16 rows and this one's stays.
-constexpr int kSbLeastRows = 17;
+// Whether this kernel takes a product the mma.sync kernel serves too: from that one's second tile of 8 rows on (us at 9 rows,
+// mma.sync / this, sb6 4 bits: [2048, 2048] 10.3 / 8.0, [8192, 2048] 14.3 / 12.0, [2048, 8192] 17.5 / 15.1, [2560, 10240] 29.5 / 17.5; at 8
+// mma.sync 8.8, 12.6, 17.1 and 21.7).  Up to 8 rows it keeps its main sum in an accumulator without the low terms
+// and is the more precise.
+constexpr int kSbLeastRows = 9;
 bool gemm_sb_pays(const rwkvq_qtensor& t, int N) {
     return tcb_enabled() && gemm_sb_ok(t) && N >= kSbLeastRows;
 }
@@ -672,6 +677,16 @@ int launch_gemm_sb(const rwkvq_qtensor* ts, int n_mats, const SbRows* rows, int 
         int rc = make_half_map(&maps.hi[k], rows[k].hi, N, ts[0].cols, rows[k].pitch, nt);
         if (rc) return rc;
         rc = make_half_map(&maps.lo[k], rows[k].lo, N, ts[0].cols, rows[k].pitch, nt);
+        if (rc) return rc;
+        const rwkvq_qtensor& t = ts[k];
+        const long long nsb = t.cols / 256;
+        const bool sb6 = t.kind == RWKVQ_KIND_SB6, byte_codes = !sb6 && t.bits == 8;
+        const int plane_row = sb6 ? (t.bits == 5 ? 32 : t.bits == 6 ? 64 : 0) : (t.bits == 6 ? 64 : 0);
+        rc = make_byte_map(&maps.codes[k], t.codes, t.rows, nsb * (byte_codes ? 256 : 128), 128, kGmRows);
+        if (rc) return rc;
+        rc = make_byte_map(&maps.rec[k], sb6 ? t.dev_meta : t.qs, t.rows, nsb * 16, 16, kGmRows);
+        if (rc) return rc;
+        if (plane_row) rc = make_byte_map(&maps.planes[k], t.dev_planes, t.rows, nsb * plane_row, plane_row, kGmRows);
         if (rc) return rc;
     }
     a.ldy = ldy; a.n_tokens = N; a.epilogue = epilogue; a.status = status;

@@ -71,5 +71,8 @@ bool gemm_sb_ok(const rwkvq_qtensor& t);                  // sb6 / sym with the 
 bool gemm_sb_pays(const rwkvq_qtensor& t, int N);
 // tensor map of an fp16 matrix: boxes of 64 columns x box_rows, 128-byte swizzle, zero fill (rwkvq_gemm_f16.cu)
 int make_half_map(CUtensorMap* map, const __half* base, long long rows, long long cols, long long pitch, int box_rows);
+// tensor map of packed rows of row_bytes (a multiple of 16): boxes of 16, 32, 64 or 128 bytes x box_rows, swizzled by their width
+// (16: not), zero fill
+int make_byte_map(CUtensorMap* map, const void* base, long long rows, long long row_bytes, int box_bytes, int box_rows);
 
 }  // namespace rwkvq

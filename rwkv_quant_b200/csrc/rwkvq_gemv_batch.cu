@@ -1,4 +1,4 @@
-// Quantized linear for a small batch of right-hand sides (2 to 16 decode streams, short verify
+// Quantized linear for a small batch of right-hand sides (2 to 8 decode streams, short verify
 // runs; more on tensors without the tcgen05 form or with single-term operands): every packed weight byte is read ONCE for the whole batch.
 //
 //     y[n, o] = epi( sum_c W[o, c] x[n, c] ),   n < N
@@ -755,6 +755,7 @@ extern "C" void rwkvq_profiling_batch_force(int force_ks, int rows, int cols) {
 // [status word, padded to 256 bytes][N floats: max|x| per row, or 2^-s of the pairs][pairs of up to kPairCols columns]
 namespace {
 constexpr int kPairCols = 16384;
+constexpr int kPairsOptional = 16;
 inline size_t batch_ws_pairs(int N) { return 256 + ((static_cast<size_t>(N) * sizeof(float) + 255) / 256) * 256; }
 }
 // whether the product runs on the tcgen05 pipeline, which reads the rows as pairs
@@ -766,23 +767,25 @@ bool batch_on_pipeline(const rwkvq_qtensor& t, int N) {
 extern "C" size_t rwkvq_gemv_batch_workspace_bytes(int N) { return N > 0 ? batch_ws_pairs(N) + sb_halves(N, kPairCols) * sizeof(__half) : 0; }
 extern "C" size_t rwkvq_gemv_batch_workspace_bytes_of(const rwkvq_qtensor* t, int N) {
     if (!t || N < 1) return 0;
-    return 256 + gemv_batch_rows_bytes(*t, N);
+    // what a call needs: up to 16 rows the row maxima (with room for the pairs it takes the pipeline from 9 on all the same)
+    return N <= kPairsOptional ? batch_ws_pairs(N) : 256 + gemv_batch_rows_bytes(*t, N);
 }
 size_t rwkvq::gemv_batch_rows_bytes(const rwkvq_qtensor& t, int N) {
     return batch_ws_pairs(N) - 256 + (batch_on_pipeline(t, N) ? sb_halves(N, t.cols) * sizeof(__half) : 0);
 }
 
 // The product on rows whose scale is not known: a pass that measures (or splits) them, then the kernel that pays
-// (scratch: gemv_batch_rows_bytes, 16-byte aligned; clear, optional: a status word of the product's own).
+// (scratch: gemv_batch_rows_bytes, without `pairs` that of the row maxima, 16-byte aligned; clear, optional: a status word of the
+// product's own).
 int rwkvq::launch_gemv_batch_rows(const rwkvq_qtensor& t, const float* x, int N, long long ldx, float* y, long long ldy, int epilogue,
-                                  const float* resid, void* scratch, int* status, int* clear, cudaStream_t s) {
+                                  const float* resid, void* scratch, int* status, int* clear, cudaStream_t s, bool pairs) {
     // default: the two-term mma.sync kernel below kSbLeastRows rows, the tcgen05 pipeline from there on (gemm_sb_pays);
     // single-term operands: mma.sync up to 32 rows, the single-buffer tcgen05 kernel above
     const bool tcb_ok = tcb_enabled() && gemm_tcb_ok(t);
     // tensors without the relayouted streams: the tcgen05 kernel that reads the file buffers, in either precision
     const bool bare = mma_layout_of(t) < 0;
     const bool tcb = tcb_ok && ldx % 8 == 0 && (bare || (batch_fast() && (N > 32 || tcb_forced())));
-    const bool sb = batch_on_pipeline(t, N);
+    const bool sb = pairs && batch_on_pipeline(t, N);
     RWKVQ_REQUIRE(tcb || sb || mma_layout_of(t) >= 0, RWKVQ_E_DTYPE,
                   "rwkvq_gemv_batch: needs an sb6 tensor, a sym tensor or per-row int8 with columns in multiples of 128");
     float* amax = static_cast<float*>(scratch);
@@ -816,6 +819,6 @@ extern "C" int rwkvq_gemv_batch(const rwkvq_qtensor* t, const float* x, int N, i
                   "rwkvq_gemv_batch: workspace of %zu bytes, %zu needed", workspace_bytes, rwkvq_gemv_batch_workspace_bytes_of(t, N));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     rc = launch_gemv_batch_rows(*t, x, N, ldx, y, ldy, epilogue, resid, static_cast<char*>(workspace) + 256, static_cast<int*>(workspace),
-                                static_cast<int*>(workspace), s);
+                                static_cast<int*>(workspace), s, workspace_bytes >= 256 + gemv_batch_rows_bytes(*t, N));
     return rc ? rc : check_launch("rwkvq_gemv_batch");
 }

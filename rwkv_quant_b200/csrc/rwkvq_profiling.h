@@ -30,7 +30,7 @@ void rwkvq_profiling_batch_fast(int fast);
 void rwkvq_profiling_zero_skip(int on);
 /* Decode step in the default precision: 1 runs every linear on the tcgen05 pipeline from 3 streams on (what
  * RWKVQ_TCB_EXACT=1 selects), 0 keeps them on mma.sync (RWKVQ_TCB_EXACT=0), -1 reads the environment again
- * (unset: from 17 streams on). */
+ * (unset: from 9 streams on). */
 void rwkvq_profiling_tcb_exact(int on);
 #ifdef __cplusplus
 }

@@ -36,6 +36,21 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
     }
     return false;
 }
+// The same for waits that are mostly short: a wait that may suspend takes some 150 cycles longer to notice a phase, complete
+// already or not.
+constexpr unsigned kGmPolls = 64;
+__device__ __forceinline__ bool mbar_poll_bounded(uint64_t* bar, uint32_t parity) {
+    const uint32_t a = smem_addr(bar);
+    for (unsigned i = 0; i < kGmPolls; ++i) {
+        uint32_t done;
+        asm volatile("{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+                     : "=r"(done)
+                     : "r"(a), "r"(parity)
+                     : "memory");
+        if (done) return true;
+    }
+    return mbar_wait_bounded(bar, parity);
+}
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
 }

@@ -55,3 +55,25 @@ def test_error_of_a_long_chain(cuda_lib, N):
     want = x.double() @ dq.dequant().double().t()
     err = (ops.gemv_batch(dq, x, check=True).double() - want).norm() / want.norm()
     assert err <= 128 * 2.0 ** -25, float(err)
+
+
+@pytest.mark.parametrize("layout,bits", [("sb6", 5), ("sym", 6)])
+@pytest.mark.parametrize("N", [8, 9, 16, 17])
+def test_either_workspace_serves_a_call(cuda_lib, layout, bits, N):
+    """9 to 16 rows take the kernel that the scratch has room for; both are fp32 grade (2e-5, as above)."""
+    import ctypes as C
+    from rwkv_quant_b200 import _lib
+    from rwkv_quant_b200.backends.cuda import ops
+    lib, dq = _lib.load(), ops.DeviceQT(_synth_linear(layout, bits, 300, 768, seed=N))
+    x = _x(N, 768, seed=N)
+    ref = x.cpu().numpy().astype(np.float64) @ _oracle_w(_synth_linear(layout, bits, 300, 768, seed=N)).astype(np.float64).T
+    least = lib.rwkvq_gemv_batch_workspace_bytes_of(dq.struct_ref, N)
+    for nws in (least, lib.rwkvq_gemv_batch_workspace_bytes(N)):
+        y, ws = torch.empty(N, 300, device="cuda"), torch.empty(nws, dtype=torch.uint8, device="cuda")
+        _lib.check(lib.rwkvq_gemv_batch(dq.struct_ref, x.data_ptr(), N, x.stride(0), y.data_ptr(), 300, 0, None, ws.data_ptr(), nws,
+                                        _lib.stream_ptr()), "rwkvq_gemv_batch")
+        assert int(ws[:4].view(torch.int32).item()) == 0
+        assert relmax(y.cpu().numpy(), ref) <= 2e-5
+    ws = torch.empty(least - 1, dtype=torch.uint8, device="cuda")
+    assert lib.rwkvq_gemv_batch(dq.struct_ref, x.data_ptr(), N, x.stride(0), y.data_ptr(), 300, 0, None, ws.data_ptr(), least - 1,
+                                _lib.stream_ptr()) != 0
