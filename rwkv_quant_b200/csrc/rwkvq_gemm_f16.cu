@@ -189,26 +189,42 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// bound of the squared norm of any row of W (fp16 hidden rows only)
+__device__ __forceinline__ float warp_w_n2(const HgDev& p, int lane) {
+    float w2 = 0.f;
+    if (p.out == HG_RELU2_F16) {
+        for (int i = lane; i < p.n_w_n2; i += 32) w2 += __ldcg(p.w_n2 + i);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) w2 += __shfl_xor_sync(0xFFFFFFFFu, w2, o);
+    }
+    return w2;
+}
 // Power of two that brings relu(y)^2 of a token below 2^14 whatever row of W meets it (Cauchy-Schwarz);
 // rows without a finite bound keep 1 and propagate.
-__device__ __forceinline__ float relu2_scale(const HgDev& p, int tok) {
-    float w2 = 0.f;
-    for (int i = 0; i < p.n_w_n2; ++i) w2 += __ldcg(p.w_n2 + i);
-    const float b2 = w2 * __ldcg(p.x_n2 + tok);          // bound of y^2
+__device__ __forceinline__ float relu2_scale(float w2, float x_n2) {
+    const float b2 = w2 * x_n2;                          // bound of y^2
     int e = 0;
     if (!(b2 > 0.f && b2 < INFINITY)) return 1.f;
     frexpf(b2, &e);                                      // b2 < 2^e; rounding of the sums stays within the headroom to 65504
     return ldexpf(1.f, max(-100, min(100, 14 - e)));
 }
 
-// Per-token factors of a tile, one token per lane: what the accumulator is multiplied with, and (fp16
-// output) the scale of the stored value.
-__device__ __forceinline__ void token_factors(const HgDev& p, int tok, int M, float& un, float& so) {
-    un = 1.f;
-    so = 1.f;
-    if (tok < M) {
-        if (p.row_scale != nullptr) un = 1.0f / __ldcg(p.row_scale + tok);      // exact: powers of two
-        if (p.out == HG_RELU2_F16) so = relu2_scale(p, tok);
+// Per-token factors of N blocks of 32 tokens `step` apart, one token per lane and block: what the accumulator is multiplied
+// with, and (fp16 output) the scale of the stored value.
+template <int N>
+__device__ __forceinline__ void token_factors(const HgDev& p, int tok, int step, int M, int lane, float (&un)[N], float (&so)[N]) {
+    float rs[N], n2[N];
+    const float w2 = warp_w_n2(p, lane);
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const int t = tok + i * step;
+        rs[i] = t < M && p.row_scale != nullptr ? __ldcg(p.row_scale + t) : 1.f;
+        n2[i] = t < M && p.out == HG_RELU2_F16 ? __ldcg(p.x_n2 + t) : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        un[i] = 1.0f / rs[i];                            // exact: powers of two
+        so[i] = relu2_scale(w2, n2[i]);
     }
 }
 
@@ -326,14 +342,17 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
 
 constexpr int kHgABytes = kGmRows * 128;                 // one CTA's weight tile of a stage: 128 rows x 64 columns
 constexpr int kHgThreads = 256;
-constexpr int kPairStages = 6, kPairTok = 256;
+constexpr int kPairStages = 6, kPairTok = 256, kPairEpiWarps = 8, kPairThreads = 128 + 32 * kPairEpiWarps;
 constexpr int kPairBBytes = (kPairTok / 2) * 128;
 constexpr size_t kPairSmem = static_cast<size_t>(kPairStages) * (kHgABytes + kPairBBytes) + 1024;
 
-// Warp 0: TMA (both CTAs, own halves).  Warp 1 of the first CTA: MMAs for the pair.  Warps 4-7: epilogue
-// of the CTA's 128 rows.  192 KB of operands in flight per SM cover the L2 latency; the 256-token tile
-// makes a stage 512 tensor cycles.
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kHgThreads, 1)
+// Warp 0: TMA (both CTAs, own halves).  Warp 1 of the first CTA: MMAs for the pair.  Warps 4-11: epilogue
+// of the CTA's 128 rows, two warps a quadrant of them with half the tokens each.  Four warps that fetched the factors of
+// each block of tokens behind its accumulators (up to four L2 round trips in a row) took longer for a tile than its products:
+// 4 x 1024 tokens 23.1 -> 22.5 ms (1.5B) and 48.7 -> 47.0 (2.9B).  (The single-CTA tiles, several to an SM's turn, lose 1 to 2 %
+// with their factors fetched ahead.)  192 KB of operands in flight per SM cover the L2 latency; the 256-token tile makes a
+// stage 512 tensor cycles.
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     gemm_pair_kernel(const __grid_constant__ HgArgs a, const __grid_constant__ HgMaps maps) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -347,7 +366,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kHgThreads, 1)
 
     if (tid == 0) {
         for (int s = 0; s < kPairStages; ++s) { mbar_init(&bar_full[s], 1); mbar_init(&bar_empty[s], 1); }
-        for (int s = 0; s < 2; ++s) { mbar_init(&bar_tfull[s], 1); mbar_init(&bar_tempty[s], 8); }
+        for (int s = 0; s < 2; ++s) { mbar_init(&bar_tfull[s], 1); mbar_init(&bar_tempty[s], 2 * kPairEpiWarps); }
         s_fail = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -415,31 +434,36 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kHgThreads, 1)
         }
     } else if (warp >= 4) {
         int acc = 0, aph = 0;
-        const int q = warp & 3;
+        constexpr int TOKS = kPairTok / (kPairEpiWarps / 4), BLOCKS = TOKS / 32;
+        const int q = warp & 3, share = ((warp - 4) >> 2) * TOKS;
         for (int tile = pair; tile < a.n_tiles; tile += n_pairs) {
             int pi;
             const HgDev p = problem_of(a, tile, pi);
             const int lt = tile - p.first_tile, rt = lt % p.row_tiles, tt = lt / p.row_tiles;
-            const int row = rt * 256 + rank * 128 + q * 32 + lane, tok0 = tt * kPairTok;
+            const int row = rt * 256 + rank * 128 + q * 32 + lane, tok0 = tt * kPairTok + share;
+            float un[BLOCKS], so[BLOCKS];
+            token_factors<BLOCKS>(p, tok0 + lane, 32, a.M, lane, un, so);
+            if (p.out == HG_RELU2_F16 && rt == 0 && rank == 0 && q == 0) {
+#pragma unroll
+                for (int i = 0; i < BLOCKS; ++i)
+                    if (tok0 + 32 * i + lane < a.M) p.out_scale[tok0 + 32 * i + lane] = so[i];
+            }
             int got = 1;
             if (lane == 0) got = mbar_wait_bounded(&bar_tfull[acc], aph) ? 1 : 0;
             got = __shfl_sync(0xFFFFFFFFu, got, 0);
             if (!got) { s_fail = 1; break; }
             tc_fence_after();
-            const uint32_t base = tmem + acc * kPairTok + (static_cast<uint32_t>(q * 32) << 16);
-            for (int c0 = 0; c0 < kPairTok; c0 += 32) {
+            const uint32_t base = tmem + acc * kPairTok + share + (static_cast<uint32_t>(q * 32) << 16);
+#pragma unroll
+            for (int i = 0; i < BLOCKS; ++i) {
                 float v[32];
-                tmem_ld32(base + c0, v);
-                if (c0 + 32 == kPairTok) {               // the accumulator is in registers: the MMA warp may overwrite it
+                tmem_ld32(base + 32 * i, v);
+                if (i == BLOCKS - 1) {                   // the accumulator is in registers: the MMA warp may overwrite it
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive_cluster(mapa(smem_addr(&bar_tempty[acc]), 0));
                 }
-                if (tok0 + c0 >= a.M) continue;
-                float un, so;
-                token_factors(p, tok0 + c0 + lane, a.M, un, so);
-                if (p.out == HG_RELU2_F16 && rt == 0 && rank == 0 && q == 0 && tok0 + c0 + lane < a.M) p.out_scale[tok0 + c0 + lane] = so;
-                finish_block<32>(p, v, un, so, tok0 + c0, row, a.M);
+                if (tok0 + 32 * i < a.M) finish_block<32>(p, v, un[i], so[i], tok0 + 32 * i, row, a.M);
             }
             if (++acc == 2) { acc = 0; aph ^= 1; }
         }
@@ -476,10 +500,10 @@ __device__ __forceinline__ void reduce_share(const HgDev& p, cg::cluster_group& 
 #pragma unroll
         for (int j = 0; j < NB; ++j) v[j] += src[j * pitch];
     }
-    float un = 1.f, so = 1.f;
-    if (lane < NB) token_factors(p, tok + lane, M, un, so);
-    if (p.out == HG_RELU2_F16 && rt == 0 && rl < 32 && lane < NB && tok + lane < M) p.out_scale[tok + lane] = so;
-    if (good) finish_block<NB>(p, v, un, so, tok, row0 + rl, M);
+    float un[1], so[1];
+    token_factors<1>(p, tok + lane, 0, lane < NB ? M : 0, lane, un, so);
+    if (p.out == HG_RELU2_F16 && rt == 0 && rl < 32 && lane < NB && tok + lane < M) p.out_scale[tok + lane] = so[0];
+    if (good) finish_block<NB>(p, v, un[0], so[0], tok, row0 + rl, M);
 }
 
 template <int NT>
@@ -566,12 +590,11 @@ __global__ void __launch_bounds__(kHgThreads, 1) gemm_one_kernel(const __grid_co
         if (good) {
             for (int c0 = half * 32; c0 < NT; c0 += 64) {
                 if (tok0 + c0 >= a.M) break;
-                float v[32];
+                float v[32], un[1], so[1];
                 tmem_ld32(base + c0, v);
-                float un, so;
-                token_factors(p, tok0 + c0 + lane, a.M, un, so);
-                if (p.out == HG_RELU2_F16 && rt == 0 && q == 0 && tok0 + c0 + lane < a.M) p.out_scale[tok0 + c0 + lane] = so;
-                finish_block<32>(p, v, un, so, tok0 + c0, row0 + rl, a.M);
+                token_factors<1>(p, tok0 + c0 + lane, 0, a.M, lane, un, so);
+                if (p.out == HG_RELU2_F16 && rt == 0 && q == 0 && tok0 + c0 + lane < a.M) p.out_scale[tok0 + c0 + lane] = so[0];
+                finish_block<32>(p, v, un[0], so[0], tok0 + c0, row0 + rl, a.M);
             }
         }
     } else {
@@ -797,7 +820,7 @@ int launch_gemm_f16(const HgProb* probs, int n_probs, int M, int* status, cudaSt
     int rc = smem_attr(gemm_pair_kernel, kPairSmem, configured);
     if (rc) return rc;
     const int grid_pairs = a.n_tiles < kSms / 2 ? a.n_tiles : kSms / 2;
-    cudaError_t e = launch_pdl(gemm_pair_kernel, dim3(2 * grid_pairs), dim3(kHgThreads), kPairSmem, s, a, maps);
+    cudaError_t e = launch_pdl(gemm_pair_kernel, dim3(2 * grid_pairs), dim3(kPairThreads), kPairSmem, s, a, maps);
     if (e != cudaSuccess) return fail(RWKVQ_E_LAUNCH, "gemm_f16(pair): %s", cudaGetErrorString(e));
     return RWKVQ_OK;
 }
