@@ -296,7 +296,12 @@ struct SideLane {
     cudaStream_t stream = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
     int start(cudaStream_t caller) const;        // the side stream waits for what the caller has issued
-    int finish(cudaStream_t caller) const;       // the caller waits for the side stream
+    int mark() const;                            // a point of the side stream
+    int wait(cudaStream_t caller) const;         // the caller waits for the last point marked
+    int finish(cudaStream_t caller) const {      // the caller waits for the side stream
+        const int rc = mark();
+        return rc ? rc : wait(caller);
+    }
 };
 SideLane* side_lane(cudaStream_t caller);
 // A fork onto a lane (or none): joined on every way out, so that what ran beside is ordered before the caller's next work
@@ -309,6 +314,8 @@ struct Fork {
         open = true;
         return lane->start(caller);
     }
+    int mark() const { return open ? lane->mark() : RWKVQ_OK; }
+    int wait() const { return open ? lane->wait(caller) : RWKVQ_OK; }
     int join() {
         if (!open) return RWKVQ_OK;
         open = false;

@@ -809,10 +809,11 @@ int SideLane::start(cudaStream_t caller) const {
         return fail(RWKVQ_E_LAUNCH, "fork onto the side stream failed");
     return RWKVQ_OK;
 }
-int SideLane::finish(cudaStream_t caller) const {
-    if (cudaEventRecord(join, stream) != cudaSuccess || cudaStreamWaitEvent(caller, join, 0) != cudaSuccess)
-        return fail(RWKVQ_E_LAUNCH, "join of the side stream failed");
-    return RWKVQ_OK;
+int SideLane::mark() const {
+    return cudaEventRecord(join, stream) == cudaSuccess ? RWKVQ_OK : fail(RWKVQ_E_LAUNCH, "join of the side stream failed");
+}
+int SideLane::wait(cudaStream_t caller) const {
+    return cudaStreamWaitEvent(caller, join, 0) == cudaSuccess ? RWKVQ_OK : fail(RWKVQ_E_LAUNCH, "join of the side stream failed");
 }
 
 }  // namespace rwkvq

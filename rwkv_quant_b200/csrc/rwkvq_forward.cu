@@ -23,6 +23,13 @@ constexpr int kSmallRows = 64;
 constexpr int kChunkedT = 16;        // tokens per sequence from which long calls take the chunked scan (two chunks)
 
 bool chunked(size_t rows, int T) { return rows > kSmallRows && T >= kChunkedT; }
+// Long calls turn every weight matrix into fp16 in front of its product.  Where the scan is long and leaves most of the chip idle, the
+// conversions run on the side lane under it, r / k / v and the LoRA matrices a layer ahead: 1.5B, 1 x 512 tokens 6.78 -> 6.35 ms,
+// 2 x 256 6.30 -> 5.93, 1 x 256 4.52 -> 4.34 (fp16 rows from the tail, some 0.1 ms, included).  Where it is short (3 x 77: 4.26 -> 4.4 ms,
+// also with the conversions of the time mix alone) they outlast it and keep the shared memory that the products behind it
+// want; where it fills the chip (16 x 512: 40.4 -> 41.3) there is nothing to run under.
+constexpr int kBesideT = 256;        // tokens a sequence from which the scan outlasts a layer's conversions
+bool convert_beside(int B, int T, int H) { return chunked(static_cast<size_t>(B) * T, T) && T >= kBesideT && wkv_chunked_f16(B, H); }
 
 struct ForwardWs {
     size_t bytes = 0;
@@ -30,7 +37,10 @@ struct ForwardWs {
     float *x, *xs, *rkv, *yl, *wkv, *out, *og, *v_first, *amax, *tailx, *taily, *n2tok, *wn2, *hffn, *lora_h, *dp;
     float* scale;                      // [4][N] row scales of the r / k / v (or channel-mix) rows and of og
     float* hscale;                     // [N]
-    __half *x16, *og16, *h16, *split, *hl, *w16, *lw16;
+    __half *x16, *og16, *h16, *split, *hl;
+    // a layer's weights in fp16, LoRA matrices of this layer and the next: apart where they are converted beside the scan, else in
+    // one place in turn
+    __half *wrkv16, *wo16, *wfk16, *wfv16, *lw16[2];
     SbRows rkv_pair[3], d_pair, f_pair;      // operand rows of the tcgen05 pipeline (17 rows and more): r / k / v; og or xk; hffn
     void* head_ws;
     size_t head_ws_bytes;
@@ -39,11 +49,6 @@ struct ForwardWs {
 inline int up64(int n) { return (n + 63) / 64 * 64; }
 inline size_t pitch16(size_t cols) { return cols + 64; }
 
-// fp16 weights of one launch: r / k / v together, or one of the others
-size_t w16_halves(const rwkvq_model& m) {
-    const size_t D = m.n_embd, F = m.ffn_dim;
-    return std::max(3 * D * D, F * D);
-}
 size_t lora16_halves(const rwkvq_model& m) { return static_cast<size_t>(8) * up64(m.max_rank) * up64(m.n_embd); }
 
 ForwardWs carve(const rwkvq_model& m, int B, int T, size_t n_tail, void* base) {
@@ -78,7 +83,11 @@ ForwardWs carve(const rwkvq_model& m, int B, int T, size_t n_tail, void* base) {
         w.x16 = f16(3 * N * pitch16(D)); w.og16 = f16(N * pitch16(D)); w.h16 = f16(N * pitch16(F));
         w.split = f16(4 * N * 2 * D); w.hl = f16(4 * N * 2 * up64(m.max_rank));
         w.scale = f32(4 * N); w.hscale = f32(N); w.n2tok = f32(N);
-        w.w16 = f16(w16_halves(m)); w.lw16 = f16(lora16_halves(m));
+        const bool apart = convert_beside(B, T, static_cast<int>(D / 64));
+        w.wrkv16 = f16(apart ? 3 * D * D : std::max(3 * D * D, F * D));
+        w.wo16 = apart ? f16(D * D) : w.wrkv16; w.wfk16 = apart ? f16(F * D) : w.wrkv16; w.wfv16 = apart ? f16(F * D) : w.wrkv16;
+        w.lw16[0] = f16(lora16_halves(m));
+        w.lw16[1] = apart ? f16(lora16_halves(m)) : w.lw16[0];
     }
     if (n_tail > 0) {
         w.tailx = f32(n_tail * D); w.taily = f32(n_tail * D);
@@ -115,6 +124,7 @@ bool same_shape(const rwkvq_qtensor& a, const rwkvq_qtensor& b) {
 }
 
 constexpr int kForkRows = 1024;
+constexpr int kBesideCtas = 3;       // CTAs an SM of a conversion beside the scan
 
 struct Pass {
     const rwkvq_model& m;
@@ -129,48 +139,61 @@ struct Pass {
         return p;
     }
 
-    // the six LoRA-side and the r / k / v products of a layer from its prepared rows
-    // (s_rkv: the stream of the latter)
-    int mix_large(const rwkvq_layer& L, bool layer0, float* const* y3, cudaStream_t s_rkv) const {
-        const size_t ND = static_cast<size_t>(N) * D, NP = static_cast<size_t>(N) * pitch16(D);
+    // matrices of layer l to fp16
+    int convert_rkv(int l, cudaStream_t s, int per_sm) const {
+        const rwkvq_layer& L = m.layers[l];
         const rwkvq_qtensor* t3[3] = {&L.Wr, &L.Wk, &L.Wv};
+        for (int k = 0; k < 3; ++k) {
+            int rc = launch_dequant_f16(*t3[k], 0, D, w.wrkv16 + static_cast<size_t>(k) * D * D, nullptr, s, per_sm);
+            if (rc) return rc;
+        }
+        return RWKVQ_OK;
+    }
+    int convert_lora(int l, cudaStream_t s) const {
+        const rwkvq_layer& L = m.layers[l];
+        const rwkvq_qtensor* t12[8] = {&L.w1, &L.w2, &L.a1, &L.a2, &L.g1, &L.g2, &L.v1, &L.v2};
+        TransposeJob jobs[8];
+        const int n = l == 0 ? 6 : 8;
+        __half* o = w.lw16[l & 1];
+        for (int i = 0; i < n; ++i) {
+            jobs[i] = {t12[i], o};
+            o += i & 1 ? static_cast<size_t>(D) * up64(t12[i]->rows) : static_cast<size_t>(t12[i]->cols) * up64(D);
+        }
+        return launch_dequant_f16_t(jobs, n, s);
+    }
+    int rkv_large(float* const* y3, cudaStream_t s) const {
+        const size_t NP = static_cast<size_t>(N) * pitch16(D);
         HgProb p[kHgMaxProbs];
         for (int k = 0; k < 3; ++k) {
-            __half* wk = w.w16 + static_cast<size_t>(k) * D * D;
-            int rc = launch_dequant_f16(*t3[k], 0, D, wk, nullptr, s_rkv);
-            if (rc) return rc;
-            p[k] = prob(wk, D, D, w.x16 + k * NP, w.scale + k * N);
+            p[k] = prob(w.wrkv16 + static_cast<size_t>(k) * D * D, D, D, w.x16 + k * NP, w.scale + k * N);
             p[k].out = HG_F32; p[k].epilogue = RWKVQ_EPI_NONE; p[k].y32 = y3[k]; p[k].ldy = D;
         }
-        int rc = launch_gemm_f16(p, 3, N, w.status, s_rkv);
-        if (rc) return rc;
-        // LoRA branches: both products with x (then h) as an fp16 pair, the matrices exact in fp16
+        return launch_gemm_f16(p, 3, N, w.status, s);
+    }
+    // LoRA branches: both products with x (then h) as an fp16 pair, the matrices exact in fp16
+    int lora_large(int l) const {
+        const rwkvq_layer& L = m.layers[l];
+        const size_t ND = static_cast<size_t>(N) * D;
         const rwkvq_qtensor* t1[4] = {&L.w1, &L.a1, &L.g1, &L.v1};
-        const rwkvq_qtensor* t2[4] = {&L.w2, &L.a2, &L.g2, &L.v2};
-        const int act[4] = {1, 0, 2, 0}, n_br = layer0 ? 3 : 4;
-        TransposeJob jobs[8];
+        const int act[4] = {1, 0, 2, 0}, n_br = l == 0 ? 3 : 4;
         HgProb dn[kHgMaxProbs], up[kHgMaxProbs];
-        __half* o = w.lw16;
+        __half* o = w.lw16[l & 1];
         const int Rp = up64(m.max_rank);
         for (int i = 0; i < n_br; ++i) {
             const int r = t1[i]->cols, rp = up64(r);
             __half* hl = w.hl + static_cast<size_t>(i) * N * 2 * Rp;
-            jobs[2 * i] = {t1[i], o};
             dn[i] = HgProb{};
             dn[i].w = o; dn[i].w_pitch = up64(D); dn[i].rows = rp; dn[i].w_rows = r; dn[i].k = D; dn[i].terms = 2;
             dn[i].x = w.split + static_cast<size_t>(i) * N * 2 * D; dn[i].x_pitch = 2 * D;
             dn[i].out = HG_SPLIT; dn[i].act = act[i]; dn[i].y16 = hl; dn[i].ldy = 2 * rp; dn[i].lo_off = rp;
             o += static_cast<size_t>(r) * up64(D);
-            jobs[2 * i + 1] = {t2[i], o};
             up[i] = HgProb{};
             up[i].w = o; up[i].w_pitch = rp; up[i].rows = D; up[i].k = rp; up[i].terms = 2;
             up[i].x = hl; up[i].x_pitch = 2 * rp;
             up[i].out = HG_F32; up[i].epilogue = RWKVQ_EPI_NONE; up[i].y32 = w.yl + i * ND; up[i].ldy = D;
             o += static_cast<size_t>(D) * rp;
         }
-        rc = launch_dequant_f16_t(jobs, 2 * n_br, s);
-        if (rc) return rc;
-        rc = launch_gemm_f16(dn, n_br, N, w.status, s);
+        int rc = launch_gemm_f16(dn, n_br, N, w.status, s);
         if (rc) return rc;
         return launch_gemm_f16(up, n_br, N, w.status, s);
     }
@@ -262,8 +285,11 @@ int rwkvq_forward_seq_status(const rwkvq_model* m, int B, int T, const int64_t* 
     if (rc) return rc;
     // r / k / v beside the LoRA branches while neither fills the chip (5 rows 2.07 -> 2.00 ms, 231 rows 4.46 -> 4.30,
     // 512 rows 6.93 -> 6.78, 1024 rows 8.73 -> 8.58)
-    SideLane* lane = N <= kForkRows ? side_lane(s) : nullptr;
-    const cudaStream_t s_rkv = lane ? lane->stream : s;
+    SideLane* lane = side_lane(s);
+    const cudaStream_t s_side = lane ? lane->stream : s, s_rkv = N <= kForkRows ? s_side : s;
+    const bool beside = lane && convert_beside(B, T, H);
+    if (beside && ((rc = ps.convert_rkv(0, s, 0)) != 0 || (rc = ps.convert_lora(0, s)) != 0)) return rc;
+    Fork fork{lane, s};
     for (int l = 0; l < m->n_layer; ++l) {
         const rwkvq_layer& L = m->layers[l];
         const bool layer0 = l == 0;
@@ -278,7 +304,6 @@ int rwkvq_forward_seq_status(const rwkvq_model* m, int B, int T, const int64_t* 
         // mix rows: r, w, k, v, a, g
         const bool sb = small && D % 256 == 0 && same_shape(L.Wr, L.Wk) && same_shape(L.Wr, L.Wv) && gemm_sb_pays(L.Wr, N) &&
                         gemm_sb_pays(L.Wo, N) && gemm_sb_pays(L.Wfk, N) && gemm_sb_pays(L.Wfv, N);
-        Fork fork{lane, s};
         const LayerAhead ahead(L, l + 1 < m->n_layer ? &L + 1 : nullptr, layer0, wkv_in[l], static_cast<size_t>(B) * D * 64 * sizeof(float));
         if (small) {
             for (int q = 0; q < 6; ++q) {
@@ -325,16 +350,28 @@ int rwkvq_forward_seq_status(const rwkvq_model* m, int B, int T, const int64_t* 
             }
             rc = launch_seq_prep(a, N, s);
             if (rc) return rc;
-            if ((rc = fork.start()) != 0) return rc;
-            rc = ps.mix_large(L, layer0, y3, s_rkv);
+            if (beside && (rc = fork.wait()) != 0) return rc;
+            if (s_rkv != s && (rc = fork.start()) != 0) return rc;
+            if (!beside && (rc = ps.convert_rkv(l, s_rkv, 0)) != 0) return rc;
+            if ((rc = ps.rkv_large(y3, s_rkv)) != 0) return rc;
+            if (s_rkv == s && beside && (rc = fork.start()) != 0) return rc;
+            if (!beside && (rc = ps.convert_lora(l, s)) != 0) return rc;
+            rc = ps.lora_large(l);
         }
         if (rc) return rc;
-        if ((rc = fork.join()) != 0) return rc;
+        if (!beside) {
+            if ((rc = fork.join()) != 0) return rc;
+        } else {
+            if (s_rkv != s && ((rc = fork.mark()) != 0 || (rc = fork.wait()) != 0)) return rc;
+            if ((rc = launch_dequant_f16(L.Wo, 0, D, w.wo16, nullptr, s_side, kBesideCtas)) != 0) return rc;
+            if ((rc = fork.mark()) != 0) return rc;
+        }
         if (chunked(N, T)) {
             WkvChunkArgs q{};
             q.r = r; q.k = k; q.v = v; q.yw = yw; q.ya = ya; q.yv = layer0 ? nullptr : yv; q.v_first = layer0 ? nullptr : w.v_first; q.g = yg;
             q.w0 = L.w0; q.a0 = L.a0; q.v0 = L.v0; q.k_k = L.k_k; q.k_a = L.k_a; q.r_k = L.r_k; q.ln_w = L.lnx_w; q.ln_b = L.lnx_b;
-            q.h_in = wkv_in[l]; q.h_out = wkv_out[l]; q.og = w.og; q.ops = w.wkv; q.dp = w.dp; q.y = w.out; q.status = w.status;
+            q.h_in = wkv_in[l]; q.h_out = wkv_out[l]; q.og = w.og; q.og16 = w.og16; q.og_scale = w.scale + 3 * N;
+            q.og_pitch = static_cast<long long>(pitch16(D)); q.ops = w.wkv; q.dp = w.dp; q.spread = beside; q.y = w.out; q.status = w.status;
             q.B = B; q.T = T; q.H = H;
             rc = launch_wkv_chunked(q, s);
             if (rc) return rc;
@@ -384,28 +421,39 @@ int rwkvq_forward_seq_status(const rwkvq_model* m, int B, int T, const int64_t* 
             if (rc) return rc;
             continue;
         }
-        rc = launch_dequant_f16(L.Wo, 0, D, w.w16, nullptr, s);
-        if (rc) return rc;
-        rc = launch_row_scale(w.og, D, D, N, w.scale + 3 * N, w.og16, static_cast<long long>(pitch16(D)), nullptr, s);
-        if (rc) return rc;
-        HgProb p = ps.prob(w.w16, D, D, w.og16, w.scale + 3 * N);
+        if (!beside && (rc = launch_dequant_f16(L.Wo, 0, D, w.wo16, nullptr, s)) != 0) return rc;
+        if (!(chunked(N, T) && wkv_chunked_f16(B, H))) {
+            rc = launch_row_scale(w.og, D, D, N, w.scale + 3 * N, w.og16, static_cast<long long>(pitch16(D)), nullptr, s);
+            if (rc) return rc;
+        }
+        if (beside && (rc = fork.wait()) != 0) return rc;
+        HgProb p = ps.prob(w.wo16, D, D, w.og16, w.scale + 3 * N);
         p.out = HG_F32; p.epilogue = RWKVQ_EPI_ADD; p.y32 = w.x; p.resid = w.x; p.ldy = D;
         rc = launch_gemm_f16(&p, 1, N, w.status, s);
         if (rc) return rc;
+        float* wn2 = w.wn2 + static_cast<size_t>(l) * 128;
+        if (beside) {
+            if ((rc = launch_dequant_f16(L.Wfk, 0, F, w.wfk16, wn2, s_side, kBesideCtas)) != 0) return rc;
+            if ((rc = launch_dequant_f16(L.Wfv, 0, D, w.wfv16, nullptr, s_side, kBesideCtas)) != 0) return rc;
+        }
         c.mode[0] = kPrepScaled; c.x16[0] = w.x16; c.scale[0] = w.scale; c.n2 = w.n2tok;
         rc = launch_seq_prep(c, N, s);
         if (rc) return rc;
-        float* wn2 = w.wn2 + static_cast<size_t>(l) * 128;
-        rc = launch_dequant_f16(L.Wfk, 0, F, w.w16, wn2, s);
-        if (rc) return rc;
-        p = ps.prob(w.w16, F, D, w.x16, w.scale);
+        if (beside) {
+            if ((rc = fork.mark()) != 0 || (rc = fork.wait()) != 0) return rc;
+            if (l + 1 < m->n_layer && ((rc = ps.convert_rkv(l + 1, s_side, kBesideCtas)) != 0 || (rc = ps.convert_lora(l + 1, s_side)) != 0 ||
+                                       (rc = fork.mark()) != 0))
+                return rc;                                   // waited for in front of the next layer's products
+        } else if ((rc = launch_dequant_f16(L.Wfk, 0, F, w.wfk16, wn2, s)) != 0) {
+            return rc;
+        }
+        p = ps.prob(w.wfk16, F, D, w.x16, w.scale);
         p.out = HG_RELU2_F16; p.y16 = w.h16; p.ldy = static_cast<long long>(pitch16(F)); p.w_n2 = wn2; p.n_w_n2 = D / 256; p.x_n2 = w.n2tok;
         p.out_scale = w.hscale;
         rc = launch_gemm_f16(&p, 1, N, w.status, s);
         if (rc) return rc;
-        rc = launch_dequant_f16(L.Wfv, 0, D, w.w16, nullptr, s);
-        if (rc) return rc;
-        p = ps.prob(w.w16, D, F, w.h16, w.hscale);
+        if (!beside && (rc = launch_dequant_f16(L.Wfv, 0, D, w.wfv16, nullptr, s)) != 0) return rc;
+        p = ps.prob(w.wfv16, D, F, w.h16, w.hscale);
         p.out = HG_F32; p.epilogue = RWKVQ_EPI_ADD; p.y32 = w.x; p.resid = w.x; p.ldy = D;
         rc = launch_gemm_f16(&p, 1, N, w.status, s);
         if (rc) return rc;

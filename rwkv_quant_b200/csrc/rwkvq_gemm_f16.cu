@@ -93,13 +93,20 @@ __global__ void __launch_bounds__(256) dequant_f16_kernel(const QView t, int row
     }
 }
 
-int launch_dequant_f16(const rwkvq_qtensor& t, int row0, int rows, __half* out, float* n2, cudaStream_t s) {
+int launch_dequant_f16(const rwkvq_qtensor& t, int row0, int rows, __half* out, float* n2, cudaStream_t s, int per_sm) {
     RWKVQ_REQUIRE((t.kind == RWKVQ_KIND_SB6 || t.kind == RWKVQ_KIND_SYM) && t.cols % 256 == 0 && (n2 == nullptr || t.cols <= 32768), RWKVQ_E_DTYPE,
                   "dequant_f16: sb6 / sym tensors (with norms of at most 32768 columns)");
     const long long items = static_cast<long long>(rows) * (t.cols >> 5);
     const long long want = (items + 255) / 256;
-    const unsigned grid = static_cast<unsigned>(want < 148 * 6 ? want : 148 * 6);
-    cudaError_t e = launch_pdl(dequant_f16_kernel, dim3(grid), dim3(256), 0, s, make_view(t), row0, items, out, n2);
+    // beside another kernel: room for its CTAs on every SM, and no launch before the one in front has ended (four conversions
+    // at once held the threads of every SM, and the scan's operands waited 30 us for them)
+    const int most = 148 * (per_sm > 0 ? per_sm : 6);
+    const dim3 grid(static_cast<unsigned>(want < most ? want : most));
+    if (per_sm > 0) {
+        dequant_f16_kernel<<<grid, 256, 0, s>>>(make_view(t), row0, items, out, n2);
+        return check_launch("dequant_f16");
+    }
+    cudaError_t e = launch_pdl(dequant_f16_kernel, grid, dim3(256), 0, s, make_view(t), row0, items, out, n2);
     if (e != cudaSuccess) return fail(RWKVQ_E_LAUNCH, "dequant_f16: %s", cudaGetErrorString(e));
     return RWKVQ_OK;
 }

@@ -47,7 +47,8 @@ int launch_row_scale(const float* x, long long ldx, int cols, int M, float* scal
 // Packed sb6 / sym rows [row0, row0 + rows) -> fp16(q * s + m) [rows, cols] (pitch cols).
 // n2 (optional, [cols / 256], zeroed by the caller): merged with the largest squared norm of a row's
 // 256-column pieces.
-int launch_dequant_f16(const rwkvq_qtensor& t, int row0, int rows, __half* out, float* n2, cudaStream_t s);
+// per_sm: CTAs an SM where other kernels of the same call run beside this one (0: none do)
+int launch_dequant_f16(const rwkvq_qtensor& t, int row0, int rows, __half* out, float* n2, cudaStream_t s, int per_sm = 0);
 
 // Up to 8 matrices stored [in, out] -> fp16 transposed [out, in_pad] (in_pad = in rounded up to 64, the
 // padding zero), in the loader's precision fp16(bf16(w)).

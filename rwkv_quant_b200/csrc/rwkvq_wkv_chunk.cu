@@ -20,6 +20,8 @@
 // registers on small grids (128 bytes per clock and SM), issue latency at 7 warps per SM on large ones.
 #include "rwkvq_wkv_chunk.cuh"
 
+#include <algorithm>
+
 #include "rwkvq_decode_parts.cuh"
 #include "rwkvq_tc.cuh"
 
@@ -499,43 +501,77 @@ __global__ void __launch_bounds__(ScanGeo<R, SPLIT>::THREADS) wkv_scan_kernel(co
     }
 }
 
-// The tail where a scan CTA does not see whole heads: a warp per (token, head), v' from the operand blocks.
-__global__ void __launch_bounds__(128) wkv_chunk_tail_kernel(const WkvChunkArgs p, int n_chunks, long long n_pairs) {
-    const long long pair = blockIdx.x * 4ll + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
+// The tail where a scan CTA does not see whole heads: a CTA per token, a thread per 8 channels (v' from the operand blocks),
+// whose rows leave as the output projection reads them: fp16 under a power of two per token.  Bound: latency, then L2 (four
+// arrays read, one of halves written; as a pass of its own behind an fp32 tail the scaling cost a launch and 8 bytes a value).
+__global__ void __launch_bounds__(512) wkv_chunk_tail_kernel(const WkvChunkArgs p, int n_chunks) {
+    __shared__ float red[16];
+    const bool live = static_cast<int>(threadIdx.x) * 8 < p.H * kS;     // whole warps: H need not be a multiple of 4
+    const int c = live ? threadIdx.x * 8 : 0, hd = c / kS, ci = c % kS, b = blockIdx.x / p.T, t = blockIdx.x % p.T;
+    const size_t at = static_cast<size_t>(blockIdx.x) * p.H * kS + c;
     pdl_launch_dependents();
+    auto load8 = [](const float* q, float (&o)[8]) {
+        const float4 lo = __ldcg(reinterpret_cast<const float4*>(q)), hi = __ldcg(reinterpret_cast<const float4*>(q) + 1);
+        o[0] = lo.x; o[1] = lo.y; o[2] = lo.z; o[3] = lo.w; o[4] = hi.x; o[5] = hi.y; o[6] = hi.z; o[7] = hi.w;
+    };
+    float lw[8], lb[8], y[8], g[8], v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) { lw[i] = __ldg(p.ln_w + c + i); lb[i] = __ldg(p.ln_b + c + i); }
     pdl_wait();
-    if (pair >= n_pairs) return;
-    const int hd = static_cast<int>(pair % p.H), b = static_cast<int>(pair / p.H / p.T), t = static_cast<int>(pair / p.H % p.T);
-    const size_t at = static_cast<size_t>(pair) * kS + 2 * lane;
-    const float* v = p.ops + ((static_cast<size_t>(b) * p.H + hd) * n_chunks + t / kC) * kChunkFloats + kOffV + (t % kC) * kS + 2 * lane;
-    const float2 y = __ldcg(reinterpret_cast<const float2*>(p.y + at)), g = __ldcg(reinterpret_cast<const float2*>(p.g + at));
-    const float2 vv = __ldcg(reinterpret_cast<const float2*>(v));
-    const float dp = __ldcg(p.dp + pair);
-    const float2 lw = __ldg(reinterpret_cast<const float2*>(p.ln_w + hd * kS) + lane), lb = __ldg(reinterpret_cast<const float2*>(p.ln_b + hd * kS) + lane);
-    float m = y.x + y.y;
+    load8(p.y + at, y);
+    load8(p.g + at, g);
+    load8(p.ops + ((static_cast<size_t>(b) * p.H + hd) * n_chunks + t / kC) * kChunkFloats + kOffV + (t % kC) * kS + ci, v);
+    const float dp = __ldcg(p.dp + static_cast<size_t>(blockIdx.x) * p.H + hd);
+    auto head_sum = [](const float (&x)[8]) {                       // 8 lanes hold a head
+        float s = ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m += __shfl_xor_sync(0xFFFFFFFFu, m, o);
-    m /= kS;
-    const float d0 = y.x - m, d1 = y.y - m;
-    float var = d0 * d0 + d1 * d1;
+        for (int o = 1; o < 8; o <<= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
+        return s;
+    };
+    const float m = head_sum(y) / kS;
+    float d2[8];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) var += __shfl_xor_sync(0xFFFFFFFFu, var, o);
-    const float inv = 1.0f / sqrtf(var / kS + 64e-5f);
-    *reinterpret_cast<float2*>(p.og + at) = make_float2((d0 * inv * lw.x + lb.x + dp * vv.x) * g.x, (d1 * inv * lw.y + lb.y + dp * vv.y) * g.y);
+    for (int i = 0; i < 8; ++i) { y[i] -= m; d2[i] = y[i] * y[i]; }
+    const float inv = 1.0f / sqrtf(head_sum(d2) / kS + 64e-5f);
+    float amax = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        y[i] = (y[i] * inv * lw[i] + lb[i] + dp * v[i]) * g[i];
+        if (live) amax = fmaxf(amax, fabsf(y[i]));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
+    __syncthreads();
+    amax = red[0];
+    for (int w = 1; w < static_cast<int>(blockDim.x >> 5); ++w) amax = fmaxf(amax, red[w]);
+    int e = 0;                                                      // |x 2^(14 - e)| <= 2^14, as row_scale_kernel
+    if (amax > 0.f && amax < INFINITY) frexpf(amax, &e);
+    const float sc = ldexpf(1.f, 14 - e);
+    if (threadIdx.x == 0) p.og_scale[blockIdx.x] = sc;
+    uint32_t h[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const __half2 x = __floats2half2_rn(y[2 * i] * sc, y[2 * i + 1] * sc);
+        h[i] = *reinterpret_cast<const uint32_t*>(&x);
+    }
+    if (live) *reinterpret_cast<uint4*>(p.og16 + static_cast<size_t>(blockIdx.x) * p.og_pitch + c) = make_uint4(h[0], h[1], h[2], h[3]);
 }
 
 template <int R, int SPLIT>
 static int launch_scan(const WkvChunkArgs& p, int n_chunks, cudaStream_t s) {
     using G = ScanGeo<R, SPLIT>;
-    cudaError_t e = cudaFuncSetAttribute(wkv_scan_kernel<R, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(G::SMEM));
-    if (e != cudaSuccess) return fail(RWKVQ_E_LIMIT, "wkv_scan: %zu bytes of shared memory: %s", G::SMEM, cudaGetErrorString(e));
+    // A scan is as slow as its fullest SM: beside the conversions of the side lane CTAs would pile up where those leave room first
+    // (1 x 512 tokens 56 -> 95 us), so a grid of up to one or two CTAs per SM asks for as much shared memory as keeps it to that.
+    const int ctas = p.B * p.H * SPLIT;
+    const size_t smem = std::max(G::SMEM, static_cast<size_t>(!p.spread ? 0 : ctas <= 148 ? 116 : ctas <= 296 ? 78 : 0) * 1024);
+    cudaError_t e = cudaFuncSetAttribute(wkv_scan_kernel<R, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 116 * 1024);
+    if (e != cudaSuccess) return fail(RWKVQ_E_LIMIT, "wkv_scan: %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
     // a plain launch: CTAs that start while the kernel before still fills the chip pile up on the SMs it leaves
     // first, and the scan of one batch element takes three times as long
-    wkv_scan_kernel<R, SPLIT><<<p.B * p.H * SPLIT, G::THREADS, G::SMEM, s>>>(p, n_chunks);
+    wkv_scan_kernel<R, SPLIT><<<ctas, G::THREADS, smem, s>>>(p, n_chunks);
     if (SPLIT == 1) return RWKVQ_OK;
-    const long long pairs = static_cast<long long>(p.B) * p.T * p.H;
-    e = launch_pdl(wkv_chunk_tail_kernel, dim3(static_cast<unsigned>((pairs + 3) / 4)), dim3(128), 0, s, p, n_chunks, pairs);
+    e = launch_pdl(wkv_chunk_tail_kernel, dim3(static_cast<unsigned>(p.B * p.T)), dim3((p.H * kS / 8 + 31) / 32 * 32), 0, s, p, n_chunks);
     if (e != cudaSuccess) return fail(RWKVQ_E_LAUNCH, "wkv_chunk_tail: %s", cudaGetErrorString(e));
     return RWKVQ_OK;
 }
@@ -545,8 +581,8 @@ int launch_wkv_chunked(const WkvChunkArgs& p, cudaStream_t s) {
     static_assert(sizeof(PreSmem) * kPreUnits <= kPreStage, "operands over the staged rows");
     const long long blocks = static_cast<long long>(p.B) * n_chunks * groups;
     RWKVQ_REQUIRE(blocks < (1ll << 31), RWKVQ_E_LIMIT, "wkv_chunked: too many tokens");
-    RWKVQ_REQUIRE(aligned(p.h_in, 16) && aligned(p.h_out, 16) && aligned(p.ln_w, 8) && aligned(p.ln_b, 8), RWKVQ_E_ALIGN,
-                  "wkv_chunked: states on 16-byte boundaries, group-norm parameters on 8-byte ones");
+    RWKVQ_REQUIRE(aligned(p.h_in, 16) && aligned(p.h_out, 16) && p.H <= 64, RWKVQ_E_ALIGN,
+                  "wkv_chunked: states on 16-byte boundaries, at most 64 heads");
     cudaError_t e = cudaFuncSetAttribute(wkv_operands_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kPreStage));
     if (e != cudaSuccess) return fail(RWKVQ_E_LIMIT, "wkv_operands: shared memory: %s", cudaGetErrorString(e));
     e = launch_pdl(wkv_operands_kernel, dim3(static_cast<unsigned>(blocks)), dim3(64 * kPreUnits), kPreStage, s, p, n_chunks);
@@ -555,6 +591,7 @@ int launch_wkv_chunked(const WkvChunkArgs& p, cudaStream_t s) {
     // shared-memory reads, 64 against 56 us at 32 heads; four: one warp per CTA); full grids: the largest tile with
     // the tail inside (4 rows per thread, twice the warps: 302 against 296 us)
     const int pairs = p.B * p.H;
+    static_assert(kChunkSplitPairs == 148, "the lines below");
     if (pairs <= 74) return launch_scan<2, 4>(p, n_chunks, s);
     if (pairs <= 148) return launch_scan<2, 2>(p, n_chunks, s);
     return launch_scan<8, 1>(p, n_chunks, s);

@@ -99,9 +99,35 @@ def test_time_mix_of_short_sequences_matches_its_steps(cuda_lib, B, T):
     model = _model("reduction", n_embd=256, ffn=1024)
     idx = torch.randint(1, 512, (B, T), generator=torch.Generator().manual_seed(T)).cuda()
     for st in (_states(model, B), model.init_state(B)):
-        got = model.forward_stateful(idx, [tuple(t.clone() for t in s) for s in st])
+        got = model.forward_stateful(idx, [tuple(t if t is None else t.clone() for t in s) for s in st])
         rows = []
         for t in range(T):
             lo, st = model.forward_stateful(idx[:, t:t + 1], st)
             rows.append(lo)
         _same(got, (torch.cat(rows, 1), st), 1e-4)
+
+
+@pytest.mark.parametrize("B,T", [(1, 255), (1, 256), (2, 300), (37, 256), (38, 256)])
+def test_weights_converted_beside_the_scan(cuda_lib, B, T):
+    """Calls on each side of the lines from which the weights become fp16 on the side stream, against the per-operator path; a
+    second call over the first one's buffers; and as a graph, whose forks are those of the captured stream."""
+    model = _model("compression", n_embd=256, ffn=1024)
+    idx = torch.randint(1, 512, (B, T), generator=torch.Generator().manual_seed(T)).cuda()
+    model.fused_prep = False
+    ref = model.forward_stateful(idx, _states(model, B), last_only=True)
+    model.fused_prep = True
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        for _ in range(2):
+            got = model.forward_stateful(idx, _states(model, B), last_only=True)
+        stream.synchronize()
+        _same(got, ref, 1e-3)
+        st, g = _states(model, B), torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=stream):
+            got = model.forward_stateful(idx, st, last_only=True)
+        for _ in range(2):
+            g.replay()
+        stream.synchronize()
+        _same(got, ref, 1e-3)
+    model.check()
