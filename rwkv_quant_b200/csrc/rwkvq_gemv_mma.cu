@@ -286,7 +286,7 @@ static int launch_one(MmaArgs& a, int rows, int cols, int n_mats, int KS, cudaSt
 }
 
 // Work split: a single wave of co-resident CTAs whenever the matrix allows it.
-//   * few row tiles, long rows  -> K is also split across CTAs (a cluster of 2 or 4; `split`)
+//   * few row tiles, long rows  -> K is also split across CTAs (a cluster of 2 or 4, one or two tiles each; `split`)
 //   * tiles * n_mats <= resident CTAs -> one tile per CTA, its 8 warps split K
 //   * more tiles -> WT tiles per CTA so that the grid still fits one wave
 //   * very many tiles (head) -> persistent CTAs, 8 warps split K of each tile
@@ -301,6 +301,12 @@ static int launch_wk(MmaArgs& a, int rows, int cols, int n_mats, bool split, con
     // shorter ones only where the caller has nothing else to fill the chip with (`split`).
     const int ctas = tiles * (cols >= kSplitAnyCols ? 1 : n_mats);
     if ((split || cols >= kSplitAnyCols) && n_iters >= 16 && rows <= kSplitMaxRows) {
+        // One tile and K in four is more than a wave: two tiles a CTA and K in four leave each CTA half the activations to
+        // prepare that one tile and K in two do (us, before / now: sb6 4 bits [2048, 8192] 6.7 / 6.3, [1200, 10240] 6.9 / 6.4, sym 8 bits
+        // [2560, 10240] 12.0 / 10.6, [3072, 8192] 10.7 / 9.7; 1.5B step of one stream 913 / 885, 2.9B 1671 / 1645).  From 32 iterations on (sb6
+        // [2048, 4096]: 4.7 / 4.9) and up to 7/8 of the resident CTAs: clusters do not fill every GPC ([2368, 8192], 296 CTAs: 7.0 / 10.4).
+        if (cols >= kSplitAnyCols && ctas * 4 > kResident && (tiles + 1) / 2 * 4 <= kResident * 7 / 8 && n_iters >= 32 && n_iters % 4 == 0)
+            return launch_one<L, 4, true>(a, rows, cols, n_mats, 4, s, ahead);
         if (ctas * 4 <= kResident && n_iters >= 32 && n_iters % 4 == 0) KS = 4;
         else if (ctas * 2 <= kResident && n_iters % 2 == 0) KS = 2;
     }

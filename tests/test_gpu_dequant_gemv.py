@@ -102,6 +102,25 @@ def test_gemv_shapes_and_uncovered_rows(cuda_lib, layout, bits, rows, cols):
     assert relmax(y, ref) <= TOL, relmax(y, ref)
 
 
+@pytest.mark.parametrize("layout,bits", [("sb6", 4), ("sym", 8)])
+@pytest.mark.parametrize("rows,cols", [(1184, 8192), (1185, 8192), (1776, 4096), (1777, 4096), (1777, 8192), (2048, 8192), (2080, 8192),
+                                       (3104, 4096), (3105, 4096)])
+def test_gemv_two_tiles_and_four_slices(cuda_lib, layout, bits, rows, cols):
+    """Long rows on each side of the lines between one tile and two tiles a CTA, odd numbers of tiles and ragged last ones; three
+    fused matrices equal their single calls bit for bit where K is split at all (sb6 [3104, 4096] has a split by the warps of a CTA,
+    as many as its tiles leave)."""
+    from rwkv_quant_b200 import synth
+    from rwkv_quant_b200.backends import cuda as be
+    g = torch.Generator().manual_seed(rows)
+    lins = [be.linear_for(getattr(synth, "quant_" + layout)("w", "g", torch.randn(rows, cols, generator=g) * 0.02, bits)) for _ in range(3)]
+    xs = _x(3, cols, rows)
+    out = (be.GwQuantLinearFused if layout == "sb6" else be.SymQuantLinearFused)(lins)(xs)
+    for lin, x, y in zip(lins, xs, out):
+        assert rows > 3000 or torch.equal(lin(x), y)
+        ref = x.double() @ lin._dequant_w(torch.float32).double().T
+        assert relmax(y.cpu().numpy(), ref.cpu().numpy()) <= TOL
+
+
 @pytest.mark.parametrize("layout,bits", LAYOUTS[:6])
 def test_batch_invariance_and_epilogues(cuda_lib, layout, bits):
     """Column n of an N-column call equals the single-vector call bit for bit;
