@@ -602,10 +602,9 @@ __device__ __forceinline__ float warp_sum64(const float* v, int lane) {
     return s;
 }
 
-// UP (one stream): the LoRA up projections of the head's 64 channels run here, their weights staged before the wait.
-template <bool UP>
-__global__ void __launch_bounds__(256) tmix_core_kernel(const TmixCoreArgs p, const std::conditional_t<UP, LoraVecArgs, int> up) {
-    extern __shared__ __align__(16) unsigned char up_smem[];         // UP: [ranks][64] fp16, [ranks] h, [8][4][64] partial sums
+// One stream: the LoRA up projections of the head's 64 channels run here too, their weights staged before the wait.
+__global__ void __launch_bounds__(256) tmix_core_up_kernel(const TmixCoreArgs p, const LoraVecArgs up) {
+    extern __shared__ __align__(16) unsigned char up_smem[];         // [ranks][64] fp16, [ranks] h, [8][4][64] partial sums
     // per-column operands of the state update, written once by warps 0 and 1 and read as float4 by all:
     // sA = -kk / |kk|, sB = (kk / |kk|) * a_gate, sW decay, sK key, sR receptance
     __shared__ __align__(16) float sA[64], sB[64], sW[64], sK[64], sR[64];
@@ -634,43 +633,34 @@ __global__ void __launch_bounds__(256) tmix_core_kernel(const TmixCoreArgs p, co
         prk0 = __ldg(p.r_k + hi * 64 + lane); prk1 = __ldg(p.r_k + hi * 64 + lane + 32);
         plw = __ldg(p.lnx_w + c); plb = __ldg(p.lnx_b + c);
     }
-    float* part_up = nullptr;
-    if constexpr (UP) {
-        const int ranks = up.first[up.n_br];
-        __half* wt = reinterpret_cast<__half*>(up_smem);
-        float* h = reinterpret_cast<float*>(wt + ranks * 64);
-        part_up = h + ranks;
-        lora_up_stage(up, hi * 64, wt);
-        pdl_wait();
-        for (int i = tid; i < ranks; i += 256) h[i] = __ldcg(up.h + i);
-        __syncthreads();
-        lora_up_vec(up, wt, h, part_up);
-        __syncthreads();
-    } else {
-        pdl_wait();            // the state above was written a whole token ago
-    }
+    const int ranks = up.first[up.n_br];
+    __half* wt = reinterpret_cast<__half*>(up_smem);
+    float* hl = reinterpret_cast<float*>(wt + ranks * 64);
+    float* part_up = hl + ranks;
+    lora_up_stage(up, hi * 64, wt);
+    pdl_wait();                // the state above was written a whole token ago
+    for (int i = tid; i < ranks; i += 256) hl[i] = __ldcg(up.h + i);
+    __syncthreads();
+    lora_up_vec(up, wt, hl, part_up);
+    __syncthreads();
     // LoRA output `br` (decay, rate, gate, value-residual) of the thread's channel
-    auto lora = [&](int br, const float* y) {
-        if constexpr (UP) {
-            float v = 0.f;
+    auto lora = [&](int br) {
+        float v = 0.f;
 #pragma unroll
-            for (int w = 0; w < 8; ++w) v += part_up[w * 256 + br * 64 + tid];
-            return v;
-        } else {
-            return __ldcg(y + row + tid);
-        }
+        for (int w = 0; w < 8; ++w) v += part_up[w * 256 + br * 64 + tid];
+        return v;
     };
     if (tid < 64) {
         const float r = __ldcg(p.r + row + tid), k = __ldcg(p.k + row + tid);
         float v = __ldcg(p.v + row + tid);
-        const float w = expf(-0.606531f * sigmoidf_(lora(0, p.yw) + pw0));
-        const float av = sigmoidf_(lora(1, p.ya) + pa0);
+        const float w = expf(-0.606531f * sigmoidf_(lora(0) + pw0));
+        const float av = sigmoidf_(lora(1) + pa0);
         const float k2 = k * (1.0f + (av - 1.0f) * pka);
         if (p.layer0) p.v_first[row + tid] = v;
-        else v = v + (__ldcg(p.v_first + row + tid) - v) * sigmoidf_(lora(3, p.yv) + pv0);
+        else v = v + (__ldcg(p.v_first + row + tid) - v) * sigmoidf_(lora(3) + pv0);
         const float kk = k * pkk;
         sT[tid] = kk * kk;
-        sW[tid] = w; sK[tid] = k2; sR[tid] = r; sV[tid] = v; sG[tid] = lora(2, p.g);
+        sW[tid] = w; sK[tid] = k2; sR[tid] = r; sV[tid] = v; sG[tid] = lora(2);
         asm volatile("bar.sync 1, 64;" ::: "memory");        // warps 0 and 1 only: sT is complete
         // both warps reduce the head-wide sum themselves; a = -kk / |kk|, b = -a * a_gate
         const float kn = kk * (1.0f / sqrtf(warp_sum64(sT, lane) + 1e-12f));
@@ -729,6 +719,110 @@ __global__ void __launch_bounds__(256) tmix_core_kernel(const TmixCoreArgs p, co
             for (int of = 16; of > 0; of >>= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, of));
             if ((tid & 31) == 0) atomicMax(reinterpret_cast<int*>(p.og_amax) + b, __float_as_int(m));
         }
+    }
+}
+
+// Several streams: two warps a (head, stream) pair.  Bound: latency of the chain rows -> gates -> row sums -> update -> group norm up to
+// some 20 streams, then the state (64 streams, 67 MB read and written: 20 -> 12 us a layer, 100 streams 35 -> 24).  A thread's tile is
+// 8 state rows x 8 columns: the five vectors of a step cost it 10 shared-memory loads for 64 state values (20 for 16 with eight warps
+// a pair, as above), the arithmetic goes in pairs, and a barrier waits for one other warp; a pair takes a quarter of the
+// instructions and of an SM's threads.  Against eight warps a pair, ms a step: 1.5B 4 streams 1.64 / 1.64, 16 1.79 / 1.76, 20 1.95 / 1.82,
+// 64 2.64 / 2.46, 100 3.63 / 3.39; 2.9B 2 streams 2.81 / 2.78, 16 3.08 / 2.95, 128 7.57 / 7.11.  Persistent CTAs of eight warps with the state and
+// rows of the next pair in registers lost 1 to 2 % (64 streams 2.67).
+__global__ void __launch_bounds__(64, 8) tmix_core_kernel(const TmixCoreArgs p) {
+    __shared__ __align__(16) float sA[64], sB[64], sW[64], sK[64], sR[64], sV[64];
+    __shared__ float sY[64], sT[64];
+    const int hi = blockIdx.x, b = blockIdx.y, tid = threadIdx.x, lane = tid & 31;
+    const size_t row = static_cast<size_t>(b) * p.D + hi * 64 + tid;
+    const int c = tid & 7, dv0 = (tid >> 3) * 8;
+    float* hp = p.state + ((static_cast<size_t>(b) * p.H + hi) * 64 + dv0) * 64 + 4 * c;     // columns 4 c .. and 32 + 4 c ..
+    float2 h[8][4];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const float4 lo = __ldcs(reinterpret_cast<const float4*>(hp + 64 * j)), hj = __ldcs(reinterpret_cast<const float4*>(hp + 64 * j + 32));
+        h[j][0] = make_float2(lo.x, lo.y); h[j][1] = make_float2(lo.z, lo.w);
+        h[j][2] = make_float2(hj.x, hj.y); h[j][3] = make_float2(hj.z, hj.w);
+    }
+    pdl_launch_dependents();
+    const int ch = hi * 64 + tid;
+    const float pw0 = __ldg(p.w0 + ch), pa0 = __ldg(p.a0 + ch), pka = __ldg(p.k_a + ch), pkk = __ldg(p.k_k + ch);
+    const float pv0 = p.layer0 ? 0.f : __ldg(p.v0 + ch);
+    const float prk0 = __ldg(p.r_k + hi * 64 + lane), prk1 = __ldg(p.r_k + hi * 64 + lane + 32), plw = __ldg(p.lnx_w + ch), plb = __ldg(p.lnx_b + ch);
+    pdl_wait();                              // the state above was written a whole token ago
+    const float r = __ldcg(p.r + row), k = __ldcg(p.k + row), yw = __ldcg(p.yw + row), ya = __ldcg(p.ya + row), g = __ldcg(p.g + row);
+    float v = __ldcg(p.v + row);
+    if (p.layer0) p.v_first[row] = v;
+    else v = v + (__ldcg(p.v_first + row) - v) * sigmoidf_(__ldcg(p.yv + row) + pv0);
+    const float w = expf(-0.606531f * sigmoidf_(yw + pw0)), av = sigmoidf_(ya + pa0), kk = k * pkk;
+    sT[tid] = kk * kk;
+    sW[tid] = w; sK[tid] = k * (1.0f + (av - 1.0f) * pka); sR[tid] = r; sV[tid] = v;
+    __syncthreads();
+    const float kn = kk * (1.0f / sqrtf(warp_sum64(sT, lane) + 1e-12f));
+    sA[tid] = -kn;
+    sB[tid] = kn * av;
+    __syncthreads();
+    float2 x[4];
+    float sa[8], y[8];
+    cols8(sA, c, x);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) sa[j] = dot8(h[j], x);
+    {
+        float2 wc[4], kc[4];                 // decay and v k^T while the sums cross the lanes
+        cols8(sW, c, wc);
+        cols8(sK, c, kc);
+        const float4 va = *reinterpret_cast<const float4*>(sV + dv0), vb = *reinterpret_cast<const float4*>(sV + dv0 + 4);
+        const float vs[8] = {va.x, va.y, va.z, va.w, vb.x, vb.y, vb.z, vb.w};
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const float2 vj = make_float2(vs[j], vs[j]);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) h[j][q] = __ffma2_rn(wc[q], h[j][q], __fmul2_rn(vj, kc[q]));
+        }
+    }
+#pragma unroll
+    for (int m = 1; m < 8; m <<= 1)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) sa[j] += __shfl_xor_sync(0xFFFFFFFFu, sa[j], m);
+    cols8(sB, c, x);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const float2 s2 = make_float2(sa[j], sa[j]);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) h[j][q] = __ffma2_rn(s2, x[q], h[j][q]);
+        *reinterpret_cast<float4*>(hp + 64 * j) = make_float4(h[j][0].x, h[j][0].y, h[j][1].x, h[j][1].y);
+        *reinterpret_cast<float4*>(hp + 64 * j + 32) = make_float4(h[j][2].x, h[j][2].y, h[j][3].x, h[j][3].y);
+    }
+    cols8(sR, c, x);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) y[j] = dot8(h[j], x);
+    // eight sums over eight lanes, half of them handed over at each of the three steps: lane bit 0 picks rows 0-3 or 4-7, bit 1 and 2 the row
+#pragma unroll
+    for (int n = 4, m = 1; n > 0; n >>= 1, m <<= 1)
+#pragma unroll
+        for (int j = 0; j < n; ++j) {
+            const bool up = (c & m) != 0;
+            const float keep = up ? y[j + n] : y[j], give = up ? y[j] : y[j + n];
+            y[j] = keep + __shfl_xor_sync(0xFFFFFFFFu, give, m);
+        }
+    sY[dv0 + (c & 1) * 4 + (c & 2) + (c >> 2)] = y[0];
+    __syncthreads();
+    // group norm over the head (two-pass), bonus, gate
+    const float mean = warp_sum64(sY, lane) / 64.f;
+    const float d0 = sY[lane] - mean, d1 = sY[lane + 32] - mean;
+    float var = d0 * d0 + d1 * d1, dp = sR[lane] * sK[lane] * prk0 + sR[lane + 32] * sK[lane + 32] * prk1;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        var += __shfl_xor_sync(0xFFFFFFFFu, var, o);
+        dp += __shfl_xor_sync(0xFFFFFFFFu, dp, o);
+    }
+    const float nrm = (sY[tid] - mean) * (1.0f / sqrtf(var / 64.f + 64e-5f));
+    const float o = (nrm * plw + plb + dp * v) * g;
+    p.og[row] = o;
+    if (p.og_amax != nullptr) {
+        float m = fabsf(o);
+#pragma unroll
+        for (int of = 16; of > 0; of >>= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, of));
+        if (lane == 0) atomicMax(reinterpret_cast<int*>(p.og_amax) + b, __float_as_int(m));
     }
 }
 
@@ -968,13 +1062,13 @@ int linear(const rwkvq_qtensor* t, const float* x, int B, int in, float* y, int 
 }
 
 int launch_tmix_core_up(const TmixCoreArgs& tc, const LoraVecArgs& up, int H, cudaStream_t s) {
-    decode_carveout<tmix_core_kernel<true>>();
+    decode_carveout<tmix_core_up_kernel>();
     const size_t smem = lora_vec_smem(up.first[up.n_br]);
     if (smem > 40 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(tmix_core_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLvMaxSmem);
+        cudaError_t e = cudaFuncSetAttribute(tmix_core_up_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kLvMaxSmem);
         if (e != cudaSuccess) return fail(RWKVQ_E_LIMIT, "tmix_core: %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
     }
-    cudaError_t e = launch_pdl(tmix_core_kernel<true>, dim3(H, 1), dim3(256), smem, s, tc, up);
+    cudaError_t e = launch_pdl(tmix_core_up_kernel, dim3(H, 1), dim3(256), smem, s, tc, up);
     if (e != cudaSuccess) return fail(RWKVQ_E_LAUNCH, "tmix_core: %s", cudaGetErrorString(e));
     return RWKVQ_OK;
 }
@@ -1224,7 +1318,7 @@ int rwkvq_decode_step(const rwkvq_model* m, int B, const int64_t* tokens, float*
             }
             rc = fork.join();                            // before the time-mix core
             if (rc) return rc;
-            launch_pdl(tmix_core_kernel<false>, dim3(H, B), dim3(256), 0, s, tc, 0);
+            launch_pdl(tmix_core_kernel, dim3(H, B), dim3(64), 0, s, tc);
         }
         if (sb) {
             const float* res[1] = {w.x};

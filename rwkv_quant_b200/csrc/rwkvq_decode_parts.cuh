@@ -17,6 +17,17 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
     return s;
 }
 
+// columns 4 c .. 4 c + 3 and 32 + 4 c .. of a row of 64: eight lanes read a row without bank conflicts
+__device__ __forceinline__ void cols8(const float* row, int c, float2 (&d)[4]) {
+    const float4 lo = *reinterpret_cast<const float4*>(row + 4 * c), hi = *reinterpret_cast<const float4*>(row + 32 + 4 * c);
+    d[0] = make_float2(lo.x, lo.y); d[1] = make_float2(lo.z, lo.w);
+    d[2] = make_float2(hi.x, hi.y); d[3] = make_float2(hi.z, hi.w);
+}
+__device__ __forceinline__ float dot8(const float2 (&h)[4], const float2 (&x)[4]) {
+    const float2 p = __ffma2_rn(h[1], x[1], __fmul2_rn(h[0], x[0])), q = __ffma2_rn(h[3], x[3], __fmul2_rn(h[2], x[2]));
+    return (p.x + p.y) + (q.x + q.y);
+}
+
 // 4 consecutive weights of stored row i at column c, in the loader's precision.
 // MODE 0: asym, cols % 4 == 0;  1: per-row int8, cols % 4 == 0;  2: anything (slow).
 template <int MODE>

@@ -23,17 +23,6 @@ struct TsSmem {
     float red[2][2][kTsChunk / 2];
 };
 
-// columns 4 c .. 4 c + 3 and 32 + 4 c .. of a row: eight lanes read a row without bank conflicts
-__device__ __forceinline__ void ts_cols(const float* row, int c, float2 (&d)[4]) {
-    const float4 lo = *reinterpret_cast<const float4*>(row + 4 * c), hi = *reinterpret_cast<const float4*>(row + 32 + 4 * c);
-    d[0] = make_float2(lo.x, lo.y); d[1] = make_float2(lo.z, lo.w);
-    d[2] = make_float2(hi.x, hi.y); d[3] = make_float2(hi.z, hi.w);
-}
-__device__ __forceinline__ float ts_dot(const float2 (&h)[4], const float2 (&x)[4]) {
-    const float2 p = __ffma2_rn(h[1], x[1], __fmul2_rn(h[0], x[0])), q = __ffma2_rn(h[3], x[3], __fmul2_rn(h[2], x[2]));
-    return (p.x + p.y) + (q.x + q.y);
-}
-
 // all warps of both roles
 __device__ __forceinline__ void ts_sync() { asm volatile("bar.sync 4, %0;" ::"n"(kTsThreads) : "memory"); }
 
@@ -82,7 +71,7 @@ __global__ void __launch_bounds__(kTsThreads, 2) tmix_seq_kernel(const TmixSeqAr
         float2 h[4][4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {                // written before the first kernel of this pass started
-            if (p.h_in) ts_cols(p.h_in + hbase + j * 64, c, h[j]);
+            if (p.h_in) cols8(p.h_in + hbase + j * 64, c, h[j]);
             else h[j][0] = h[j][1] = h[j][2] = h[j][3] = make_float2(0.f, 0.f);
         }
         pdl_wait();                                  // what this kernel stores may be read by the kernels before it
@@ -94,15 +83,15 @@ __global__ void __launch_bounds__(kTsThreads, 2) tmix_seq_kernel(const TmixSeqAr
             for (int t = 0; t < n; ++t) {
                 float2 x[4];
                 float sa[4], y[4];
-                ts_cols(o.a[t], c, x);
+                cols8(o.a[t], c, x);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) sa[j] = ts_dot(h[j], x);
+                for (int j = 0; j < 4; ++j) sa[j] = dot8(h[j], x);
                 const float4 v4 = *reinterpret_cast<const float4*>(&o.v[t][dv0]);
                 const float v[4] = {v4.x, v4.y, v4.z, v4.w};
                 {
                     float2 w[4], k[4];               // decay and v k^T while the sums cross the lanes
-                    ts_cols(o.w[t], c, w);
-                    ts_cols(o.k[t], c, k);
+                    cols8(o.w[t], c, w);
+                    cols8(o.k[t], c, k);
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         const float2 vj = make_float2(v[j], v[j]);
@@ -114,16 +103,16 @@ __global__ void __launch_bounds__(kTsThreads, 2) tmix_seq_kernel(const TmixSeqAr
                 for (int m = 1; m < 8; m <<= 1)
 #pragma unroll
                     for (int j = 0; j < 4; ++j) sa[j] += __shfl_xor_sync(0xFFFFFFFFu, sa[j], m);
-                ts_cols(o.b[t], c, x);
+                cols8(o.b[t], c, x);
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const float2 s2 = make_float2(sa[j], sa[j]);
 #pragma unroll
                     for (int q = 0; q < 4; ++q) h[j][q] = __ffma2_rn(s2, x[q], h[j][q]);
                 }
-                ts_cols(o.r[t], c, x);
+                cols8(o.r[t], c, x);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) y[j] = ts_dot(h[j], x);
+                for (int j = 0; j < 4; ++j) y[j] = dot8(h[j], x);
                 // four sums over eight lanes, halving the values: lane bits 0 and 1 pick the row
                 const float k0 = (c & 1) ? y[2] : y[0], k1 = (c & 1) ? y[3] : y[1], g0 = (c & 1) ? y[0] : y[2], g1 = (c & 1) ? y[1] : y[3];
                 const float u0 = k0 + __shfl_xor_sync(0xFFFFFFFFu, g0, 1), u1 = k1 + __shfl_xor_sync(0xFFFFFFFFu, g1, 1);

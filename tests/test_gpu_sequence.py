@@ -107,6 +107,23 @@ def test_time_mix_of_short_sequences_matches_its_steps(cuda_lib, B, T):
         _same(got, (torch.cat(rows, 1), st), 1e-4)
 
 
+@pytest.mark.parametrize("recipe,D,B,T", [("compression", 256, 2, 3), ("compression", 768, 3, 3), ("reduction", 256, 16, 3),
+                                          ("compression", 256, 17, 3), ("reduction", 768, 21, 3)])
+def test_steps_of_several_streams_match_the_sequence(cuda_lib, recipe, D, B, T):
+    """The time mix of a step against the per-operator path (64 rows at most: above, its linears have fp16 operands): logits and
+    all states after T tokens."""
+    model = _model(recipe, n_embd=D, ffn=1024)
+    idx = torch.randint(1, 512, (B, T), generator=torch.Generator().manual_seed(B)).cuda()
+    st = _states(model, B)
+    dec = model.decoder(B, states=[tuple(t.clone() for t in s) for s in st])
+    steps = []
+    for t in range(T):
+        dec.step(idx[:, t])
+        steps.append(dec.logits.clone())
+    model.fused_prep = False
+    _same((torch.stack(steps, 1), dec.states), model.forward_stateful(idx, st), 1e-4)
+
+
 @pytest.mark.parametrize("B,T", [(1, 255), (1, 256), (2, 300), (37, 256), (38, 256)])
 def test_weights_converted_beside_the_scan(cuda_lib, B, T):
     """Calls on each side of the lines from which the weights become fp16 on the side stream, against the per-operator path; a
