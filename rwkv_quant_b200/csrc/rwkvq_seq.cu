@@ -10,6 +10,8 @@
 //                      -kk and kk*a, the operands of the WKV-7 scan       (quant_model.py:700-712)
 #include "rwkvq_seq.cuh"
 
+#include <algorithm>
+
 #include "rwkvq_decode_parts.cuh"
 
 namespace rwkvq {
@@ -376,6 +378,102 @@ __global__ void __launch_bounds__(kSeqVecWarps * 32) seq_prep_vec_kernel(const S
     }
 }
 
+// One token of each stream, the shift state in place: all mixes of a token in one CTA, which holds the row and the state it
+// replaces.  Bound: the latency of three block reductions (two sums, the maxima of all mixes together) and of a thread's 6 x 8 columns
+// out; the form of many streams, see the dispatch.
+__global__ void __launch_bounds__(kSeqVecWarps * 32) seq_prep_step_kernel(const SeqPrepArgs a) {
+    constexpr int M = 6;
+    __shared__ float red_s[kSeqVecWarps], red_q[kSeqVecWarps], red_n[kSeqVecWarps], red_m[kSeqVecWarps][M];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
+    const int D = a.D, d0 = tid * 8;
+    const long long tok = blockIdx.x;
+    float lw[8], lb[8], mx[M][8];
+    prep_load8(a.ln_w + d0, lw);
+    prep_load8(a.ln_b + d0, lb);
+#pragma unroll
+    for (int m = 0; m < M; ++m)
+        if (m < a.n_mix) prep_load8(a.mix + static_cast<size_t>(m) * D + d0, mx[m]);
+    pdl_launch_dependents();
+    pdl_wait();
+    if (tid == 0) {
+        if (a.zero_a != nullptr) a.zero_a[tok] = 0.f;
+        if (a.zero_b != nullptr) a.zero_b[tok] = 0.f;
+    }
+    float v[8], pv[8];
+    prep_load8cg(a.x + tok * D + d0, v);
+    prep_load8cg(a.shift_in + tok * D + d0, pv);
+    float r = warp_add(((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7])));
+    if (lane == 0) red_s[warp] = r;
+    __syncthreads();
+    r = 0.f;
+    for (int w = 0; w < nw; ++w) r += red_s[w];
+    const float mean = r / D;
+    r = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) { const float c = v[i] - mean; r = fmaf(c, c, r); }
+    r = warp_add(r);
+    if (lane == 0) red_q[warp] = r;
+    __syncthreads();
+    r = 0.f;
+    for (int w = 0; w < nw; ++w) r += red_q[w];
+    const float inv = 1.0f / sqrtf(r / D + 1e-5f);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        v[i] = (v[i] - mean) * inv * lw[i] + lb[i];
+        pv[i] -= v[i];                                   // xx = prev - cur
+    }
+    prep_store8(a.shift_out + tok * D + d0, v);
+    float am[M], n2 = 0.f;
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+        am[m] = 0.f;
+        if (m >= a.n_mix) continue;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float o = v[i] + pv[i] * mx[m][i];
+            am[m] = fmaxf(am[m], fabsf(o));
+            if (m == 0) n2 = fmaf(o, o, n2);
+        }
+    }
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+#pragma unroll
+        for (int q = 16; q > 0; q >>= 1) am[m] = fmaxf(am[m], __shfl_xor_sync(0xFFFFFFFFu, am[m], q));
+        if (lane == 0) red_m[warp][m] = am[m];
+    }
+    n2 = warp_add(n2);
+    if (lane == 0) red_n[warp] = n2;
+    __syncthreads();
+    if (a.n2 != nullptr && tid == 0) {
+        n2 = 0.f;
+        for (int w = 0; w < nw; ++w) n2 += red_n[w];
+        a.n2[tok] = n2;
+    }
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+        if (m >= a.n_mix) break;
+        const int mode = a.mode[m];
+        float o[8], sc = 1.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) o[i] = v[i] + pv[i] * mx[m][i];
+        if (mode & (kPrepScaled | kPrepAmax | kPrepPair)) {
+            float top = 0.f;
+            for (int w = 0; w < nw; ++w) top = fmaxf(top, red_m[w][m]);
+            sc = prep_scale(top);
+            if (tid == 0 && (mode & (kPrepScaled | kPrepAmax))) a.scale[m][tok] = (mode & kPrepScaled) ? sc : top;
+            if (mode & kPrepPair) {                      // the mode goes alone or with kPrepF32
+                float s1, u1, q[8];
+                sb_scale(top, s1, u1);
+                if (tid == 0) a.pair[m].unscale[tok] = u1;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) q[i] = o[i] * s1;
+                sb_store_pair(a.pair[m], static_cast<int>(tok), static_cast<int>(gridDim.x), tid, q);
+            }
+        }
+        prep_emit8(a, m, mode, tok, d0, o, sc);
+    }
+}
+
 // Many tokens, D a multiple of 512: 64 threads per token (a barrier of two warps, not of a CTA, behind
 // every sum), four tokens side by side in a CTA that share the parameters and lerp vectors in shared
 // memory; a group walks a run of consecutive tokens and keeps the normalised row for its successor.
@@ -540,7 +638,7 @@ int launch_seq_prep(const SeqPrepArgs& a, long long n_tokens, cudaStream_t s) {
     RWKVQ_REQUIRE(aligned(a.x, 8) && aligned(a.ln_w, 8) && aligned(a.ln_b, 8) && aligned(a.mix, 8) && aligned(a.shift_in, 8) && aligned(a.shift_out, 8),
                   RWKVQ_E_ALIGN, "seq_ln_shift_mix_prep: 8-byte aligned rows required");       // the scalar form reads pairs
     RWKVQ_REQUIRE(!in_place || a.T == 1, RWKVQ_E_SHAPE, "seq_ln_shift_mix_prep: the shift state in place needs T = 1");
-    // (in place: the scalar form has a token's mixes in one CTA, the vector form in one cluster)
+    // (in place: the scalar and the step form have a token's mixes in one CTA, the vector form in one cluster)
     // Which form (us, scalar / vector / groups, six mixes and one):
     //   few      the vector form while its CTAs, one per token and mix, are one wave: two an SM up to 2048 columns, one above (six
     //            mixes: still ahead at two a slot).  2048 columns, 49 tokens: 7.6 / 4.1, one mix 296: 4.8 / 4.2; 2304, 231: 4.9 / 7.1
@@ -562,6 +660,11 @@ int launch_seq_prep(const SeqPrepArgs& a, long long n_tokens, cudaStream_t s) {
             case 5: e = launch_prep_group<5>(a, n_tokens, s); break;
             default: e = launch_prep_group<6>(a, n_tokens, s); break;
         }
+    } else if (vec && in_place && a.n_mix > 1 && 2 * n_tokens * a.n_mix > 3 * 148 * std::max(1, 65536 / (112 * a.D / 8))) {
+        // A CTA per token instead of a cluster of one per mix, which normalises the row six times, from where the clusters are one
+        // and a half waves (by registers: two CTAs an SM at 2048 columns, one above).  us a step, cluster / this: 1.5B 16 streams 1760 /
+        // 1855, 64 2447 / 2485, 100 3369 / 3315, 200 5049 / 4810; 2.9B 32 streams 3418 / 3453, 64 4492 / 4281, 128 7074 / 6565
+        e = launch_pdl(seq_prep_step_kernel, dim3(static_cast<unsigned>(n_tokens)), dim3(a.D / 8), 0, s, a);
     } else if (vec && in_place && a.n_mix > 1) {
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(static_cast<unsigned>(n_tokens), a.n_mix);

@@ -108,9 +108,10 @@ def test_time_mix_of_short_sequences_matches_its_steps(cuda_lib, B, T):
 
 
 @pytest.mark.parametrize("recipe,D,B,T", [("compression", 256, 2, 3), ("compression", 768, 3, 3), ("reduction", 256, 16, 3),
-                                          ("compression", 256, 17, 3), ("reduction", 768, 21, 3)])
+                                          ("compression", 256, 17, 3), ("reduction", 768, 21, 3), ("compression", 2304, 37, 1),
+                                          ("compression", 2304, 38, 1), ("reduction", 4096, 40, 1), ("compression", 256, 46, 1)])
 def test_steps_of_several_streams_match_the_sequence(cuda_lib, recipe, D, B, T):
-    """The time mix of a step against the per-operator path (64 rows at most: above, its linears have fp16 operands): logits and
+    """The time mix and the LayerNorms of a step against the per-operator path (64 rows at most: above, its linears have fp16 operands): logits and
     all states after T tokens."""
     model = _model(recipe, n_embd=D, ffn=1024)
     idx = torch.randint(1, 512, (B, T), generator=torch.Generator().manual_seed(B)).cuda()
