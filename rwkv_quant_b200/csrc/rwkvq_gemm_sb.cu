@@ -600,8 +600,10 @@ int launch_sb(SbArgs& a, const SbMaps& maps, int groups, int force_ks, const Ahe
         if (dev < 64) configured[dev] = true;
     }
     // K split into up to 8 slices of whole super-blocks, by a model of the slowest CTA in microseconds fitted to
-    // [2048, 2048] .. [65536, 2048] at 8 to 128 rows: 0.37 to 0.55 a stage by the tile's width, 5 for ramp and store, 3.5 for the cluster
-    // reduction; without a split the CTAs are persistent and pay the ramp once
+    // [2048, 2048] .. [65536, 2048] at 8 to 128 rows: 0.37 to 0.55 per 64 columns by the tile's width, 5 for ramp and store, 3.5 for the
+    // cluster reduction; without a split the CTAs are persistent and pay the ramp once.  (Fitted to units of 64 columns; with units of
+    // 128, 0.30, 0.33 and 0.41 per 64 at 13, 64 and 100 rows, it still picks the fastest split or one within 2 % of it: 8 shapes
+    // [2048, 2048] .. [10240, 2560] and [2560, 10240], sb6 4 bits and sym 8 bits, at those rows, every split from 1 to 8)
     const double stage = std::max(0.37, 0.41 + 0.0022 * (a.nt - 64));
     double best = 1e300;
     a.ks = 1;
