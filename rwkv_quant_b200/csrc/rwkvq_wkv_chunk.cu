@@ -522,17 +522,26 @@ __global__ void __launch_bounds__(512) wkv_chunk_tail_kernel(const WkvChunkArgs 
     load8(p.g + at, g);
     load8(p.ops + ((static_cast<size_t>(b) * p.H + hd) * n_chunks + t / kC) * kChunkFloats + kOffV + (t % kC) * kS + ci, v);
     const float dp = __ldcg(p.dp + static_cast<size_t>(blockIdx.x) * p.H + hd);
-    auto head_sum = [](const float (&x)[8]) {                       // 8 lanes hold a head
-        float s = ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));
+    // A head's sum over its 8 lanes, from sums of neighbours, in the order of a butterfly over 32 lanes of two channels each: the fp16
+    // rounding behind it carries another order's 1e-7 into 2^-11 of a value, 7e-4 of the logits 24 layers on.
+    auto head_sum = [](float (&x)[4]) {
 #pragma unroll
-        for (int o = 1; o < 8; o <<= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
-        return s;
+        for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) x[i] += __shfl_xor_sync(0xFFFFFFFFu, x[i], o);
+        return (x[0] + x[2]) + (x[1] + x[3]);
     };
-    const float m = head_sum(y) / kS;
-    float d2[8];
+    float two[4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) { y[i] -= m; d2[i] = y[i] * y[i]; }
-    const float inv = 1.0f / sqrtf(head_sum(d2) / kS + 64e-5f);
+    for (int i = 0; i < 4; ++i) two[i] = y[2 * i] + y[2 * i + 1];
+    const float m = head_sum(two) / kS;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float d0 = y[2 * i] - m, d1 = y[2 * i + 1] - m;
+        two[i] = d0 * d0 + d1 * d1;
+        y[2 * i] = d0; y[2 * i + 1] = d1;
+    }
+    const float inv = 1.0f / sqrtf(head_sum(two) / kS + 64e-5f);
     float amax = 0.f;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
