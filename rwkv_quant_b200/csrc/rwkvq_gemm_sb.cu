@@ -25,8 +25,9 @@
 // the first bytes were asked for, 0.5 by TMA.
 // The mma.sync form of the same product (rwkvq_gemv_batch.cu) issues 3 MMAs of 16 x 8 x 16 per warp and step and tops out
 // at 0.92 G MMA/s per SM.
-// Every mbarrier wait is bounded; a warp whose wait ran out waits no more, the status word is set and all roles run to the
-// common end.
+// Every mbarrier wait is bounded.  A warp whose wait ran out waits and arrives no more (an arrival for a unit that it did not wait for
+// would count towards a phase whose copies are still on their way), the status word is set and all roles run to the common end.
+// The two warps that issue copies leave their part only when those have landed, or a wait for them has run out too.
 #include "rwkvq_gemm_sb.cuh"
 
 #include <cooperative_groups.h>
@@ -219,7 +220,6 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
 
     int sb_before = 0;                                               // super-blocks of the tiles before
     bool alive = true;                                               // no wait of this warp has run out
-    int raw_issued = 0;                                              // super-blocks asked for (the thread that does)
     uint32_t done_phase = 0;
     for (int ti = 0; ti < n_my; ++ti) {
         const int tile = first_tile + ti * tile_step, mat = tile / a.row_tiles, row0 = (tile % a.row_tiles) * kGmRows;
@@ -260,9 +260,10 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
             if (alive && elected) umma_commit(&bar_done);
         } else if (warp == kSbRawWarp) {
             // ------------------------------------------------------------------ packed weights: do not depend on the producer of x
-            if (lane == 0) {
-                for (int sb = 0; sb < n_super; ++sb) {
-                    const int qi = sb_before + sb, slot = qi % G::AHEAD;
+            if (lane == 0 && alive) {
+                int qi = sb_before;
+                for (; qi < sb_before + n_super; ++qi) {
+                    const int sb = qi - sb_before, slot = qi % G::AHEAD;
                     alive = alive && (qi < G::AHEAD || mbar_poll_bounded(&raw_empty[slot], (qi / G::AHEAD - 1) & 1));
                     if (!alive) break;
                     unsigned char* w = smem + G::OFF_RAW + slot * Y::RAW;
@@ -272,14 +273,16 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
                         tma_load_2d(w + c * (kGmRows * 128), &maps.codes[mat], (sb0 + sb) * Y::CODE_ROW + c * 128, row0, &raw_full[slot]);
                     if (Y::PLANE_ROW > 0) tma_load_2d(w + Y::OFF_P, &maps.planes[mat], (sb0 + sb) * Y::PLANE_ROW, row0, &raw_full[slot]);
                     tma_load_2d(w + Y::OFF_R, &maps.rec[mat], (sb0 + sb) * 16, row0, &raw_full[slot]);
-                    raw_issued = qi + 1;
                 }
+                if (!alive || ti == n_my - 1)                        // the last copy of each slot: all others were waited for
+                    for (int q = max(0, qi - G::AHEAD); q < qi; ++q) mbar_poll_bounded(&raw_full[q % G::AHEAD], (q / G::AHEAD) & 1);
             }
         } else if (warp == kSbTmaWarp) {
             // ------------------------------------------------------------------ activation pairs
-            if (lane == 0) {
-                for (int u = 0; u < 2 * n_super; ++u) {
-                    const int g = 2 * sb_before + u, buf = g % G::U;
+            if (lane == 0 && alive) {
+                int g = 2 * sb_before;
+                for (; g < 2 * (sb_before + n_super); ++g) {
+                    const int u = g - 2 * sb_before, buf = g % G::U;
                     alive = alive && (g < G::U || mbar_poll_bounded(&bar_empty[buf], (g / G::U - 1) & 1));
                     if (!alive) break;
                     unsigned char* b = smem + buf * G::BSLAB;
@@ -302,6 +305,8 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
                                          : "memory");
                     }
                 }
+                if (!alive || ti == n_my - 1)                        // the last unit of each buffer has been multiplied
+                    for (int d = max(0, g - G::U); d < g; ++d) mbar_poll_bounded(&bar_empty[d % G::U], (d / G::U) & 1);
             }
         } else {
             // ------------------------------------------------------------------ weights
@@ -339,7 +344,7 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
                 }
                 const uint4 rec = *reinterpret_cast<const uint4*>(raw + Y::OFF_R + wrow * 16);
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&raw_empty[slot]);        // the super-block is in registers
+                if (lane == 0 && alive) mbar_arrive(&raw_empty[slot]);        // the super-block is in registers
                 const uint32_t dd = d_next * 0x00010001u;
                 if (!Y::SB6 && sb + 1 < n_super) d_next = __half_as_ushort(__ldg(dp + sb + 1));
 #pragma unroll
@@ -382,7 +387,7 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
                     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                     tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(&bar_full[buf]);
+                    if (lane == 0 && alive) mbar_arrive(&bar_full[buf]);
                 }
             }
         }
@@ -498,9 +503,6 @@ __global__ void __launch_bounds__(kSbThreads, 1) gemm_sb_kernel(const __grid_con
             cluster.sync();                                          // nobody leaves while a peer still reads its partial tile
         }
     }
-    // where a wait ran out, copies may still be on their way
-    if (s_fail && warp == kSbRawWarp && lane == 0)
-        for (int qi = max(0, raw_issued - G::AHEAD); qi < raw_issued; ++qi) mbar_poll_bounded(&raw_full[qi % G::AHEAD], (qi / G::AHEAD) & 1);
     __syncthreads();
     if (tid == 0 && s_fail) atomicCAS(a.status, 0, RWKVQ_E_TIMEOUT);
     tc_fence_after();
