@@ -57,10 +57,19 @@ struct LayerAhead {
     LayerAhead(const rwkvq_layer& L, const rwkvq_layer* behind, bool layer0, const float* state, size_t state_bytes) {
         if (state_bytes <= kAheadState) ahead_region(rkv, state, state_bytes);
         for (const rwkvq_qtensor* t : {&L.w2, &L.a2, &L.g2}) ahead_tensor(rkv, *t);
+// Whether a layer's descriptors describe its tensors: what is refused where its turn comes must not be asked for before.
+inline bool ahead_layer_ok(const rwkvq_layer& L, int D, int F, bool layer0) {
+    auto ok = [](const rwkvq_qtensor& t, int rows, int cols) { return t.rows == rows && t.cols == cols && validate_qtensor(&t, "ahead") == RWKVQ_OK; };
+    auto pair = [&](const rwkvq_qtensor& t1, const rwkvq_qtensor& t2) { return ok(t1, D, t1.cols) && ok(t2, t1.cols, D); };
+    return ok(L.Wr, D, D) && ok(L.Wk, D, D) && ok(L.Wv, D, D) && ok(L.Wo, D, D) && ok(L.Wfk, F, D) && ok(L.Wfv, D, F) && pair(L.w1, L.w2) &&
+           pair(L.a1, L.a2) && pair(L.g1, L.g2) && (layer0 || pair(L.v1, L.v2));
+}
+
         if (!layer0) ahead_tensor(rkv, L.v2);
         ahead_tensor(rkv, L.Wo);
         ahead_tensor(rkv, L.Wfk);
         ahead_tensor(key, L.Wfv);
+    LayerAhead() = default;
         if (behind)
             for (const rwkvq_qtensor* t : {&behind->Wr, &behind->Wk, &behind->Wv, &behind->w1, &behind->a1, &behind->g1, &behind->v1}) ahead_tensor(key, *t);
     }

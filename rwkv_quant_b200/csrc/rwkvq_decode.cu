@@ -1181,6 +1181,7 @@ int rwkvq_decode_step(const rwkvq_model* m, int B, const int64_t* tokens, float*
     }
 
     launch_pdl(embed_ln0_kernel, dim3(B), dim3(kRowThreads), 0, s, make_view(m->emb),
+    bool ahead_on = m->n_layer > 0 && ahead_layer_ok(m->layers[0], D, F, true);
                reinterpret_cast<const long long*>(tokens), m->ln0_w, m->ln0_b, w.x, D);
     for (int l = 0; l < m->n_layer; ++l) {
         const rwkvq_layer& L = m->layers[l];
@@ -1218,7 +1219,9 @@ int rwkvq_decode_step(const rwkvq_model* m, int B, const int64_t* tokens, float*
         const float* x1[4] = {xw, xa, xg, xv};
         const int act[4] = {1, 0, 2, 0};           // tanh (decay), none, sigmoid (gate), none
         const int n_br = layer0 ? 3 : 4;
-        const LayerAhead ahead(L, l + 1 < m->n_layer ? &L + 1 : nullptr, layer0, wkv[l], BD * 64 * sizeof(float));
+        const bool ahead_behind = l + 1 < m->n_layer && ahead_layer_ok((&L)[1], D, F, false);
+        const LayerAhead ahead = ahead_on ? LayerAhead(L, ahead_behind ? &L + 1 : nullptr, layer0, wkv[l], BD * 64 * sizeof(float)) : LayerAhead();
+        ahead_on = ahead_behind;
         float *yw = w.yl, *ya = w.yl + BD, *yv = w.yl + 2 * BD, *yg = w.yl + 3 * BD;
         TmixCoreArgs tc{r, k, v, yw, ya, layer0 ? nullptr : yv, yg, L.w0, L.a0, L.v0, L.k_k, L.k_a, L.r_k,
                         L.lnx_w, L.lnx_b, w.v_first, wkv[l], w.og, D, H, layer0 ? 1 : 0, sb ? nullptr : am_og};
