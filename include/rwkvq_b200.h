@@ -193,17 +193,17 @@ int rwkvq_quantize_sym6_packed(const float* w, int64_t ldw, int rows, int cols, 
  * activations; activations: hi + lo of x scaled per token by a power of two chosen from its max|x|),
  * fp32 accumulation: the result agrees with an fp32 dequantise-and-multiply, and with rwkvq_gemv,
  * to ~1e-6 of max|y| (a column's last bits may depend on the batch it is computed in; two calls on
- * the same input give the same bits).  The K split is reduced across a thread-block cluster through
+ * the same input and with equal workspace_bytes give the same bits).  The K split is reduced across a thread-block cluster through
  * distributed shared memory: no scratch for partial sums.
  * Up to 8 rows the products run on mma.sync; from 9 rows on sb6 / sym tensors with whole 256-column
  * super-blocks (up to 16384 columns) run on the tcgen05 tensor cores in the same arithmetic (rows of 128
- * as the UMMA M, the converted weights as its operand in tensor memory, the batch as its N); 9 to 16 rows
- * where the workspace is that of rwkvq_gemv_batch_workspace_bytes(N) or has as much room, else on mma.sync.
+ * as the UMMA M, the converted weights as its operand in tensor memory, the batch as its N).
  * With RWKVQ_BATCH_FAST=1 in the environment (read once per process) single fp16 operands are used
  * instead (weights fp16(q*s+m)): results within ~3e-4 of max|y| per call (the precision of rwkvq_gemm),
  * and sb6 / sym tensors with more than 32 rows run on a single-term tcgen05 form.
  *   workspace: rwkvq_gemv_batch_workspace_bytes_of(t, N) bytes (rwkvq_gemv_batch_workspace_bytes(N): whatever
- *   the tensor), 16-byte aligned: a status word (first
+ *   the tensor; with 9 to 16 rows a call that has room for the status word and the row maxima only,
+ *   256 + 256 bytes, is served by mma.sync, whose last bits differ), 16-byte aligned: a status word (first
  *   int32: RWKVQ_E_TIMEOUT if a bounded wait on the tensor-core pipeline ran out; read it after
  *   synchronising the stream, 0 = ok), one float per row (max|x|, or the inverse scale of the pairs) and
  *   the rows as fp16 pairs, which a one-block-per-row pre-pass writes before the product kernel starts.

@@ -306,7 +306,7 @@ def has_batch_layout(dq: "DeviceQT") -> bool:
 def gemv_batch(dq: "DeviceQT", x: torch.Tensor, epilogue: int = 0, resid: Optional[torch.Tensor] = None,
                check: bool = False) -> torch.Tensor:
     """x [N, IN] -> y [N, OUT] fp32 with the packed weights read once for up to 128 rows: tokens as the MMA columns, both
-    operands as fp16 pairs, fp32 accumulation (mma.sync up to 16 rows, the tcgen05 pipeline above)."""
+    operands as fp16 pairs, fp32 accumulation (mma.sync up to 8 rows, the tcgen05 pipeline above)."""
     _require_cuda(dq.bufs[0], x, resid)
     lib = _lib.load()
     x = x.float()
@@ -314,8 +314,7 @@ def gemv_batch(dq: "DeviceQT", x: torch.Tensor, epilogue: int = 0, resid: Option
         x = x.contiguous()
     n = x.shape[0]
     y = torch.empty((n, dq.rows), dtype=torch.float32, device=x.device)
-    # 9 to 16 rows: with room for operand pairs the product takes the tcgen05 pipeline
-    nws = lib.rwkvq_gemv_batch_workspace_bytes(n) if 9 <= n <= 16 else lib.rwkvq_gemv_batch_workspace_bytes_of(dq.struct_ref, n)
+    nws = lib.rwkvq_gemv_batch_workspace_bytes_of(dq.struct_ref, n)
     ws = torch.empty(nws, dtype=torch.uint8, device=x.device)
     _lib.check(lib.rwkvq_gemv_batch(dq.struct_ref, x.data_ptr(), n, x.stride(0), y.data_ptr(), y.stride(0),
                                     epilogue, _lib.ptr(resid), ws.data_ptr(), nws, _lib.stream_ptr()), "rwkvq_gemv_batch")

@@ -766,9 +766,11 @@ bool batch_on_pipeline(const rwkvq_qtensor& t, int N) {
 }
 extern "C" size_t rwkvq_gemv_batch_workspace_bytes(int N) { return N > 0 ? batch_ws_pairs(N) + sb_halves(N, kPairCols) * sizeof(__half) : 0; }
 extern "C" size_t rwkvq_gemv_batch_workspace_bytes_of(const rwkvq_qtensor* t, int N) {
-    if (!t || N < 1) return 0;
-    // what a call needs: up to 16 rows the row maxima (with room for the pairs it takes the pipeline from 9 on all the same)
-    return N <= kPairsOptional ? batch_ws_pairs(N) : 256 + gemv_batch_rows_bytes(*t, N);
+    return t && N >= 1 ? 256 + gemv_batch_rows_bytes(*t, N) : 0;
+}
+// What a call is accepted with: up to 16 rows the row maxima alone, for the mma.sync kernel
+static size_t batch_ws_least(const rwkvq_qtensor& t, int N) {
+    return N <= kPairsOptional && !tcb_forced() ? batch_ws_pairs(N) : 256 + gemv_batch_rows_bytes(t, N);
 }
 size_t rwkvq::gemv_batch_rows_bytes(const rwkvq_qtensor& t, int N) {
     return batch_ws_pairs(N) - 256 + (batch_on_pipeline(t, N) ? sb_halves(N, t.cols) * sizeof(__half) : 0);
@@ -815,7 +817,7 @@ extern "C" int rwkvq_gemv_batch(const rwkvq_qtensor* t, const float* x, int N, i
     RWKVQ_REQUIRE(x && y, RWKVQ_E_NULL, "rwkvq_gemv_batch: x or y is null");
     RWKVQ_REQUIRE(aligned(x, 16) && ldx % 4 == 0, RWKVQ_E_ALIGN, "rwkvq_gemv_batch: x rows must be 16-byte aligned");
     RWKVQ_REQUIRE(aligned(workspace, 16), RWKVQ_E_ALIGN, "rwkvq_gemv_batch: workspace must be 16-byte aligned");
-    RWKVQ_REQUIRE(workspace && workspace_bytes >= rwkvq_gemv_batch_workspace_bytes_of(t, N), RWKVQ_E_LIMIT,
+    RWKVQ_REQUIRE(workspace && workspace_bytes >= batch_ws_least(*t, N), RWKVQ_E_LIMIT,
                   "rwkvq_gemv_batch: workspace of %zu bytes, %zu needed", workspace_bytes, rwkvq_gemv_batch_workspace_bytes_of(t, N));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     rc = launch_gemv_batch_rows(*t, x, N, ldx, y, ldy, epilogue, resid, static_cast<char*>(workspace) + 256, static_cast<int*>(workspace),

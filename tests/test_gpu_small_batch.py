@@ -42,7 +42,7 @@ def test_token_tiles_and_k_splits(cuda_lib, layout, bits, rows, cols, ks):
         force(0)
 
 
-@pytest.mark.parametrize("N", [2, 8, 17, 64, 128])
+@pytest.mark.parametrize("N", [2, 8, 9, 16, 17, 64, 128])
 def test_error_of_a_long_chain(cuda_lib, N):
     """Rows without a K split: 2048 columns are 128 steps of an accumulator that the tensor cores truncate, 2^-24 of the
     partial sum on average at the end of the chain and half of that over it.  The terms with a low half stay out of that chain
@@ -59,21 +59,37 @@ def test_error_of_a_long_chain(cuda_lib, N):
 
 @pytest.mark.parametrize("layout,bits", [("sb6", 5), ("sym", 6)])
 @pytest.mark.parametrize("N", [8, 9, 16, 17])
-def test_either_workspace_serves_a_call(cuda_lib, layout, bits, N):
-    """9 to 16 rows take the kernel that the scratch has room for; both are fp32 grade (2e-5, as above)."""
-    import ctypes as C
+def test_which_kernel_serves_a_call(cuda_lib, layout, bits, N):
+    """With the workspace of the tensor a call of 9 rows and more has the bits of the pipeline, one of 8 those of mma.sync; up to 16
+    rows the row maxima alone are enough, for mma.sync.  All are fp32 grade (2e-5, as above)."""
     from rwkv_quant_b200 import _lib
     from rwkv_quant_b200.backends.cuda import ops
     lib, dq = _lib.load(), ops.DeviceQT(_synth_linear(layout, bits, 300, 768, seed=N))
     x = _x(N, 768, seed=N)
     ref = x.cpu().numpy().astype(np.float64) @ _oracle_w(_synth_linear(layout, bits, 300, 768, seed=N)).astype(np.float64).T
-    least = lib.rwkvq_gemv_batch_workspace_bytes_of(dq.struct_ref, N)
-    for nws in (least, lib.rwkvq_gemv_batch_workspace_bytes(N)):
+    force = lib.rwkvq_profiling_tcb_force
+    force.restype, force.argtypes = None, [C.c_int]
+
+    def call(nws, forced=0):
         y, ws = torch.empty(N, 300, device="cuda"), torch.empty(nws, dtype=torch.uint8, device="cuda")
-        _lib.check(lib.rwkvq_gemv_batch(dq.struct_ref, x.data_ptr(), N, x.stride(0), y.data_ptr(), 300, 0, None, ws.data_ptr(), nws,
-                                        _lib.stream_ptr()), "rwkvq_gemv_batch")
+        force(forced)
+        try:
+            rc = lib.rwkvq_gemv_batch(dq.struct_ref, x.data_ptr(), N, x.stride(0), y.data_ptr(), 300, 0, None, ws.data_ptr(), nws,
+                                      _lib.stream_ptr())
+        finally:
+            force(0)
+        if rc:
+            return None
         assert int(ws[:4].view(torch.int32).item()) == 0
         assert relmax(y.cpu().numpy(), ref) <= 2e-5
-    ws = torch.empty(least - 1, dtype=torch.uint8, device="cuda")
-    assert lib.rwkvq_gemv_batch(dq.struct_ref, x.data_ptr(), N, x.stride(0), y.data_ptr(), 300, 0, None, ws.data_ptr(), least - 1,
-                                _lib.stream_ptr()) != 0
+        return y
+
+    rows, room = 256 + 256, lib.rwkvq_gemv_batch_workspace_bytes(N)
+    own = call(lib.rwkvq_gemv_batch_workspace_bytes_of(dq.struct_ref, N))
+    mma, pipeline = call(room, -1), call(room, 1000)
+    assert not torch.equal(mma, pipeline)
+    for y in (own, call(room), ops.gemv_batch(dq, x)):
+        assert torch.equal(y, pipeline if N >= 9 else mma)
+    least = call(rows)
+    assert least is None if N > 16 else torch.equal(least, mma)
+    assert call(rows - 1) is None and call(rows, 1000) is None

@@ -40,7 +40,8 @@ def test_gemm_holds_its_own_weights():
         assert of(t, 500, 1) <= lib.rwkvq_gemm_workspace_bytes_for(500, t.cols) and of(t, 500, 0) <= lib.rwkvq_gemm_workspace_bytes_for(500, 0)
 
 
-@pytest.mark.parametrize("tensor,n,pairs", [(("sb6", 4, 2048, 2048), 16, False), (("sb6", 4, 2048, 2048), 17, True),
+@pytest.mark.parametrize("tensor,n,pairs", [(("sb6", 4, 2048, 2048), 8, False), (("sb6", 4, 2048, 2048), 9, True),
+                                            (("sb6", 4, 2048, 2048), 16, True), (("sb6", 4, 2048, 2048), 17, True),
                                             (("sb6", 4, 2048, 2048, False), 100, False), (("rtn", 8, 2048, 2048), 4096, False),
                                             (("sym", 8, 256, 16640), 100, False)])
 def test_pairs_only_where_the_pipeline_reads_them(tensor, n, pairs):
