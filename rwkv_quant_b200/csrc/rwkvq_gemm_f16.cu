@@ -357,7 +357,9 @@ constexpr size_t kPairSmem = static_cast<size_t>(kPairStages) * (kHgABytes + kPa
 // of the CTA's 128 rows, two warps a quadrant of them with half the tokens each.  Four warps that fetched the factors of
 // each block of tokens behind its accumulators (up to four L2 round trips in a row) took longer for a tile than its products:
 // 4 x 1024 tokens 23.1 -> 22.5 ms (1.5B) and 48.7 -> 47.0 (2.9B).  (The single-CTA tiles, several to an SM's turn, lose 1 to 2 %
-// with their factors fetched ahead.)  192 KB of operands in flight per SM cover the L2 latency; the 256-token tile makes a
+// with their factors fetched ahead.)  A block's code, 32 tokens of three epilogues, stands once: four copies of it are fetched by
+// every launch, which costs a launch of one tile a CTA 3 to 7 us (2.9B 4 x 33 tokens 7.20 -> 6.96 ms, 3 x 77 7.63 -> 7.13, 1.5B
+// 1 x 512 6.37 -> 6.12, 4 x 1024 22.5 -> 21.9).  192 KB of operands in flight per SM cover the L2 latency; the 256-token tile makes a
 // stage 512 tensor cycles.
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     gemm_pair_kernel(const __grid_constant__ HgArgs a, const __grid_constant__ HgMaps maps) {
@@ -461,16 +463,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
             if (!got) { s_fail = 1; break; }
             tc_fence_after();
             const uint32_t base = tmem + acc * kPairTok + share + (static_cast<uint32_t>(q * 32) << 16);
-#pragma unroll
+#pragma unroll 1
             for (int i = 0; i < BLOCKS; ++i) {
-                float v[32];
+                float v[32], u = un[0], s = so[0];       // a select each: one copy of the block's code
+#pragma unroll
+                for (int k = 1; k < BLOCKS; ++k) { u = i == k ? un[k] : u; s = i == k ? so[k] : s; }
                 tmem_ld32(base + 32 * i, v);
                 if (i == BLOCKS - 1) {                   // the accumulator is in registers: the MMA warp may overwrite it
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive_cluster(mapa(smem_addr(&bar_tempty[acc]), 0));
                 }
-                if (tok0 + 32 * i < a.M) finish_block<32>(p, v, un[i], so[i], tok0 + 32 * i, row, a.M);
+                if (tok0 + 32 * i < a.M) finish_block<32>(p, v, u, s, tok0 + 32 * i, row, a.M);
             }
             if (++acc == 2) { acc = 0; aph ^= 1; }
         }
