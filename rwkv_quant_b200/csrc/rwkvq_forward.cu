@@ -23,6 +23,11 @@ constexpr int kSmallRows = 64;
 constexpr int kChunkedT = 16;        // tokens per sequence from which long calls take the chunked scan (two chunks)
 
 bool chunked(size_t rows, int T) { return rows > kSmallRows && T >= kChunkedT; }
+// Shorter calls of many sequences: operands, scan and tail as three launches, whose smaller CTAs fill the chip better than the one
+// kernel's (ms, three / one: 1.5B, 32 heads, 44 x 2 tokens 3.81 / 3.75, 50 x 3 3.82 / 3.85, 50 x 9 5.48 / 5.45, 70 x 5 4.97 / 5.21,
+// 128 x 2 4.42 / 4.70, 128 x 9 9.26 / 9.61; 2.9B, 40 heads, 36 x 5 6.95 / 7.05, 44 x 9 9.85 / 9.85, 64 x 3 7.17 / 7.43).
+constexpr int kSeqPairs = 1600;      // heads of all sequences up to which the one kernel serves
+bool three_launches(size_t rows, int B, int T, int H) { return rows > kSmallRows && T < kChunkedT && static_cast<long long>(B) * H > kSeqPairs; }
 // Long calls turn every weight matrix into fp16 in front of its product.  Where the scan is long and leaves most of the chip idle, the
 // conversions run on the side lane under it, r / k / v and the LoRA matrices a layer ahead: 1.5B, 1 x 512 tokens 6.78 -> 6.35 ms,
 // 2 x 256 6.30 -> 5.93, 1 x 256 4.52 -> 4.34 (fp16 rows from the tail, some 0.1 ms, included).  Where it is short (3 x 77: 4.26 -> 4.4 ms,
@@ -41,7 +46,7 @@ struct ForwardWs {
     // a layer's weights in fp16, LoRA matrices of this layer and the next: apart where they are converted beside the scan, else in
     // one place in turn
     __half *wrkv16, *wo16, *wfk16, *wfv16, *lw16[2];
-    SbRows rkv_pair[3], d_pair, f_pair;      // operand rows of the tcgen05 pipeline (17 rows and more): r / k / v; og or xk; hffn
+    SbRows rkv_pair[3], d_pair, f_pair;      // operand rows of the tcgen05 pipeline (9 to 64 rows): r / k / v; og or xk; hffn
     void* head_ws;
     size_t head_ws_bytes;
 };
@@ -65,6 +70,7 @@ ForwardWs carve(const rwkvq_model& m, int B, int T, size_t n_tail, void* base) {
     w.status = reinterpret_cast<int*>(take(256));
     w.wn2 = f32(static_cast<size_t>(m.n_layer) * 128);
     w.x = f32(N * D); w.rkv = f32(3 * N * D); w.yl = f32(4 * N * D);
+    if (three_launches(N, B, T, static_cast<int>(D / 64))) { w.wkv = f32(5 * N * D); w.out = f32(N * D); }
     if (chunked(N, T)) { w.wkv = f32(wkv_chunk_floats(B, T, static_cast<int>(D / 64))); w.dp = f32(N * D / 64); w.out = f32(N * D); }
     w.og = f32(N * D); w.v_first = f32(N * D);
     if (N <= kSmallRows) {
@@ -374,6 +380,15 @@ int rwkvq_forward_seq_status(const rwkvq_model* m, int B, int T, const int64_t* 
             q.og_pitch = static_cast<long long>(pitch16(D)); q.ops = w.wkv; q.dp = w.dp; q.spread = beside; q.y = w.out; q.status = w.status;
             q.B = B; q.T = T; q.H = H;
             rc = launch_wkv_chunked(q, s);
+            if (rc) return rc;
+        } else if (three_launches(N, B, T, H)) {
+            float *dw = w.wkv, *k2 = w.wkv + ND, *v2 = w.wkv + 2 * ND, *na = w.wkv + 3 * ND, *nb = w.wkv + 4 * ND;
+            rc = rwkvq_seq_tmix_pre(k, v, yw, ya, layer0 ? nullptr : yv, layer0 ? nullptr : w.v_first, L.w0, L.a0, L.v0, L.k_k, L.k_a, dw,
+                                    k2, v2, na, nb, N, H, stream);
+            if (rc) return rc;
+            rc = rwkvq_wkv7(r, dw, k2, v2, na, nb, wkv_in[l], w.out, wkv_out[l], B, T, H, 64, stream);
+            if (rc) return rc;
+            rc = rwkvq_wkv_tail(w.out, r, k2, v2, L.r_k, L.lnx_w, L.lnx_b, yg, w.og, N, H, 64, 64e-5f, stream);
             if (rc) return rc;
         } else {
             TmixSeqArgs q{};

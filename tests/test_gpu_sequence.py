@@ -51,7 +51,7 @@ def test_forward_calls_match_the_oracle(cuda_lib, tmp_path, recipe):
     save_rwkvq(ck, str(tmp_path / "m.rwkvq"))
     model, oracle = QuantRWKV7(ck, device="cuda"), OracleRWKV7(*oc.open_rwkvq(str(tmp_path / "m.rwkvq")))
     for B, T in [(1, 2), (1, 16), (1, 17), (2, 32), (1, 65), (5, 15), (5, 16), (4, 17), (3, 23), (3, 24), (3, 25), (3, 31), (19, 15),
-                 (18, 17), (19, 17), (37, 33), (38, 33)]:
+                 (18, 17), (19, 17), (37, 33), (38, 33), (400, 3), (401, 3)]:
         idx = torch.randint(1, 512, (B, T), generator=torch.Generator().manual_seed(B * 100 + T))
         st = _states(model, B)
         got = model.forward_stateful(idx.cuda(), st)
