@@ -50,13 +50,6 @@ __host__ inline void ahead_tensor(Ahead& a, const rwkvq_qtensor& t) {
     }
 }
 
-// What a layer's launches ask for: its r / k / v launch the state, the LoRA up matrices, the output projection and the ffn key, its
-// ffn key the ffn value and the r / k / v and LoRA down matrices of the layer behind it (null: none).
-struct LayerAhead {
-    Ahead rkv{}, key{};
-    LayerAhead(const rwkvq_layer& L, const rwkvq_layer* behind, bool layer0, const float* state, size_t state_bytes) {
-        if (state_bytes <= kAheadState) ahead_region(rkv, state, state_bytes);
-        for (const rwkvq_qtensor* t : {&L.w2, &L.a2, &L.g2}) ahead_tensor(rkv, *t);
 // Whether a layer's descriptors describe its tensors: what is refused where its turn comes must not be asked for before.
 inline bool ahead_layer_ok(const rwkvq_layer& L, int D, int F, bool layer0) {
     auto ok = [](const rwkvq_qtensor& t, int rows, int cols) { return t.rows == rows && t.cols == cols && validate_qtensor(&t, "ahead") == RWKVQ_OK; };
@@ -65,11 +58,18 @@ inline bool ahead_layer_ok(const rwkvq_layer& L, int D, int F, bool layer0) {
            pair(L.a1, L.a2) && pair(L.g1, L.g2) && (layer0 || pair(L.v1, L.v2));
 }
 
+// What a layer's launches ask for: its r / k / v launch the state, the LoRA up matrices, the output projection and the ffn key, its
+// ffn key the ffn value and the r / k / v and LoRA down matrices of the layer behind it (null: none).
+struct LayerAhead {
+    Ahead rkv{}, key{};
+    LayerAhead() = default;
+    LayerAhead(const rwkvq_layer& L, const rwkvq_layer* behind, bool layer0, const float* state, size_t state_bytes) {
+        if (state_bytes <= kAheadState) ahead_region(rkv, state, state_bytes);
+        for (const rwkvq_qtensor* t : {&L.w2, &L.a2, &L.g2}) ahead_tensor(rkv, *t);
         if (!layer0) ahead_tensor(rkv, L.v2);
         ahead_tensor(rkv, L.Wo);
         ahead_tensor(rkv, L.Wfk);
         ahead_tensor(key, L.Wfv);
-    LayerAhead() = default;
         if (behind)
             for (const rwkvq_qtensor* t : {&behind->Wr, &behind->Wk, &behind->Wv, &behind->w1, &behind->a1, &behind->g1, &behind->v1}) ahead_tensor(key, *t);
     }

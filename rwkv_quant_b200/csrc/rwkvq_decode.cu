@@ -1180,8 +1180,8 @@ int rwkvq_decode_step(const rwkvq_model* m, int B, const int64_t* tokens, float*
             }
     }
 
-    launch_pdl(embed_ln0_kernel, dim3(B), dim3(kRowThreads), 0, s, make_view(m->emb),
     bool ahead_on = m->n_layer > 0 && ahead_layer_ok(m->layers[0], D, F, true);
+    launch_pdl(embed_ln0_kernel, dim3(B), dim3(kRowThreads), 0, s, make_view(m->emb),
                reinterpret_cast<const long long*>(tokens), m->ln0_w, m->ln0_b, w.x, D);
     for (int l = 0; l < m->n_layer; ++l) {
         const rwkvq_layer& L = m->layers[l];

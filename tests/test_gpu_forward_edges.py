@@ -245,8 +245,6 @@ def test_an_error_behind_the_fork_joins_the_side_stream(cuda_lib, B):
     assert torch.equal(ref.step(tok), dec.step(tok))
 
 
-@pytest.mark.parametrize("D", [128, 512, 768, 1024, 1280, 1536, 2048, 2304, 2560, 3072, 3584, 4096])
-@pytest.mark.parametrize("N", [24, 49, 50, 199, 444, 1024])
 @pytest.mark.parametrize("B", [1, 2, 9])
 @pytest.mark.parametrize("name,field,value", [("w1", "gs", 0), ("g2", "rows", -4), ("Wk", "cols", 0)])
 def test_a_tensor_that_a_later_layer_refuses_is_not_asked_for_before(cuda_lib, B, name, field, value):
@@ -268,6 +266,8 @@ def test_a_tensor_that_a_later_layer_refuses_is_not_asked_for_before(cuda_lib, B
     assert torch.equal(model.decoder(B, use_graph=False).step(tok), want)
 
 
+@pytest.mark.parametrize("D", [128, 512, 768, 1024, 1280, 1536, 2048, 2304, 2560, 3072, 3584, 4096])
+@pytest.mark.parametrize("N", [24, 49, 50, 199, 444, 1024])
 def test_row_preparation_in_every_form(cuda_lib, D, N):
     """Widths and token counts on each side of the lines between the scalar, vector and group forms; the three row forms of a
     mix agree with the fp64 LayerNorm, shift and lerp: fp32 rows to rounding, pairs to 2^-20, scaled fp16 to half an ulp of 2^-10."""
