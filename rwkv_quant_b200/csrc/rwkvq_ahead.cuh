@@ -3,8 +3,7 @@
 // The chain is a series of short dependent kernels: one stream reads 34 MB of weights a layer in 39 us, a seventh of the HBM
 // rate, and each linear still waits for DRAM when it starts, since its CTAs become resident only as those of the
 // kernel before leave.  A linear therefore asks L2 (126 MB) for the weights of the linears behind it while it runs its own:
-// one cp.async.bulk.prefetch.L2 per region and CTA, whose bytes no SM ever sees.  1.5B: one stream 956 -> 903 us, 64 streams
-// 2.81 -> 2.76 ms, 5 drafts 1.94 -> 1.91 ms; 13 and 100 streams and one of the 2.9B model stay as they were.
+// one cp.async.bulk.prefetch.L2 per region and CTA, whose bytes no SM ever sees.
 #pragma once
 #include <algorithm>
 
@@ -13,7 +12,15 @@
 namespace rwkvq {
 
 constexpr int kAheadRegions = 32;            // a lane each
-constexpr size_t kAheadState = 64u << 20;    // WKV state of a layer up to which it is asked for: half of L2
+// Weights and WKV state of a layer, together, up to which they are asked for: somewhat more than half of L2.  What has to stay there
+// until it is used is then thrown out by what flows through.  us a step without / with (MiB of a layer with one stream, and more a stream):
+//   1.5B compression (31.6, 0.5)  1 stream 908 / 906, 13 1777 / 1727, 32 2000 / 1966, 64 2480 / 2441, 72 2944 / 2946, 80 3021 / 3043, 128 3622 / 3636
+//   1.5B reduction   (46.0, 0.5)  1 1074 / 1082, 13 1728 / 1686, 32 1966 / 1964, 48 2336 / 2341, 72 2930 / 2964, 128 3589 / 3655
+//   2.9B compression (48.9, 0.6)  1 1658 / 1557, 13 3003 / 2923, 32 3509 / 3451, 40 4054 / 4056, 64 4288 / 4355, 128 6486 / 6577
+//   2.9B reduction   (71.4, 0.6)  1 1610 / 1633, 13 2912 / 2937, 32 3398 / 3411, 64 4203 / 4330, 128 6468 / 6652
+// Steps of 2 to 8 streams, on the mma.sync kernel beside the LoRA pair, ask for nothing (without / with, 1.5B compression 2 streams 1600 /
+// 1617, 4 1623 / 1635, reduction 1632 / 1654, 1662 / 1677, 2.9B 2645 / 2689, 2701 / 2699); its forward calls do (1.5B 5 drafts 1930 / 1908).
+constexpr size_t kAheadMost = 70u << 20;
 
 struct Ahead {
     const unsigned char* p[kAheadRegions];
@@ -64,7 +71,7 @@ struct LayerAhead {
     Ahead rkv{}, key{};
     LayerAhead() = default;
     LayerAhead(const rwkvq_layer& L, const rwkvq_layer* behind, bool layer0, const float* state, size_t state_bytes) {
-        if (state_bytes <= kAheadState) ahead_region(rkv, state, state_bytes);
+        ahead_region(rkv, state, state_bytes);
         for (const rwkvq_qtensor* t : {&L.w2, &L.a2, &L.g2}) ahead_tensor(rkv, *t);
         if (!layer0) ahead_tensor(rkv, L.v2);
         ahead_tensor(rkv, L.Wo);
@@ -72,6 +79,10 @@ struct LayerAhead {
         ahead_tensor(key, L.Wfv);
         if (behind)
             for (const rwkvq_qtensor* t : {&behind->Wr, &behind->Wk, &behind->Wv, &behind->w1, &behind->a1, &behind->g1, &behind->v1}) ahead_tensor(key, *t);
+        size_t all = 0;
+        for (int i = 0; i < rkv.count; ++i) all += rkv.n[i];
+        for (int i = 0; i < key.count; ++i) all += key.n[i];
+        if (all > kAheadMost) rkv.count = key.count = 0;
     }
 };
 

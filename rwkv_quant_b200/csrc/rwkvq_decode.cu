@@ -1030,7 +1030,7 @@ Workspace carve(const rwkvq_model& m, int B, void* base) {
 // the K split, everything else goes through the public entry point.
 // x16 / x_scale: the fp16 form of x with its per-row scale inverses (what the LayerNorm kernels write
 // in fast mode), or null with x_scale = max|x| per row for fp32 rows; y_amax: optional slots max|y| per row is
-// merged into.
+// merged into; ahead: one stream only.
 int linear(const rwkvq_qtensor* t, const float* x, int B, int in, float* y, int out, int epi, const float* resid,
            void* gemm_ws, void* stream, const __half* x16 = nullptr, const float* x_scale = nullptr,
            float* y_amax = nullptr, int* status = nullptr, const Ahead* ahead = nullptr) {
@@ -1051,7 +1051,7 @@ int linear(const rwkvq_qtensor* t, const float* x, int B, int in, float* y, int 
         float* ao[1] = {y_amax};
         if (tcb_pays(B) && gemm_tcb_ok(*t))
             return launch_gemm_tcb(t, 1, xs, x16 != nullptr, sc, B, in, ys, out, epi, rs, ao, status, static_cast<cudaStream_t>(stream));
-        return launch_gemv_batch(t, 1, xs, x16 != nullptr, sc, B, in, ys, out, epi, rs, ao, static_cast<cudaStream_t>(stream), ahead);
+        return launch_gemv_batch(t, 1, xs, x16 != nullptr, sc, B, in, ys, out, epi, rs, ao, static_cast<cudaStream_t>(stream));
     }
     if (linear_on_gemm(*t, B)) {                            // tcgen05 path for large batches
         int rc = validate_qtensor(t, "rwkvq_decode_step(linear)");
@@ -1303,7 +1303,7 @@ int rwkvq_decode_step(const rwkvq_model* m, int B, const int64_t* tokens, float*
                 if (tcb_pays(B) && gemm_tcb_ok(L.Wr))
                     rc = launch_gemm_tcb(three, 3, x3, h16, a3, B, D, y3, D, RWKVQ_EPI_NONE, nullptr, nullptr, w.status, s_rkv);
                 else
-                    rc = launch_gemv_batch(three, 3, x3, h16, a3, B, D, y3, D, RWKVQ_EPI_NONE, nullptr, nullptr, s_rkv, &ahead.rkv);
+                    rc = launch_gemv_batch(three, 3, x3, h16, a3, B, D, y3, D, RWKVQ_EPI_NONE, nullptr, nullptr, s_rkv);
                 if (rc) return rc;
             } else {
                 rc = linear(&L.Wr, xr, B, D, r, D, RWKVQ_EPI_NONE, nullptr, w.gemm_ws, s_rkv, h16 ? w.xs16 : nullptr, am, nullptr, w.status);
