@@ -660,10 +660,11 @@ int launch_seq_prep(const SeqPrepArgs& a, long long n_tokens, cudaStream_t s) {
             case 5: e = launch_prep_group<5>(a, n_tokens, s); break;
             default: e = launch_prep_group<6>(a, n_tokens, s); break;
         }
-    } else if (vec && in_place && a.n_mix > 1 && 2 * n_tokens * a.n_mix > 3 * 148 * std::max(1, 65536 / (112 * a.D / 8))) {
+    } else if (vec && in_place && a.n_mix > 1 && a.mix != nullptr && 2 * n_tokens * a.n_mix > 3 * 148 * std::max(1, 65536 / (112 * a.D / 8))) {
         // A CTA per token instead of a cluster of one per mix, which normalises the row six times, from where the clusters are one
-        // and a half waves (by registers: two CTAs an SM at 2048 columns, one above).  us a step, cluster / this: 1.5B 16 streams 1760 /
-        // 1855, 64 2447 / 2485, 100 3369 / 3315, 200 5049 / 4810; 2.9B 32 streams 3418 / 3453, 64 4492 / 4281, 128 7074 / 6565
+        // and a half waves (by registers two CTAs an SM up to 2304 columns, one above: from 75 streams on at 2048 and 2304, from 38 at
+        // 2560).  us a step, cluster / this: 1.5B 16 streams 1760 / 1855, 64 2447 / 2485, 100 3369 / 3315, 200 5049 / 4810; 2.9B 32 streams
+        // 3418 / 3453, 64 4492 / 4281, 128 7074 / 6565
         e = launch_pdl(seq_prep_step_kernel, dim3(static_cast<unsigned>(n_tokens)), dim3(a.D / 8), 0, s, a);
     } else if (vec && in_place && a.n_mix > 1) {
         cudaLaunchConfig_t cfg{};

@@ -91,12 +91,14 @@ def test_wide_tensor_without_relayouted_streams(cuda_lib, layout, bits, N):
         assert relmax(y.cpu().numpy(), want) <= 2e-5, relayout
 
 
-@pytest.mark.parametrize("D", [256, 384, 2048])
-def test_shift_state_updated_in_place(cuda_lib, D):
-    """One token a sequence: the row preparation may write the shift state over its input, whatever the width."""
+@pytest.mark.parametrize("D,B", [(256, 70), (384, 70), (2048, 70), (256, 666), (256, 667), (2048, 74), (2048, 75), (2304, 75), (2560, 37),
+                                 (2560, 38), (4096, 38)])
+def test_shift_state_updated_in_place(cuda_lib, D, B):
+    """One token a sequence: the row preparation may write the shift state over its input, whatever the width; streams on each side of
+    the line from which one CTA makes all rows of a token."""
     import ctypes as C
     from rwkv_quant_b200 import _lib
-    B, gen = 70, torch.Generator(device="cuda").manual_seed(D)
+    gen = torch.Generator(device="cuda").manual_seed(D)
     draw = lambda *s: torch.randn(s, generator=gen, device="cuda")
     x, w, b, mix, shift = draw(B, D), draw(D), draw(D), draw(6, D), draw(B, D)
     xn = torch.nn.functional.layer_norm(x.double(), (D,), w.double(), b.double())

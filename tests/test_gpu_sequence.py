@@ -111,10 +111,13 @@ def test_time_mix_of_short_sequences_matches_its_steps(cuda_lib, B, T):
 
 @pytest.mark.parametrize("recipe,D,B,T", [("compression", 256, 2, 3), ("compression", 768, 3, 3), ("reduction", 256, 16, 3),
                                           ("compression", 256, 17, 3), ("reduction", 768, 21, 3), ("compression", 2304, 37, 1),
-                                          ("compression", 2304, 38, 1), ("reduction", 4096, 40, 1), ("compression", 256, 46, 1)])
+                                          ("compression", 2304, 38, 1), ("reduction", 4096, 40, 1), ("compression", 256, 46, 1),
+                                          # each side of the line from which a CTA normalises a token for all its mixes
+                                          ("compression", 2048, 74, 1), ("compression", 2048, 75, 1), ("reduction", 2304, 75, 2),
+                                          ("reduction", 2560, 37, 1), ("reduction", 2560, 38, 1)])
 def test_steps_of_several_streams_match_the_sequence(cuda_lib, recipe, D, B, T):
-    """The time mix and the LayerNorms of a step against the per-operator path (64 rows at most: above, its linears have fp16 operands): logits and
-    all states after T tokens."""
+    """The time mix and the LayerNorms of a step against the per-operator path (a few streams at a time: above 64 rows its linears have fp16
+    operands): logits and all states after T tokens."""
     model = _model(recipe, n_embd=D, ffn=1024)
     idx = torch.randint(1, 512, (B, T), generator=torch.Generator().manual_seed(B)).cuda()
     st = _states(model, B)
@@ -124,7 +127,10 @@ def test_steps_of_several_streams_match_the_sequence(cuda_lib, recipe, D, B, T):
         dec.step(idx[:, t])
         steps.append(dec.logits.clone())
     model.fused_prep = False
-    _same((torch.stack(steps, 1), dec.states), model.forward_stateful(idx, st), 1e-4)
+    few = 64 // T
+    ref = [model.forward_stateful(idx[i:i + few], [tuple(t[i:i + few] for t in s) for s in st]) for i in range(0, B, few)]
+    states = [tuple(torch.cat([r[1][l][k] for r in ref]) for k in range(3)) for l in range(model.n_layer)]
+    _same((torch.stack(steps, 1), dec.states), (torch.cat([r[0] for r in ref]), states), 1e-4)
 
 
 @pytest.mark.parametrize("B,T", [(1, 255), (1, 256), (2, 300), (37, 256), (38, 256)])
