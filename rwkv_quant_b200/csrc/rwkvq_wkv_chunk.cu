@@ -573,8 +573,10 @@ static int launch_scan(const WkvChunkArgs& p, int n_chunks, cudaStream_t s) {
     // A scan is as slow as its fullest SM: beside the conversions of the side lane CTAs would pile up where those leave room first
     // (1 x 512 tokens 56 -> 95 us), so a grid of up to one or two CTAs per SM asks for as much shared memory as keeps it to that.
     const int ctas = p.B * p.H * SPLIT;
-    const size_t smem = std::max(G::SMEM, static_cast<size_t>(!p.spread ? 0 : ctas <= 148 ? 116 : ctas <= 296 ? 78 : 0) * 1024);
-    cudaError_t e = cudaFuncSetAttribute(wkv_scan_kernel<R, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 116 * 1024);
+    constexpr size_t kOne = 116 * 1024, kTwo = 78 * 1024;
+    static_assert(G::SMEM <= kOne, "the largest a launch may ask for");
+    const size_t smem = std::max(G::SMEM, !p.spread ? 0 : ctas <= 148 ? kOne : ctas <= 296 ? kTwo : 0);
+    cudaError_t e = cudaFuncSetAttribute(wkv_scan_kernel<R, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kOne));
     if (e != cudaSuccess) return fail(RWKVQ_E_LIMIT, "wkv_scan: %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
     // a plain launch: CTAs that start while the kernel before still fills the chip pile up on the SMs it leaves
     // first, and the scan of one batch element takes three times as long
