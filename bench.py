@@ -237,7 +237,7 @@ NCU_GEMV_PHASE_DRAM_BYTES_B1 = 856284928 + 68864 - 26591232
 def kernel_name(B, fast):
     if fast:
         return "row_amax_kernel + " + ("gemm_tcb_kernel" if B > 32 else "gemv_batch_kernel")
-    return "split_rows_kernel + gemm_sb_kernel" if B > 16 else "row_amax_kernel + gemv_batch_kernel"
+    return "split_rows_kernel + gemm_sb_kernel" if B > 8 else "row_amax_kernel + gemv_batch_kernel"
 
 
 def time_decode(model, B, prompt, steps, warmup, sync_all, clock_index=None, groups=None):

@@ -922,8 +922,9 @@ constexpr int kBatchMax = 256;     // streams up to which the small-batch kernel
 inline bool batch_path(int B) { return B > (batch_fast() ? 2 : 1) && B <= kBatchMax; }
 // Single-term operands (RWKVQ_BATCH_FAST=1): the tcgen05 form wins over the mma.sync one from 33 streams on (1.5B, whole
 // step, 64 streams: 3.77 against 4.43 ms) and loses below (32: 2.87 / 2.68 ms, 8: 2.42 / 2.01): its pass (dependent weight
-// loads -> conversion -> MMA) is longer than a warp-iteration.  The default precision is faster from 9 streams on (64: 2.60
-// ms).
+// loads -> conversion -> MMA) is longer than a warp-iteration.  The default precision is faster from 20 streams on, with sym tensors
+// from 9 (ms, default / this: 1.5B sb6 8 streams 1.67 / 1.49, 16 1.77 / 1.66, 20 1.82 / 1.99, 64 2.44 / 3.11; sym 8 1.70 / 1.59, 9 1.65 / 1.74,
+// 64 2.43 / 3.37).
 inline bool tcb_pays(int B) { return batch_fast() && tcb_enabled() && B > 32; }
 // Default (two-term) precision: from kSbMinStreams streams on every linear of the step runs on the tcgen05 pipeline
 // (rwkvq_gemm_sb.cu), fed with fp16 pairs and block sums by the LayerNorm kernels and, for the output projection and the

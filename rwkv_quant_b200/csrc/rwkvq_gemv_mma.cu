@@ -303,7 +303,7 @@ static int launch_wk(MmaArgs& a, int rows, int cols, int n_mats, bool split, con
     if ((split || cols >= kSplitAnyCols) && n_iters >= 16 && rows <= kSplitMaxRows) {
         // One tile and K in four is more than a wave: two tiles a CTA and K in four leave each CTA half the activations to
         // prepare that one tile and K in two do (us, before / now: sb6 4 bits [2048, 8192] 6.7 / 6.3, [1200, 10240] 6.9 / 6.4, sym 8 bits
-        // [2560, 10240] 12.0 / 10.6, [3072, 8192] 10.7 / 9.7; 1.5B step of one stream 913 / 885, 2.9B 1671 / 1645).  From 32 iterations on (sb6
+        // [2560, 10240] 12.0 / 10.6, [3072, 8192] 10.7 / 9.7; 1.5B step of one stream 913 / 885, 2.9B within noise).  From 32 iterations on (sb6
         // [2048, 4096]: 4.7 / 4.9) and up to 7/8 of the resident CTAs: clusters do not fill every GPC ([2368, 8192], 296 CTAs: 7.0 / 10.4).
         if (cols >= kSplitAnyCols && ctas * 4 > kResident && (tiles + 1) / 2 * 4 <= kResident * 7 / 8 && n_iters >= 32 && n_iters % 4 == 0)
             return launch_one<L, 4, true>(a, rows, cols, n_mats, 4, s, ahead);
