@@ -308,15 +308,18 @@ def gemv_batch(dq: "DeviceQT", x: torch.Tensor, epilogue: int = 0, resid: Option
     """x [N, IN] -> y [N, OUT] fp32 with the packed weights read once for up to 128 rows: tokens as the MMA columns, both
     operands as fp16 pairs, fp32 accumulation (mma.sync up to 8 rows, the tcgen05 pipeline above)."""
     _require_cuda(dq.bufs[0], x, resid)
-    lib = _lib.load()
-    x = x.float()
-    if x.stride(-1) != 1 or x.stride(0) % 4 or x.data_ptr() % 16:
+    lib, ref, dev, rows = _lib.load(), dq.struct_ref, x.device, dq.rows
+    if x.dtype is not torch.float32:
+        x = x.float()
+    ldx = x.stride(0)
+    if x.stride(-1) != 1 or ldx % 4 or x.data_ptr() % 16:
         x = x.contiguous()
+        ldx = x.stride(0)
     n = x.shape[0]
-    y = torch.empty((n, dq.rows), dtype=torch.float32, device=x.device)
-    nws = lib.rwkvq_gemv_batch_workspace_bytes_of(dq.struct_ref, n)
-    ws = torch.empty(nws, dtype=torch.uint8, device=x.device)
-    _lib.check(lib.rwkvq_gemv_batch(dq.struct_ref, x.data_ptr(), n, x.stride(0), y.data_ptr(), y.stride(0),
+    y = torch.empty((n, rows), dtype=torch.float32, device=dev)
+    nws = lib.rwkvq_gemv_batch_workspace_bytes_of(ref, n)
+    ws = torch.empty(nws, dtype=torch.uint8, device=dev)
+    _lib.check(lib.rwkvq_gemv_batch(ref, x.data_ptr(), n, ldx, y.data_ptr(), rows,
                                     epilogue, _lib.ptr(resid), ws.data_ptr(), nws, _lib.stream_ptr()), "rwkvq_gemv_batch")
     if check:          # synchronises: the kernel's own report that a bounded pipeline wait ran out
         _lib.check(int(ws[:4].view(torch.int32).item()), "rwkvq_gemv_batch(kernel status)")
